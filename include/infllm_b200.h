@@ -271,7 +271,12 @@ int infllm_device_store_info(int device, int64_t* total_bytes, int64_t* used_byt
  * max_cached_block >= topk, context_manager.py:19 -> INFLLM_E_CAPACITY) and allocates nothing
  * large: buffers are created on the first append (context_manager.py:292-363). */
 int infllm_ctx_create(const infllm_config* cfg, infllm_ctx** out);
+/* infllm_ctx_destroy forgets the tokens and keeps the context's workspaces (device buffers, pinned host slabs, streams)
+ * for the next infllm_ctx_create with an equal configuration: at most 256 contexts, 16 GiB of pinned memory and
+ * 16 GiB of device memory (no more than a quarter of what is free), the oldest are freed first.
+ * infllm_ctx_release_idle frees all of them. */
 int infllm_ctx_destroy(infllm_ctx* ctx);
+int infllm_ctx_release_idle(void);
 /* Forget every token but keep the allocations (device buffers, pinned host store). */
 int infllm_ctx_reset(infllm_ctx* ctx);
 

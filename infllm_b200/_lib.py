@@ -151,6 +151,7 @@ SIGNATURES = {
     "infllm_ctx_load": (c_int, [c_void_p, c_char_p, c_void_p]),
     "infllm_ctx_create": (c_int, [POINTER(Config), POINTER(c_void_p)]),
     "infllm_ctx_destroy": (c_int, [c_void_p]),
+    "infllm_ctx_release_idle": (c_int, []),
     "infllm_ctx_reset": (c_int, [c_void_p]),
     "infllm_ctx_append": (c_int, [c_void_p, c_void_p, c_int64, c_int64, c_void_p, c_int64, c_int64, c_void_p,
                                   c_int64, c_int64, c_void_p, c_int64, c_int64, c_int64, c_void_p]),

@@ -40,6 +40,13 @@ def device_store_info(device=None):
     return tot.value >> 20, used.value >> 20
 
 
+def release_idle_memories():
+    """Free the workspaces of memories that were dropped (device buffers, pinned host slabs, streams).  The library
+    keeps them, within bounds, for the next ContextManager of the same shape; it also frees them itself when one of
+    its own allocations fails."""
+    _lib.check(_lib.lib.infllm_ctx_release_idle())
+
+
 class ContextManager:
     """Per-layer context memory: sliding local window, init sink, sealed memory units with
     representative keys, top-k retrieval, a GPU cache of max_cached_block units with LRU

@@ -289,6 +289,13 @@ struct infllm_ctx {
               ev_cand = nullptr, ev_seal = nullptr, ev_stage = nullptr;
   bool attn_recorded = false, attn_prev_recorded = false, spec_recorded = false;
   cudaStream_t urgent_stream = nullptr;  // copies an exec block is waiting for, past the queue of staged copies
+  // A reset waits for nothing: it marks where every stream of the context stands, and the next append orders all of
+  // them behind those marks (order_behind_reset).
+  cudaEvent_t ev_last = nullptr;  // behind the last kernel of an append on the caller's stream, where ev_attn is not
+  bool last_recorded = false;
+  cudaEvent_t ev_side[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
+  bool reset_pending = false, reset_attn = false, reset_last = false;
+  bool failed = false;  // an append gave up half-way: the context is not handed to anybody else afterwards
 
   // optional per-kernel timing (infllm_ctx_profile): CUDA events around the launches on their stream
   bool prof = false;
@@ -322,6 +329,8 @@ struct infllm_ctx {
   char* dev_unit(int64_t b) { return (char*)dev_slabs[b / slab_units] + (b % slab_units) * unit_bytes; }
   const char* unit_src(int64_t b) { return dev_resident(b) ? dev_unit(b) : host_unit(b); }
 };
+
+static int idle_trim(int64_t dev, int64_t host, int64_t dev_limit, bool all);
 
 namespace {
 
@@ -381,6 +390,24 @@ int free_buffers(TokenBuffers& tb, cudaStream_t s) {
   return INFLLM_OK;
 }
 
+// Device memory that idle contexts hold is given up before an allocation fails.
+cudaError_t dev_malloc(void** p, size_t n) {
+  cudaError_t e = cudaMalloc(p, n);
+  if (e == cudaErrorMemoryAllocation && idle_trim(0, 0, 0, true) > 0) {
+    cudaGetLastError();
+    e = cudaMalloc(p, n);
+  }
+  return e;
+}
+cudaError_t dev_malloc_async(void** p, size_t n, cudaStream_t s) {
+  cudaError_t e = cudaMallocAsync(p, n, s);
+  if (e == cudaErrorMemoryAllocation && idle_trim(0, 0, 0, true) > 0) {
+    cudaGetLastError();
+    e = cudaMallocAsync(p, n, s);
+  }
+  return e;
+}
+
 int lazy_init(infllm_ctx* c, cudaStream_t s) {
   const infllm_config& g = c->cfg;
   // keep freed device memory in the pool: the token buffers are re-created at every compaction
@@ -402,7 +429,7 @@ int lazy_init(infllm_ctx* c, cudaStream_t s) {
   INFLLM_CUDA_OK(cudaEventCreateWithFlags(&c->ev_ingest, cudaEventDisableTiming));
   c->pack_units = g.exc_block_size / g.block_size + 2;
   for (int i = 0; i < 2; ++i) {
-    INFLLM_CUDA_OK(cudaMalloc(&c->pack_buf[i], (int64_t)c->pack_units * c->unit_bytes));
+    INFLLM_CUDA_OK(dev_malloc((void**)&c->pack_buf[i], (int64_t)c->pack_units * c->unit_bytes));
     INFLLM_CUDA_OK(cudaEventCreateWithFlags(&c->ev_pack[i], cudaEventDisableTiming));
   }
   INFLLM_CUDA_OK(cudaEventCreateWithFlags(&c->ev_main, cudaEventDisableTiming));
@@ -419,14 +446,16 @@ int lazy_init(infllm_ctx* c, cudaStream_t s) {
   INFLLM_CUDA_OK(cudaEventCreateWithFlags(&c->ev_cand, cudaEventDisableTiming));
   INFLLM_CUDA_OK(cudaEventCreateWithFlags(&c->ev_seal, cudaEventDisableTiming));
   INFLLM_CUDA_OK(cudaEventCreateWithFlags(&c->ev_stage, cudaEventDisableTiming));
+  INFLLM_CUDA_OK(cudaEventCreateWithFlags(&c->ev_last, cudaEventDisableTiming));
+  for (auto& e : c->ev_side) INFLLM_CUDA_OK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
 
   const int64_t D = g.head_dim, H = g.n_heads, HKV = g.n_kv_heads;
   c->sub_max = round_up(std::max<int64_t>(16384, 2 * g.exc_block_size), g.exc_block_size);
   // RoPE table: positions of a call stay below n_local + sub_max; twice that so that the origin
   // moves (and the window is re-rotated) only every sub_max tokens
   c->tab_len = g.n_local + 2 * c->sub_max + 1;
-  INFLLM_CUDA_OK(cudaMalloc(&c->cos_t, c->tab_len * (D / 2) * sizeof(float)));
-  INFLLM_CUDA_OK(cudaMalloc(&c->sin_t, c->tab_len * (D / 2) * sizeof(float)));
+  INFLLM_CUDA_OK(dev_malloc((void**)&c->cos_t, c->tab_len * (D / 2) * sizeof(float)));
+  INFLLM_CUDA_OK(dev_malloc((void**)&c->sin_t, c->tab_len * (D / 2) * sizeof(float)));
   {
     std::vector<float> inv(D / 2);
     // rope.py:22-24: 1 / base ** (arange(0, D, 2) / D) in fp32
@@ -436,31 +465,31 @@ int lazy_init(infllm_ctx* c, cudaStream_t s) {
   // buffers that TMA tiles may over-read are zero-filled once: a tile row past the valid data must not
   // hold NaN bit patterns (0 * NaN would poison P V)
   c->init_cap = std::max<int64_t>(g.n_init, 128);
-  INFLLM_CUDA_OK(cudaMalloc(&c->init_k, HKV * c->init_cap * D * c->esz));
-  INFLLM_CUDA_OK(cudaMalloc(&c->init_v, HKV * c->init_cap * D * c->esz));
+  INFLLM_CUDA_OK(dev_malloc((void**)&c->init_k, HKV * c->init_cap * D * c->esz));
+  INFLLM_CUDA_OK(dev_malloc((void**)&c->init_v, HKV * c->init_cap * D * c->esz));
   INFLLM_CUDA_OK(cudaMemsetAsync(c->init_k, 0, HKV * c->init_cap * D * c->esz, s));
   INFLLM_CUDA_OK(cudaMemsetAsync(c->init_v, 0, HKV * c->init_cap * D * c->esz, s));
-  INFLLM_CUDA_OK(cudaMalloc(&c->q_loc, H * c->sub_max * D * c->esz));
-  INFLLM_CUDA_OK(cudaMalloc(&c->q_glb, H * c->sub_max * D * c->esz));
+  INFLLM_CUDA_OK(dev_malloc((void**)&c->q_loc, H * c->sub_max * D * c->esz));
+  INFLLM_CUDA_OK(dev_malloc((void**)&c->q_glb, H * c->sub_max * D * c->esz));
   INFLLM_CUDA_OK(cudaMemsetAsync(c->q_loc, 0, H * c->sub_max * D * c->esz, s));
   INFLLM_CUDA_OK(cudaMemsetAsync(c->q_glb, 0, H * c->sub_max * D * c->esz, s));
-  INFLLM_CUDA_OK(cudaMalloc(&c->qbar, (c->sub_max / g.exc_block_size + 1) * c->width * sizeof(float)));
-  INFLLM_CUDA_OK(cudaMalloc(&c->lse, H * g.exc_block_size * sizeof(float)));
-  INFLLM_CUDA_OK(cudaMalloc(&c->st_acc, H * g.exc_block_size * D * sizeof(float)));
-  INFLLM_CUDA_OK(cudaMalloc(&c->st_m, H * g.exc_block_size * sizeof(float)));
-  INFLLM_CUDA_OK(cudaMalloc(&c->st_l, H * g.exc_block_size * sizeof(float)));
-  INFLLM_CUDA_OK(cudaMalloc(&c->d_topk, std::max(1, g.topk) * sizeof(int32_t)));
-  INFLLM_CUDA_OK(cudaMalloc((void**)&c->d_miss, sizeof(int32_t)));
+  INFLLM_CUDA_OK(dev_malloc((void**)&c->qbar, (c->sub_max / g.exc_block_size + 1) * c->width * sizeof(float)));
+  INFLLM_CUDA_OK(dev_malloc((void**)&c->lse, H * g.exc_block_size * sizeof(float)));
+  INFLLM_CUDA_OK(dev_malloc((void**)&c->st_acc, H * g.exc_block_size * D * sizeof(float)));
+  INFLLM_CUDA_OK(dev_malloc((void**)&c->st_m, H * g.exc_block_size * sizeof(float)));
+  INFLLM_CUDA_OK(dev_malloc((void**)&c->st_l, H * g.exc_block_size * sizeof(float)));
+  INFLLM_CUDA_OK(dev_malloc((void**)&c->d_topk, std::max(1, g.topk) * sizeof(int32_t)));
+  INFLLM_CUDA_OK(dev_malloc((void**)&c->d_miss, sizeof(int32_t)));
   INFLLM_CUDA_OK(cudaMemsetAsync(c->d_miss, 0, sizeof(int32_t), s));
   {
     const int per = std::max(1, g.topk);
-    INFLLM_CUDA_OK(cudaMalloc((void**)&c->d_topk_ring, (size_t)infllm_ctx::kPendSlots * per * sizeof(int32_t)));
+    INFLLM_CUDA_OK(dev_malloc((void**)&c->d_topk_ring, (size_t)infllm_ctx::kPendSlots * per * sizeof(int32_t)));
     for (auto& pt : c->pend) {
       INFLLM_CUDA_OK(cudaHostAlloc((void**)&pt.h_ids, per * sizeof(int32_t), cudaHostAllocDefault));
       INFLLM_CUDA_OK(cudaEventCreateWithFlags(&pt.ev, cudaEventDisableTiming));
     }
   }
-  INFLLM_CUDA_OK(cudaMalloc((void**)&c->tickets, 2 * sizeof(unsigned int)));
+  INFLLM_CUDA_OK(dev_malloc((void**)&c->tickets, 2 * sizeof(unsigned int)));
   INFLLM_CUDA_OK(cudaMemsetAsync(c->tickets, 0, 2 * sizeof(unsigned int), s));
   INFLLM_CUDA_OK(cudaHostAlloc((void**)&c->h_topk, std::max(1, g.topk) * sizeof(int32_t),
                                cudaHostAllocDefault));
@@ -473,19 +502,19 @@ int lazy_init(infllm_ctx* c, cudaStream_t s) {
   }
   INFLLM_CUDA_OK(cudaHostAlloc((void**)&c->h_cand_rows, c->cand_cap * sizeof(int32_t), cudaHostAllocDefault));
   INFLLM_CUDA_OK(cudaHostAlloc((void**)&c->h_cand_scores, c->cand_cap * sizeof(float), cudaHostAllocDefault));
-  INFLLM_CUDA_OK(cudaMalloc((void**)&c->d_cand_scores, c->cand_cap * sizeof(float)));
-  INFLLM_CUDA_OK(cudaMalloc((void**)&c->d_spec, (c->look_depth + 1) * std::max(1, g.topk) * sizeof(int32_t)));
+  INFLLM_CUDA_OK(dev_malloc((void**)&c->d_cand_scores, c->cand_cap * sizeof(float)));
+  INFLLM_CUDA_OK(dev_malloc((void**)&c->d_spec, (c->look_depth + 1) * std::max(1, g.topk) * sizeof(int32_t)));
   INFLLM_CUDA_OK(cudaStreamCreateWithFlags(&c->mail_stream, cudaStreamNonBlocking));
   // decode partials: window + units + sink + overflow, each segment may add one ragged chunk
   int64_t dec_keys = (int64_t)g.n_local + (int64_t)g.topk * g.block_size + g.n_init + g.block_size + g.exc_block_size;
   (void)dec_keys;
   c->max_parts = 2 * 148;  // the decode attention launches at most two CTAs per SM, one partial each
-  INFLLM_CUDA_OK(cudaMalloc(&c->part_o, (int64_t)c->max_parts * H * D * sizeof(float)));
-  INFLLM_CUDA_OK(cudaMalloc(&c->part_lse, (int64_t)c->max_parts * H * sizeof(float)));
-  INFLLM_CUDA_OK(cudaMalloc(&c->dec_logits, H * ((int64_t)g.n_local + 1) * sizeof(float)));
+  INFLLM_CUDA_OK(dev_malloc((void**)&c->part_o, (int64_t)c->max_parts * H * D * sizeof(float)));
+  INFLLM_CUDA_OK(dev_malloc((void**)&c->part_lse, (int64_t)c->max_parts * H * sizeof(float)));
+  INFLLM_CUDA_OK(dev_malloc((void**)&c->dec_logits, H * ((int64_t)g.n_local + 1) * sizeof(float)));
   // max_cached_block slots hold the cache proper; topk more per look-ahead step hold the copies staged ahead
   const int64_t n_slots = (int64_t)g.max_cached_block + (int64_t)c->look_depth * g.topk;
-  INFLLM_CUDA_OK(cudaMalloc(&c->cache, n_slots * c->unit_bytes));
+  INFLLM_CUDA_OK(dev_malloc((void**)&c->cache, n_slots * c->unit_bytes));
   INFLLM_CUDA_OK(cudaMemsetAsync(c->cache, 0, n_slots * c->unit_bytes, s));
   c->use_tc = D == 128 && g.block_size % 128 == 0 && !(g.debug_flags & 1);
   if (c->use_tc) {
@@ -511,6 +540,23 @@ int lazy_init(infllm_ctx* c, cudaStream_t s) {
   c->slab_units = std::max<int64_t>(16, (128ll << 20) / c->unit_bytes);
   c->dev_cap = (int64_t)g.device_store_mb * (1ll << 20) / c->unit_bytes;  // device copy of the store, in units
   c->initialized = true;
+  return INFLLM_OK;
+}
+
+// After a reset: s and the context's own streams continue behind everything that was enqueued before it, and the sink
+// starts from zeros again (a tile may reach past its last row).
+int order_behind_reset(infllm_ctx* c, cudaStream_t s) {
+  if (!c->reset_pending) return INFLLM_OK;
+  c->reset_pending = false;
+  cudaStream_t side[5] = {c->copy_stream, c->urgent_stream, c->aux_stream, c->d2h_stream, c->mail_stream};
+  for (cudaEvent_t e : c->ev_side) INFLLM_CUDA_OK(cudaStreamWaitEvent(s, e, 0));
+  if (c->reset_attn) INFLLM_CUDA_OK(cudaStreamWaitEvent(s, c->ev_attn, 0));
+  if (c->reset_last) INFLLM_CUDA_OK(cudaStreamWaitEvent(s, c->ev_last, 0));
+  const size_t sink = (size_t)c->cfg.n_kv_heads * c->init_cap * c->cfg.head_dim * c->esz;
+  INFLLM_CUDA_OK(cudaMemsetAsync(c->init_k, 0, sink, s));
+  INFLLM_CUDA_OK(cudaMemsetAsync(c->init_v, 0, sink, s));
+  INFLLM_CUDA_OK(cudaEventRecord(c->ev_main, s));
+  for (cudaStream_t t : side) INFLLM_CUDA_OK(cudaStreamWaitEvent(t, c->ev_main, 0));
   return INFLLM_OK;
 }
 
@@ -555,10 +601,10 @@ int ensure_tokens(infllm_ctx* c, int64_t add, cudaStream_t s) {
   TokenBuffers nb;
   nb.cap = round_up(need + std::max<int64_t>(4096, g.n_local), 256);
   nb.t0 = live0;
-  INFLLM_CUDA_OK(cudaMallocAsync(&nb.k_raw, HKV * nb.cap * D * c->esz, s));
-  INFLLM_CUDA_OK(cudaMallocAsync(&nb.k_rot, HKV * nb.cap * D * c->esz, s));
-  INFLLM_CUDA_OK(cudaMallocAsync(&nb.v, HKV * nb.cap * D * c->esz, s));
-  INFLLM_CUDA_OK(cudaMallocAsync((void**)&nb.score, H * nb.cap * sizeof(float), s));
+  INFLLM_CUDA_OK(dev_malloc_async((void**)&nb.k_raw, HKV * nb.cap * D * c->esz, s));
+  INFLLM_CUDA_OK(dev_malloc_async((void**)&nb.k_rot, HKV * nb.cap * D * c->esz, s));
+  INFLLM_CUDA_OK(dev_malloc_async((void**)&nb.v, HKV * nb.cap * D * c->esz, s));
+  INFLLM_CUDA_OK(dev_malloc_async((void**)&nb.score, H * nb.cap * sizeof(float), s));
   if (live > 0) {
     const int64_t off = (live0 - tb.t0) * D * c->esz;
     const size_t w = live * D * c->esz;
@@ -590,7 +636,7 @@ int ensure_block_k(infllm_ctx* c, int64_t n, cudaStream_t s) {
   int64_t cap = std::max<int64_t>(16, c->block_k_cap);
   while (cap < n) cap *= 2;  // VectorTensor.append_cache doubles (context_manager.py:128-138)
   void* nb = nullptr;
-  INFLLM_CUDA_OK(cudaMallocAsync(&nb, cap * c->width * c->esz, s));
+  INFLLM_CUDA_OK(dev_malloc_async((void**)&nb, cap * c->width * c->esz, s));
   if (c->num_blocks > 0)
     INFLLM_CUDA_OK(cudaMemcpyAsync(nb, c->block_k, c->num_blocks * c->width * c->esz, cudaMemcpyDeviceToDevice, s));
   if (c->block_k) {
@@ -622,6 +668,10 @@ int ensure_host_units(infllm_ctx* c, int64_t n) {
     }
     if (!p) {
       cudaError_t e = cudaHostAlloc(&p, bytes, cudaHostAllocDefault);
+      if (e == cudaErrorMemoryAllocation && idle_trim(0, 0, 0, true) > 0) {
+        cudaGetLastError();
+        e = cudaHostAlloc(&p, bytes, cudaHostAllocDefault);
+      }
       if (e != cudaSuccess) return fail(INFLLM_E_NOMEM, "pinned host store: cudaHostAlloc of %lld bytes failed: %s",
                                         (long long)bytes, cudaGetErrorString(e));
     }
@@ -640,7 +690,7 @@ int ensure_scores(infllm_ctx* c, int64_t n, cudaStream_t s) {
   int64_t cap = std::max<int64_t>(1024, c->scores_cap);
   while (cap < n) cap *= 2;
   if (c->scores) INFLLM_CUDA_OK(cudaFreeAsync(c->scores, s));
-  INFLLM_CUDA_OK(cudaMallocAsync((void**)&c->scores, cap * sizeof(float), s));
+  INFLLM_CUDA_OK(dev_malloc_async((void**)&c->scores, cap * sizeof(float), s));
   c->scores_cap = cap;
   return INFLLM_OK;
 }
@@ -699,7 +749,7 @@ int lookahead_launch(infllm_ctx* c, int64_t target, cudaStream_t s) {
     int64_t cap = std::max<int64_t>(1024, c->scores_aux_cap);
     while (cap < la.n_spec) cap *= 2;
     if (c->scores_aux) INFLLM_CUDA_OK(cudaFreeAsync(c->scores_aux, c->aux_stream));
-    INFLLM_CUDA_OK(cudaMallocAsync((void**)&c->scores_aux, cap * sizeof(float), c->aux_stream));
+    INFLLM_CUDA_OK(dev_malloc_async((void**)&c->scores_aux, cap * sizeof(float), c->aux_stream));
     c->scores_aux_cap = cap;
   }
   trace_mark(c, c->aux_stream, TR_SPEC_BEGIN, target);
@@ -1005,7 +1055,7 @@ int flush_table(infllm_ctx* c, cudaStream_t s) {
     if (c->d_unit_ptrs) INFLLM_CUDA_OK(cudaFreeAsync(c->d_unit_ptrs, s));
     c->tab_cap = std::max<int64_t>(c->block_k_cap, 1024);
     // entries [tab_cap, tab_cap + topk): the landing slot of every retrieval position
-    INFLLM_CUDA_OK(cudaMallocAsync((void**)&c->d_unit_ptrs, (c->tab_cap + topk) * sizeof(unsigned long long), s));
+    INFLLM_CUDA_OK(dev_malloc_async((void**)&c->d_unit_ptrs, (c->tab_cap + topk) * sizeof(unsigned long long), s));
     c->table_valid = false;
   }
   // a free slot set aside for every retrieval position (fewer when the pool runs dry: those positions deposit nothing)
@@ -1290,7 +1340,7 @@ int unit_score_update(infllm_ctx* c, const std::vector<int32_t>& ids, const char
   const int64_t D = g.head_dim, H = g.n_heads, HKV = g.n_kv_heads, bs = g.block_size;
   const int64_t cols = (int64_t)g.topk * bs, n = (int64_t)ids.size();
   if (!c->unit_prob) {
-    INFLLM_CUDA_OK(cudaMalloc((void**)&c->unit_prob, H * cols * sizeof(float)));
+    INFLLM_CUDA_OK(dev_malloc((void**)&c->unit_prob, H * cols * sizeof(float)));
     INFLLM_CUDA_OK(cudaHostAlloc((void**)&c->h_unit_prob, H * cols * sizeof(float), cudaHostAllocDefault));
   }
   for (int64_t i = 0; i < n; ++i) {
@@ -1559,7 +1609,7 @@ int append_sub(infllm_ctx* c, const char* q, int64_t q_hs, int64_t q_ts, const c
           const size_t need = attn_tc2_scratch_floats(TP.n_split, (int)H, lq);
           if (need > c->tc_part_floats) {
             if (c->tc_part) INFLLM_CUDA_OK(cudaFreeAsync(c->tc_part, s));
-            INFLLM_CUDA_OK(cudaMallocAsync((void**)&c->tc_part, need * sizeof(float), s));
+            INFLLM_CUDA_OK(dev_malloc_async((void**)&c->tc_part, need * sizeof(float), s));
             c->tc_part_floats = need;
           }
           if (TP.n_split > 1) {
@@ -1692,53 +1742,24 @@ int append_sub(infllm_ctx* c, const char* q, int64_t q_hs, int64_t q_ts, const c
 
 }  // namespace
 
-extern "C" int infllm_ctx_create(const infllm_config* cfg, infllm_ctx** out) {
-  if (!cfg || !out) return fail(INFLLM_E_BADARG, "ctx_create: null pointer");
-  const infllm_config& g = *cfg;
-  if (g.n_heads <= 0 || g.n_kv_heads <= 0 || g.n_heads % g.n_kv_heads)
-    return fail(INFLLM_E_BADARG, "ctx_create: %d heads / %d kv heads", g.n_heads, g.n_kv_heads);
-  if (g.head_dim != 128 && g.head_dim != 64)
-    return fail(INFLLM_E_UNSUPPORTED, "ctx_create: head_dim %d (64 and 128 are built)", g.head_dim);
-  if (g.n_init < 0 || g.n_local <= 0 || g.block_size <= 0 || g.topk <= 0 || g.exc_block_size <= 0 || g.repr_topk <= 0)
-    return fail(INFLLM_E_BADARG, "ctx_create: sizes must be positive");
-  if (g.exc_block_size > g.n_local)  // context_manager.py:219
-    return fail(INFLLM_E_BADARG, "ctx_create: exc_block_size %d > n_local %d", g.exc_block_size, g.n_local);
-  if (g.max_cached_block < g.topk)  // CudaCache.alloc would assert (context_manager.py:19)
-    return fail(INFLLM_E_CAPACITY, "ctx_create: max_cached_block %d < topk %d: a retrieval could not be held in the cache",
-                g.max_cached_block, g.topk);
-  if (g.repr_topk > g.block_size) return fail(INFLLM_E_BADARG, "ctx_create: repr_topk %d > block_size %d", g.repr_topk, g.block_size);
-  if (g.block_size % 8) return fail(INFLLM_E_BADARG, "ctx_create: block_size %d must be a multiple of 8", g.block_size);
-  if (g.dtype != INFLLM_BF16 && g.dtype != INFLLM_FP16) return fail(INFLLM_E_UNSUPPORTED, "ctx_create: dtype code %d", g.dtype);
-  if (g.cache_strategy != INFLLM_CACHE_LRU && g.cache_strategy != INFLLM_CACHE_LRU_S)
-    return fail(INFLLM_E_UNSUPPORTED, "ctx_create: cache strategy code %d", g.cache_strategy);
-  if (g.topk > 1024) return fail(INFLLM_E_UNSUPPORTED, "ctx_create: topk %d > 1024", g.topk);
-  if (g.chunk_topk_calc != 0 && g.chunk_topk_calc < g.exc_block_size)
-    return fail(INFLLM_E_BADARG, "ctx_create: chunk_topk_calc %d < exc_block_size %d", g.chunk_topk_calc, g.exc_block_size);
-  infllm_ctx* c = new (std::nothrow) infllm_ctx();
-  if (!c) return fail(INFLLM_E_NOMEM, "ctx_create: out of host memory");
-  c->cfg = g;
-  // lru-s: the cache plan of an exec block depends on the attention of the one before it (context_manager.py:
-  // 454-470), so nothing is ranked, staged or attended ahead of the host
-  if (g.cache_strategy == INFLLM_CACHE_LRU_S) c->cfg.debug_flags |= 2 | 16 | 32;
-  c->esz = 2;
-  c->width = (int64_t)g.n_heads * g.head_dim;
-  c->unit_elems = (int64_t)g.n_kv_heads * g.block_size * g.head_dim;
-  c->unit_bytes = 2 * c->unit_elems * c->esz;
-  c->lru = LruTable(g.max_cached_block);
-  if (g.look_depth > 0) c->look_depth = std::min<int>(g.look_depth, infllm_ctx::kMaxLookDepth);
-  *out = c;
-  return INFLLM_OK;
-}
-
-extern "C" int infllm_ctx_reset(infllm_ctx* c) {
-  if (!c) return fail(INFLLM_E_BADARG, "ctx_reset: null context");
+// Forget every token.  `wait`: also wait until nothing the context has enqueued is still running (the caller is about
+// to write the host store, or slabs of the device store go back to a pool that others take from); otherwise the
+// streams are only marked and the next append orders itself behind the marks.
+static int ctx_reset(infllm_ctx* c, bool wait) {
   if (c->initialized) {
     INFLLM_CUDA_OK(cudaSetDevice(c->cfg.device));
-    INFLLM_CUDA_OK(cudaStreamSynchronize(c->copy_stream));
-    INFLLM_CUDA_OK(cudaStreamSynchronize(c->urgent_stream));
-    INFLLM_CUDA_OK(cudaStreamSynchronize(c->aux_stream));
-    INFLLM_CUDA_OK(cudaStreamSynchronize(c->d2h_stream));
-    INFLLM_CUDA_OK(cudaStreamSynchronize(c->mail_stream));
+    cudaStream_t side[5] = {c->copy_stream, c->urgent_stream, c->aux_stream, c->d2h_stream, c->mail_stream};
+    if (wait || !c->dev_slabs.empty()) {
+      for (cudaStream_t s : side) INFLLM_CUDA_OK(cudaStreamSynchronize(s));
+      if (c->attn_recorded) INFLLM_CUDA_OK(cudaEventSynchronize(c->ev_attn));
+      if (c->last_recorded) INFLLM_CUDA_OK(cudaEventSynchronize(c->ev_last));
+    } else {
+      for (int i = 0; i < 5; ++i) INFLLM_CUDA_OK(cudaEventRecord(c->ev_side[i], side[i]));
+      // (marks of an earlier reset that no append has followed still stand)
+      c->reset_attn = c->attn_recorded || (c->reset_pending && c->reset_attn);
+      c->reset_last = c->last_recorded || (c->reset_pending && c->reset_last);
+    }
+    c->reset_pending = true;
   }
   c->pend_head = c->pend_count = 0;  // retrievals not yet applied belong to the tokens that are forgotten
   c->landing_slots.clear();
@@ -1753,6 +1774,7 @@ extern "C" int infllm_ctx_reset(infllm_ctx* c) {
   c->init_full = false;
   c->rope_origin = -1;
   c->tb.t0 = 0;
+  c->tb.zero_upto = 0;  // the rows hold what the forgotten tokens left there
   c->lru.clear();
   c->slot_of.clear();
   c->table_valid = false;
@@ -1768,12 +1790,17 @@ extern "C" int infllm_ctx_reset(infllm_ctx* c) {
   c->attn_recorded = false;
   c->attn_prev_recorded = false;
   c->spec_recorded = false;
+  c->last_recorded = false;
   c->counters = infllm_ctx_info{};
   return INFLLM_OK;
 }
 
-extern "C" int infllm_ctx_destroy(infllm_ctx* c) {
-  if (!c) return INFLLM_OK;
+extern "C" int infllm_ctx_reset(infllm_ctx* c) {
+  if (!c) return fail(INFLLM_E_BADARG, "ctx_reset: null context");
+  return ctx_reset(c, false);
+}
+
+static void ctx_free(infllm_ctx* c) {
   if (c->initialized) {
     cudaSetDevice(c->cfg.device);
     cudaDeviceSynchronize();
@@ -1836,10 +1863,165 @@ extern "C" int infllm_ctx_destroy(infllm_ctx* c) {
     cudaEventDestroy(c->ev_attn);
     cudaEventDestroy(c->ev_attn_prev);
     cudaStreamDestroy(c->urgent_stream);
+    cudaEventDestroy(c->ev_last);
+    for (cudaEvent_t e : c->ev_side) cudaEventDestroy(e);
     for (cudaEvent_t e : c->ev_pool) cudaEventDestroy(e);
+    for (auto& m : c->marks) cudaEventDestroy(m.ev);
     cudaDeviceSynchronize();
   }
   delete c;
+}
+
+// ------------------------------------------------------------------------------------ idle contexts
+// A program that drops a memory and starts another of the same shape (a new prompt in a generation loop, once per
+// layer) would pay for its workspaces again: some twenty device allocations and as many frees, five streams, and a
+// slab of page-locked host memory, which alone costs 50 ms and more.  A destroyed context therefore becomes idle, its
+// tokens forgotten, and infllm_ctx_create hands it out again for an equal configuration.  Measured: an 8192-token prompt
+// into a new memory 140 -> 4.8 ms, a 32768-token prompt 217 -> 13 ms.  The bounds: at most kIdleContexts contexts, kIdleBytes of device memory (and no more than a
+// quarter of what is free on the device) and kIdleBytes of pinned host memory; past them the oldest are freed.
+// infllm_ctx_release_idle frees all of them, and an allocation of the library that fails does so before it tries
+// again.  The list is behind a mutex; the streams' order is kept by the marks of ctx_reset, whichever stream the next
+// owner appends on.
+constexpr size_t kIdleContexts = 256;
+constexpr int64_t kIdleBytes = 16ll << 30;
+
+struct IdleContext {
+  infllm_ctx* c;
+  int64_t dev_bytes, host_bytes;
+};
+struct IdlePool {
+  std::mutex mu;
+  std::list<IdleContext> list;  // oldest first
+  int64_t dev_bytes = 0, host_bytes = 0;
+};
+static IdlePool& idle_pool() {
+  static IdlePool* p = new IdlePool();  // never destroyed: the CUDA runtime may be gone when static objects are
+  return *p;
+}
+
+static int64_t ctx_device_bytes(const infllm_ctx* c) {
+  const infllm_config& g = c->cfg;
+  const int64_t D = g.head_dim, H = g.n_heads, HKV = g.n_kv_heads, exc = g.exc_block_size;
+  int64_t n = 2 * c->pack_units * c->unit_bytes + c->tab_len * D * 4 + 2 * HKV * c->init_cap * D * c->esz;
+  n += 2 * H * c->sub_max * D * c->esz + (c->sub_max / exc + 1) * c->width * 4 + H * exc * (D + 3) * 4;
+  n += (int64_t)c->max_parts * H * (D + 1) * 4 + H * ((int64_t)g.n_local + 1) * 4;
+  n += ((int64_t)g.max_cached_block + (int64_t)c->look_depth * g.topk) * c->unit_bytes;
+  n += HKV * c->tb.cap * D * c->esz * 3 + H * c->tb.cap * 4 + c->block_k_cap * c->width * c->esz;
+  n += (int64_t)c->tc_part_floats * 4 + (c->scores_cap + c->scores_aux_cap) * 4 + c->tab_cap * 8;
+  return n;
+}
+
+// frees the oldest idle contexts until the pool's bounds hold with `dev` and `host` bytes more (all: every context)
+static int idle_trim(int64_t dev, int64_t host, int64_t dev_limit, bool all) {
+  std::vector<infllm_ctx*> gone;
+  {
+    IdlePool& p = idle_pool();
+    std::lock_guard<std::mutex> lk(p.mu);
+    while (!p.list.empty() && (all || p.list.size() >= kIdleContexts || p.dev_bytes + dev > dev_limit ||
+                               p.host_bytes + host > kIdleBytes)) {
+      p.dev_bytes -= p.list.front().dev_bytes;
+      p.host_bytes -= p.list.front().host_bytes;
+      gone.push_back(p.list.front().c);
+      p.list.pop_front();
+    }
+  }
+  int cur = -1;
+  if (!gone.empty()) cudaGetDevice(&cur);
+  for (infllm_ctx* c : gone) ctx_free(c);
+  if (cur >= 0) cudaSetDevice(cur);
+  return (int)gone.size();
+}
+
+extern "C" int infllm_ctx_release_idle(void) {
+  idle_trim(0, 0, kIdleBytes, true);
+  return INFLLM_OK;
+}
+
+extern "C" int infllm_ctx_destroy(infllm_ctx* c) {
+  if (!c) return INFLLM_OK;
+  bool keep = c->initialized && !c->failed;
+  if (keep) {
+    int cur = 0;
+    cudaGetDevice(&cur);
+    const int64_t dev = ctx_device_bytes(c), host = (int64_t)c->slabs.size() * c->slab_units * c->unit_bytes;
+    size_t free_b = 0, total_b = 0;
+    keep = cudaSetDevice(c->cfg.device) == cudaSuccess && cudaMemGetInfo(&free_b, &total_b) == cudaSuccess;
+    IdlePool& p = idle_pool();
+    int64_t limit = 0;
+    if (keep) {
+      std::lock_guard<std::mutex> lk(p.mu);
+      limit = std::min<int64_t>(kIdleBytes, ((int64_t)free_b + p.dev_bytes + dev) / 4);
+    }
+    keep = keep && dev <= limit && host <= kIdleBytes && ctx_reset(c, false) == INFLLM_OK;
+    if (keep) {
+      c->comm = nullptr;
+      c->prof = c->trace_on = false;
+      c->pending.clear();
+      c->ev_used = 0;
+      for (auto& m : c->marks) cudaEventDestroy(m.ev);
+      c->marks.clear();
+      for (int i = 0; i < INFLLM_PROF_SLOTS; ++i) c->prof_ms[i] = c->prof_work[i] = 0, c->prof_launches[i] = 0;
+      for (double& us : c->host_us) us = 0;
+      idle_trim(dev, host, limit, false);
+      std::lock_guard<std::mutex> lk(p.mu);
+      p.list.push_back({c, dev, host});
+      p.dev_bytes += dev;
+      p.host_bytes += host;
+    }
+    cudaSetDevice(cur);
+  }
+  if (!keep) ctx_free(c);
+  return INFLLM_OK;
+}
+
+extern "C" int infllm_ctx_create(const infllm_config* cfg, infllm_ctx** out) {
+  if (!cfg || !out) return fail(INFLLM_E_BADARG, "ctx_create: null pointer");
+  const infllm_config& g = *cfg;
+  if (g.n_heads <= 0 || g.n_kv_heads <= 0 || g.n_heads % g.n_kv_heads)
+    return fail(INFLLM_E_BADARG, "ctx_create: %d heads / %d kv heads", g.n_heads, g.n_kv_heads);
+  if (g.head_dim != 128 && g.head_dim != 64)
+    return fail(INFLLM_E_UNSUPPORTED, "ctx_create: head_dim %d (64 and 128 are built)", g.head_dim);
+  if (g.n_init < 0 || g.n_local <= 0 || g.block_size <= 0 || g.topk <= 0 || g.exc_block_size <= 0 || g.repr_topk <= 0)
+    return fail(INFLLM_E_BADARG, "ctx_create: sizes must be positive");
+  if (g.exc_block_size > g.n_local)  // context_manager.py:219
+    return fail(INFLLM_E_BADARG, "ctx_create: exc_block_size %d > n_local %d", g.exc_block_size, g.n_local);
+  if (g.max_cached_block < g.topk)  // CudaCache.alloc would assert (context_manager.py:19)
+    return fail(INFLLM_E_CAPACITY, "ctx_create: max_cached_block %d < topk %d: a retrieval could not be held in the cache",
+                g.max_cached_block, g.topk);
+  if (g.repr_topk > g.block_size) return fail(INFLLM_E_BADARG, "ctx_create: repr_topk %d > block_size %d", g.repr_topk, g.block_size);
+  if (g.block_size % 8) return fail(INFLLM_E_BADARG, "ctx_create: block_size %d must be a multiple of 8", g.block_size);
+  if (g.dtype != INFLLM_BF16 && g.dtype != INFLLM_FP16) return fail(INFLLM_E_UNSUPPORTED, "ctx_create: dtype code %d", g.dtype);
+  if (g.cache_strategy != INFLLM_CACHE_LRU && g.cache_strategy != INFLLM_CACHE_LRU_S)
+    return fail(INFLLM_E_UNSUPPORTED, "ctx_create: cache strategy code %d", g.cache_strategy);
+  if (g.topk > 1024) return fail(INFLLM_E_UNSUPPORTED, "ctx_create: topk %d > 1024", g.topk);
+  if (g.chunk_topk_calc != 0 && g.chunk_topk_calc < g.exc_block_size)
+    return fail(INFLLM_E_BADARG, "ctx_create: chunk_topk_calc %d < exc_block_size %d", g.chunk_topk_calc, g.exc_block_size);
+  infllm_config use = g;
+  // lru-s: the cache plan of an exec block depends on the attention of the one before it (context_manager.py:
+  // 454-470), so nothing is ranked, staged or attended ahead of the host
+  if (g.cache_strategy == INFLLM_CACHE_LRU_S) use.debug_flags |= 2 | 16 | 32;
+  {
+    IdlePool& p = idle_pool();
+    std::lock_guard<std::mutex> lk(p.mu);
+    for (auto it = p.list.rbegin(); it != p.list.rend(); ++it)
+      if (memcmp(&it->c->cfg, &use, sizeof(use)) == 0) {  // the one that became idle last: its memory is warm
+        *out = it->c;
+        p.dev_bytes -= it->dev_bytes;
+        p.host_bytes -= it->host_bytes;
+        p.list.erase(std::next(it).base());
+        return INFLLM_OK;
+      }
+  }
+  infllm_ctx* c = new (std::nothrow) infllm_ctx();
+  if (!c) return fail(INFLLM_E_NOMEM, "ctx_create: out of host memory");
+  c->cfg = use;
+  c->esz = 2;
+  c->width = (int64_t)g.n_heads * g.head_dim;
+  c->unit_elems = (int64_t)g.n_kv_heads * g.block_size * g.head_dim;
+  c->unit_bytes = 2 * c->unit_elems * c->esz;
+  c->lru = LruTable(g.max_cached_block);
+  if (g.look_depth > 0) c->look_depth = std::min<int>(g.look_depth, infllm_ctx::kMaxLookDepth);
+  *out = c;
   return INFLLM_OK;
 }
 
@@ -1854,12 +2036,15 @@ extern "C" int infllm_ctx_append(infllm_ctx* c, const void* d_q, int64_t q_hs, i
   cudaStream_t s = (cudaStream_t)stream;
   INFLLM_CUDA_OK(cudaSetDevice(c->cfg.device));
   if (!c->initialized) INFLLM_TRY(lazy_init(c, s));
+  INFLLM_TRY(order_behind_reset(c, s));
   INFLLM_TRY(poll_device_error(c, s));
+  c->failed = true;  // until the call has gone through
   c->call_serial += 1;
   c->last_stream = s;
   c->trace_topk.clear();
   c->counters.exec_blocks = 0;
   const int esz = c->esz;
+  const int64_t units_before = c->num_blocks;
   c->chunk_mode = c->cfg.chunk_topk_calc > 0 && len > 1;  // context_manager.py:749
   for (int64_t off = 0; off < len; off += c->sub_max) {
     const int64_t n = std::min<int64_t>(c->sub_max, len - off);
@@ -1869,6 +2054,11 @@ extern "C" int infllm_ctx_append(infllm_ctx* c, const void* d_q, int64_t q_hs, i
                           o_ts, n, s));
   }
   if (c->use_tc && len > 64) INFLLM_TRY(send_device_error(c, s, s));  // read by the next call (or by get_info)
+  if (len > 1 || c->num_blocks != units_before) {  // a token that seals nothing ends with its attention: ev_attn
+    INFLLM_CUDA_OK(cudaEventRecord(c->ev_last, s));
+    c->last_recorded = true;
+  }
+  c->failed = false;
   return INFLLM_OK;
 }
 
@@ -2004,7 +2194,8 @@ extern "C" int infllm_ctx_load_synthetic(infllm_ctx* c, int64_t n_units, const v
   cudaStream_t s = (cudaStream_t)stream;
   INFLLM_CUDA_OK(cudaSetDevice(g.device));
   if (!c->initialized) INFLLM_TRY(lazy_init(c, s));
-  INFLLM_TRY(infllm_ctx_reset(c));
+  INFLLM_TRY(ctx_reset(c, true));
+  INFLLM_TRY(order_behind_reset(c, s));
   const int64_t D = g.head_dim, HKV = g.n_kv_heads;
   INFLLM_TRY(ensure_host_units(c, n_units));
   for (int64_t b = 0; b < n_units; ++b) memcpy(c->host_unit(b), (const char*)h_units + b * c->unit_bytes, c->unit_bytes);
@@ -2029,7 +2220,7 @@ extern "C" int infllm_ctx_load_synthetic(infllm_ctx* c, int64_t n_units, const v
   const int64_t kv_hs = tb.cap * D;
   void* tmp = nullptr;
   const size_t wbytes = HKV * (int64_t)g.n_local * D * c->esz;
-  INFLLM_CUDA_OK(cudaMallocAsync(&tmp, 2 * wbytes, s));
+  INFLLM_CUDA_OK(dev_malloc_async((void**)&tmp, 2 * wbytes, s));
   INFLLM_CUDA_OK(cudaMemcpyAsync(tmp, h_win_k, wbytes, cudaMemcpyHostToDevice, s));
   INFLLM_CUDA_OK(cudaMemcpyAsync((char*)tmp + wbytes, h_win_v, wbytes, cudaMemcpyHostToDevice, s));
   const int64_t at = c->length - tb.t0;
@@ -2284,7 +2475,8 @@ extern "C" int infllm_ctx_load(infllm_ctx* c, const char* path, void* stream) {
   }
   INFLLM_CUDA_OK(cudaSetDevice(g.device));
   if (!c->initialized) INFLLM_TRY(lazy_init(c, s));
-  INFLLM_TRY(infllm_ctx_reset(c));
+  INFLLM_TRY(ctx_reset(c, true));
+  INFLLM_TRY(order_behind_reset(c, s));
   bool ok = true;
   std::vector<char> buf;
   auto fill2d = [&](void* dev, int64_t pitch, int64_t width, int64_t rows) -> bool {
@@ -2344,7 +2536,7 @@ extern "C" int infllm_device_store_reserve(int device, int64_t bytes) {
   const int64_t n = bytes / (int64_t)kPoolSlabBytes;
   for (int64_t i = 0; i < n; ++i) {
     void* p = nullptr;
-    cudaError_t e = cudaMalloc(&p, kPoolSlabBytes);
+    cudaError_t e = dev_malloc(&p, kPoolSlabBytes);
     if (e != cudaSuccess) {
       cudaGetLastError();
       return fail(INFLLM_E_NOMEM, "device_store_reserve: cudaMalloc failed after %lld of %lld slabs of 128 MiB: %s",

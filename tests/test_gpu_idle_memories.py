@@ -1,0 +1,72 @@
+"""Workspaces of dropped memories are handed out again (infllm_ctx_destroy / infllm_ctx_create): a memory that starts
+in them, on another stream and behind work that is still running, behaves like the first one, and nothing of the old
+sequence is left - not even values that no arithmetic would wipe out."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+H, HKV, D = 8, 2, 128
+
+
+def _tokens(n, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    return [torch.randn((1, h, n, D), generator=g, device="cuda").to(torch.bfloat16) for h in (H, HKV, HKV)]
+
+
+def _run(calls, stream=None, device_store_mb=0):
+    from infllm_b200.attention import ContextManager, RotaryEmbeddingESM
+
+    cm = ContextManager(RotaryEmbeddingESM(D, 1e6, 1.0), 64, 512, 128, 6, 4, 256, None, True, 4,
+                        device_store_mb=device_store_mb)
+    with torch.cuda.stream(stream) if stream is not None else torch.cuda.stream(torch.cuda.current_stream()):
+        outs = [cm.append(q, k, v, q, k, v) for q, k, v in calls]
+    return cm, outs
+
+
+@pytest.mark.parametrize("tail", [1, 37, 300])
+def test_a_reused_memory_equals_a_new_one(tail):
+    from infllm_b200.attention import release_idle_memories
+
+    calls = [_tokens(2300, 1), _tokens(tail, 2), _tokens(1, 3)]
+    torch.cuda.synchronize()
+    release_idle_memories()
+    cm, want = _run(calls)
+    ids = cm.last_topk()
+    torch.cuda.synchronize()
+    # another sequence in the same workspaces: longer, with infinities in its keys and values, dropped while it runs
+    other = [_tokens(4000, 4)]
+    other[0][1][:, :, 100::7] = float("inf")
+    other[0][2][:, :, ::5] = float("nan")
+    torch.cuda.synchronize()
+    del cm
+    cm, _ = _run(other)
+    del cm
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    cm, got = _run(calls, side)
+    assert cm.last_topk() == ids
+    torch.cuda.synchronize()
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
+
+
+def test_idle_memories_are_bounded_by_their_shape_and_given_back():
+    from infllm_b200.attention import release_idle_memories
+
+    torch.cuda.synchronize()
+    release_idle_memories()
+    calls = [_tokens(1500, 5)]
+    cm, _ = _run(calls)
+    torch.cuda.synchronize()
+    held = torch.cuda.mem_get_info()[0]
+    for _ in range(3):  # one at a time: the same workspaces every time
+        del cm
+        cm, _ = _run(calls)
+    torch.cuda.synchronize()
+    # (the stream-ordered pool behind the token buffers may grow by a buffer while the old one is still in use)
+    assert torch.cuda.mem_get_info()[0] >= held - (64 << 20)
+    del cm
+    release_idle_memories()
+    torch.cuda.synchronize()
+    assert torch.cuda.mem_get_info()[0] > held
