@@ -91,6 +91,19 @@ int infllm_attn_stage(const void* d_q, int64_t q_hs, int64_t q_ts,
                       int n_heads, int n_kv_heads, int64_t lq, int64_t lk, int head_dim,
                       int mask_mode, int64_t mask_offset, int64_t mask_size,
                       float* d_acc, float* d_m, float* d_l, int first, int dtype, void* stream);
+/* infllm_attn_stage_ex: the same with two additions.  d_scratch (scratch_floats of them, may be NULL): room for partial
+ *   results, with which a stage that has few queries is cut along its keys so that it fills the GPU;
+ *   infllm_attn_stage_scratch says how much makes a difference.  d_out (may be NULL): this is the last stage — the
+ *   normalised rows go to d_out and their log-sum-exp to d_lse (may be NULL) instead of the state, which with
+ *   first != 0 may then be NULL too. */
+int64_t infllm_attn_stage_scratch(int n_heads, int n_kv_heads, int64_t lq, int64_t lk, int head_dim);
+int infllm_attn_stage_ex(const void* d_q, int64_t q_hs, int64_t q_ts,
+                         const void* d_k, int64_t k_hs, int64_t k_ts,
+                         const void* d_v, int64_t v_hs, int64_t v_ts,
+                         int n_heads, int n_kv_heads, int64_t lq, int64_t lk, int head_dim,
+                         int mask_mode, int64_t mask_offset, int64_t mask_size,
+                         float* d_acc, float* d_m, float* d_l, int first, float* d_scratch, int64_t scratch_floats,
+                         void* d_out, int64_t o_hs, int64_t o_ts, float* d_lse, int dtype, void* stream);
 int infllm_attn_finalize(const float* d_acc, const float* d_m, const float* d_l,
                          void* d_out, int64_t o_hs, int64_t o_ts, float* d_lse,
                          int n_heads, int64_t lq, int head_dim, int dtype, void* stream);

@@ -99,6 +99,11 @@ SIGNATURES = {
     "infllm_attn_stage": (c_int, [c_void_p, c_int64, c_int64, c_void_p, c_int64, c_int64, c_void_p, c_int64, c_int64,
                                   c_int, c_int, c_int64, c_int64, c_int, c_int, c_int64, c_int64,
                                   c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p]),
+    "infllm_attn_stage_scratch": (c_int64, [c_int, c_int, c_int64, c_int64, c_int]),
+    "infllm_attn_stage_ex": (c_int, [c_void_p, c_int64, c_int64, c_void_p, c_int64, c_int64, c_void_p, c_int64, c_int64,
+                                     c_int, c_int, c_int64, c_int64, c_int, c_int, c_int64, c_int64,
+                                     c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int64, c_void_p, c_int64, c_int64,
+                                     c_void_p, c_int, c_void_p]),
     "infllm_attn_finalize": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_void_p,
                                      c_int, c_int64, c_int, c_int, c_void_p]),
     "infllm_attn_colsum": (c_int, [c_void_p, c_int64, c_int64, c_void_p, c_int64, c_int64, c_int, c_int, c_int64,

@@ -20,11 +20,8 @@ class CudaMultiStageDotProductionAttention:
         self.dtype = dtype
         self.device = torch.device(device)
         self._code = _lib.dtype_code(dtype)
-        b, h, lq, d = self.q_shape
-        self._acc = torch.empty((b, h, lq, d), dtype=torch.float32, device=self.device)
-        self._m = torch.empty((b, h, lq), dtype=torch.float32, device=self.device)
-        self._l = torch.empty((b, h, lq), dtype=torch.float32, device=self.device)
-        self._stages = []
+        self._state = None  # (acc, m, l) between stages, fp32; a single stage needs none
+        self._stages, self._scored = [], []
         self._first = True
         self.end = False
         self.ret = None
@@ -55,27 +52,38 @@ class CudaMultiStageDotProductionAttention:
         if k.stride(-1) != 1 or k.stride() != v.stride():
             k, v = k.contiguous(), v.contiguous()
         stream = _lib.stream_ptr(self.device)
+        lib, f32 = _lib.lib, torch.float32
+        if get_score:
+            self._scored.append(len(self._stages))
+        if self._state is None and not end:
+            self._state = (torch.empty((b, h, lq, d), dtype=f32, device=self.device),
+                           torch.empty((2, b, h, lq), dtype=f32, device=self.device))
+        lse = None
+        if end:
+            self.ret = torch.empty(self.q_shape, dtype=self.dtype, device=self.device)
+            lse = torch.empty((b, h, lq), dtype=f32, device=self.device) if self._scored else None
+        n_scratch = lib.infllm_attn_stage_scratch(h, hkv, lq, lk, d)
+        scratch = torch.empty(n_scratch, dtype=f32, device=self.device) if n_scratch > 0 else None
+        out = self.ret
         for bi in range(b):
-            _lib.check(_lib.lib.infllm_attn_stage(
+            acc, m, l = (None, None, None) if self._state is None else (
+                self._state[0][bi].data_ptr(), self._state[1][0, bi].data_ptr(), self._state[1][1, bi].data_ptr())
+            _lib.check(lib.infllm_attn_stage_ex(
                 q[bi].data_ptr(), q.stride(1), q.stride(2), k[bi].data_ptr() if lk else None, k.stride(1), k.stride(2),
                 v[bi].data_ptr() if lk else None, v.stride(1), v.stride(2), h, hkv, lq, lk, d, mode, off, size,
-                self._acc[bi].data_ptr(), self._m[bi].data_ptr(), self._l[bi].data_ptr(), int(self._first),
-                self._code, stream))
+                acc, m, l, int(self._first), None if scratch is None else scratch.data_ptr(), n_scratch,
+                out[bi].data_ptr() if end else None, out.stride(1) if end else 0, out.stride(2) if end else 0,
+                lse[bi].data_ptr() if lse is not None else None, self._code, stream))
         self._first = False
         self._stages.append((q, k, mode, off, size) if get_score else None)
         if end:
-            self._finalize()
+            self._finalize(lse)
 
-    def _finalize(self):
+    def _finalize(self, lse):
+        """The per-key scores of the stages that asked for them, from the final log-sum-exp of every row."""
         self.end = True
         b, h, lq, d = self.q_shape
-        self.ret = torch.empty(self.q_shape, dtype=self.dtype, device=self.device)
-        lse = torch.empty((b, h, lq), dtype=torch.float32, device=self.device)
         stream = _lib.stream_ptr(self.device)
-        for bi in range(b):
-            _lib.check(_lib.lib.infllm_attn_finalize(
-                self._acc[bi].data_ptr(), self._m[bi].data_ptr(), self._l[bi].data_ptr(), self.ret[bi].data_ptr(),
-                self.ret.stride(1), self.ret.stride(2), lse[bi].data_ptr(), h, lq, d, self._code, stream))
         for st in self._stages:
             if st is None:
                 self.score_list.append(None)
@@ -83,7 +91,8 @@ class CudaMultiStageDotProductionAttention:
                 continue
             q, k, mode, off, size = st
             lk, hkv = k.size(2), k.size(1)
-            score = torch.zeros((b, h, lk), dtype=torch.float32, device=self.device)
+            # every column is written, unless there is nothing to sum
+            score = (torch.empty if lq and lk else torch.zeros)((b, h, lk), dtype=torch.float32, device=self.device)
             for bi in range(b):
                 _lib.check(_lib.lib.infllm_attn_colsum(
                     q[bi].data_ptr(), q.stride(1), q.stride(2), k[bi].data_ptr() if lk else None, k.stride(1),

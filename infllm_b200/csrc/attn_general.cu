@@ -6,6 +6,8 @@
 // the reference's append()/get_result() (dot_production_attention/base.py:18-30).  The 512-query
 // exec-block fast path of the context memory uses the tcgen05 kernel in attn_tc.cu instead; this
 // one serves ragged shapes, short query blocks and the column-sum (per-key score) pass.
+#include <algorithm>
+
 #include "attn_common.cuh"
 #include "attn_tc.cuh"
 #include "mma_common.cuh"
@@ -393,17 +395,29 @@ int launch_colsum(const void* q, int64_t q_hs, int64_t q_ts, const void* k, int6
   return INFLLM_OK;
 }
 
+// out = acc / l: HBM-bound, four columns per thread (8 MB in and 4 MB out at 512 queries x 32 heads: 11 us with one CTA
+// per row, 3.2 us like this)
 template <typename T>
-__global__ void attn_finalize_kernel(const float* __restrict__ acc, const float* __restrict__ m,
-                                     const float* __restrict__ l, T* __restrict__ out, int64_t o_hs, int64_t o_ts,
-                                     float* __restrict__ lse, int64_t lq, int head_dim) {
-  int64_t row = blockIdx.x;  // h * lq + i
-  int64_t h = row / lq, i = row - h * lq;
-  float lv = l[row];
-  float inv = lv > 0.f ? 1.f / lv : 0.f;
-  for (int d = threadIdx.x; d < head_dim; d += blockDim.x)
-    out[h * o_hs + i * o_ts + d] = Act<T>::from_f(acc[row * head_dim + d] * inv);
-  if (lse && threadIdx.x == 0) lse[row] = lv > 0.f ? m[row] + log2f(lv) : -INFINITY;
+__global__ void __launch_bounds__(256)
+attn_finalize_kernel(const float* __restrict__ acc, const float* __restrict__ m, const float* __restrict__ l,
+                     T* __restrict__ out, int64_t o_hs, int64_t o_ts, float* __restrict__ lse, int64_t rows, int64_t lq,
+                     int head_dim, int vec) {
+  const int per_row = head_dim / 4;
+  const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, row = idx / per_row;  // row = h * lq + i
+  if (row >= rows) return;
+  const int d = (int)(idx - row * per_row) * 4;
+  const int64_t h = row / lq, i = row - h * lq;
+  const float lv = l[row], inv = lv > 0.f ? 1.f / lv : 0.f;
+  const float2 a = *reinterpret_cast<const float2*>(acc + row * head_dim + d),
+               b = *reinterpret_cast<const float2*>(acc + row * head_dim + d + 2);
+  T* o = out + h * o_hs + i * o_ts + d;
+  const typename Act<T>::T2 v01 = Act<T>::from_f2(a.x * inv, a.y * inv), v23 = Act<T>::from_f2(b.x * inv, b.y * inv);
+  if (vec) {
+    *reinterpret_cast<uint2*>(o) = make_uint2(*reinterpret_cast<const uint32_t*>(&v01), *reinterpret_cast<const uint32_t*>(&v23));
+  } else {  // rows that are not 8-byte aligned
+    o[0] = v01.x, o[1] = v01.y, o[2] = v23.x, o[3] = v23.y;
+  }
+  if (lse && d == 0) lse[row] = lv > 0.f ? m[row] + log2f(lv) : -INFINITY;
 }
 
 }  // namespace
@@ -439,24 +453,117 @@ static int check_rows(const void* p, int64_t hs, int64_t ts, const char* what) {
   return INFLLM_OK;
 }
 
-extern "C" int infllm_attn_stage(const void* d_q, int64_t q_hs, int64_t q_ts, const void* d_k, int64_t k_hs,
-                                 int64_t k_ts, const void* d_v, int64_t v_hs, int64_t v_ts, int n_heads,
-                                 int n_kv_heads, int64_t lq, int64_t lk, int head_dim, int mask_mode,
-                                 int64_t mask_offset, int64_t mask_size, float* d_acc, float* d_m, float* d_l,
-                                 int first, int dtype, void* stream) {
+namespace infllm {
+
+// Which kernel a stage runs on (head_dim 128, rows aligned for TMA; everything else: the shape-generic one above).
+//   one query    the split-K decode kernel, up to 8 query heads per KV head: it is bound by the K/V bytes
+//   others       the tcgen05 kernel.  Its fixed cost is one 128-key tile; the generic kernel takes 3.9 us per 64 keys
+//                whatever the number of queries (one CTA per 64 of them walks the keys alone), so a stage has to be as
+//                short as one tile, with at most one tile of queries, before that one is the cheaper.
+enum StageKernel { STAGE_GENERIC, STAGE_ONE, STAGE_TC };
+static StageKernel stage_kernel(int n_heads, int n_kv_heads, int64_t lq, int64_t lk, int head_dim) {
+  if (head_dim != 128 || n_heads % n_kv_heads || lk <= 0 || lk > INT32_MAX) return STAGE_GENERIC;
+  if (lq == 1 && n_heads / n_kv_heads <= 8) return STAGE_ONE;
+  if (lk > kTile || lq > kTile) return STAGE_TC;
+  return STAGE_GENERIC;
+}
+
+static int stage_tc(const void* d_q, int64_t q_hs, int64_t q_ts, const void* d_k, const void* d_v, int64_t k_hs,
+                    int64_t k_ts, int n_heads, int n_kv_heads, int64_t lq, int64_t lk, int mask_mode,
+                    int64_t mask_offset, int64_t mask_size, float* d_acc, float* d_m, float* d_l, int first,
+                    float* scratch, int64_t scratch_floats, void* out, int64_t o_hs, int64_t o_ts, float* lse, int dtype,
+                    cudaStream_t s) {
+  AttnTcParams P{};
+  INFLLM_TRY(encode_rows_map(&P.maps[0], dtype, d_q, lq, n_heads, q_hs, q_ts));
+  INFLLM_TRY(encode_rows_map(&P.maps[1], dtype, d_k, lk, n_kv_heads, k_hs, k_ts));
+  INFLLM_TRY(encode_rows_map(&P.maps[2], dtype, d_v, lk, n_kv_heads, k_hs, k_ts));
+  INFLLM_TRY(tc_get_error_ptr(&P.err));
+  P.n_stage = 1; P.n_heads = n_heads; P.n_kv_heads = n_kv_heads; P.lq = lq;
+  P.scale_log2 = kLog2e / sqrtf(128.f);
+  P.stage[0] = {0, 0, mask_mode, 0, 1, 0, mask_offset, mask_size, lk};
+  P.seg[0] = {1, 2, 0, -1, -1, (int32_t)lk};
+  P.n_split = attn_tc3_splits(lq, n_heads, lk);
+  const int64_t rows = n_heads * lq;
+  if (P.n_split > 1 && (int64_t)P.n_split * rows * 130 > scratch_floats) P.n_split = 1;
+  if (P.n_split > 1) {
+    P.part_acc = scratch;
+    P.part_m = scratch + P.n_split * rows * 128;
+    P.part_l = P.part_m + P.n_split * rows;
+    INFLLM_TRY(attn_tc3_launch(P, dtype, s));
+    return attn_tc_combine_launch(P.part_acc, P.part_m, P.part_l, P.n_split, n_heads, lq, out, o_hs, o_ts, lse,
+                                  first ? nullptr : d_acc, d_m, d_l, d_acc, d_m, d_l, dtype, s);
+  }
+  if (!first) P.st_acc = d_acc, P.st_m = d_m, P.st_l = d_l;
+  if (out) {
+    P.out = out; P.o_hs = o_hs; P.o_ts = o_ts; P.lse = lse;
+  } else {
+    P.part_acc = d_acc; P.part_m = d_m; P.part_l = d_l;
+  }
+  return attn_tc3_launch(P, dtype, s);
+}
+
+}  // namespace infllm
+
+// Floats of scratch with which infllm_attn_stage_ex splits a stage of these sizes over the whole GPU (0: none needed).
+extern "C" int64_t infllm_attn_stage_scratch(int n_heads, int n_kv_heads, int64_t lq, int64_t lk, int head_dim) {
   using namespace infllm;
-  if (!d_q || !d_acc || !d_m || !d_l || lq < 0 || lk < 0 || n_heads <= 0 || n_kv_heads <= 0)
+  if (n_heads <= 0 || n_kv_heads <= 0 || lq <= 0 || lk <= 0) return 0;
+  switch (stage_kernel(n_heads, n_kv_heads, lq, lk, head_dim)) {
+    case STAGE_ONE: return infllm_attn_decode_max_parts(1, lk) * n_heads * 129;
+    case STAGE_TC: {
+      const int n = attn_tc3_splits(lq, n_heads, lk);
+      return n > 1 ? (int64_t)n * n_heads * lq * 130 : 0;
+    }
+    default: return 0;
+  }
+}
+
+extern "C" int infllm_attn_stage_ex(const void* d_q, int64_t q_hs, int64_t q_ts, const void* d_k, int64_t k_hs,
+                                    int64_t k_ts, const void* d_v, int64_t v_hs, int64_t v_ts, int n_heads,
+                                    int n_kv_heads, int64_t lq, int64_t lk, int head_dim, int mask_mode,
+                                    int64_t mask_offset, int64_t mask_size, float* d_acc, float* d_m, float* d_l,
+                                    int first, float* d_scratch, int64_t scratch_floats, void* d_out, int64_t o_hs,
+                                    int64_t o_ts, float* d_lse, int dtype, void* stream) {
+  using namespace infllm;
+  if (!d_q || ((!first || !d_out) && (!d_acc || !d_m || !d_l)) || lq < 0 || lk < 0 || n_heads <= 0 || n_kv_heads <= 0)
     return fail(INFLLM_E_BADARG, "attn_stage: bad argument");
   if (lk > 0 && (!d_k || !d_v)) return fail(INFLLM_E_BADARG, "attn_stage: null keys/values");
-  if (k_hs != v_hs || k_ts != v_ts) return fail(INFLLM_E_BADARG, "attn_stage: k and v must share strides");
+  if (lk > 0 && (k_hs != v_hs || k_ts != v_ts)) return fail(INFLLM_E_BADARG, "attn_stage: k and v must share strides");
   if (k_ts > INT32_MAX) return fail(INFLLM_E_BADARG, "attn_stage: token stride too large");
   INFLLM_TRY(check_rows(d_q, q_hs, q_ts, "attn_stage q"));
   if (lk > 0) {
     INFLLM_TRY(check_rows(d_k, k_hs, k_ts, "attn_stage k"));
     INFLLM_TRY(check_rows(d_v, v_hs, v_ts, "attn_stage v"));
   }
+  if (d_out) INFLLM_TRY(check_rows(d_out, o_hs, o_ts, "attn_stage out"));
   if (mask_mode < INFLLM_MASK_NONE || mask_mode > INFLLM_MASK_COMPLEMENT)
     return fail(INFLLM_E_BADARG, "attn_stage: mask mode %d", mask_mode);
+  if (lq == 0) return INFLLM_OK;
+  cudaStream_t s = (cudaStream_t)stream;
+  if ((uintptr_t)d_scratch % 16) d_scratch = nullptr;
+  const bool rows_ok = ((uintptr_t)d_acc % 16) == 0 && tc_rows_ok(d_q, q_hs, q_ts) && (lk == 0 || (tc_rows_ok(d_k, k_hs, k_ts) && tc_rows_ok(d_v, v_hs, v_ts)));
+  const StageKernel kern = rows_ok ? stage_kernel(n_heads, n_kv_heads, lq, lk, head_dim) : STAGE_GENERIC;
+  if (kern == STAGE_ONE) {
+    const int64_t parts = std::min<int64_t>(scratch_floats / ((int64_t)n_heads * 129), infllm_attn_decode_max_parts(1, lk));
+    if (d_scratch && parts > 0) {
+      int64_t lo, hi;  // what the one query sees is one run of keys
+      visible_key_range(mask_mode, mask_offset, mask_size, 0, 0, lk, &lo, &hi);
+      int n = 0;
+      float* plse = d_scratch + parts * n_heads * 128;
+      if (lo <= hi) {
+        const KvSeg seg = {(const char*)d_k + lo * k_ts * 2, (const char*)d_v + lo * v_ts * 2, k_hs, (int32_t)k_ts,
+                           (int32_t)(hi - lo + 1)};
+        const int32_t qsel = 0;
+        INFLLM_TRY(attn_decode_launch(d_q, d_q, q_hs, n_heads, n_kv_heads, head_dim, 1, &seg, &qsel, d_scratch, plse,
+                                      (int)parts, &n, -1, nullptr, dtype, s, nullptr));
+      }
+      return attn_tc_combine_launch(d_scratch, plse, nullptr, n, n_heads, 1, d_out, o_hs, o_ts, d_lse,
+                                    first ? nullptr : d_acc, d_m, d_l, d_acc, d_m, d_l, dtype, s);
+    }
+  }
+  if (kern == STAGE_TC)
+    return stage_tc(d_q, q_hs, q_ts, d_k, d_v, k_hs, k_ts, n_heads, n_kv_heads, lq, lk, mask_mode, mask_offset, mask_size,
+                    d_acc, d_m, d_l, first, d_scratch, d_scratch ? scratch_floats : 0, d_out, o_hs, o_ts, d_lse, dtype, s);
   AttnParams p{};
   p.n_stage = 1;
   p.stage[0].q = d_q; p.stage[0].q_hs = q_hs; p.stage[0].q_ts = q_ts;
@@ -471,10 +578,20 @@ extern "C" int infllm_attn_stage(const void* d_q, int64_t q_hs, int64_t q_ts, co
     pos += n;
   }
   p.stage[0].seg_begin = 0; p.stage[0].seg_end = nseg;
-  p.n_heads = n_heads; p.n_kv_heads = n_kv_heads; p.first = first; p.last = 0; p.lq = lq;
-  p.acc = d_acc; p.m = d_m; p.l = d_l; p.out = nullptr; p.lse = nullptr;
+  p.n_heads = n_heads; p.n_kv_heads = n_kv_heads; p.first = first; p.last = d_out ? 1 : 0; p.lq = lq;
+  p.acc = d_acc; p.m = d_m; p.l = d_l; p.out = d_out; p.o_hs = o_hs; p.o_ts = o_ts; p.lse = d_lse;
   p.scale_log2 = kLog2e / sqrtf((float)head_dim);
-  return attn_general_launch(p, head_dim, dtype, (cudaStream_t)stream);
+  return attn_general_launch(p, head_dim, dtype, s);
+}
+
+extern "C" int infllm_attn_stage(const void* d_q, int64_t q_hs, int64_t q_ts, const void* d_k, int64_t k_hs,
+                                 int64_t k_ts, const void* d_v, int64_t v_hs, int64_t v_ts, int n_heads,
+                                 int n_kv_heads, int64_t lq, int64_t lk, int head_dim, int mask_mode,
+                                 int64_t mask_offset, int64_t mask_size, float* d_acc, float* d_m, float* d_l,
+                                 int first, int dtype, void* stream) {
+  return infllm_attn_stage_ex(d_q, q_hs, q_ts, d_k, k_hs, k_ts, d_v, v_hs, v_ts, n_heads, n_kv_heads, lq, lk, head_dim,
+                              mask_mode, mask_offset, mask_size, d_acc, d_m, d_l, first, nullptr, 0, nullptr, 0, 0,
+                              nullptr, dtype, stream);
 }
 
 extern "C" int infllm_attn_finalize(const float* d_acc, const float* d_m, const float* d_l, void* d_out, int64_t o_hs,
@@ -482,10 +599,13 @@ extern "C" int infllm_attn_finalize(const float* d_acc, const float* d_m, const 
                                     void* stream) {
   using namespace infllm;
   if (!d_acc || !d_m || !d_l || !d_out) return fail(INFLLM_E_BADARG, "attn_finalize: null pointer");
+  if (head_dim <= 0 || head_dim % 4) return fail(INFLLM_E_BADARG, "attn_finalize: head_dim %d", head_dim);
+  const int vec = (uintptr_t)d_out % 8 == 0 && o_hs % 4 == 0 && o_ts % 4 == 0;
   if (lq <= 0) return INFLLM_OK;
   INFLLM_DISPATCH_DTYPE(dtype, T, {
-    attn_finalize_kernel<T><<<(unsigned)(n_heads * lq), 128, 0, (cudaStream_t)stream>>>(
-        d_acc, d_m, d_l, (T*)d_out, o_hs, o_ts, d_lse, lq, head_dim);
+    const int64_t rows = (int64_t)n_heads * lq;
+    attn_finalize_kernel<T><<<(unsigned)ceil_div(rows * (head_dim / 4), 256), 256, 0, (cudaStream_t)stream>>>(
+        d_acc, d_m, d_l, (T*)d_out, o_hs, o_ts, d_lse, rows, lq, head_dim, vec);
   });
   INFLLM_LAUNCH_OK("attn_finalize_kernel");
   return INFLLM_OK;

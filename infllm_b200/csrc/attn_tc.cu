@@ -616,6 +616,20 @@ __global__ void __launch_bounds__(352, 1) attn_tc3_kernel(const __grid_constant_
   const int h = blockIdx.y, hkv = h / (P.n_heads / P.n_kv_heads);
   const int64_t i0 = (int64_t)blockIdx.x * kTile;
   const int rows_q = (int)((P.lq - i0) < kTile ? (P.lq - i0) : kTile);
+  const int split = blockIdx.z;
+
+  // this CTA's run [g0, g1) of the work item's key tiles, numbered over all stages
+  int g0 = 0, g1 = 1 << 30;
+  if (P.n_split > 1) {
+    int n_total = 0;
+    for (int st = 0; st < P.n_stage; ++st) {
+      const TcStage& S = P.stage[st];
+      int64_t vis_lo, vis_hi;
+      visible_key_range(S.mask_mode, S.mask_offset, S.mask_size, i0, i0 + rows_q - 1, S.lk, &vis_lo, &vis_hi);
+      if (vis_lo <= vis_hi) n_total += stage_tiles(P, S, vis_lo, vis_hi);
+    }
+    g0 = (int)((int64_t)n_total * split / P.n_split), g1 = (int)((int64_t)n_total * (split + 1) / P.n_split);
+  }
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < T3_N_BARS; ++i) mbar_init(bar(i), (i >= T3_P_FULL0 && i <= T3_P_FULL2) ? 256u : 1u);
@@ -641,7 +655,7 @@ __global__ void __launch_bounds__(352, 1) attn_tc3_kernel(const __grid_constant_
     // when the P V product of tile t-2 has run, late in the tile's cycle; asked for in tile order, K(t+1) queued
     // behind that wait and S(t+1) was not ready when the softmax warps came for it.
     if (lane == 0) {
-      int it = 0, sidx = 0;
+      int g = 0, it = 0, sidx = 0;
       bool ok = true;
       struct { int it, tok, c3, map; } pend = {-1, 0, 0, 0};  // the V tile that has not been asked for yet
       auto load_v = [&]() {
@@ -664,7 +678,11 @@ __global__ void __launch_bounds__(352, 1) attn_tc3_kernel(const __grid_constant_
         int64_t vis_lo, vis_hi;
         visible_key_range(S.mask_mode, S.mask_offset, S.mask_size, i0, i0 + rows_q - 1, S.lk, &vis_lo, &vis_hi);
         if (vis_lo > vis_hi) continue;
-        if (stage_tiles(P, S, vis_lo, vis_hi) == 0) continue;
+        const int n_st = stage_tiles(P, S, vis_lo, vis_hi);
+        if ((g > g0 ? g : g0) >= (g + n_st < g1 ? g + n_st : g1)) {  // none of this run's tiles
+          g += n_st;
+          continue;
+        }
         if (sidx >= 1) ok = wait_or_abort(bar(T3_Q_EMPTY), (sidx - 1) & 1, abort_flag, P.err, 600);
         if (!ok) break;
         mbar_expect_tx(bar(T3_Q_FULL), 2 * kSubTileBytes);
@@ -676,7 +694,9 @@ __global__ void __launch_bounds__(352, 1) attn_tc3_kernel(const __grid_constant_
           const TcSeg& G = P.seg[sg];
           int tf, tl;
           if (seg_tiles(vis_lo, vis_hi, seg_j0, G.len, &tf, &tl)) {
-            for (int t = tf; t <= tl && ok; ++t, ++it) {
+            const int skip = g0 > g ? g0 - g : 0;  // tiles of earlier runs
+            for (int t = tf + skip; t <= tl && ok; ++t) {
+              if (g + t - tf >= g1) break;
               const int b = it & 1, tok = G.tok0 + t * kTile;
               if (it >= 2) ok = wait_or_abort(bar(T3_K_EMPTY0 + b), ((it >> 1) - 1) & 1, abort_flag, P.err, 601);
               if (!ok) break;
@@ -692,7 +712,9 @@ __global__ void __launch_bounds__(352, 1) attn_tc3_kernel(const __grid_constant_
               if (pend.it >= 0) load_v();
               if (!ok) break;
               pend.it = it, pend.tok = tok, pend.c3 = G.c3_v, pend.map = G.map_v;
+              ++it;
             }
+            g += tl - tf + 1;
           }
           seg_j0 += G.len;
         }
@@ -714,13 +736,15 @@ __global__ void __launch_bounds__(352, 1) attn_tc3_kernel(const __grid_constant_
     // before - S of tile t+2 may overwrite its buffer only when P V of tile t has read P from it - is now the
     // wait for that product's commit.
     if (lane == 0) {
-      int nt[kMaxStage], n_act = 0, n = 0;  // tiles per stage that has any, in order
+      int nt[kMaxStage], n_act = 0, n = 0, g = 0;  // this run's tiles per stage that has any, in order
       for (int st = 0; st < P.n_stage; ++st) {
         const TcStage& S = P.stage[st];
         int64_t vis_lo, vis_hi;
         visible_key_range(S.mask_mode, S.mask_offset, S.mask_size, i0, i0 + rows_q - 1, S.lk, &vis_lo, &vis_hi);
         if (vis_lo > vis_hi) continue;
-        const int c = stage_tiles(P, S, vis_lo, vis_hi);
+        const int n_st = stage_tiles(P, S, vis_lo, vis_hi);
+        const int c = (g + n_st < g1 ? g + n_st : g1) - (g > g0 ? g : g0);
+        g += n_st;
         if (c > 0) nt[n_act++] = c, n += c;
       }
       bool ok = true;
@@ -782,7 +806,7 @@ __global__ void __launch_bounds__(352, 1) attn_tc3_kernel(const __grid_constant_
     const int64_t qrow[2] = {i0 + rbase, i0 + rbase + 8};
     const bool valid[2] = {qrow[0] < P.lq, qrow[1] < P.lq};
     float m_ref[2] = {-INFINITY, -INFINITY}, l_part[2] = {0.f, 0.f};
-    int it = 0;
+    int g = 0, it = 0;
     bool ok = true;
     for (int st = 0; st < P.n_stage && ok; ++st) {
       const TcStage& S = P.stage[st];
@@ -806,7 +830,9 @@ __global__ void __launch_bounds__(352, 1) attn_tc3_kernel(const __grid_constant_
         const TcSeg& G = P.seg[sg];
         int tf, tl;
         if (seg_tiles(vis_lo, vis_hi, seg_j0, G.len, &tf, &tl)) {
-          for (int t = tf; t <= tl && ok; ++t, ++it) {
+          const int skip = g0 > g ? g0 - g : 0;
+          for (int t = tf + skip; t <= tl && ok; ++t, ++it) {
+            if (g + t - tf >= g1) break;
             const int b3 = it % 3;
             const uint32_t tS = tmem + b3 * 128 + lane_base;
             ok = __all_sync(0xffffffffu, wait_or_abort(bar(T3_S_FULL0 + b3), (it / 3) & 1, abort_flag, P.err, 620));
@@ -898,6 +924,7 @@ __global__ void __launch_bounds__(352, 1) attn_tc3_kernel(const __grid_constant_
             tc_fence_before();
             mbar_arrive(bar(T3_P_FULL0 + b3));
           }
+          g += tl - tf + 1;
         }
         seg_j0 += G.len;
       }
@@ -920,11 +947,27 @@ __global__ void __launch_bounds__(352, 1) attn_tc3_kernel(const __grid_constant_
     const bool row_valid = qi < P.lq;
     const uint32_t row_base = ((uint32_t)(quad * 32)) << 16;
     const float l_sum = xsum[row], m_row = xmax[row];
+    // Three ways out: a run of a split work item leaves its un-normalised partial; a stage of a multi-stage attention
+    // leaves the state (acc, m, l); everything else is normalised.  A state that came in is folded in first.
+    const int64_t srow = (int64_t)h * P.lq + qi;
+    float ws = 1.f, wp = 0.f, m_out = m_row, l_out = it >= 1 ? l_sum : 0.f;
+    if (P.st_acc) {
+      if (row_valid) {
+        const float mp = P.st_m[srow], mm = fmaxf(mp, m_row), ms = mm == -INFINITY ? 0.f : mm;
+        ws = exp2f(m_row - ms);
+        wp = exp2f(mp - ms);
+        l_out = ws * l_out + wp * P.st_l[srow];
+        m_out = mm;
+      }
+      asm volatile("bar.sync 1, 256;" ::: "memory");  // both halves of a row have read (m, l): they may be overwritten
+    }
     if (ok && it >= 1) ok = __all_sync(0xffffffffu, wait_or_abort(bar(T3_O_FULL), 0, abort_flag, P.err, 624));
     if (ok) {
       tc_fence_after();
-      const float inv = (it >= 1 && l_sum > 0.f) ? 1.f / l_sum : 0.f;
-      T* orow = (T*)P.out + (int64_t)h * P.o_hs + qi * P.o_ts + col0;
+      const bool raw = P.part_acc != nullptr;
+      const int64_t prow = (int64_t)split * P.n_heads * P.lq + srow;
+      const float inv = l_out > 0.f ? 1.f / l_out : 0.f;
+      T* orow = raw ? nullptr : (T*)P.out + (int64_t)h * P.o_hs + qi * P.o_ts + col0;
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
         uint32_t o[32];
@@ -936,21 +979,45 @@ __global__ void __launch_bounds__(352, 1) attn_tc3_kernel(const __grid_constant_
           for (int k = 0; k < 32; ++k) o[k] = 0;
         }
         if (row_valid) {
+          if (P.st_acc) {
+            const float4* sp = reinterpret_cast<const float4*>(P.st_acc + srow * 128 + col0 + c * 32);
 #pragma unroll
-          for (int k = 0; k < 32; k += 8) {
-            uint4 v;
-            uint32_t* pv = reinterpret_cast<uint32_t*>(&v);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              typename Act<T>::T2 v2 = Act<T>::from_f2(__uint_as_float(o[k + 2 * e]) * inv,
-                                                       __uint_as_float(o[k + 2 * e + 1]) * inv);
-              pv[e] = *reinterpret_cast<uint32_t*>(&v2);
+            for (int k = 0; k < 32; k += 4) {
+              const float4 v = sp[k >> 2];
+              o[k] = __float_as_uint(fmaf(wp, v.x, ws * __uint_as_float(o[k])));
+              o[k + 1] = __float_as_uint(fmaf(wp, v.y, ws * __uint_as_float(o[k + 1])));
+              o[k + 2] = __float_as_uint(fmaf(wp, v.z, ws * __uint_as_float(o[k + 2])));
+              o[k + 3] = __float_as_uint(fmaf(wp, v.w, ws * __uint_as_float(o[k + 3])));
             }
-            *reinterpret_cast<uint4*>(orow + c * 32 + k) = v;
+          }
+          if (raw) {
+            uint4* ap = reinterpret_cast<uint4*>(P.part_acc + prow * 128 + col0 + c * 32);
+#pragma unroll
+            for (int k = 0; k < 32; k += 4) ap[k >> 2] = make_uint4(o[k], o[k + 1], o[k + 2], o[k + 3]);
+          } else {
+#pragma unroll
+            for (int k = 0; k < 32; k += 8) {
+              uint4 v;
+              uint32_t* pv = reinterpret_cast<uint32_t*>(&v);
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                typename Act<T>::T2 v2 = Act<T>::from_f2(__uint_as_float(o[k + 2 * e]) * inv,
+                                                         __uint_as_float(o[k + 2 * e + 1]) * inv);
+                pv[e] = *reinterpret_cast<uint32_t*>(&v2);
+              }
+              *reinterpret_cast<uint4*>(orow + c * 32 + k) = v;
+            }
           }
         }
       }
-      if (half == 0 && row_valid && P.lse) P.lse[(int64_t)h * P.lq + qi] = l_sum > 0.f ? m_row + log2f(l_sum) : -INFINITY;
+      if (half == 0 && row_valid) {
+        if (raw) {
+          P.part_m[prow] = m_out;
+          P.part_l[prow] = l_out;
+        } else if (P.lse) {
+          P.lse[srow] = l_out > 0.f ? m_out + log2f(l_out) : -INFINITY;
+        }
+      }
     }
   }
   // ---- teardown
@@ -959,38 +1026,50 @@ __global__ void __launch_bounds__(352, 1) attn_tc3_kernel(const __grid_constant_
   if (warp == 9) tmem_dealloc(tmem, 512);
 }
 
-// out = sum_s acc_s 2^(m_s - m) / sum_s l_s 2^(m_s - m), lse = m + log2(denominator); one warp per row
+// Merge of n_split partials (acc, m, l) per row, and of a state that came in (st_*, may be null): the sum of
+// acc_s 2^(m_s - m), normalised into out / lse, or, when out is null, left as the new state (which may overwrite the
+// old one in place).  l == null: the partials are normalised and m is their log-sum-exp.  One warp per row.
 template <typename T>
 __global__ void attn_tc_combine_kernel(const float* __restrict__ acc, const float* __restrict__ m,
                                        const float* __restrict__ l, int n_split, int n_heads, int64_t lq,
-                                       T* __restrict__ out, int64_t o_hs, int64_t o_ts, float* __restrict__ lse) {
+                                       T* __restrict__ out, int64_t o_hs, int64_t o_ts, float* __restrict__ lse,
+                                       const float* st_acc, const float* st_m, const float* st_l, float* new_acc,
+                                       float* new_m, float* new_l) {
   const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);  // h * lq + i
   if (row >= (int64_t)n_heads * lq) return;
   const int lane = threadIdx.x & 31;
   const int64_t h = row / lq, i = row - h * lq;
   const int64_t stride = (int64_t)n_heads * lq;
-  float mx = -INFINITY;
+  float mx = st_acc ? st_m[row] : -INFINITY;
   for (int s = 0; s < n_split; ++s) mx = fmaxf(mx, m[s * stride + row]);
   float den = 0.f;
   float4 num = make_float4(0.f, 0.f, 0.f, 0.f);
   if (mx != -INFINITY) {
-    for (int s = 0; s < n_split; ++s) {
-      const float ms = m[s * stride + row];
-      if (ms == -INFINITY) continue;
+    auto fold = [&](float ms, float ls, const float* ap) {
+      if (ms == -INFINITY) return;
       const float w = exp2f(ms - mx);
-      den = fmaf(w, l[s * stride + row], den);
-      const float4 a = *reinterpret_cast<const float4*>(acc + (s * stride + row) * 128 + lane * 4);
+      den = fmaf(w, ls, den);
+      const float4 a = *reinterpret_cast<const float4*>(ap + row * 128 + lane * 4);
       num.x = fmaf(w, a.x, num.x);
       num.y = fmaf(w, a.y, num.y);
       num.z = fmaf(w, a.z, num.z);
       num.w = fmaf(w, a.w, num.w);
-    }
+    };
+    if (st_acc) fold(st_m[row], st_l[row], st_acc);
+#pragma unroll 4
+    for (int s = 0; s < n_split; ++s) fold(m[s * stride + row], l ? l[s * stride + row] : 1.f, acc + s * stride * 128);
   }
-  const float inv = den > 0.f ? 1.f / den : 0.f;
-  typename Act<T>::T2 v01 = Act<T>::from_f2(num.x * inv, num.y * inv), v23 = Act<T>::from_f2(num.z * inv, num.w * inv);
-  uint2 v = make_uint2(*reinterpret_cast<uint32_t*>(&v01), *reinterpret_cast<uint32_t*>(&v23));
-  *reinterpret_cast<uint2*>(out + h * o_hs + i * o_ts + lane * 4) = v;
-  if (lane == 0 && lse) lse[row] = den > 0.f ? mx + log2f(den) : -INFINITY;
+  if (out) {
+    const float inv = den > 0.f ? 1.f / den : 0.f;
+    typename Act<T>::T2 v01 = Act<T>::from_f2(num.x * inv, num.y * inv), v23 = Act<T>::from_f2(num.z * inv, num.w * inv);
+    uint2 v = make_uint2(*reinterpret_cast<uint32_t*>(&v01), *reinterpret_cast<uint32_t*>(&v23));
+    *reinterpret_cast<uint2*>(out + h * o_hs + i * o_ts + lane * 4) = v;
+    if (lane == 0 && lse) lse[row] = den > 0.f ? mx + log2f(den) : -INFINITY;
+  } else {
+    __syncwarp();  // every lane has read the old state of this row
+    *reinterpret_cast<float4*>(new_acc + row * 128 + lane * 4) = num;
+    if (lane == 0) new_m[row] = mx, new_l[row] = den;
+  }
 }
 
 // ------------------------------------------------------------------------------------ column sums
@@ -1302,9 +1381,32 @@ int tc_get_error_ptr(int** p) {
   return INFLLM_OK;
 }
 
+int attn_tc_combine_launch(const float* acc, const float* m, const float* l, int n_split, int n_heads, int64_t lq, void* out,
+                           int64_t o_hs, int64_t o_ts, float* lse, const float* st_acc, const float* st_m,
+                           const float* st_l, float* new_acc, float* new_m, float* new_l, int dtype, cudaStream_t s) {
+  const int64_t rows = (int64_t)n_heads * lq;
+  const int threads = rows >= 4096 ? 256 : 64;  // few rows: spread over the SMs
+  INFLLM_DISPATCH_DTYPE(dtype, T, {
+    attn_tc_combine_kernel<T><<<(unsigned)ceil_div(rows, threads / 32), threads, 0, s>>>(
+        acc, m, l, n_split, n_heads, lq, (T*)out, o_hs, o_ts, lse, st_acc, st_m, st_l, new_acc, new_m, new_l);
+  });
+  INFLLM_LAUNCH_OK("attn_tc_combine_kernel");
+  return INFLLM_OK;
+}
+
+// Runs of key tiles per (128-query tile, head): one while the grid covers more than half of the SMs, else as many as
+// fill them with at least two tiles each.
+int attn_tc3_splits(int64_t lq, int n_heads, int64_t keys) {
+  const int64_t items = ceil_div(lq, kTile) * n_heads, tiles = ceil_div(keys, kTile);
+  if (items > 74) return 1;
+  return (int)std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(148 / items, tiles / 2), 32));
+}
+
 int attn_tc3_launch(const AttnTcParams& P, int dtype, cudaStream_t s) {
   if (P.lq <= 0) return INFLLM_OK;
-  dim3 grid((unsigned)ceil_div(P.lq, kTile), P.n_heads);
+  if (P.n_split < 1 || (P.n_split > 1 && (!P.part_acc || !P.part_m || !P.part_l || P.st_acc)))
+    return fail(INFLLM_E_BADARG, "attn_tc3: split %d without partial buffers", P.n_split);
+  dim3 grid((unsigned)ceil_div(P.lq, kTile), P.n_heads, P.n_split);
   const size_t smem = tc3::kTotal + 1024;
   INFLLM_DISPATCH_DTYPE(dtype, T, {
     auto kern = attn_tc3_kernel<T>;
@@ -1343,14 +1445,9 @@ int attn_tc2_launch(const AttnTcParams& P, int dtype, cudaStream_t s) {
                   fa.maxThreadsPerBlock);
     }
   });
-  if (P.n_split > 1) {
-    const int64_t rows = (int64_t)P.n_heads * P.lq;
-    INFLLM_DISPATCH_DTYPE(dtype, T, {
-      attn_tc_combine_kernel<T><<<(unsigned)ceil_div(rows, 8), 256, 0, s>>>(
-          P.part_acc, P.part_m, P.part_l, P.n_split, P.n_heads, P.lq, (T*)P.out, P.o_hs, P.o_ts, P.lse);
-    });
-    INFLLM_LAUNCH_OK("attn_tc_combine_kernel");
-  }
+  if (P.n_split > 1)
+    return attn_tc_combine_launch(P.part_acc, P.part_m, P.part_l, P.n_split, P.n_heads, P.lq, P.out, P.o_hs, P.o_ts, P.lse,
+                                  nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, dtype, s);
   return INFLLM_OK;
 }
 

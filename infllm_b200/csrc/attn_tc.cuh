@@ -32,12 +32,14 @@ struct AttnTcParams {
   float* lse;
   float scale_log2;
   int* err;
-  // two-head kernel only: the key tiles of a work item are cut into n_split runs; with n_split > 1 every run
-  // writes an un-normalised partial (acc, m, l) and attn_tc_combine merges them
+  // The key tiles of a work item are cut into n_split runs; with n_split > 1 every run writes an un-normalised
+  // partial (acc, m, l) and attn_tc_combine merges them.  With n_split == 1 the one-head kernel writes its state here
+  // instead of out / lse when part_acc is set, and folds in the state st_* when that is set (it may be the same memory).
   int32_t n_split, pad2;
   float* part_acc;  // (n_split, H, lq, 128)
   float* part_m;    // (n_split, H, lq)
   float* part_l;    // (n_split, H, lq)
+  const float *st_acc, *st_m, *st_l;
 };
 
 struct ColsumTcParams {
@@ -60,6 +62,10 @@ bool tc_rows_ok(const void* base, int64_t hs, int64_t ts);
 int tc_get_error_ptr(int** p);
 // one CTA per (128-query tile, head)
 int attn_tc3_launch(const AttnTcParams& P, int dtype, cudaStream_t s);
+int attn_tc3_splits(int64_t lq, int n_heads, int64_t keys);
+int attn_tc_combine_launch(const float* acc, const float* m, const float* l, int n_split, int n_heads, int64_t lq, void* out,
+                           int64_t o_hs, int64_t o_ts, float* lse, const float* st_acc, const float* st_m,
+                           const float* st_l, float* new_acc, float* new_m, float* new_l, int dtype, cudaStream_t s);
 // two query heads of one KV head per CTA (needs an even number of query heads per KV head)
 int attn_tc2_launch(const AttnTcParams& P, int dtype, cudaStream_t s);
 size_t attn_tc2_scratch_floats(int n_split, int n_heads, int64_t lq);
