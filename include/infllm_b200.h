@@ -114,6 +114,28 @@ int infllm_attn_colsum(const void* d_q, int64_t q_hs, int64_t q_ts,
                        const float* d_lse, float* d_score, int64_t score_hs, int accumulate,
                        int dtype, void* stream);
 
+/* ------------------------------------------------ sink + window attention
+ * Replaces one forward of "infinite-lm" / "stream-llm" (inf_llm/attention/infinite_lm.py:6-100, stream_llm.py:6-111)
+ * for one sequence, between its projections: [cache of the previous call | new tokens] -> output rows and new cache.
+ * q (n_heads, len_q, head_dim), k and v (n_kv_heads, len_q, head_dim) are the new tokens, un-rotated, k and v with the
+ * same strides; past_k/v (n_kv_heads, past_len, head_dim) the cache (past_len 0: none); `seen` counts every token of
+ * the sequence, the new ones included.  The window stage rotates keys to their positions among the last
+ * len_q + n_local rows; the sink stage (once seen > n_local) attends to the first n_init rows that have left a
+ * query's window, with queries at position n_local - 1 and raw keys, or, with stream_positions != 0, with queries at
+ * n_local + n_init - 1 and keys at their own positions.  d_cache_k/v (may be NULL) receive, contiguous, the first
+ * cache_head rows and the last cache_rows - cache_head rows of [cache | new].  d_cos / d_sin are an infllm_rope_table.
+ * infllm_sink_window_scratch: bytes of d_scratch the call needs (-1: bad sizes; only the sizes and d_cache_v are read). */
+typedef struct infllm_sink_window {
+  const void *d_q, *d_k, *d_v, *d_past_k, *d_past_v;
+  void *d_cache_k, *d_cache_v, *d_out, *d_scratch;
+  const float *d_cos, *d_sin;
+  int64_t q_hs, q_ts, k_hs, k_ts, past_hs, past_ts, o_hs, o_ts; /* element strides: heads, tokens */
+  int64_t len_q, past_len, seen, cache_head, cache_rows, table_len, scratch_bytes;
+  int32_t n_heads, n_kv_heads, head_dim, n_local, n_init, stream_positions, dtype, pad;
+} infllm_sink_window;
+int64_t infllm_sink_window_scratch(const infllm_sink_window* args);
+int infllm_sink_window_run(const infllm_sink_window* args, void* stream);
+
 /* ------------------------------------------------------ retrieval kernels
  * infllm_block_topk replaces calc_block_topk / VectorTensor.get_topk
  *   (context_manager.py:366-383, 159-163): scores[b] = <block_k[b, :], qbar> for b < n_blocks

@@ -43,6 +43,15 @@ class Config(ctypes.Structure):
     ]
 
 
+class SinkWindow(ctypes.Structure):
+    _fields_ = [(n, c_void_p) for n in ("d_q", "d_k", "d_v", "d_past_k", "d_past_v", "d_cache_k", "d_cache_v", "d_out",
+                                        "d_scratch", "d_cos", "d_sin")] + \
+               [(n, c_int64) for n in ("q_hs", "q_ts", "k_hs", "k_ts", "past_hs", "past_ts", "o_hs", "o_ts", "len_q", "past_len",
+                                       "seen", "cache_head", "cache_rows", "table_len", "scratch_bytes")] + \
+               [(n, c_int32) for n in ("n_heads", "n_kv_heads", "head_dim", "n_local", "n_init", "stream_positions", "dtype",
+                                       "pad")]
+
+
 class CtxInfo(ctypes.Structure):
     _fields_ = [(n, c_int64) for n in (
         "length", "frontier", "num_blocks", "init_len", "num_cached", "load_count", "exec_blocks",
@@ -104,6 +113,8 @@ SIGNATURES = {
                                      c_int, c_int, c_int64, c_int64, c_int, c_int, c_int64, c_int64,
                                      c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int64, c_void_p, c_int64, c_int64,
                                      c_void_p, c_int, c_void_p]),
+    "infllm_sink_window_scratch": (c_int64, [POINTER(SinkWindow)]),
+    "infllm_sink_window_run": (c_int, [POINTER(SinkWindow), c_void_p]),
     "infllm_attn_finalize": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_void_p,
                                      c_int, c_int64, c_int, c_int, c_void_p]),
     "infllm_attn_colsum": (c_int, [c_void_p, c_int64, c_int64, c_void_p, c_int64, c_int64, c_int, c_int, c_int64,

@@ -51,6 +51,8 @@ class CudaMultiStageDotProductionAttention:
             q = q.contiguous()
         if k.stride(-1) != 1 or k.stride() != v.stride():
             k, v = k.contiguous(), v.contiguous()
+        # (the strides of dimensions of one element are arbitrary, also behind contiguous())
+        k_hs, k_ts = (k.stride(1) if hkv > 1 else max(lk, 1) * d), (k.stride(2) if lk > 1 else d)
         stream = _lib.stream_ptr(self.device)
         lib, f32 = _lib.lib, torch.float32
         if get_score:
@@ -69,13 +71,13 @@ class CudaMultiStageDotProductionAttention:
             acc, m, l = (None, None, None) if self._state is None else (
                 self._state[0][bi].data_ptr(), self._state[1][0, bi].data_ptr(), self._state[1][1, bi].data_ptr())
             _lib.check(lib.infllm_attn_stage_ex(
-                q[bi].data_ptr(), q.stride(1), q.stride(2), k[bi].data_ptr() if lk else None, k.stride(1), k.stride(2),
-                v[bi].data_ptr() if lk else None, v.stride(1), v.stride(2), h, hkv, lq, lk, d, mode, off, size,
+                q[bi].data_ptr(), q.stride(1), q.stride(2), k[bi].data_ptr() if lk else None, k_hs, k_ts,
+                v[bi].data_ptr() if lk else None, k_hs, k_ts, h, hkv, lq, lk, d, mode, off, size,
                 acc, m, l, int(self._first), None if scratch is None else scratch.data_ptr(), n_scratch,
                 out[bi].data_ptr() if end else None, out.stride(1) if end else 0, out.stride(2) if end else 0,
                 lse[bi].data_ptr() if lse is not None else None, self._code, stream))
         self._first = False
-        self._stages.append((q, k, mode, off, size) if get_score else None)
+        self._stages.append((q, k, k_hs, k_ts, mode, off, size) if get_score else None)
         if end:
             self._finalize(lse)
 
@@ -89,14 +91,14 @@ class CudaMultiStageDotProductionAttention:
                 self.score_list.append(None)
                 self.score_list_fp32.append(None)
                 continue
-            q, k, mode, off, size = st
+            q, k, k_hs, k_ts, mode, off, size = st
             lk, hkv = k.size(2), k.size(1)
             # every column is written, unless there is nothing to sum
             score = (torch.empty if lq and lk else torch.zeros)((b, h, lk), dtype=torch.float32, device=self.device)
             for bi in range(b):
                 _lib.check(_lib.lib.infllm_attn_colsum(
-                    q[bi].data_ptr(), q.stride(1), q.stride(2), k[bi].data_ptr() if lk else None, k.stride(1),
-                    k.stride(2), h, hkv, lq, lk, d, mode, off, size, lse[bi].data_ptr(), score[bi].data_ptr(),
+                    q[bi].data_ptr(), q.stride(1), q.stride(2), k[bi].data_ptr() if lk else None, k_hs, k_ts, h, hkv,
+                    lq, lk, d, mode, off, size, lse[bi].data_ptr(), score[bi].data_ptr(),
                     score.stride(1), 0, self._code, stream))
             self.score_list_fp32.append(score)
             self.score_list.append(score.to(self.dtype))

@@ -4,13 +4,15 @@
 
 namespace infllm {
 
-// One contiguous run of keys/values of a stage.  Tokens are `ts` elements apart, heads `hs`.
+// One contiguous run of keys/values of a stage.  Tokens are `ts` elements apart, heads `hs`; the decode kernel also
+// takes values whose heads are v_hs apart (0: hs).
 struct KvSeg {
   const void* k;
   const void* v;
   int64_t hs;
   int32_t ts;
   int32_t len;
+  int64_t v_hs = 0;
 };
 
 constexpr int kMaxSeg = 80;    // segments per launch (retrieved units + init sink + overflow + window)

@@ -39,7 +39,7 @@ constexpr int kDecMaxRuns = 2 * 148;  // CTAs of one launch over all KV heads: t
 struct DecodeSeg {
   const void* k;
   const void* v;
-  int64_t hs;
+  int64_t hs, v_hs;
   int32_t ts;
   int32_t len;
 };
@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(kDecThreads, 2) attn_decode_kernel(const __gri
         if (!seg_ok && mine && P.ind.miss && lane == 0) *P.ind.miss = 1;
       }
       kbase = reinterpret_cast<const char*>(sk) + (int64_t)hkv * S.hs * 2;
-      vbase = reinterpret_cast<const char*>(sv) + (int64_t)hkv * S.hs * 2;
+      vbase = reinterpret_cast<const char*>(sv) + (int64_t)hkv * S.v_hs * 2;
       if ((int)P.qsel[sg] != cur_q) {
         cur_q = P.qsel[sg];
         const char* qp = reinterpret_cast<const char*>(P.q[cur_q]) + (int64_t)hq * P.q_hs * 2;
@@ -443,9 +443,9 @@ int attn_decode_launch(const void* q0, const void* q1, int64_t q_hs, int n_heads
   for (int i = 0; i < n_seg; ++i) {
     if (segs[i].len <= 0) continue;  // empty segments contribute nothing
     if (ind && ind->n_units > 0 && i == ind->first_seg) P.ind.first_seg = ns;
-    if (((uintptr_t)segs[i].k | (uintptr_t)segs[i].v) % 16 || segs[i].hs % 8 || segs[i].ts % 8)
+    if (((uintptr_t)segs[i].k | (uintptr_t)segs[i].v) % 16 || segs[i].hs % 8 || segs[i].v_hs % 8 || segs[i].ts % 8)
       return fail(INFLLM_E_BADARG, "decode attention: segment %d rows are not 16-byte aligned", i);
-    P.seg[ns] = {segs[i].k, segs[i].v, segs[i].hs, segs[i].ts, segs[i].len};
+    P.seg[ns] = {segs[i].k, segs[i].v, segs[i].hs, segs[i].v_hs ? segs[i].v_hs : segs[i].hs, segs[i].ts, segs[i].len};
     P.qsel[ns] = (uint8_t)(seg_q[i] ? 1 : 0);
     P.item_begin[ns] = items;
     if (i == logit_seg) logit_seg_packed = ns;

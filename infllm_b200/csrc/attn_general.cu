@@ -557,6 +557,9 @@ extern "C" int infllm_attn_stage_ex(const void* d_q, int64_t q_hs, int64_t q_ts,
         INFLLM_TRY(attn_decode_launch(d_q, d_q, q_hs, n_heads, n_kv_heads, head_dim, 1, &seg, &qsel, d_scratch, plse,
                                       (int)parts, &n, -1, nullptr, dtype, s, nullptr));
       }
+      if (first && d_out && n > 0)
+        return lse_merge_launch(d_scratch, plse, n, n_heads, head_dim, d_out, o_hs, d_lse, dtype, s, nullptr, 0, nullptr, 0,
+                                nullptr);
       return attn_tc_combine_launch(d_scratch, plse, nullptr, n, n_heads, 1, d_out, o_hs, o_ts, d_lse,
                                     first ? nullptr : d_acc, d_m, d_l, d_acc, d_m, d_l, dtype, s);
     }
