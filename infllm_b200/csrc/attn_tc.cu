@@ -75,17 +75,30 @@ __device__ __forceinline__ float2 fadd2(float2 a, float2 b) {
 
 // exp2 of a pair on the FMA and integer pipes (the special-function unit does 16 per clock per SM, which bounds the
 // softmax when every exponential goes there): x = n + f with n the nearest integer (magic-number rounding) and f in
-// [-0.5, 0.5], 2^f by a cubic (relative error 7e-4, below the rounding of a 16-bit P), n added into the exponent
+// [-0.5, 0.5], 2^f by a polynomial whose relative error was minimised over that interval (weighted least squares on
+// Chebyshev points), n added into the exponent.  Cubic: 7.5e-5, a twentieth of the rounding of a 16-bit P; quartic:
+// 2.6e-6, for sums that stay fp32.
+template <int kDegree>
 __device__ __forceinline__ float2 ex2_poly2(float2 x) {
+  static_assert(kDegree == 3 || kDegree == 4, "");
   x.x = fmaxf(x.x, -126.f);
   x.y = fmaxf(x.y, -126.f);
   const float2 magic = make_float2(12582912.f, 12582912.f), neg_magic = make_float2(-12582912.f, -12582912.f);
   const float2 t = fadd2(x, magic);
   const float2 n = fadd2(t, neg_magic);
   const float2 f = fadd2(x, make_float2(-n.x, -n.y));
-  float2 p = ffma2(f.x, f.y, make_float2(0.0555041f, 0.0555041f), make_float2(0.2402265f, 0.2402265f));
-  p = ffma2(p.x, p.y, f, make_float2(0.6931472f, 0.6931472f));
-  p = ffma2(p.x, p.y, f, make_float2(1.f, 1.f));
+  auto c2 = [](float c) { return make_float2(c, c); };
+  float2 p;
+  if (kDegree == 3) {
+    p = ffma2(f.x, f.y, c2(0.05517167f), c2(0.24261113f));
+    p = ffma2(p.x, p.y, f, c2(0.69326097f));
+    p = ffma2(p.x, p.y, f, c2(0.99992806f));
+  } else {
+    p = ffma2(f.x, f.y, c2(0.0095701022f), c2(0.055917859f));
+    p = ffma2(p.x, p.y, f, c2(0.24024744f));
+    p = ffma2(p.x, p.y, f, c2(0.69312179f));
+    p = ffma2(p.x, p.y, f, c2(0.99999928f));
+  }
   return make_float2(__int_as_float(__float_as_int(p.x) + (__float_as_int(t.x) << 23)),
                      __int_as_float(__float_as_int(p.y) + (__float_as_int(t.y) << 23)));
 }
@@ -191,7 +204,7 @@ __global__ void __launch_bounds__(576, 1) attn_tc2_kernel(const __grid_constant_
   const int g0 = (int)((int64_t)n_total * split / P.n_split), g1 = (int)((int64_t)n_total * (split + 1) / P.n_split);
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < T2_N_BARS; ++i) mbar_init(bar(i), (i == T2_P_FULLA || i == T2_P_FULLB) ? 256u : 1u);
+    for (int i = 0; i < T2_N_BARS; ++i) mbar_init(bar(i), (i == T2_P_FULLA || i == T2_P_FULLB) ? 8u : 1u);
     *abort_flag = 0;
     mbar_fence_init();
   }
@@ -486,7 +499,8 @@ __global__ void __launch_bounds__(576, 1) attn_tc2_kernel(const __grid_constant_
             l_part += (rs4[0] + rs4[1]) + (rs4[2] + rs4[3]);
             tmem_wait_st();
             tc_fence_before();
-            mbar_arrive(bar(T2_P_FULLA + x));
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar(T2_P_FULLA + x));
             ++it;
           }
         }
@@ -632,7 +646,7 @@ __global__ void __launch_bounds__(352, 1) attn_tc3_kernel(const __grid_constant_
   }
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < T3_N_BARS; ++i) mbar_init(bar(i), (i >= T3_P_FULL0 && i <= T3_P_FULL2) ? 256u : 1u);
+    for (int i = 0; i < T3_N_BARS; ++i) mbar_init(bar(i), (i >= T3_P_FULL0 && i <= T3_P_FULL2) ? 8u : 1u);
     *abort_flag = 0;
     mbar_fence_init();
   }
@@ -823,7 +837,8 @@ __global__ void __launch_bounds__(352, 1) attn_tc3_kernel(const __grid_constant_
         } else if (S.mask_mode == INFLLM_MASK_COMPLEMENT) {
           jhi[r] = qrow[r] + S.mask_offset - S.mask_size;
         }
-        if (!valid[r]) jhi[r] = -1, jlo[r] = 0;
+        // rows past the last query are not masked, so that whole tiles stay whole: nothing of them is written
+        if (!valid[r]) jhi[r] = S.lk - 1, jlo[r] = 0;
       }
       int64_t seg_j0 = 0;
       for (int sg = S.seg_begin; sg < S.seg_end && ok; ++sg) {
@@ -895,7 +910,7 @@ __global__ void __launch_bounds__(352, 1) attn_tc3_kernel(const __grid_constant_
               const float2 a = ffma2(s[2 * k], s[2 * k + 1], sc2, nm2[r]);
               float2 p;
               if ((k % kPolyEvery) == kPolyEvery - 1) {
-                p = ex2_poly2(a);  // one pair in kPolyEvery off the special-function unit
+                p = ex2_poly2<3>(a);  // one pair in kPolyEvery off the special-function unit
               } else {
                 p = make_float2(ex2_approx(a.x), ex2_approx(a.y));
               }
@@ -922,7 +937,8 @@ __global__ void __launch_bounds__(352, 1) attn_tc3_kernel(const __grid_constant_
             tmem_st_16x128b_x16(tS, pk);
             tmem_wait_st();
             tc_fence_before();
-            mbar_arrive(bar(T3_P_FULL0 + b3));
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar(T3_P_FULL0 + b3));  // per warp: 256 arrivals on one word took turns
           }
           g += tl - tf + 1;
         }
@@ -1075,44 +1091,47 @@ __global__ void attn_tc_combine_kernel(const float* __restrict__ acc, const floa
 // ------------------------------------------------------------------------------------ column sums
 // One CTA owns one query head and a run of 128-key tiles.  The head's query tiles (at most four, 512 queries)
 // and their log-sum-exps stay in shared memory for the whole CTA; the key tiles stream through a two-stage TMA
-// ring; every (key tile, visible query tile) pair is one S^T = K Q^T into one of four TMEM buffers, which 16
-// compute warps (four threads per key row, 32 query columns each) turn into sum_q exp2(s - lse_q).  A key
-// tile is loaded once per head and a query tile once per CTA, which keeps the L2 traffic an order of magnitude
-// below one load per pair.
+// ring; every (key tile, visible query tile) pair is one S^T = K Q^T into one of four TMEM buffers, and each buffer has
+// four of the sixteen compute warps of its own, which turn it into sum_q exp2(s - lse_q).  A key tile is loaded once
+// per head and a query tile once per CTA, which keeps the L2 traffic an order of magnitude below one load per pair.
+// Bound: 16384 exponentials per pair, 768 cycles of the special-function unit with every fourth pair of them as a
+// quartic on the FMA pipe, and the product, 514; a pair takes 1150.  512 queries x 32 heads over 4608 keys: 30.7 us.
+// (37.6 us with one issuing thread and all sixteen warps on one buffer at a time, whose exponentials were two at a
+// time in fp16: 1.4e-3 off in a sum, now 1e-6.)
 namespace colsum_smem {
 constexpr int kQTiles = 4;                     // resident query tiles
 constexpr int kMaxKeyTiles = 10;               // key tiles per CTA
 constexpr int kBufs = 4;                       // TMEM accumulators in flight
+constexpr int kIssuers = 2;                    // threads that issue products (a divisor of kBufs)
+constexpr int kThreads = (16 + 1 + kIssuers) * 32;
 constexpr int kQ = 0;
 constexpr int kK = kQ + kQTiles * 2 * kSubTileBytes;   // two stages
 constexpr int kLse = kK + 2 * 2 * kSubTileBytes;       // kQTiles x 128 fp32
 constexpr int kBar = kLse + kQTiles * 512;
-constexpr int kAcc = kBar + 128;               // [key tile][column quarter][key] partial sums
+constexpr int kAcc = kBar + 256;               // [key tile][TMEM buffer][key] partial sums
 constexpr int kTotal = kAcc + kMaxKeyTiles * 4 * 128 * 4;
 }  // namespace colsum_smem
 
-// query tiles [tf, tl] that can see a key of the tile starting at j0 (tl < tf: none)
-__device__ __forceinline__ void colsum_q_tiles(const ColsumTcParams& P, int64_t j0, int keys, int* tf, int* tl) {
-  int64_t lo = 0, hi = P.lq - 1;
-  if (P.mask_mode == INFLLM_MASK_WINDOW) {
-    lo = j0 - P.mask_offset;
-    hi = j0 + keys - 1 - P.mask_offset + P.mask_size - 1;
-  } else if (P.mask_mode == INFLLM_MASK_COMPLEMENT) {
-    lo = j0 - P.mask_offset + P.mask_size;
-  }
-  if (lo < 0) lo = 0;
-  if (hi > P.lq - 1) hi = P.lq - 1;
-  if (lo > hi) {
-    *tf = 0;
-    *tl = -1;
-  } else {
-    *tf = (int)(lo / kTile);
-    *tl = (int)(hi / kTile);
-  }
+// Queries [lo, hi] that see key j, before clamping to [0, lq): with d = j - mask_offset a window gives
+// [d, d + mask_size - 1], a complement [d + mask_size, lq - 1], no mask everything; P.lo_add / hi_add hold the
+// constants (clamped to 2^30 on the host, so that 32-bit arithmetic is enough).
+__device__ __forceinline__ void colsum_range(const ColsumTcParams& P, int j, int* lo, int* hi) {
+  *lo = P.lo_add == kNoBound ? 0 : j + P.lo_add;
+  *hi = P.hi_add == kNoBound ? (int)P.lq - 1 : j + P.hi_add;
+}
+// query tiles [tf, tl] that can see a key of the tile [j0, j0 + keys) (tl < tf: none)
+__device__ __forceinline__ void colsum_q_tiles(const ColsumTcParams& P, int j0, int keys, int* tf, int* tl) {
+  int lo, hi, x;
+  colsum_range(P, j0, &lo, &x);
+  colsum_range(P, j0 + keys - 1, &x, &hi);
+  lo = lo < 0 ? 0 : lo;
+  hi = hi > (int)P.lq - 1 ? (int)P.lq - 1 : hi;
+  *tf = lo <= hi ? lo / kTile : 0;
+  *tl = lo <= hi ? hi / kTile : -1;
 }
 
 template <typename T>
-__global__ void __launch_bounds__(576, 1) colsum_tc_kernel(const __grid_constant__ ColsumTcParams P) {
+__global__ void __launch_bounds__(colsum_smem::kThreads, 1) colsum_tc_kernel(const __grid_constant__ ColsumTcParams P) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const uint32_t s_base = smem_u32(smem);
@@ -1121,49 +1140,23 @@ __global__ void __launch_bounds__(576, 1) colsum_tc_kernel(const __grid_constant
   float* s_acc = reinterpret_cast<float*>(smem + colsum_smem::kAcc);
   const uint32_t bars = s_base + colsum_smem::kBar;
   constexpr int NB = colsum_smem::kBufs;
-  // barriers: 0 q_full, 1-2 k_full, 3-4 k_free, then s_full[NB], free[NB]
-  constexpr int KF = 1, KE = 3, SF = 5, FR = 5 + NB;
+  // barriers: k_full[2], k_free[2], s_full[NB], free[NB], q_full[query tile]
+  constexpr int KF = 0, KE = 2, SF = 4, FR = 4 + NB, QF = 4 + 2 * NB, N_BARS = QF + colsum_smem::kQTiles;
   auto bar = [&](int i) { return bars + 8u * (uint32_t)i; };
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + colsum_smem::kBar + 112);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + colsum_smem::kBar + 120);
+  static_assert(N_BARS * 8 <= 144, "");
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + colsum_smem::kBar + 144);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + colsum_smem::kBar + 152);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int h = blockIdx.y, hkv = h / P.group;
   const int n_key_tiles = (int)((P.lk + kTile - 1) / kTile);
   const int kt0 = blockIdx.x * P.tiles_per_cta;
   const int kt1 = kt0 + P.tiles_per_cta < n_key_tiles ? kt0 + P.tiles_per_cta : n_key_tiles;
-  if (threadIdx.x == 0) {
-    mbar_init(bar(0), 1);
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(bar(KF + i), 1);
-      mbar_init(bar(KE + i), 1);
-    }
-    for (int i = 0; i < NB; ++i) {
-      mbar_init(bar(SF + i), 1);
-      mbar_init(bar(FR + i), 512);
-    }
-    *abort_flag = 0;
-    mbar_fence_init();
-  }
-  for (int i = threadIdx.x; i < colsum_smem::kMaxKeyTiles * 4 * 128; i += blockDim.x) s_acc[i] = 0.f;
-  for (int i = threadIdx.x; i < colsum_smem::kQTiles * 128; i += blockDim.x)
-    s_lse[i] = i < P.lq ? P.lse[(int64_t)h * P.lq + i] : INFINITY;
-  if (warp == 17) {
-    tmem_alloc(smem_u32(tmem_slot), 128 * NB);
-    tmem_relinquish();
-  }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
-  constexpr bool kBf16 = !std::is_same<T, __half>::value;
-  constexpr uint32_t idesc = make_idesc(kBf16, 128, 128, false);
-
   // the query tiles any key tile of this CTA needs
   int q_first = 1 << 30, q_last = -1;
   for (int kt = kt0; kt < kt1; ++kt) {
-    const int64_t j0 = (int64_t)kt * kTile;
-    const int keys = (int)((P.lk - j0) < kTile ? (P.lk - j0) : kTile);
+    const int j0 = kt * kTile;
+    const int keys = (int)P.lk - j0 < kTile ? (int)P.lk - j0 : kTile;
     int tf, tl;
     colsum_q_tiles(P, j0, keys, &tf, &tl);
     if (tl >= tf) {
@@ -1172,40 +1165,104 @@ __global__ void __launch_bounds__(576, 1) colsum_tc_kernel(const __grid_constant
     }
   }
   const bool any = q_last >= q_first;
-
-  if (warp == 16) {
-    // ============================================================== producer: query tiles once, then key tiles
-    if (lane == 0 && any) {
-      mbar_expect_tx(bar(0), (uint32_t)(q_last - q_first + 1) * 2 * kSubTileBytes);
-      for (int t = q_first; t <= q_last; ++t) {
-        tma_load_3d(sQ + t * 2 * kSubTileBytes, &P.map_q, bar(0), 0, P.q_row0 + t * kTile, h);
-        tma_load_3d(sQ + t * 2 * kSubTileBytes + kSubTileBytes, &P.map_q, bar(0), 64, P.q_row0 + t * kTile, h);
-      }
-      bool ok = true;
-      int n = 0;  // key tiles with work, in order
-      for (int kt = kt0; kt < kt1 && ok; ++kt) {
-        const int64_t j0 = (int64_t)kt * kTile;
-        const int keys = (int)((P.lk - j0) < kTile ? (P.lk - j0) : kTile);
+  auto load_q = [&](int t) {
+    mbar_expect_tx(bar(QF + t), 2 * kSubTileBytes);
+    tma_load_3d(sQ + t * 2 * kSubTileBytes, &P.map_q, bar(QF + t), 0, P.q_row0 + t * kTile, h);
+    tma_load_3d(sQ + t * 2 * kSubTileBytes + kSubTileBytes, &P.map_q, bar(QF + t), 64, P.q_row0 + t * kTile, h);
+  };
+  auto load_k = [&](int b, int j0) {
+    mbar_expect_tx(bar(KF + b), 2 * kSubTileBytes);
+    tma_load_3d(sK + b * 2 * kSubTileBytes, &P.map_k, bar(KF + b), 0, P.k_tok0 + j0, hkv);
+    tma_load_3d(sK + b * 2 * kSubTileBytes + kSubTileBytes, &P.map_k, bar(KF + b), 64, P.k_tok0 + j0, hkv);
+  };
+  if (warp == 16 && lane == 0) {
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(bar(KF + i), 1);
+      mbar_init(bar(KE + i), colsum_smem::kIssuers);
+    }
+    for (int i = 0; i < NB; ++i) {
+      mbar_init(bar(SF + i), 1);
+      mbar_init(bar(FR + i), 4);  // the warps of the group that reads the buffer
+    }
+    for (int i = 0; i < colsum_smem::kQTiles; ++i) mbar_init(bar(QF + i), 1);
+    *abort_flag = 0;
+    mbar_fence_init();
+    chain_enter();
+    // what the first products need is on its way while the CTA sets up; they run as soon as a query tile is there
+    if (any) {
+      int n = 0;
+      for (int kt = kt0; kt < kt1 && n < 2; ++kt) {
+        const int j0 = kt * kTile;
+        const int keys = (int)P.lk - j0 < kTile ? (int)P.lk - j0 : kTile;
         int tf, tl;
         colsum_q_tiles(P, j0, keys, &tf, &tl);
         if (tl < tf) continue;
-        const int b = n & 1;
-        if (n >= 2) ok = wait_or_abort(bar(KE + b), ((n >> 1) - 1) & 1, abort_flag, P.err, 410);
-        if (!ok) break;
-        mbar_expect_tx(bar(KF + b), 2 * kSubTileBytes);
-        tma_load_3d(sK + b * 2 * kSubTileBytes, &P.map_k, bar(KF + b), 0, P.k_tok0 + (int)j0, hkv);
-        tma_load_3d(sK + b * 2 * kSubTileBytes + kSubTileBytes, &P.map_k, bar(KF + b), 64, P.k_tok0 + (int)j0, hkv);
+        if (n == 0) {
+          load_q(tf);
+          load_k(0, j0);
+          for (int t = q_first; t <= q_last; ++t)
+            if (t != tf) load_q(t);
+        } else {
+          load_k(1, j0);
+        }
         ++n;
       }
     }
-  } else if (warp == 17) {
-    // ======================================================================================= MMA issuer
+  }
+  for (int i = threadIdx.x; i < (kt1 - kt0) * NB * 128; i += blockDim.x) s_acc[i] = 0.f;
+  if (warp == 17) {
+    tmem_alloc(smem_u32(tmem_slot), 128 * NB);
+    tmem_relinquish();
+  }
+  chain_enter();
+  for (int i = threadIdx.x; i < colsum_smem::kQTiles * 128; i += blockDim.x)
+    s_lse[i] = i < P.lq ? -P.lse[(int64_t)h * P.lq + i] : -INFINITY;
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+  constexpr bool kBf16 = !std::is_same<T, __half>::value;
+  constexpr uint32_t idesc = make_idesc(kBf16, 128, 128, false);
+
+  if (warp == 16) {
+    // ==================================================== producer: the key tiles after the first two
     if (lane == 0 && any) {
-      bool ok = wait_or_abort(bar(0), 0, abort_flag, P.err, 411);
-      int n = 0, step = 0;
+      bool ok = true;
+      int n = 0;  // key tiles with work, in order
       for (int kt = kt0; kt < kt1 && ok; ++kt) {
-        const int64_t j0 = (int64_t)kt * kTile;
-        const int keys = (int)((P.lk - j0) < kTile ? (P.lk - j0) : kTile);
+        const int j0 = kt * kTile;
+        const int keys = (int)P.lk - j0 < kTile ? (int)P.lk - j0 : kTile;
+        int tf, tl;
+        colsum_q_tiles(P, j0, keys, &tf, &tl);
+        if (tl < tf) continue;
+        if (n >= 2) {
+          ok = wait_or_abort(bar(KE + (n & 1)), ((n >> 1) - 1) & 1, abort_flag, P.err, 410);
+          if (!ok) break;
+          load_k(n & 1, j0);
+        }
+        ++n;
+      }
+      if (!ok) {
+        // give loads that are still in flight a bounded chance to land before the CTA's memory goes away
+        for (int b = 0; b < 2; ++b)
+          for (uint32_t i = 0; i < 4096 && !mbar_try_wait(bar(KF + b), 0) && !mbar_try_wait(bar(KF + b), 1); ++i) __nanosleep(64);
+        for (int t = q_first; t <= q_last; ++t)
+          for (uint32_t i = 0; i < 4096 && !mbar_try_wait(bar(QF + t), 0); ++i) __nanosleep(64);
+      }
+    }
+  } else if (warp > 16) {
+    // ====================================================================================== MMA issuers
+    // Two threads take the products in turn.  A product keeps the pipe busy for 514 cycles and the thread that issues
+    // it for 1385 (waits that are already over cost 200 cycles each, the eight instructions leave at the pipe's pace,
+    // then the commit): one thread for all of them was what the whole kernel waited for.  A TMEM buffer always has the
+    // same issuer, which therefore never gets a whole turn ahead of the buffer's phases.
+    if (lane == 0 && any) {
+      const int me = warp - 17;
+      bool ok = true;
+      int n = 0, step = 0, q_there = 0;
+      for (int kt = kt0; kt < kt1 && ok; ++kt) {
+        const int j0 = kt * kTile;
+        const int keys = (int)P.lk - j0 < kTile ? (int)P.lk - j0 : kTile;
         int tf, tl;
         colsum_q_tiles(P, j0, keys, &tf, &tl);
         if (tl < tf) continue;
@@ -1214,102 +1271,101 @@ __global__ void __launch_bounds__(576, 1) colsum_tc_kernel(const __grid_constant
         const uint32_t kt_s = sK + kb * 2 * kSubTileBytes;
         for (int t = tf; t <= tl && ok; ++t, ++step) {
           const int b = step % NB;
+          if (b % colsum_smem::kIssuers != me) continue;
           if (step >= NB) ok = wait_or_abort(bar(FR + b), ((step / NB) - 1) & 1, abort_flag, P.err, 413);
+          if (ok && !(q_there >> t & 1)) ok = wait_or_abort(bar(QF + t), 0, abort_flag, P.err, 411);
+          q_there |= 1 << t;
           if (!ok) break;
           tc_fence_after();
-          const uint32_t qt = sQ + t * 2 * kSubTileBytes;
+          const uint64_t ad = make_sdesc(kt_s, 16, 1024), bd = make_sdesc(sQ + t * 2 * kSubTileBytes, 16, 1024);
 #pragma unroll
           for (int ks = 0; ks < 8; ++ks) {
             // S^T = K Q^T: keys are the M rows (TMEM lanes), queries the N columns
-            uint64_t ad = make_sdesc(kt_s + (ks >> 2) * kSubTileBytes + (ks & 3) * 32, 16, 1024);
-            uint64_t bd = make_sdesc(qt + (ks >> 2) * kSubTileBytes + (ks & 3) * 32, 16, 1024);
-            mma_ss(tmem + b * 128, ad, bd, idesc, ks > 0);
+            const uint64_t off = (uint64_t)(((ks >> 2) * kSubTileBytes + (ks & 3) * 32) >> 4);
+            mma_ss(tmem + b * 128, ad + off, bd + off, idesc, ks > 0);
           }
           tc_commit(bar(SF + b));
         }
-        if (ok) tc_commit(bar(KE + kb));  // every product that reads this key tile has been issued
+        if (ok) tc_commit(bar(KE + kb));  // this thread's products with this key tile have been issued
         ++n;
       }
     }
   } else {
     // ========================================================================================== compute
+    // Group `part` of four warps takes every fourth product - TMEM buffer `part` - whole: a thread owns one key and all
+    // 128 queries of it, in four loads of 32 columns (asking for the next columns ahead costs registers and gained nothing: the
+    // other groups' warps fill the wait).
     const int quad = warp & 3, part = warp >> 2;
     const int krow = quad * 32 + lane;
-    const int col0 = part * 32;
-    const uint32_t lane_base = ((uint32_t)(quad * 32)) << 16;
+    const uint32_t tS = tmem + part * 128 + (((uint32_t)(quad * 32)) << 16);
     bool ok = true;
-    int step = 0, n = 0;
+    int step = 0;
     for (int kt = kt0; kt < kt1 && ok; ++kt) {
-      const int64_t j0 = (int64_t)kt * kTile;
-      const int keys = (int)((P.lk - j0) < kTile ? (P.lk - j0) : kTile);
+      const int j0 = kt * kTile;
+      const int keys = (int)P.lk - j0 < kTile ? (int)P.lk - j0 : kTile;
       int tf, tl;
       colsum_q_tiles(P, j0, keys, &tf, &tl);
       if (tl < tf) continue;
-      // queries that see this thread's key
-      const int64_t kj = j0 + krow;
-      int64_t vi_lo = 0, vi_hi = P.lq - 1;
-      if (P.mask_mode == INFLLM_MASK_WINDOW) {
-        vi_lo = kj - P.mask_offset;
-        vi_hi = kj - P.mask_offset + P.mask_size - 1;
-      } else if (P.mask_mode == INFLLM_MASK_COMPLEMENT) {
-        vi_lo = kj - P.mask_offset + P.mask_size;
-      }
-      if (vi_lo < 0) vi_lo = 0;
-      if (vi_hi > P.lq - 1) vi_hi = P.lq - 1;
-      if (kj >= P.lk) vi_hi = -1;
+      // queries [vi_lo, vi_hi] see this thread's key
+      int vi_lo, vi_hi;
+      colsum_range(P, j0 + krow, &vi_lo, &vi_hi);
+      if (krow >= keys) vi_hi = -1;
       float total = 0.f;
       for (int t = tf; t <= tl && ok; ++t, ++step) {
-        const int b = step % NB;
-        ok = __all_sync(0xffffffffu, wait_or_abort(bar(SF + b), (step / NB) & 1, abort_flag, P.err, 414));
+        if ((step % NB) != part) continue;
+        ok = __all_sync(0xffffffffu, wait_or_abort(bar(SF + part), (step / NB) & 1, abort_flag, P.err, 414));
         if (!ok) break;
         tc_fence_after();
-        float sv[32];
-        tmem_ld32(tmem + b * 128 + lane_base + col0, reinterpret_cast<uint32_t*>(sv));
-        tmem_wait_ld();
-        tc_fence_before();
-        mbar_arrive(bar(FR + b));  // the accumulator is in registers: the buffer can be overwritten
-        const int64_t q0 = (int64_t)t * kTile + col0;
-        const int64_t a = vi_lo > q0 ? vi_lo : q0, e = vi_hi < q0 + 31 ? vi_hi : q0 + 31;
-        const int c_lo = (int)(a - q0), c_hi = (int)(e - q0);
-        const float* ls = s_lse + t * kTile + col0;
-        float acc4[4] = {0.f, 0.f, 0.f, 0.f};
-        if (c_lo == 0 && c_hi == 31) {
-#pragma unroll
-          for (int c = 0; c < 32; c += 4) {
-            const float4 l4 = *reinterpret_cast<const float4*>(ls + c);
-            const float2 p01 = ex2_pair(fmaf(sv[c], P.scale_log2, -l4.x), fmaf(sv[c + 1], P.scale_log2, -l4.y));
-            const float2 p23 = ex2_pair(fmaf(sv[c + 2], P.scale_log2, -l4.z), fmaf(sv[c + 3], P.scale_log2, -l4.w));
-            acc4[0] += p01.x;
-            acc4[1] += p01.y;
-            acc4[2] += p23.x;
-            acc4[3] += p23.y;
+        const int q_end = (int)P.lq - 1 - t * kTile, c_lo = vi_lo - t * kTile,
+                  c_hi = vi_hi - t * kTile < q_end ? vi_hi - t * kTile : q_end;
+        // a query row without any visible key has lse = -inf; it cannot see this key either, so it is masked
+        const bool full = __all_sync(0xffffffffu, c_lo <= 0 && c_hi >= kTile - 1);
+        const float* ls = s_lse + t * kTile;
+        const float2 sc2 = make_float2(P.scale_log2, P.scale_log2);
+        float2 acc[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+#pragma unroll 1
+        for (int cc = 0; cc < 4; ++cc) {
+          float sc[32];
+          tmem_ld32(tS + cc * 32, reinterpret_cast<uint32_t*>(sc));
+          tmem_wait_ld();
+          if (cc == 3) {  // everything is in registers: the buffer can be overwritten
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar(FR + part));
           }
-        } else if (c_lo <= c_hi) {
+          if (full) {
 #pragma unroll
-          for (int c = 0; c < 32; ++c) {
-            const float pv = ex2_approx(fmaf(sv[c], P.scale_log2, -ls[c]));
-            acc4[c & 3] += (c >= c_lo && c <= c_hi) ? pv : 0.f;
+            for (int c = 0; c < 32; c += 4) {
+              const float4 l4 = *reinterpret_cast<const float4*>(ls + cc * 32 + c);  // negated
+              const float2 a0 = ffma2(sc[c], sc[c + 1], sc2, make_float2(l4.x, l4.y));
+              const float2 a1 = ffma2(sc[c + 2], sc[c + 3], sc2, make_float2(l4.z, l4.w));
+              acc[0] = fadd2(acc[0], make_float2(ex2_approx(a0.x), ex2_approx(a0.y)));
+              acc[1] = fadd2(acc[1], (c & 4) ? ex2_poly2<4>(a1) : make_float2(ex2_approx(a1.x), ex2_approx(a1.y)));
+            }
+          } else {
+#pragma unroll
+            for (int c = 0; c < 32; ++c) {
+              const float pv = ex2_approx(fmaf(sc[c], P.scale_log2, ls[cc * 32 + c]));
+              if (cc * 32 + c >= c_lo && cc * 32 + c <= c_hi) acc[c & 1].x += pv;
+            }
           }
         }
-        // a query row without any visible key has lse = -inf; it cannot see this key either, so it is masked above
-        total += (acc4[0] + acc4[1]) + (acc4[2] + acc4[3]);
+        total += (acc[0].x + acc[0].y) + (acc[1].x + acc[1].y);
       }
       // every thread owns one slot per key tile: no atomics, and the final sum below has a fixed order
       s_acc[((kt - kt0) * 4 + part) * 128 + krow] = total;
-      ++n;
     }
-    (void)n;
   }
   tc_fence_before();
   __syncthreads();
-  if (threadIdx.x < 128 && !(*abort_flag)) {
-    for (int kt = kt0; kt < kt1; ++kt) {
-      const int64_t kj = (int64_t)kt * kTile + threadIdx.x;
-      if (kj >= P.lk) break;
-      const float* sa = s_acc + ((kt - kt0) * 4) * 128 + threadIdx.x;
+  if (!(*abort_flag)) {
+    // every column in a thread of its own: one round of reads and writes
+    const int cols = (int)((P.lk < (int64_t)kt1 * kTile ? P.lk : (int64_t)kt1 * kTile) - (int64_t)kt0 * kTile);
+    float* dst = P.score + (int64_t)h * P.score_hs + (int64_t)kt0 * kTile;
+    for (int i = threadIdx.x; i < cols; i += blockDim.x) {
+      const float* sa = s_acc + (i >> 7) * NB * 128 + (i & 127);
       const float v = (sa[0] + sa[128]) + (sa[256] + sa[384]);
-      float* dst = P.score + (int64_t)h * P.score_hs + kj;
-      *dst = P.accumulate ? *dst + v : v;
+      dst[i] = P.accumulate ? dst[i] + v : v;
     }
   }
   if (warp == 17) tmem_dealloc(tmem, 128 * NB);
@@ -1395,11 +1451,12 @@ int attn_tc_combine_launch(const float* acc, const float* m, const float* l, int
 }
 
 // Runs of key tiles per (128-query tile, head): one while the grid covers more than half of the SMs, else as many as
-// fill them with at least two tiles each.
+// fill them with at least eight tiles each (a run has the fixed cost of about four, and the partials are merged by a
+// launch of their own).
 int attn_tc3_splits(int64_t lq, int n_heads, int64_t keys) {
   const int64_t items = ceil_div(lq, kTile) * n_heads, tiles = ceil_div(keys, kTile);
   if (items > 74) return 1;
-  return (int)std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(148 / items, tiles / 2), 32));
+  return (int)std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(148 / items, tiles / 8), 32));
 }
 
 int attn_tc3_launch(const AttnTcParams& P, int dtype, cudaStream_t s) {
@@ -1416,10 +1473,6 @@ int attn_tc3_launch(const AttnTcParams& P, int dtype, cudaStream_t s) {
   });
   INFLLM_LAUNCH_OK("attn_tc3_kernel");
   return INFLLM_OK;
-}
-
-size_t attn_tc2_scratch_floats(int n_split, int n_heads, int64_t lq) {
-  return n_split > 1 ? (size_t)n_split * n_heads * lq * (128 + 2) : 0;
 }
 
 int attn_tc2_launch(const AttnTcParams& P, int dtype, cudaStream_t s) {
@@ -1455,14 +1508,19 @@ int colsum_tc_launch_maps(const CUtensorMap& map_q, const CUtensorMap& map_k, in
                           int n_kv_heads, int64_t lq, int64_t lk, int mask_mode, int64_t mask_offset,
                           int64_t mask_size, const float* lse, float* score, int64_t score_hs, int accumulate,
                           int dtype, cudaStream_t s) {
+  if (lk > (1 << 29)) return fail(INFLLM_E_UNSUPPORTED, "colsum (tensor-core kernel): %lld keys", (long long)lk);
   if (lq > colsum_smem::kQTiles * kTile)
     return fail(INFLLM_E_UNSUPPORTED, "colsum (tensor-core kernel): %lld queries, at most %d", (long long)lq,
                 colsum_smem::kQTiles * kTile);
   ColsumTcParams P{};
   P.map_q = map_q; P.map_k = map_k;
   P.q_row0 = q_row0; P.k_tok0 = k_tok0; P.n_heads = n_heads; P.group = n_heads / n_kv_heads;
-  P.lq = lq; P.lk = lk; P.mask_mode = mask_mode; P.accumulate = accumulate;
-  P.mask_offset = mask_offset; P.mask_size = mask_size; P.lse = lse; P.score = score; P.score_hs = score_hs;
+  P.lq = lq; P.lk = lk; P.accumulate = accumulate;
+  auto clamp = [](int64_t v) { return (int)std::max<int64_t>(-(1 << 30) + 1, std::min<int64_t>(1 << 30, v)); };
+  P.lo_add = P.hi_add = kNoBound;
+  if (mask_mode == INFLLM_MASK_WINDOW) P.lo_add = clamp(-mask_offset), P.hi_add = clamp(-mask_offset + mask_size - 1);
+  if (mask_mode == INFLLM_MASK_COMPLEMENT) P.lo_add = clamp(-mask_offset + mask_size);
+  P.lse = lse; P.score = score; P.score_hs = score_hs;
   P.scale_log2 = kLog2e / sqrtf(128.f);
   INFLLM_TRY(tc_get_error_ptr(&P.err));
   // one CTA per (head, run of key tiles): about one CTA per SM, never more than kMaxKeyTiles tiles each
@@ -1478,7 +1536,7 @@ int colsum_tc_launch_maps(const CUtensorMap& map_q, const CUtensorMap& map_k, in
     auto kern = colsum_tc_kernel<T>;
     // the opt-in holds for the current device only, and a process may drive several: asked for at every launch
     INFLLM_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kern<<<grid, 576, smem, s>>>(P);
+    kern<<<grid, colsum_smem::kThreads, smem, s>>>(P);
   });
   INFLLM_LAUNCH_OK("colsum_tc_kernel");
   return INFLLM_OK;

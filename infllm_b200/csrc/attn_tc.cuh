@@ -42,13 +42,13 @@ struct AttnTcParams {
   const float *st_acc, *st_m, *st_l;
 };
 
+constexpr int kNoBound = -(1 << 30);
 struct ColsumTcParams {
   alignas(64) CUtensorMap map_q, map_k;
   int32_t q_row0, k_tok0, n_heads, group;
   int64_t lq, lk;
-  int32_t mask_mode, accumulate;
-  int32_t tiles_per_cta, pad;
-  int64_t mask_offset, mask_size;
+  int32_t accumulate, tiles_per_cta;
+  int32_t lo_add, hi_add;  // queries [j + lo_add, j + hi_add] see key j; kNoBound: no bound on that side
   const float* lse;
   float* score;
   int64_t score_hs;
@@ -68,7 +68,6 @@ int attn_tc_combine_launch(const float* acc, const float* m, const float* l, int
                            const float* st_l, float* new_acc, float* new_m, float* new_l, int dtype, cudaStream_t s);
 // two query heads of one KV head per CTA (needs an even number of query heads per KV head)
 int attn_tc2_launch(const AttnTcParams& P, int dtype, cudaStream_t s);
-size_t attn_tc2_scratch_floats(int n_split, int n_heads, int64_t lq);
 int colsum_tc_launch_maps(const CUtensorMap& map_q, const CUtensorMap& map_k, int q_row0, int k_tok0, int n_heads,
                           int n_kv_heads, int64_t lq, int64_t lk, int mask_mode, int64_t mask_offset,
                           int64_t mask_size, const float* lse, float* score, int64_t score_hs, int accumulate,

@@ -1324,7 +1324,7 @@ int local_scores(infllm_ctx* c, cudaStream_t s, int64_t st, int64_t ks, int64_t 
   const int64_t D = g.head_dim, H = g.n_heads, HKV = g.n_kv_heads;
   const int64_t n = j_end - j_begin, tok = ks - tb.t0 + j_begin, off = (lk - lq) - j_begin;
   ProfScope ps(c, s, INFLLM_PROF_COLSUM, work);
-  if (c->use_tc && lq > 64 && lq <= 512)
+  if (c->use_tc && lq > 1 && lq <= 512)
     return colsum_tc_launch_maps(c->m_qloc, c->m_krot, (int)st, (int)tok, (int)H, (int)HKV, lq, n, INFLLM_MASK_WINDOW,
                                  off, g.n_local, c->lse, tb.score + tok, tb.cap, 1, g.dtype, s);
   return attn_colsum_launch((const char*)c->q_loc + st * D * c->esz, c->sub_max * D, D,
@@ -1574,7 +1574,7 @@ int append_sub(infllm_ctx* c, const char* q, int64_t q_hs, int64_t q_ts, const c
       for (int64_t i = 0; i < lq; ++i) local_pairs += (double)std::min<int64_t>(S + i + 1, g.n_local);
       for (auto& sgm : gsegs) all_glk += sgm.len;
       local_pairs_eb = local_pairs;
-      const bool tc_now = c->use_tc && lq > 64 && gsegs.size() + 1 <= (size_t)kMaxSeg;
+      const bool tc_now = c->use_tc && lq > 1 && gsegs.size() + 1 <= (size_t)kMaxSeg;
       if (tc_now) {
         AttnTcParams TP{};
         TP.maps[0] = c->m_qloc; TP.maps[1] = c->m_qglb; TP.maps[2] = c->m_krot; TP.maps[3] = c->m_kraw;
@@ -1598,29 +1598,32 @@ int append_sub(infllm_ctx* c, const char* q, int64_t q_hs, int64_t q_ts, const c
         TP.stage[1].map_q = 1; TP.stage[1].q_row0 = (int)st; TP.stage[1].mask_mode = INFLLM_MASK_NONE;
         TP.stage[1].lk = (int64_t)all_glk; TP.stage[1].seg_begin = 1; TP.stage[1].seg_end = ns;
         ProfScope ps(c, s, INFLLM_PROF_ATTN, 4.0 * D * H * (local_pairs + (double)lq * all_glk));
-        // The one-head kernel runs one CTA per (128-query tile, head): with few heads on this GPU (a KV-head-group
-        // shard) its grid leaves most SMs idle, and the two-head kernel, which also cuts the key tiles into runs,
-        // fills them.  Flag bit 3 forces the two-head kernel.
-        const bool few_ctas = lq >= 256 && ((lq + 127) / 128) * H <= 74;
-        if ((H / HKV) % 2 == 0 && ((g.debug_flags & 8) || few_ctas)) {
-          // two heads of a KV head per CTA; cut the key tiles into runs until the grid covers the SMs
-          const int items = (int)((lq + 127) / 128) * (int)(H / 2);
-          TP.n_split = std::max(1, std::min(8, 148 / items));
-          const size_t need = attn_tc2_scratch_floats(TP.n_split, (int)H, lq);
-          if (need > c->tc_part_floats) {
-            if (c->tc_part) INFLLM_CUDA_OK(cudaFreeAsync(c->tc_part, s));
-            INFLLM_CUDA_OK(dev_malloc_async((void**)&c->tc_part, need * sizeof(float), s));
-            c->tc_part_floats = need;
-          }
-          if (TP.n_split > 1) {
-            TP.part_acc = c->tc_part;
-            TP.part_m = c->tc_part + (size_t)TP.n_split * H * lq * 128;
-            TP.part_l = TP.part_m + (size_t)TP.n_split * H * lq;
-          }
+        // One CTA per (128-query tile, head); few queries or few heads on this GPU (a short call, a KV-head-group shard)
+        // leave most SMs idle that way, and the key tiles are cut into runs until the grid fills them.  Flag bit 3
+        // forces the kernel that takes two heads of a KV head per CTA.
+        const bool two = (H / HKV) % 2 == 0 && (g.debug_flags & 8);
+        const int items = (int)((lq + 127) / 128) * (int)(H / 2);
+        TP.n_split = two ? std::max(1, std::min(8, 148 / items)) : attn_tc3_splits(lq, (int)H, lk + (int64_t)all_glk);
+        const size_t need = TP.n_split > 1 ? (size_t)TP.n_split * H * lq * (128 + 2) : 0;
+        if (need > c->tc_part_floats) {
+          if (c->tc_part) INFLLM_CUDA_OK(cudaFreeAsync(c->tc_part, s));
+          c->tc_part = nullptr;
+          c->tc_part_floats = 0;
+          INFLLM_CUDA_OK(dev_malloc_async((void**)&c->tc_part, need * sizeof(float), s));
+          c->tc_part_floats = need;
+        }
+        if (TP.n_split > 1) {
+          TP.part_acc = c->tc_part;
+          TP.part_m = c->tc_part + (size_t)TP.n_split * H * lq * 128;
+          TP.part_l = TP.part_m + (size_t)TP.n_split * H * lq;
+        }
+        if (two) {
           INFLLM_TRY(attn_tc2_launch(TP, g.dtype, s));
         } else {
-          TP.n_split = 1;
           INFLLM_TRY(attn_tc3_launch(TP, g.dtype, s));
+          if (TP.n_split > 1)
+            INFLLM_TRY(attn_tc_combine_launch(TP.part_acc, TP.part_m, TP.part_l, TP.n_split, (int)H, lq, out_eb, o_hs, o_ts,
+                                              c->lse, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, g.dtype, s));
         }
       } else {
       AttnParams P{};
