@@ -41,8 +41,17 @@ int qbar_launch(const void* q, int64_t q_hs, int64_t q_ts, int n_heads, int64_t 
 int block_topk_launch(const void* bk, int64_t n, int width, const float* qbar, float* scores, int k, int id_base,
                       int32_t* out_ids, float* out_scores, int dtype, cudaStream_t s, unsigned int* ticket,
                       int32_t* out_ids_copy = nullptr);
-int block_score_rows_launch(const void* bk, const int32_t* rows, int n, int width, const float* qbar, float* scores,
-                            int dtype, cudaStream_t s);
+int seal_score_launch(const void* k, int64_t k_hs, int64_t k_ts, const float* score, int64_t score_hs, int64_t tok0, int n_new,
+                      int first_new, int block_size, int repr_topk, int n_heads, int n_kv_heads, int head_dim, void* bk,
+                      const int32_t* rows, int n_old, const float* qbar, float* scores, const int32_t* err, int32_t* err_out,
+                      int dtype, cudaStream_t s);
+bool seal_score_ok(int block_size, int head_dim, int64_t k_hs, int64_t k_ts, const void* k);
+int mail_words_launch(const int32_t* src, int32_t* dst, cudaStream_t s);
+int ingest_rows_launch(const void* q, int64_t q_hs, int64_t q_ts, const void* k, int64_t k_hs, int64_t k_ts, const void* v,
+                       int64_t v_hs, int64_t v_ts, void* q_loc, void* q_glb, int64_t qs_hs, float* qbar, int64_t qbar_stride,
+                       void* k_raw, void* k_rot, void* v_out, int64_t kv_hs, float* score, int64_t score_hs, int n_heads,
+                       int n_kv_heads, int64_t len, int exc, const float* cos_t, const float* sin_t, int64_t table_len,
+                       int64_t pos_loc, int64_t pos_glb, bool first_only, int dtype, cudaStream_t s);
 int repr_select_launch(const void* k, int64_t k_hs, int64_t k_ts, const float* score, int64_t score_hs,
                        int64_t tok0, int n_new, int block_size, int repr_topk, int n_heads, int n_kv_heads,
                        int head_dim, void* out, int dtype, cudaStream_t s);
@@ -285,6 +294,11 @@ struct infllm_ctx {
   int64_t d2h_synced_upto = 0;  // units below this id are known to be in the host store as far as copy_stream is concerned
 
   cudaStream_t copy_stream = nullptr, aux_stream = nullptr;
+  // Sealing and the ranking of the next exec block's candidates run beside the main stream, which goes on with the rest
+  // of the column sums; ev_seal is behind the last sealing (on whichever stream it ran), ev_urgent behind the sums it needs.
+  cudaStream_t seal_stream = nullptr;
+  cudaEvent_t ev_urgent = nullptr;
+  bool seal_aside = false;  // the last sealing ran on seal_stream: the main stream has not waited for it
   cudaEvent_t ev_main = nullptr, ev_copy = nullptr, ev_sync = nullptr, ev_attn = nullptr, ev_attn_prev = nullptr, ev_spec = nullptr,
               ev_cand = nullptr, ev_seal = nullptr, ev_stage = nullptr;
   bool attn_recorded = false, attn_prev_recorded = false, spec_recorded = false;
@@ -293,7 +307,7 @@ struct infllm_ctx {
   // them behind those marks (order_behind_reset).
   cudaEvent_t ev_last = nullptr;  // behind the last kernel of an append on the caller's stream, where ev_attn is not
   bool last_recorded = false;
-  cudaEvent_t ev_side[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
+  cudaEvent_t ev_side[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
   bool reset_pending = false, reset_attn = false, reset_last = false;
   bool failed = false;  // an append gave up half-way: the context is not handed to anybody else afterwards
 
@@ -423,8 +437,10 @@ int lazy_init(infllm_ctx* c, cudaStream_t s) {
     INFLLM_CUDA_OK(cudaDeviceGetStreamPriorityRange(&lo, &hi));
     INFLLM_CUDA_OK(cudaStreamCreateWithPriority(&c->copy_stream, cudaStreamNonBlocking, hi));
     INFLLM_CUDA_OK(cudaStreamCreateWithPriority(&c->urgent_stream, cudaStreamNonBlocking, hi));
+    // so is the packing of sealed units: a few microseconds on the SMs that an attention grid leaves free, ahead of the
+    // look-ahead scoring that would take them for longer
+    INFLLM_CUDA_OK(cudaStreamCreateWithPriority(&c->d2h_stream, cudaStreamNonBlocking, hi));
   }
-  INFLLM_CUDA_OK(cudaStreamCreateWithFlags(&c->d2h_stream, cudaStreamNonBlocking));
   INFLLM_CUDA_OK(cudaEventCreateWithFlags(&c->ev_d2h, cudaEventDisableTiming));
   INFLLM_CUDA_OK(cudaEventCreateWithFlags(&c->ev_ingest, cudaEventDisableTiming));
   c->pack_units = g.exc_block_size / g.block_size + 2;
@@ -441,12 +457,14 @@ int lazy_init(infllm_ctx* c, cudaStream_t s) {
     int lo = 0, hi = 0;  // the look-ahead kernels are short and latency matters: highest priority
     INFLLM_CUDA_OK(cudaDeviceGetStreamPriorityRange(&lo, &hi));
     INFLLM_CUDA_OK(cudaStreamCreateWithPriority(&c->aux_stream, cudaStreamNonBlocking, hi));
+    INFLLM_CUDA_OK(cudaStreamCreateWithPriority(&c->seal_stream, cudaStreamNonBlocking, hi));
   }
   INFLLM_CUDA_OK(cudaEventCreateWithFlags(&c->ev_spec, cudaEventDisableTiming));
   INFLLM_CUDA_OK(cudaEventCreateWithFlags(&c->ev_cand, cudaEventDisableTiming));
   INFLLM_CUDA_OK(cudaEventCreateWithFlags(&c->ev_seal, cudaEventDisableTiming));
   INFLLM_CUDA_OK(cudaEventCreateWithFlags(&c->ev_stage, cudaEventDisableTiming));
   INFLLM_CUDA_OK(cudaEventCreateWithFlags(&c->ev_last, cudaEventDisableTiming));
+  INFLLM_CUDA_OK(cudaEventCreateWithFlags(&c->ev_urgent, cudaEventDisableTiming));
   for (auto& e : c->ev_side) INFLLM_CUDA_OK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
 
   const int64_t D = g.head_dim, H = g.n_heads, HKV = g.n_kv_heads;
@@ -548,7 +566,7 @@ int lazy_init(infllm_ctx* c, cudaStream_t s) {
 int order_behind_reset(infllm_ctx* c, cudaStream_t s) {
   if (!c->reset_pending) return INFLLM_OK;
   c->reset_pending = false;
-  cudaStream_t side[5] = {c->copy_stream, c->urgent_stream, c->aux_stream, c->d2h_stream, c->mail_stream};
+  cudaStream_t side[6] = {c->copy_stream, c->urgent_stream, c->aux_stream, c->d2h_stream, c->mail_stream, c->seal_stream};
   for (cudaEvent_t e : c->ev_side) INFLLM_CUDA_OK(cudaStreamWaitEvent(s, e, 0));
   if (c->reset_attn) INFLLM_CUDA_OK(cudaStreamWaitEvent(s, c->ev_attn, 0));
   if (c->reset_last) INFLLM_CUDA_OK(cudaStreamWaitEvent(s, c->ev_last, 0));
@@ -560,34 +578,34 @@ int order_behind_reset(infllm_ctx* c, cudaStream_t s) {
   return INFLLM_OK;
 }
 
-// Sends a copy of the tensor-core kernels' error record to the host on `copy_on`, ordered behind what stream s has
-// enqueued so far (copy_on == s: no extra ordering needed).
-int send_device_error(infllm_ctx* c, cudaStream_t s, cudaStream_t copy_on) {
+// Sends the tensor-core kernels' error record to the host, behind what stream s has enqueued so far.
+int send_device_error(infllm_ctx* c, cudaStream_t s) {
   if (!c->tc_err || !c->h_tc_err) return INFLLM_OK;
-  if (copy_on != s) {
-    INFLLM_CUDA_OK(cudaEventRecord(c->ev_main, s));
-    INFLLM_CUDA_OK(cudaStreamWaitEvent(copy_on, c->ev_main, 0));
-  }
-  INFLLM_CUDA_OK(cudaMemcpyAsync(c->h_tc_err, c->tc_err, 4 * sizeof(int32_t), cudaMemcpyDeviceToHost, copy_on));
-  INFLLM_CUDA_OK(cudaEventRecord(c->ev_err, copy_on));
+  INFLLM_TRY(mail_words_launch(c->tc_err, c->h_tc_err, s));
+  INFLLM_CUDA_OK(cudaEventRecord(c->ev_err, s));
   c->err_pending = true;
   return INFLLM_OK;
 }
 
-// Reads the last copy of the record if it has landed (never waits): a recorded error becomes INFLLM_E_TIMEOUT,
-// and the device-side record is cleared on s so that the next report names a new event.
+// A copy of the record that has landed: a recorded error becomes INFLLM_E_TIMEOUT, and the device-side record is
+// cleared on s so that the next report names a new event.
+int check_device_error(infllm_ctx* c, cudaStream_t s) {
+  if (!c->h_tc_err || c->h_tc_err[0] == 0) return INFLLM_OK;
+  const int code = c->h_tc_err[0], where = c->h_tc_err[1], bx = c->h_tc_err[2], by = c->h_tc_err[3];
+  c->h_tc_err[0] = 0;
+  INFLLM_CUDA_OK(cudaMemsetAsync(c->tc_err, 0, 4 * sizeof(int32_t), s));
+  return fail(INFLLM_E_TIMEOUT, "a bounded wait of a tensor-core kernel ran out (code %d, wait %d, CTA %d,%d): the rows "
+              "that CTA was to write are not valid", code, where, bx, by);
+}
+
+// Reads the last copy of the record if it has landed (never waits).
 int poll_device_error(infllm_ctx* c, cudaStream_t s) {
   if (!c->err_pending || cudaEventQuery(c->ev_err) != cudaSuccess) {
     cudaGetLastError();  // cudaErrorNotReady is not an error of ours
     return INFLLM_OK;
   }
   c->err_pending = false;
-  if (c->h_tc_err[0] == 0) return INFLLM_OK;
-  const int code = c->h_tc_err[0], where = c->h_tc_err[1], bx = c->h_tc_err[2], by = c->h_tc_err[3];
-  c->h_tc_err[0] = 0;
-  INFLLM_CUDA_OK(cudaMemsetAsync(c->tc_err, 0, 4 * sizeof(int32_t), s));
-  return fail(INFLLM_E_TIMEOUT, "a bounded wait of a tensor-core kernel ran out (code %d, wait %d, CTA %d,%d): the rows "
-              "that CTA was to write are not valid", code, where, bx, by);
+  return check_device_error(c, s);
 }
 
 // make room for tokens [frontier, length + add) in the token buffers
@@ -710,8 +728,25 @@ int score_topk(infllm_ctx* c, int64_t n, const float* qbar, float* scores, int32
   return topk_launch(scores, n, k, 0, d_ids, nullptr, s);
 }
 
-// ids of one exec block straight from the device scorer: scoring + top-k, then a host sync on the result
-int retrieve_now(infllm_ctx* c, int eb_in_call, std::vector<int32_t>* ids, cudaStream_t s) {
+// the scorer's one-launch form can write the ids into pinned host words itself (no copy, which would queue behind the
+// units on their way out)
+bool ids_direct(const infllm_ctx* c, int64_t n) { return !c->comm && c->cfg.topk <= 64 && n <= 16384; }
+
+// ids of one exec block straight from the device scorer, in two halves: scoring + top-k on s, and the wait for the result
+int retrieve_launch(infllm_ctx* c, int eb_in_call, int64_t n, cudaStream_t s) {
+  const infllm_config& g = c->cfg;
+  INFLLM_TRY(ensure_scores(c, n, s));
+  const bool direct = ids_direct(c, n);
+  {
+    ProfScope ps(c, s, INFLLM_PROF_TOPK, (double)n * c->width * c->esz);
+    INFLLM_TRY(score_topk(c, n, c->qbar + (int64_t)eb_in_call * c->width, c->scores, c->d_topk, s, 0, 0, direct ? c->h_topk : nullptr));
+  }
+  if (!direct) INFLLM_CUDA_OK(cudaMemcpyAsync(c->h_topk, c->d_topk, g.topk * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+  INFLLM_CUDA_OK(cudaEventRecord(c->ev_sync, s));
+  return INFLLM_OK;
+}
+
+int retrieve_now(infllm_ctx* c, int eb_in_call, std::vector<int32_t>* ids, cudaStream_t s, bool launched) {
   const infllm_config& g = c->cfg;
   ids->clear();
   const int64_t n = c->chunk_mode ? c->chunk_n0 : c->num_blocks;
@@ -719,13 +754,7 @@ int retrieve_now(infllm_ctx* c, int eb_in_call, std::vector<int32_t>* ids, cudaS
     for (int64_t b = 0; b < n; ++b) ids->push_back((int32_t)b);
     return INFLLM_OK;
   }
-  INFLLM_TRY(ensure_scores(c, n, s));
-  {
-    ProfScope ps(c, s, INFLLM_PROF_TOPK, (double)n * c->width * c->esz);
-    INFLLM_TRY(score_topk(c, n, c->qbar + (int64_t)eb_in_call * c->width, c->scores, c->d_topk, s, 0));
-  }
-  INFLLM_CUDA_OK(cudaMemcpyAsync(c->h_topk, c->d_topk, g.topk * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-  INFLLM_CUDA_OK(cudaEventRecord(c->ev_sync, s));
+  if (!launched) INFLLM_TRY(retrieve_launch(c, eb_in_call, n, s));
   INFLLM_CUDA_OK(cudaEventSynchronize(c->ev_sync));  // the ids decide the cache plan (context_manager.py:163)
   ids->assign(c->h_topk, c->h_topk + g.topk);
   return INFLLM_OK;
@@ -755,8 +784,10 @@ int lookahead_launch(infllm_ctx* c, int64_t target, cudaStream_t s) {
   trace_mark(c, c->aux_stream, TR_SPEC_BEGIN, target);
   ProfScope ps(c, c->aux_stream, INFLLM_PROF_TOPK, (double)la.n_spec * c->width * c->esz);
   int32_t* d_ids = c->d_spec + (target % (c->look_depth + 1)) * std::max(1, g.topk);
-  INFLLM_TRY(score_topk(c, la.n_spec, c->qbar + target * c->width, c->scores_aux, d_ids, c->aux_stream, 1));
-  INFLLM_CUDA_OK(cudaMemcpyAsync(la.h_ids, d_ids, g.topk * sizeof(int32_t), cudaMemcpyDeviceToHost, c->aux_stream));
+  const bool direct = ids_direct(c, la.n_spec);
+  INFLLM_TRY(score_topk(c, la.n_spec, c->qbar + target * c->width, c->scores_aux, d_ids, c->aux_stream, 1, 0, direct ? la.h_ids : nullptr));
+  if (!direct)
+    INFLLM_CUDA_OK(cudaMemcpyAsync(la.h_ids, d_ids, g.topk * sizeof(int32_t), cudaMemcpyDeviceToHost, c->aux_stream));
   trace_mark(c, c->aux_stream, TR_SPEC_END, target);
   INFLLM_CUDA_OK(cudaEventRecord(la.ev, c->aux_stream));
   INFLLM_CUDA_OK(cudaEventRecord(c->ev_spec, c->aux_stream));
@@ -843,31 +874,20 @@ int lookahead_stage(infllm_ctx* c, int64_t target) {
   return INFLLM_OK;
 }
 
-// score the candidates of the next exec block (look-ahead ids + units sealed since) on s; results to pinned memory
-int candidates_launch(infllm_ctx* c, int64_t eb_next, int* n_cand, cudaStream_t s) {
+// the candidates of the next exec block once n_now units exist: what its look-ahead found, then the units sealed since.
+// *n_old of the *n exist already; none when every unit is retrieved anyway (context_manager.py:370-371).
+int candidates_list(infllm_ctx* c, int64_t eb_next, int64_t n_now, int* n_old, int* n) {
   const infllm_config& g = c->cfg;
   const infllm_ctx::LookAhead& la = c->la[eb_next % (c->look_depth + 1)];
-  const int64_t n_spec = la.n_spec;
-  const std::vector<int32_t>& spec_ids = la.ids;
-  const int64_t n_now = c->num_blocks;
-  *n_cand = 0;
-  if (n_now <= g.topk) return INFLLM_OK;  // all units, in id order, no scoring (context_manager.py:370-371)
-  int n = 0;
-  for (int32_t b : spec_ids) c->h_cand_rows[n++] = b;
-  for (int64_t b = n_spec; b < n_now && n < c->cand_cap; ++b) c->h_cand_rows[n++] = (int32_t)b;
-  if ((int64_t)spec_ids.size() + (n_now - n_spec) > c->cand_cap)
-    return fail(INFLLM_E_CAPACITY, "look-ahead: %lld candidates exceed %d", (long long)(spec_ids.size() + n_now - n_spec), c->cand_cap);
-  INFLLM_TRY(block_score_rows_launch(c->block_k, c->h_cand_rows, n, (int)c->width,
-                                     c->qbar + eb_next * c->width, c->d_cand_scores, g.dtype, s));
-  if (c->comm) INFLLM_TRY(comm_allreduce_sum(c->comm, 0, c->d_cand_scores, (size_t)n, s));
-  // the scores travel to the host on their own stream so that the main stream goes straight on
-  INFLLM_CUDA_OK(cudaEventRecord(c->ev_main, s));
-  INFLLM_CUDA_OK(cudaStreamWaitEvent(c->mail_stream, c->ev_main, 0));
-  INFLLM_CUDA_OK(cudaMemcpyAsync(c->h_cand_scores, c->d_cand_scores, n * sizeof(float), cudaMemcpyDeviceToHost,
-                                 c->mail_stream));
-  INFLLM_TRY(send_device_error(c, c->mail_stream, c->mail_stream));  // this exec block's attention is behind ev_main
-  INFLLM_CUDA_OK(cudaEventRecord(c->ev_cand, c->mail_stream));
-  *n_cand = n;
+  *n_old = *n = 0;
+  if (n_now <= g.topk) return INFLLM_OK;
+  if ((int64_t)la.ids.size() + (n_now - la.n_spec) > c->cand_cap)
+    return fail(INFLLM_E_CAPACITY, "look-ahead: %lld candidates exceed %d", (long long)(la.ids.size() + n_now - la.n_spec), c->cand_cap);
+  int k = 0;
+  for (int32_t b : la.ids) c->h_cand_rows[k++] = b;
+  for (int64_t b = la.n_spec; b < n_now; ++b) c->h_cand_rows[k++] = (int32_t)b;
+  *n = k;
+  *n_old = k - (int)(n_now - c->num_blocks);
   return INFLLM_OK;
 }
 
@@ -879,8 +899,8 @@ int candidates_finish(infllm_ctx* c, int n_cand, std::vector<int32_t>* ids) {
     for (int64_t b = 0; b < c->num_blocks; ++b) ids->push_back((int32_t)b);
     return INFLLM_OK;
   }
-  INFLLM_CUDA_OK(cudaEventSynchronize(c->ev_cand));
-  INFLLM_TRY(poll_device_error(c, c->mail_stream));
+  INFLLM_CUDA_OK(cudaEventSynchronize(c->comm ? c->ev_cand : c->ev_seal));
+  INFLLM_TRY(check_device_error(c, c->mail_stream));
   std::vector<int> order(n_cand);
   for (int i = 0; i < n_cand; ++i) order[i] = i;
   const int32_t* rows = c->h_cand_rows;
@@ -1177,7 +1197,10 @@ SealPlan plan_seal(const infllm_ctx* c, int64_t end) {
   return p;
 }
 
-int seal_apply(infllm_ctx* c, const SealPlan& sp, cudaStream_t s) {
+// Sealing, and, with eb_next >= 0, the scores of exec block eb_next's candidates in the same launch: *n_cand of them, on
+// their way to the host with ev_seal behind them.  When there is a next exec block this runs on seal_stream: what it reads -
+// keys, and the scores of tokens that have left every later query's window - the main stream does not write again.
+int seal_apply(infllm_ctx* c, const SealPlan& sp, int64_t eb_next, int* n_cand, cudaStream_t s) {
   const infllm_config& g = c->cfg;
   TokenBuffers& tb = c->tb;
   const int64_t D = g.head_dim, HKV = g.n_kv_heads, bs = g.block_size;
@@ -1193,15 +1216,46 @@ int seal_apply(infllm_ctx* c, const SealPlan& sp, cudaStream_t s) {
   }
   if (c->init_len == g.n_init) c->init_full = true;
   const int n_new = sp.n_new;
-  if (n_new == 0) return INFLLM_OK;
-  INFLLM_TRY(ensure_block_k(c, c->num_blocks + n_new, s));
-  INFLLM_TRY(ensure_host_units(c, c->num_blocks + n_new));
-  INFLLM_TRY(repr_select_launch(tb.k_raw, tb.cap * D, D, tb.score, tb.cap, c->frontier - tb.t0, n_new, (int)bs,
-                                g.repr_topk, g.n_heads, g.n_kv_heads, (int)D,
-                                (char*)c->block_k + c->num_blocks * c->width * c->esz, g.dtype, s));
+  const bool aside = eb_next >= 0 && !c->comm, grow = n_new > 0 && c->num_blocks + n_new > c->block_k_cap;
+  if (c->seal_aside && (!aside || grow)) INFLLM_CUDA_OK(cudaStreamWaitEvent(s, c->ev_seal, 0));
+  if (grow) INFLLM_TRY(ensure_block_k(c, c->num_blocks + n_new, s));
+  if (aside) {
+    INFLLM_CUDA_OK(cudaEventRecord(c->ev_urgent, s));
+    INFLLM_CUDA_OK(cudaStreamWaitEvent(c->seal_stream, c->ev_urgent, 0));
+    s = c->seal_stream;
+  }
+  c->seal_aside = aside;
+  int n_old = 0;
+  *n_cand = 0;
+  if (eb_next >= 0) INFLLM_TRY(candidates_list(c, eb_next, c->num_blocks + n_new, &n_old, n_cand));
+  const float* qbar = *n_cand > 0 ? c->qbar + eb_next * c->width : nullptr;
+  // the scores go straight to pinned memory, unless they are summed over ranks first
+  float* scores = c->comm ? c->d_cand_scores : c->h_cand_scores;
+  const int64_t tok0 = c->frontier - tb.t0;
+  if (seal_score_ok((int)bs, (int)D, tb.cap * D, D, tb.k_raw)) {
+    if (n_new > 0 || qbar)
+      INFLLM_TRY(seal_score_launch(tb.k_raw, tb.cap * D, D, tb.score, tb.cap, tok0, n_new, (int)c->num_blocks, (int)bs, g.repr_topk,
+                                   g.n_heads, g.n_kv_heads, (int)D, c->block_k, c->h_cand_rows, n_old, qbar, scores, c->tc_err,
+                                   qbar ? c->h_tc_err : nullptr, g.dtype, s));
+  } else {
+    INFLLM_TRY(repr_select_launch(tb.k_raw, tb.cap * D, D, tb.score, tb.cap, tok0, n_new, (int)bs, g.repr_topk, g.n_heads,
+                                  g.n_kv_heads, (int)D, (char*)c->block_k + c->num_blocks * c->width * c->esz, g.dtype, s));
+    if (qbar)  // every candidate exists by now
+      INFLLM_TRY(seal_score_launch(nullptr, 0, 0, nullptr, 0, 0, 0, 0, 1, 1, g.n_heads, g.n_kv_heads, (int)D, c->block_k, c->h_cand_rows,
+                                   *n_cand, qbar, scores, c->tc_err, c->h_tc_err, g.dtype, s));
+  }
   trace_mark(c, s, TR_REPR_END, c->num_blocks);
   c->num_blocks += n_new;
   c->frontier += n_new * bs;
+  if (qbar && c->comm) {
+    INFLLM_TRY(comm_allreduce_sum(c->comm, 0, c->d_cand_scores, (size_t)*n_cand, s));
+    INFLLM_CUDA_OK(cudaEventRecord(c->ev_main, s));
+    INFLLM_CUDA_OK(cudaStreamWaitEvent(c->mail_stream, c->ev_main, 0));
+    INFLLM_CUDA_OK(cudaMemcpyAsync(c->h_cand_scores, c->d_cand_scores, *n_cand * sizeof(float), cudaMemcpyDeviceToHost,
+                                   c->mail_stream));
+    INFLLM_CUDA_OK(cudaEventRecord(c->ev_cand, c->mail_stream));
+  }
+  if (eb_next >= 0) INFLLM_CUDA_OK(cudaEventRecord(c->ev_seal, s));
   return INFLLM_OK;
 }
 
@@ -1269,10 +1323,11 @@ int fill_dev_store(infllm_ctx* c, int64_t n_units) {
   return INFLLM_OK;
 }
 
-// second half of sealing: the new units' K/V go to the host store.  `first` is the id of the first new unit,
-// `tok0` its first token (absolute); called after the units were counted in.
+// first half of sealing: the new units' K/V go to the host store.  `first` is the id of the first new unit,
+// `tok0` its first token (absolute); called before the units are counted in.
 int seal_offload(infllm_ctx* c, int64_t first, int n_new, int64_t tok0, cudaStream_t s) {
   if (n_new <= 0) return INFLLM_OK;
+  INFLLM_TRY(ensure_host_units(c, first + n_new));
   const infllm_config& g = c->cfg;
   TokenBuffers& tb = c->tb;
   const int64_t D = g.head_dim, HKV = g.n_kv_heads, bs = g.block_size;
@@ -1390,6 +1445,8 @@ int append_sub(infllm_ctx* c, const char* q, int64_t q_hs, int64_t q_ts, const c
     }
   }
   // RoPE: keys keep the position (token - rope_origin) until the table would run out
+  if (c->chunk_mode && c->call_off % ((int64_t)(g.chunk_topk_calc / g.exc_block_size) * g.exc_block_size) == 0) c->chunk_n0 = c->num_blocks;
+  bool ranked = false;  // the first exec block's ids have been asked for
   const int64_t win0 = std::max<int64_t>(T - g.n_local, 0);  // oldest key any query of this call can see locally
   if (c->rope_origin < 0 || T + L - c->rope_origin > c->tab_len || win0 < c->rope_origin) {
     c->rope_origin = win0;
@@ -1407,21 +1464,42 @@ int append_sub(infllm_ctx* c, const char* q, int64_t q_hs, int64_t q_ts, const c
                                    c->d_miss));
     c->ingest_event_due = true;  // recorded when a sealing asks for it (seal_offload): one call less per token
   } else {
-    INFLLM_TRY(copy_rows_launch(k, k_hs, k_ts, (char*)tb.k_raw + at * D * esz, kv_hs, D, (int)HKV, L, (int)D, s));
-    INFLLM_TRY(copy_rows_launch(v, v_hs, v_ts, (char*)tb.v + at * D * esz, kv_hs, D, (int)HKV, L, (int)D, s));
-    INFLLM_CUDA_OK(cudaEventRecord(c->ev_ingest, s));
-    c->ingest_event_due = false;
-    INFLLM_CUDA_OK(cudaMemset2DAsync(tb.score + at, tb.cap * sizeof(float), 0, L * sizeof(float), H, s));
-    INFLLM_TRY(rope_apply_launch((char*)tb.k_raw + at * D * esz, kv_hs, D, (char*)tb.k_rot + at * D * esz, kv_hs, D,
-                                 (int)HKV, L, (int)D, c->cos_t, c->sin_t, c->tab_len, T - c->rope_origin, 1, g.dtype,
-                                 s));
-    // queries: window-relative rotation for the local stage, the single position n_local-1 for the
-    // global stage (context_manager.py:480 and :744-747)
-    INFLLM_TRY(rope_apply_launch(q, q_hs, q_ts, c->q_loc, q_hs_s, D, (int)H, L, (int)D, c->cos_t, c->sin_t, c->tab_len,
-                                 T - c->rope_origin, 1, g.dtype, s));
-    INFLLM_TRY(rope_apply_launch(q, q_hs, q_ts, c->q_glb, q_hs_s, D, (int)H, L, (int)D, c->cos_t, c->sin_t, c->tab_len,
-                                 g.n_local - 1, 0, g.dtype, s));
-    INFLLM_TRY(qbar_launch(c->q_glb, q_hs_s, D, (int)H, L, g.exc_block_size, (int)D, c->qbar, c->width, g.dtype, s));
+    const int64_t pos = T - c->rope_origin;
+    if (D == 128) {
+      auto ingest = [&](bool first_only) {
+        return ingest_rows_launch(q, q_hs, q_ts, k, k_hs, k_ts, v, v_hs, v_ts, c->q_loc, c->q_glb, q_hs_s, c->qbar, c->width,
+                                  (char*)tb.k_raw + at * D * esz, (char*)tb.k_rot + at * D * esz, (char*)tb.v + at * D * esz, kv_hs,
+                                  tb.score + at, tb.cap, (int)H, (int)HKV, L, g.exc_block_size, c->cos_t, c->sin_t, c->tab_len, pos,
+                                  g.n_local - 1, first_only, g.dtype, s);
+      };
+      // the first exec block's ids are on their way before the rest of the call is ingested: its missing units then
+      // cross PCIe beside that work
+      const int64_t n0 = c->chunk_mode ? c->chunk_n0 : c->num_blocks;
+      if (L > g.exc_block_size && n0 > g.topk) {
+        INFLLM_TRY(ingest(true));
+        INFLLM_TRY(retrieve_launch(c, 0, n0, s));
+        ranked = true;
+      }
+      INFLLM_TRY(ingest(false));
+      INFLLM_CUDA_OK(cudaEventRecord(c->ev_ingest, s));
+      c->ingest_event_due = false;
+    } else {
+      INFLLM_TRY(copy_rows_launch(k, k_hs, k_ts, (char*)tb.k_raw + at * D * esz, kv_hs, D, (int)HKV, L, (int)D, s));
+      INFLLM_TRY(copy_rows_launch(v, v_hs, v_ts, (char*)tb.v + at * D * esz, kv_hs, D, (int)HKV, L, (int)D, s));
+      INFLLM_CUDA_OK(cudaEventRecord(c->ev_ingest, s));
+      c->ingest_event_due = false;
+      INFLLM_CUDA_OK(cudaMemset2DAsync(tb.score + at, tb.cap * sizeof(float), 0, L * sizeof(float), H, s));
+      INFLLM_TRY(rope_apply_launch((char*)tb.k_raw + at * D * esz, kv_hs, D, (char*)tb.k_rot + at * D * esz, kv_hs, D,
+                                   (int)HKV, L, (int)D, c->cos_t, c->sin_t, c->tab_len, T - c->rope_origin, 1, g.dtype,
+                                   s));
+      // queries: window-relative rotation for the local stage, the single position n_local-1 for the
+      // global stage (context_manager.py:480 and :744-747)
+      INFLLM_TRY(rope_apply_launch(q, q_hs, q_ts, c->q_loc, q_hs_s, D, (int)H, L, (int)D, c->cos_t, c->sin_t, c->tab_len,
+                                   T - c->rope_origin, 1, g.dtype, s));
+      INFLLM_TRY(rope_apply_launch(q, q_hs, q_ts, c->q_glb, q_hs_s, D, (int)H, L, (int)D, c->cos_t, c->sin_t, c->tab_len,
+                                   g.n_local - 1, 0, g.dtype, s));
+      INFLLM_TRY(qbar_launch(c->q_glb, q_hs_s, D, (int)H, L, g.exc_block_size, (int)D, c->qbar, c->width, g.dtype, s));
+    }
   }
 
   // one-token appends whose retrieval has not been applied to the cache yet: a call that is not itself such a token
@@ -1467,13 +1545,13 @@ int append_sub(infllm_ctx* c, const char* q, int64_t q_hs, int64_t q_ts, const c
       if ((c->call_off + st) % chunk == 0) c->chunk_n0 = c->num_blocks;
     }
     const bool spec = run_ahead;
-    const bool ids_direct = !c->comm && g.topk <= 64 && c->num_blocks <= 16384;  // the scorer's one-launch form
+    const bool direct = ids_direct(c, c->num_blocks);
     cudaEvent_t token_ev = nullptr;
     int32_t* d_ids_tok = nullptr;  // the device-side ids of a run-ahead token
     if (!spec) {
       if (!have_ids) {
         HostTimer ht(&c->host_us[0]);
-        INFLLM_TRY(retrieve_now(c, eb, &ids, s));
+        INFLLM_TRY(retrieve_now(c, eb, &ids, s, ranked && eb == 0));
       }
       {
         HostTimer ht(&c->host_us[1]);
@@ -1490,9 +1568,9 @@ int append_sub(infllm_ctx* c, const char* q, int64_t q_hs, int64_t q_ts, const c
       d_ids_tok = c->d_topk_ring + (int64_t)slot * std::max(1, g.topk);
       {
         ProfScope ps(c, s, INFLLM_PROF_TOPK, (double)c->num_blocks * c->width * c->esz);
-        INFLLM_TRY(score_topk(c, c->num_blocks, c->qbar, c->scores, d_ids_tok, s, 0, g.topk, ids_direct ? pt.h_ids : nullptr));
+        INFLLM_TRY(score_topk(c, c->num_blocks, c->qbar, c->scores, d_ids_tok, s, 0, g.topk, direct ? pt.h_ids : nullptr));
       }
-      if (ids_direct) {
+      if (direct) {
         // the ranking threads wrote the ids into the pinned words themselves; the event that tells the host so is
         // recorded behind the token's last kernel, so that nothing stands between the kernels of the chain
         token_ev = pt.ev;
@@ -1694,9 +1772,13 @@ int append_sub(infllm_ctx* c, const char* q, int64_t q_hs, int64_t q_ts, const c
     }
 
     const SealPlan sp = plan_seal(c, E);
+    // The tokens about to be sealed are final: their units leave for the host store now, under the attention, so that
+    // the link is free again when the candidates' scores come back over it.
+    const int64_t first_new = c->num_blocks, tok_new = c->frontier + sp.take;
+    INFLLM_TRY(seal_offload(c, first_new, sp.n_new, tok_new, s));
     // accumulated local score of every window key (context_manager.py:488, 623-625).  Sealing only needs
     // the scores of the tokens it is about to seal, so their 128-key tiles go first; the rest of the
-    // window follows behind the sealing and overlaps the host's cache planning for the next exec block.
+    // window runs beside the sealing and overlaps the host's cache planning for the next exec block.
     int64_t j_u = 0;
     if (!decode_path) {
       j_u = std::min<int64_t>(lk, std::max<int64_t>(sp.new_frontier - ks, 0));
@@ -1705,23 +1787,18 @@ int append_sub(infllm_ctx* c, const char* q, int64_t q_hs, int64_t q_ts, const c
       INFLLM_TRY(local_scores(c, s, st, ks, lq, lk, 0, j_u, local_pairs_eb));
     }
     trace_mark(c, s, TR_URGENT_END, eb);
-    if (more) {
+    auto stage = [&](int d) -> int {  // refill copies for exec block eb + d, once its look-ahead is back
+      const int64_t tgt = eb + d;
+      infllm_ctx::LookAhead& la = c->la[tgt % (c->look_depth + 1)];
       HostTimer ht(&c->host_us[4]);
-      for (int d = 1; d <= c->look_depth; ++d) {
-        const int64_t tgt = eb + d;
-        infllm_ctx::LookAhead& la = c->la[tgt % (c->look_depth + 1)];
-        if (tgt < n_eb && la.launched && la.target == tgt && !la.staged) INFLLM_TRY(lookahead_stage(c, tgt));
-      }
-    }
-    const int64_t first_new = c->num_blocks, tok_new = c->frontier + sp.take;
+      return tgt < n_eb && la.launched && la.target == tgt && !la.staged ? lookahead_stage(c, tgt) : INFLLM_OK;
+    };
+    if (more) INFLLM_TRY(stage(1));  // the candidates contain its ids (back since the last exec block, as a rule)
     {
       HostTimer ht(&c->host_us[5]);
-      INFLLM_TRY(seal_apply(c, sp, s));
-      if (more) INFLLM_CUDA_OK(cudaEventRecord(c->ev_seal, s));
+      INFLLM_TRY(seal_apply(c, sp, more ? eb + 1 : -1, &n_cand, s));
     }
-    if (more) INFLLM_TRY(candidates_launch(c, eb + 1, &n_cand, s));
     trace_mark(c, s, TR_SEAL_END, eb);
-    INFLLM_TRY(seal_offload(c, first_new, sp.n_new, tok_new, s));  // off the ranking's critical path
     if (L == 1 && sp.n_new > 0) {
       // a one-token attention finds a unit through the table of unit addresses: the new units are listed at their
       // place in the store, which the copy-out must have reached first (once per block_size tokens)
@@ -1731,6 +1808,8 @@ int append_sub(infllm_ctx* c, const char* q, int64_t q_hs, int64_t q_ts, const c
     }
     if (!decode_path) INFLLM_TRY(local_scores(c, s, st, ks, lq, lk, j_u, lk, 0.0));
     trace_mark(c, s, TR_REST_END, eb);
+    if (more)  // behind every launch of this exec block: the host waits for the look-ahead here
+      for (int d = 2; d <= c->look_depth; ++d) INFLLM_TRY(stage(d));
     have_ids = false;
     if (more) {
       HostTimer ht(&c->host_us[6]);
@@ -1751,13 +1830,13 @@ int append_sub(infllm_ctx* c, const char* q, int64_t q_hs, int64_t q_ts, const c
 static int ctx_reset(infllm_ctx* c, bool wait) {
   if (c->initialized) {
     INFLLM_CUDA_OK(cudaSetDevice(c->cfg.device));
-    cudaStream_t side[5] = {c->copy_stream, c->urgent_stream, c->aux_stream, c->d2h_stream, c->mail_stream};
+    cudaStream_t side[6] = {c->copy_stream, c->urgent_stream, c->aux_stream, c->d2h_stream, c->mail_stream, c->seal_stream};
     if (wait || !c->dev_slabs.empty()) {
       for (cudaStream_t s : side) INFLLM_CUDA_OK(cudaStreamSynchronize(s));
       if (c->attn_recorded) INFLLM_CUDA_OK(cudaEventSynchronize(c->ev_attn));
       if (c->last_recorded) INFLLM_CUDA_OK(cudaEventSynchronize(c->ev_last));
     } else {
-      for (int i = 0; i < 5; ++i) INFLLM_CUDA_OK(cudaEventRecord(c->ev_side[i], side[i]));
+      for (int i = 0; i < 6; ++i) INFLLM_CUDA_OK(cudaEventRecord(c->ev_side[i], side[i]));
       // (marks of an earlier reset that no append has followed still stand)
       c->reset_attn = c->attn_recorded || (c->reset_pending && c->reset_attn);
       c->reset_last = c->last_recorded || (c->reset_pending && c->reset_last);
@@ -1793,6 +1872,7 @@ static int ctx_reset(infllm_ctx* c, bool wait) {
   c->attn_recorded = false;
   c->attn_prev_recorded = false;
   c->spec_recorded = false;
+  c->seal_aside = false;
   c->last_recorded = false;
   c->counters = infllm_ctx_info{};
   return INFLLM_OK;
@@ -1838,6 +1918,8 @@ static void ctx_free(infllm_ctx* c) {
     if (c->tc_part) cudaFreeAsync(c->tc_part, nullptr);
     cudaStreamDestroy(c->aux_stream);
     cudaStreamDestroy(c->mail_stream);
+    cudaStreamDestroy(c->seal_stream);
+    cudaEventDestroy(c->ev_urgent);
     if (c->d_cand_scores) cudaFree(c->d_cand_scores);
     if (c->d_spec) cudaFree(c->d_spec);
     cudaStreamDestroy(c->d2h_stream);
@@ -2042,6 +2124,10 @@ extern "C" int infllm_ctx_append(infllm_ctx* c, const void* d_q, int64_t q_hs, i
   INFLLM_TRY(order_behind_reset(c, s));
   INFLLM_TRY(poll_device_error(c, s));
   c->failed = true;  // until the call has gone through
+  if (c->seal_aside) {  // a call that gave up half-way left it so
+    INFLLM_CUDA_OK(cudaStreamWaitEvent(s, c->ev_seal, 0));
+    c->seal_aside = false;
+  }
   c->call_serial += 1;
   c->last_stream = s;
   c->trace_topk.clear();
@@ -2056,7 +2142,7 @@ extern "C" int infllm_ctx_append(infllm_ctx* c, const void* d_q, int64_t q_hs, i
                           k_ts, (const char*)d_v + off * v_ts * esz, v_hs, v_ts, (char*)d_out + off * o_ts * esz, o_hs,
                           o_ts, n, s));
   }
-  if (c->use_tc && len > 64) INFLLM_TRY(send_device_error(c, s, s));  // read by the next call (or by get_info)
+  if (c->use_tc && len > 64) INFLLM_TRY(send_device_error(c, s));  // read by the next call (or by get_info)
   if (len > 1 || c->num_blocks != units_before) {  // a token that seals nothing ends with its attention: ev_attn
     INFLLM_CUDA_OK(cudaEventRecord(c->ev_last, s));
     c->last_recorded = true;

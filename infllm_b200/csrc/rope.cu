@@ -57,6 +57,16 @@ __global__ void rope_apply_kernel(const T* __restrict__ x, int64_t x_hs, int64_t
   *reinterpret_cast<uint4*>(dst + half) = ohi;
 }
 
+// four words to pinned host memory: a copy of them would queue behind the units on their way to the host
+__global__ void mail_words_kernel(const int32_t* __restrict__ src, int32_t* __restrict__ dst) {
+  if (threadIdx.x < 4) dst[threadIdx.x] = src[threadIdx.x];
+}
+int mail_words_launch(const int32_t* src, int32_t* dst, cudaStream_t s) {
+  mail_words_kernel<<<1, 32, 0, s>>>(src, dst);
+  INFLLM_LAUNCH_OK("mail_words_kernel");
+  return INFLLM_OK;
+}
+
 // plain strided row copy (H, L, D) -> (H, L, D), 16 bytes per thread
 template <typename T>
 __global__ void copy_rows_kernel(const T* __restrict__ x, int64_t x_hs, int64_t x_ts, T* __restrict__ out,
@@ -84,6 +94,130 @@ __global__ void qbar_kernel(const T* __restrict__ q, int64_t q_hs, int64_t q_ts,
   const T* p = q + h * q_hs + d;
   for (int64_t t = st; t < ed; ++t) acc += Act<T>::to_f(p[t * q_ts]);
   qbar[e * qbar_stride + (int64_t)h * head_dim + d] = acc / (float)(ed - st);
+}
+
+// The tokens of a call, in one pass over them: K and V into the token buffers, K also rotated, Q rotated both ways, the
+// accumulated-score columns cleared and the query means of the exec blocks formed (of the rounded one-angle rotations,
+// in a fixed order).  CTA (e, h) of the first part takes exec block e of query head h, 32 rows of eight threads at a
+// time, and keeps the sums in registers; the CTAs behind them take 32 rows of a KV head each.  HBM-bound: 285 MB per 8192
+// tokens of 32 + 2 x 8 heads, 62 us; as copies, rotations, a clear and a reduction of their own they took 155 us.
+constexpr int kIngestThreads = 256, kIngestRows = kIngestThreads / 8;
+template <typename T>
+struct IngestArgs {
+  const T *q, *k, *v;
+  T *q_loc, *q_glb, *k_raw, *k_rot, *v_out;
+  float *qbar, *score;
+  const float *cos_t, *sin_t;
+  int64_t q_hs, q_ts, k_hs, k_ts, v_hs, v_ts, qs_hs, kv_hs, score_hs, qbar_stride, pos_loc, pos_glb;
+  int32_t len, exc, n_heads, n_kv, n_eb, kv_tiles;
+};
+__device__ __forceinline__ void load8(const float* p, float* x) {
+  const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
+  x[0] = a.x, x[1] = a.y, x[2] = a.z, x[3] = a.w, x[4] = b.x, x[5] = b.y, x[6] = b.z, x[7] = b.w;
+}
+template <typename T>
+__device__ __forceinline__ void rotate8(const uint4& lo, const uint4& hi, const float* cs, const float* sn, uint4* olo, uint4* ohi) {
+  const T *a = reinterpret_cast<const T*>(&lo), *b = reinterpret_cast<const T*>(&hi);
+  T *oa = reinterpret_cast<T*>(olo), *ob = reinterpret_cast<T*>(ohi);
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const float x1 = Act<T>::to_f(a[i]), x2 = Act<T>::to_f(b[i]);
+    oa[i] = Act<T>::from_f(__fadd_rn(__fmul_rn(x1, cs[i]), __fmul_rn(-x2, sn[i])));
+    ob[i] = Act<T>::from_f(__fadd_rn(__fmul_rn(x2, cs[i]), __fmul_rn(x1, sn[i])));
+  }
+}
+template <typename T>
+__global__ void __launch_bounds__(kIngestThreads) ingest_rows_kernel(const __grid_constant__ IngestArgs<T> A) {
+  __shared__ float s_sum[kIngestRows / 4][128];
+  const int tid = threadIdx.x, c = tid & 7, r = tid >> 3, lane = tid & 31, warp = tid >> 5;
+  const int n_q = A.n_eb * A.n_heads;
+  if ((int)blockIdx.x < n_q) {
+    const int h = blockIdx.x % A.n_heads, e = blockIdx.x / A.n_heads;
+    const int st = e * A.exc, ed = min(A.len, st + A.exc);
+    float cg[8], sg[8], sum[16];
+    load8(A.cos_t + A.pos_glb * 64 + c * 8, cg);
+    load8(A.sin_t + A.pos_glb * 64 + c * 8, sg);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) sum[i] = 0.f;
+#pragma unroll 2
+    for (int t = st + r; t < ed; t += kIngestRows) {
+      const T* src = A.q + h * A.q_hs + (int64_t)t * A.q_ts + c * 8;
+      const uint4 lo = __ldcs(reinterpret_cast<const uint4*>(src)), hi = __ldcs(reinterpret_cast<const uint4*>(src + 64));
+      float cs[8], sn[8];
+      load8(A.cos_t + (A.pos_loc + t) * 64 + c * 8, cs);
+      load8(A.sin_t + (A.pos_loc + t) * 64 + c * 8, sn);
+      uint4 a, b;
+      T* dl = A.q_loc + h * A.qs_hs + (int64_t)t * 128 + c * 8;
+      rotate8<T>(lo, hi, cs, sn, &a, &b);
+      *reinterpret_cast<uint4*>(dl) = a;
+      *reinterpret_cast<uint4*>(dl + 64) = b;
+      T* dg = A.q_glb + h * A.qs_hs + (int64_t)t * 128 + c * 8;
+      rotate8<T>(lo, hi, cg, sg, &a, &b);
+      *reinterpret_cast<uint4*>(dg) = a;
+      *reinterpret_cast<uint4*>(dg + 64) = b;
+      const T *xa = reinterpret_cast<const T*>(&a), *xb = reinterpret_cast<const T*>(&b);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) sum[i] += Act<T>::to_f(xa[i]), sum[8 + i] += Act<T>::to_f(xb[i]);
+    }
+    // the four rows of a warp, then the warps
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      sum[i] += __shfl_xor_sync(0xffffffffu, sum[i], 8);
+      sum[i] += __shfl_xor_sync(0xffffffffu, sum[i], 16);
+    }
+    if (lane < 8)
+#pragma unroll
+      for (int i = 0; i < 8; ++i) s_sum[warp][c * 8 + i] = sum[i], s_sum[warp][64 + c * 8 + i] = sum[8 + i];
+    __syncthreads();
+    if (tid < 128) {
+      float x = 0.f;
+#pragma unroll
+      for (int w = 0; w < kIngestThreads / 32; ++w) x += s_sum[w][tid];
+      A.qbar[e * A.qbar_stride + (int64_t)h * 128 + tid] = x / (float)(ed - st);
+    }
+    if (A.kv_tiles)  // not in a launch that takes the first exec block's queries only
+      for (int t = st + tid; t < ed; t += kIngestThreads) A.score[h * A.score_hs + t] = 0.f;
+    return;
+  }
+  const int b = blockIdx.x - n_q, h = b / A.kv_tiles, t = (b - h * A.kv_tiles) * kIngestRows + r;
+  if (t >= A.len) return;
+  const T *ks = A.k + h * A.k_hs + (int64_t)t * A.k_ts + c * 8, *vs = A.v + h * A.v_hs + (int64_t)t * A.v_ts + c * 8;
+  const uint4 k0 = __ldcs(reinterpret_cast<const uint4*>(ks)), k1 = __ldcs(reinterpret_cast<const uint4*>(ks + 64));
+  const uint4 v0 = __ldcs(reinterpret_cast<const uint4*>(vs)), v1 = __ldcs(reinterpret_cast<const uint4*>(vs + 64));
+  float cs[8], sn[8];
+  load8(A.cos_t + (A.pos_loc + t) * 64 + c * 8, cs);
+  load8(A.sin_t + (A.pos_loc + t) * 64 + c * 8, sn);
+  const int64_t at = h * A.kv_hs + (int64_t)t * 128 + c * 8;
+  uint4 a, d;
+  rotate8<T>(k0, k1, cs, sn, &a, &d);
+  *reinterpret_cast<uint4*>(A.k_raw + at) = k0;
+  *reinterpret_cast<uint4*>(A.k_raw + at + 64) = k1;
+  *reinterpret_cast<uint4*>(A.k_rot + at) = a;
+  *reinterpret_cast<uint4*>(A.k_rot + at + 64) = d;
+  *reinterpret_cast<uint4*>(A.v_out + at) = v0;
+  *reinterpret_cast<uint4*>(A.v_out + at + 64) = v1;
+}
+
+// head_dim 128 only.  first_only: only the queries of the first exec block and its mean (nothing else is written).
+int ingest_rows_launch(const void* q, int64_t q_hs, int64_t q_ts, const void* k, int64_t k_hs, int64_t k_ts, const void* v,
+                       int64_t v_hs, int64_t v_ts, void* q_loc, void* q_glb, int64_t qs_hs, float* qbar, int64_t qbar_stride,
+                       void* k_raw, void* k_rot, void* v_out, int64_t kv_hs, float* score, int64_t score_hs, int n_heads,
+                       int n_kv_heads, int64_t len, int exc, const float* cos_t, const float* sin_t, int64_t table_len,
+                       int64_t pos_loc, int64_t pos_glb, bool first_only, int dtype, cudaStream_t s) {
+  if (pos_loc < 0 || pos_loc + len > table_len || pos_glb < 0 || pos_glb >= table_len)
+    return fail(INFLLM_E_BADARG, "ingest: positions %lld..%lld / %lld outside the table of %lld rows", (long long)pos_loc,
+                (long long)(pos_loc + len - 1), (long long)pos_glb, (long long)table_len);
+  if ((q_hs | q_ts | k_hs | k_ts | v_hs | v_ts) % 8 || ((uintptr_t)q | (uintptr_t)k | (uintptr_t)v) % 16)
+    return fail(INFLLM_E_BADARG, "ingest: rows must be 16-byte aligned");
+  const int n_eb = first_only ? 1 : (int)ceil_div(len, exc), kv_tiles = first_only ? 0 : (int)ceil_div(len, kIngestRows);
+  INFLLM_DISPATCH_DTYPE(dtype, T, {
+    IngestArgs<T> A{(const T*)q, (const T*)k, (const T*)v, (T*)q_loc, (T*)q_glb, (T*)k_raw, (T*)k_rot, (T*)v_out, qbar, score,
+                    cos_t, sin_t, q_hs, q_ts, k_hs, k_ts, v_hs, v_ts, qs_hs, kv_hs, score_hs, qbar_stride, pos_loc, pos_glb,
+                    (int)len, exc, n_heads, n_kv_heads, n_eb, kv_tiles};
+    ingest_rows_kernel<T><<<n_eb * n_heads + n_kv_heads * kv_tiles, kIngestThreads, 0, s>>>(A);
+  });
+  INFLLM_LAUNCH_OK("ingest_rows_kernel");
+  return INFLLM_OK;
 }
 
 // K and V of n_new consecutive units -> the host store's unit layout [unit][K|V][head][token][d], contiguous,
