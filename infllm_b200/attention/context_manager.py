@@ -142,8 +142,10 @@ class ContextManager:
         """context_manager.py:682-813.  q (B, H, L, D); k, v (B, H_kv, L, D); returns (B, H, L, D).
         The global tensors must be the local ones (inf_llm/attention/inf_llm.py:58-59 passes the same
         projections twice); the kernels rotate them per stage themselves."""
-        if self.initialized and local_q.shape[2] == 1 and not self.perhead and local_q.shape[0] == 1 and local_q.is_cuda:
-            return self._append_token(local_q, local_k, local_v, global_q)
+        if self.initialized and local_q.dim() == 4 and local_q.size(2) == 1 and local_q.is_cuda and not self.perhead:
+            out = self._append_token(local_q, local_k, local_v, global_q)
+            if out is not None:
+                return out
         for t in (local_q, local_k, local_v):
             _lib.require_cuda(t, "ContextManager.append input")
         if global_q is not local_q and global_q.data_ptr() != local_q.data_ptr():
@@ -161,42 +163,53 @@ class ContextManager:
         if k.stride(-1) != 1 or k.stride() != v.stride():
             k, v = k.contiguous(), v.contiguous()
         out = torch.empty((batch, heads, length, dim), dtype=q.dtype, device=q.device)
-        stream = _lib.stream_ptr(q.device)
-        if self.perhead:
-            g = heads // self.num_heads_kv
-            for b in range(batch):
-                for h in range(heads):
-                    qq, kk, vv, oo = q[b, h:h + 1], k[b, h // g:h // g + 1], v[b, h // g:h // g + 1], out[b, h:h + 1]
-                    self._append_unit(self._ctx[b * heads + h], qq, kk, vv, oo, length, stream)
-        else:
-            for b in range(batch):
-                self._append_unit(self._ctx[b], q[b], k[b], v[b], out[b], length, stream)
+        self._append_units(q, k, v, out, length)
         self.length += length
         return out
 
     def _append_token(self, q, k, v, global_q):
-        """One token of one sequence: the same call with the checks that cannot fail for this shape left out (the
-        host's share of a decode step is a few tens of microseconds, of the order of the GPU's)."""
+        """One token of every sequence: the same call with the checks that cannot fail for this shape left out (the
+        host's share of a decode step is of the order of the GPU's).  None: the general path has to copy something."""
         if global_q is not q and global_q.data_ptr() != q.data_ptr():
             raise NotImplementedError("distinct global_q/k/v tensors are not supported: pass the local ones")
-        if q.shape[1] != self.num_heads or k.shape[1] != self.num_heads_kv or q.dtype != self.dtype or \
-                q.stride(-1) != 1 or k.stride(-1) != 1 or k.stride() != v.stride() or not (k.is_cuda and v.is_cuda):
+        batch, heads, _, dim = shape = q.shape
+        ks = k.stride()
+        if heads != self.num_heads or batch != self.batch_size or k.shape != (batch, self.num_heads_kv, 1, dim) or \
+                v.shape != k.shape or q.dtype != self.dtype or k.dtype != self.dtype or v.dtype != self.dtype or \
+                q.stride(3) != 1 or ks[3] != 1 or ks != v.stride() or not (k.is_cuda and v.is_cuda):
+            if batch > 1:
+                return None
             raise ValueError("ContextManager.append: a one-token call with other shapes, strides or dtype than the memory's")
-        out = torch.empty_like(q, memory_format=torch.contiguous_format)
-        rc = _lib.lib.infllm_ctx_append(
-            self._ctx[0], q.data_ptr(), q.stride(1), q.stride(2), k.data_ptr(), k.stride(1), k.stride(2), v.data_ptr(),
-            v.stride(1), v.stride(2), out.data_ptr(), out.stride(1), out.stride(2), 1,
-            torch.cuda.current_stream(q.device).cuda_stream)
-        if rc:
-            _lib.check(rc)
+        out = torch.empty(shape, dtype=q.dtype, device=q.device)
+        self._append_units(q, k, v, out, 1)
         self.length += 1
         return out
 
-    @staticmethod
-    def _append_unit(ctx, q, k, v, o, length, stream):
-        _lib.check(_lib.lib.infllm_ctx_append(
-            ctx, q.data_ptr(), q.stride(0), q.stride(1), k.data_ptr(), k.stride(0), k.stride(1), v.data_ptr(),
-            v.stride(0), v.stride(1), o.data_ptr(), o.stride(0), o.stride(1), length, stream))
+    def _append_units(self, q, k, v, out, length):
+        """One native call per unit (sequence, or head of a sequence); addresses by arithmetic, 2 bytes per element."""
+        append, stream = _lib.lib.infllm_ctx_append, torch.cuda.current_stream(q.device).cuda_stream
+        q_bs, q_hs, q_ts, _ = q.stride()
+        k_bs, k_hs, k_ts, _ = k.stride()
+        o_bs, o_hs, o_ts, _ = out.stride()
+        q_at, k_at, v_at, o_at = q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr()
+        rc = 0
+        if self.perhead:
+            heads, g = self.num_heads, self.num_heads // self.num_heads_kv
+            for i, ctx in enumerate(self._ctx):
+                b, h = divmod(i, heads)
+                kv = 2 * (b * k_bs + h // g * k_hs)
+                rc = append(ctx, q_at + 2 * (b * q_bs + h * q_hs), q_hs, q_ts, k_at + kv, k_hs, k_ts, v_at + kv, k_hs, k_ts,
+                            o_at + 2 * (b * o_bs + h * o_hs), o_hs, o_ts, length, stream)
+                if rc:
+                    break
+        else:
+            for b, ctx in enumerate(self._ctx):
+                rc = append(ctx, q_at + 2 * b * q_bs, q_hs, q_ts, k_at + 2 * b * k_bs, k_hs, k_ts, v_at + 2 * b * k_bs, k_hs,
+                            k_ts, o_at + 2 * b * o_bs, o_hs, o_ts, length, stream)
+                if rc:
+                    break
+        if rc:
+            _lib.check(rc)
 
     def size(self, *args, **kwargs):
         return self.length

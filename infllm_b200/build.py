@@ -12,7 +12,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libinfllm_b200.so")
 SOURCES = ["error.cu", "rope.cu", "retrieval.cu", "attn_general.cu", "attn_decode.cu", "attn_tc.cu", "context.cu",
-           "comm.cu", "sink_window.cu"]
+           "comm.cu", "sink_window.cu", "token.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
     "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr",

@@ -22,6 +22,7 @@
 
 #include "attn_common.cuh"
 #include "attn_tc.cuh"
+#include "token.cuh"
 
 struct infllm_comm;  // comm.cu
 
@@ -214,7 +215,9 @@ struct infllm_ctx {
   // appended — or when somebody asks for the tables.  Ring of the tokens whose ids have not been applied yet.
   struct PendingToken {
     int32_t* h_ids = nullptr;  // pinned: topk ids
-    cudaEvent_t ev = nullptr;  // on the mail stream, behind the copy of the ids
+    unsigned long long* h_words = nullptr;  // pinned, one-launch tokens: {id, seq} words, read as they arrive
+    uint32_t seq = 0;          // != 0: the ids are in h_words and carry this number
+    cudaEvent_t ev = nullptr;  // seq == 0: behind the ids
     int64_t serial = 0;        // the append call it belongs to
     std::vector<int32_t> listed;  // units the device table showed in a cache slot when the token was launched
     std::vector<int> landing;     // the landing slot of every retrieval position at that time (-1: none)
@@ -230,6 +233,13 @@ struct infllm_ctx {
   PendingToken pend[kPendSlots];
   int pend_head = 0, pend_count = 0;
   int32_t* d_topk_ring = nullptr;  // kPendSlots x topk
+  // one-launch tokens (token.cu): the words its CTAs exchange, and how many tokens have used them
+  unsigned long long *tok_scores = nullptr, *tok_ids = nullptr, *tok_parts = nullptr;
+  int64_t tok_scores_cap = 0;
+  size_t tok_part_words = 0;
+  int tok_sms = 0;  // SMs of the device
+  uint32_t tok_seq = 0;
+  bool tok_restart = false;  // a token gave up, or the numbers are used up: the words start again
   int64_t call_serial = 0;
   cudaStream_t last_stream = nullptr;  // stream of the last append (for calls that take none)
   std::vector<void*> slabs;  // pinned host memory
@@ -504,9 +514,12 @@ int lazy_init(infllm_ctx* c, cudaStream_t s) {
     INFLLM_CUDA_OK(dev_malloc((void**)&c->d_topk_ring, (size_t)infllm_ctx::kPendSlots * per * sizeof(int32_t)));
     for (auto& pt : c->pend) {
       INFLLM_CUDA_OK(cudaHostAlloc((void**)&pt.h_ids, per * sizeof(int32_t), cudaHostAllocDefault));
+      INFLLM_CUDA_OK(cudaHostAlloc((void**)&pt.h_words, per * sizeof(unsigned long long), cudaHostAllocDefault));
+      memset(pt.h_words, 0, per * sizeof(unsigned long long));
       INFLLM_CUDA_OK(cudaEventCreateWithFlags(&pt.ev, cudaEventDisableTiming));
     }
   }
+  INFLLM_CUDA_OK(cudaDeviceGetAttribute(&c->tok_sms, cudaDevAttrMultiProcessorCount, g.device));
   INFLLM_CUDA_OK(dev_malloc((void**)&c->tickets, 2 * sizeof(unsigned int)));
   INFLLM_CUDA_OK(cudaMemsetAsync(c->tickets, 0, 2 * sizeof(unsigned int), s));
   INFLLM_CUDA_OK(cudaHostAlloc((void**)&c->h_topk, std::max(1, g.topk) * sizeof(int32_t),
@@ -593,6 +606,7 @@ int check_device_error(infllm_ctx* c, cudaStream_t s) {
   if (!c->h_tc_err || c->h_tc_err[0] == 0) return INFLLM_OK;
   const int code = c->h_tc_err[0], where = c->h_tc_err[1], bx = c->h_tc_err[2], by = c->h_tc_err[3];
   c->h_tc_err[0] = 0;
+  c->tok_restart = true;
   INFLLM_CUDA_OK(cudaMemsetAsync(c->tc_err, 0, 4 * sizeof(int32_t), s));
   return fail(INFLLM_E_TIMEOUT, "a bounded wait of a tensor-core kernel ran out (code %d, wait %d, CTA %d,%d): the rows "
               "that CTA was to write are not valid", code, where, bx, by);
@@ -1068,8 +1082,9 @@ int plan_and_refill(infllm_ctx* c, const std::vector<int32_t>& ids, int64_t eb, 
   return INFLLM_OK;
 }
 
-// bring the device table of unit addresses up to date on stream s
-int flush_table(infllm_ctx* c, cudaStream_t s) {
+// bring the device table of unit addresses up to date on stream s; with `tok` the changes travel with that token's launch
+// when they fit
+int flush_table(infllm_ctx* c, cudaStream_t s, TokenParams* tok = nullptr) {
   const int topk = c->cfg.topk;
   if (c->tab_cap < c->block_k_cap || !c->d_unit_ptrs) {
     if (c->d_unit_ptrs) INFLLM_CUDA_OK(cudaFreeAsync(c->d_unit_ptrs, s));
@@ -1133,7 +1148,35 @@ int flush_table(infllm_ctx* c, cudaStream_t s) {
   }
   c->tab_updates.clear();
   if (ids.empty()) return INFLLM_OK;
+  if (tok && ids.size() <= (size_t)kTokMaxUpdates) {
+    tok->n_upd = (int)ids.size();
+    std::copy(ids.begin(), ids.end(), tok->upd_id);
+    std::copy(vals.begin(), vals.end(), tok->upd_val);
+    return INFLLM_OK;
+  }
   return ptr_table_update_launch(c->d_unit_ptrs, ids.data(), vals.data(), (int)ids.size(), s);
+}
+
+// The ids of a one-launch token, as its ranking threads write them: long before the token is through, so that the host
+// prepares the next one under its attention.  Bounded: the kernel's own waits end after a second or two and leave the
+// error record; the rest of the limit is for work ahead of the token on its stream.
+int wait_words(infllm_ctx* c, infllm_ctx::PendingToken& p) {
+  const int k = c->cfg.topk;
+  const auto t0 = std::chrono::steady_clock::now();
+  for (int i = 0; i < k;) {
+    const unsigned long long w = *(volatile unsigned long long*)(p.h_words + i);
+    if ((uint32_t)(w >> 32) == p.seq) {
+      p.h_ids[i++] = (int32_t)(uint32_t)w;
+      continue;
+    }
+    for (int spin = 0; spin < 64; ++spin) __builtin_ia32_pause();
+    if (*(volatile int32_t*)c->h_tc_err) INFLLM_TRY(check_device_error(c, c->last_stream));
+    if (std::chrono::steady_clock::now() - t0 > std::chrono::seconds(60)) {
+      c->tok_restart = true;
+      return fail(INFLLM_E_TIMEOUT, "the retrieved ids of a token did not arrive");
+    }
+  }
+  return INFLLM_OK;
 }
 
 // Apply the oldest pending retrieval of a one-token append to the cache: wait for its ids (they left the device
@@ -1144,7 +1187,11 @@ int settle_one(infllm_ctx* c, cudaStream_t s) {
   infllm_ctx::PendingToken& p = c->pend[c->pend_head];
   {
     HostTimer ht(&c->host_us[0]);
-    INFLLM_CUDA_OK(cudaEventSynchronize(p.ev));
+    if (p.seq != 0) {
+      INFLLM_TRY(wait_words(c, p));
+    } else {
+      INFLLM_CUDA_OK(cudaEventSynchronize(p.ev));
+    }
   }
   std::vector<int32_t> ids(p.h_ids, p.h_ids + g.topk);
   // the units that token's attention did not find in a cache slot were read in place and sit in the landing slots
@@ -1419,6 +1466,65 @@ int unit_score_update(infllm_ctx* c, const std::vector<int32_t>& ids, const char
   return INFLLM_OK;
 }
 
+// A one-token append as one launch: ingestion, retrieval, attention and merge (token.cu).  S is the token's absolute
+// index, `at` its slot in the token buffers; the ids go, marked, to pt.h_words.
+int token_whole(infllm_ctx* c, infllm_ctx::PendingToken& pt, int runs, const char* q, int64_t q_hs, const char* k, int64_t k_hs,
+                const char* v, int64_t v_hs, char* out, int64_t o_hs, int64_t at, int64_t S, cudaStream_t s) {
+  const infllm_config& g = c->cfg;
+  TokenBuffers& tb = c->tb;
+  const int64_t D = g.head_dim, kv_hs = tb.cap * D, wsz = sizeof(unsigned long long);
+  const int esz = c->esz;
+  TokenParams P;
+  P.n_upd = 0;
+  INFLLM_TRY(flush_table(c, s, &P));
+  if (!c->tok_ids) {
+    c->tok_part_words = (size_t)runs * g.n_heads * 129;
+    INFLLM_CUDA_OK(dev_malloc((void**)&c->tok_ids, g.topk * wsz));
+    INFLLM_CUDA_OK(dev_malloc((void**)&c->tok_parts, c->tok_part_words * wsz));
+    c->tok_restart = true;
+  }
+  if (c->tok_scores_cap < c->num_blocks) {
+    if (c->tok_scores) INFLLM_CUDA_OK(cudaFreeAsync(c->tok_scores, s));
+    c->tok_scores = nullptr;
+    c->tok_scores_cap = 0;
+    INFLLM_CUDA_OK(dev_malloc_async((void**)&c->tok_scores, std::max<int64_t>(c->block_k_cap, 1024) * wsz, s));
+    c->tok_scores_cap = std::max<int64_t>(c->block_k_cap, 1024);
+    c->tok_restart = true;
+  }
+  if (c->tok_restart) {  // no word carries a number any more
+    INFLLM_CUDA_OK(cudaMemsetAsync(c->tok_scores, 0, c->tok_scores_cap * wsz, s));
+    INFLLM_CUDA_OK(cudaMemsetAsync(c->tok_ids, 0, g.topk * wsz, s));
+    INFLLM_CUDA_OK(cudaMemsetAsync(c->tok_parts, 0, c->tok_part_words * wsz, s));
+    for (auto& o : c->pend) memset(o.h_words, 0, g.topk * wsz);
+    c->tok_seq = 0;
+    c->tok_restart = false;
+  }
+  pt.seq = ++c->tok_seq;
+  if (c->tok_seq == UINT32_MAX) c->tok_restart = true;  // 0 marks "not a one-launch token"
+  P.q = q, P.k = k, P.v = v, P.q_hs = q_hs, P.k_hs = k_hs, P.v_hs = v_hs;
+  P.k_raw = (char*)tb.k_raw + at * D * esz, P.k_rot = (char*)tb.k_rot + at * D * esz, P.v_out = (char*)tb.v + at * D * esz;
+  P.kv_hs = kv_hs;
+  P.cos_t = c->cos_t, P.sin_t = c->sin_t, P.pos_loc = S - c->rope_origin, P.pos_glb = g.n_local - 1;
+  P.bk = c->block_k, P.score_words = c->tok_scores, P.id_words = c->tok_ids, P.ids_host = pt.h_words;
+  P.n = (int)c->num_blocks, P.width = (int)c->width, P.k_top = g.topk;
+  const int64_t wlo = std::max<int64_t>(S + 1 - g.n_local, 0), ovf = std::max<int64_t>(S + 1 - c->frontier - g.n_local, 0);
+  const int64_t w_off = (wlo - tb.t0) * D * esz, f_off = (c->frontier - tb.t0) * D * esz;
+  P.rest[0] = {(char*)tb.k_rot + w_off, (char*)tb.v + w_off, kv_hs, (int32_t)(S - wlo), 0};
+  P.rest[1] = {c->init_k, c->init_v, c->init_cap * D, (int32_t)c->init_len, 0};
+  P.rest[2] = {(char*)tb.k_raw + f_off, (char*)tb.v + f_off, kv_hs, (int32_t)ovf, 0};
+  P.rest_begin[0] = 0;
+  for (int i = 0; i < 3; ++i) P.rest_begin[i + 1] = P.rest_begin[i] + (P.rest[i].len + 15) / 16;
+  P.ptrs = c->d_unit_ptrs, P.landing_at = c->tab_cap, P.unit_bytes = c->unit_bytes, P.unit_len = g.block_size;
+  P.n_heads = g.n_heads, P.n_kv = g.n_kv_heads, P.group = g.n_heads / g.n_kv_heads, P.n_runs = runs;
+  P.scale_log2 = kLog2e / sqrtf((float)D);
+  P.part_words = c->tok_parts, P.logits = c->dec_logits, P.logit_hs = (int64_t)g.n_local + 1;
+  P.win_score = tb.score + (wlo - tb.t0), P.score_hs = tb.cap;
+  P.out = out, P.o_hs = o_hs;
+  P.seq = c->tok_seq;
+  P.err = c->tc_err, P.err_host = c->h_tc_err;
+  return token_launch(P, g.dtype, s);
+}
+
 // one internal call of at most sub_max tokens whose exec-block boundaries coincide with the caller's
 int append_sub(infllm_ctx* c, const char* q, int64_t q_hs, int64_t q_ts, const char* k, int64_t k_hs, int64_t k_ts,
                const char* v, int64_t v_hs, int64_t v_ts, char* out, int64_t o_hs, int64_t o_ts, int64_t L,
@@ -1455,7 +1561,16 @@ int append_sub(infllm_ctx* c, const char* q, int64_t q_hs, int64_t q_ts, const c
                                    (char*)tb.k_rot + (win0 - tb.t0) * D * esz, kv_hs, D, (int)HKV, T - win0, (int)D,
                                    c->cos_t, c->sin_t, c->tab_len, 0, 1, g.dtype, s));
   }
-  if (L == 1) {
+  // One-token appends over more units than a retrieval takes run ahead of the host (see below); where the sizes allow it
+  // the whole token is one launch (per-kernel timing wants the kernels apart).
+  const bool run_ahead = L == 1 && D == 128 && c->num_blocks > g.topk && g.topk <= kMaxSeg - 4 && !(g.debug_flags & 16) &&
+                         g.chunk_topk_calc == 0 && g.cache_strategy == INFLLM_CACHE_LRU;
+  const int tok_runs = run_ahead && c->use_tc && !c->prof && !c->comm
+                           ? token_runs((int)H, (int)HKV, (int)D, c->num_blocks, g.topk, (int)bs, c->tok_sms) : 0;
+  const bool one_launch = tok_runs > 0;
+  if (one_launch) {
+    c->ingest_event_due = true;
+  } else if (L == 1) {
     // one token: copies, the three rotations, the query mean and the cleared score column in one launch
     INFLLM_TRY(ingest_token_launch(q, q_hs, k, k_hs, v, v_hs, c->q_loc, c->q_glb, q_hs_s, c->qbar,
                                    (char*)tb.k_raw + at * D * esz, (char*)tb.k_rot + at * D * esz,
@@ -1504,8 +1619,6 @@ int append_sub(infllm_ctx* c, const char* q, int64_t q_hs, int64_t q_ts, const c
 
   // one-token appends whose retrieval has not been applied to the cache yet: a call that is not itself such a token
   // needs the cache as the reference would have it
-  const bool run_ahead = L == 1 && D == 128 && c->num_blocks > g.topk && g.topk <= kMaxSeg - 4 && !(g.debug_flags & 16) &&
-                         g.chunk_topk_calc == 0 && g.cache_strategy == INFLLM_CACHE_LRU;
   if (!run_ahead) INFLLM_TRY(settle_all(c, s));
   if (L > 1) {  // units a previous one-token append fetched ahead are not wanted by a prefill's look-ahead
     for (auto it = c->staged.begin(); it != c->staged.end();) {
@@ -1562,15 +1675,20 @@ int append_sub(infllm_ctx* c, const char* q, int64_t q_hs, int64_t q_ts, const c
       ids.clear();
       // at most kMaxOutstanding tokens ahead of the cache: apply the older retrievals first
       while (c->pend_count >= infllm_ctx::kMaxOutstanding) INFLLM_TRY(settle_one(c, s));
-      INFLLM_TRY(ensure_scores(c, c->num_blocks, s));
       const int slot = (c->pend_head + c->pend_count) % infllm_ctx::kPendSlots;
       infllm_ctx::PendingToken& pt = c->pend[slot];
       d_ids_tok = c->d_topk_ring + (int64_t)slot * std::max(1, g.topk);
-      {
+      pt.seq = 0;
+      if (one_launch) {
+        INFLLM_TRY(token_whole(c, pt, tok_runs, q, q_hs, k, k_hs, v, v_hs, out, o_hs, at, S, s));
+      } else {
+        INFLLM_TRY(ensure_scores(c, c->num_blocks, s));
         ProfScope ps(c, s, INFLLM_PROF_TOPK, (double)c->num_blocks * c->width * c->esz);
         INFLLM_TRY(score_topk(c, c->num_blocks, c->qbar, c->scores, d_ids_tok, s, 0, g.topk, direct ? pt.h_ids : nullptr));
       }
-      if (direct) {
+      if (one_launch) {
+        // the ranking threads write the ids, marked, into the pinned words
+      } else if (direct) {
         // the ranking threads wrote the ids into the pinned words themselves; the event that tells the host so is
         // recorded behind the token's last kernel, so that nothing stands between the kernels of the chain
         token_ev = pt.ev;
@@ -1582,7 +1700,7 @@ int append_sub(infllm_ctx* c, const char* q, int64_t q_hs, int64_t q_ts, const c
       }
       pt.serial = c->call_serial;
       c->pend_count += 1;
-      INFLLM_TRY(flush_table(c, s));
+      if (!one_launch) INFLLM_TRY(flush_table(c, s));
       pt.listed.clear();
       for (auto& kv : c->dev_table) pt.listed.push_back(kv.first);
       pt.landing = c->landing_slots;
@@ -1610,7 +1728,9 @@ int append_sub(infllm_ctx* c, const char* q, int64_t q_hs, int64_t q_ts, const c
     const char* qglb_eb = (const char*)c->q_glb + st * D * esz;
     const bool decode_path = lq == 1 && D == 128;
     double local_pairs_eb = 0;
-    if (decode_path) {
+    if (one_launch) {
+      // launched above
+    } else if (decode_path) {
       // ---- one-token exec block: split-K decode over [visible window | global segments]
       const int64_t wlo = std::max<int64_t>(E - g.n_local, ks);  // window mask of the single query
       std::vector<KvSeg> segs;
@@ -1889,16 +2009,18 @@ static void ctx_free(infllm_ctx* c) {
     cudaDeviceSynchronize();
     free_buffers(c->tb, nullptr);
     void* dev[] = {c->init_k, c->init_v, c->cos_t, c->sin_t, c->q_loc, c->q_glb, c->qbar, c->lse, c->st_acc, c->st_m,
-                   c->st_l, c->d_topk, c->tickets, c->d_miss, c->part_o, c->part_lse, c->dec_logits, c->cache};
+                   c->st_l, c->d_topk, c->tok_ids, c->tok_parts, c->tickets, c->d_miss, c->part_o, c->part_lse, c->dec_logits, c->cache};
     for (void* p : dev)
       if (p) cudaFree(p);
     if (c->block_k) cudaFreeAsync(c->block_k, nullptr);
     if (c->scores) cudaFreeAsync(c->scores, nullptr);
+    if (c->tok_scores) cudaFreeAsync(c->tok_scores, nullptr);
     if (c->d_unit_ptrs) cudaFreeAsync(c->d_unit_ptrs, nullptr);
 
     if (c->d_topk_ring) cudaFree(c->d_topk_ring);
     for (auto& pt : c->pend) {
       if (pt.h_ids) cudaFreeHost(pt.h_ids);
+      if (pt.h_words) cudaFreeHost(pt.h_words);
       if (pt.ev) cudaEventDestroy(pt.ev);
     }
     if (c->unit_prob) cudaFree(c->unit_prob);
@@ -1992,7 +2114,7 @@ static int64_t ctx_device_bytes(const infllm_ctx* c) {
   n += (int64_t)c->max_parts * H * (D + 1) * 4 + H * ((int64_t)g.n_local + 1) * 4;
   n += ((int64_t)g.max_cached_block + (int64_t)c->look_depth * g.topk) * c->unit_bytes;
   n += HKV * c->tb.cap * D * c->esz * 3 + H * c->tb.cap * 4 + c->block_k_cap * c->width * c->esz;
-  n += (int64_t)c->tc_part_floats * 4 + (c->scores_cap + c->scores_aux_cap) * 4 + c->tab_cap * 8;
+  n += (int64_t)c->tc_part_floats * 4 + (int64_t)c->tok_part_words * 8 + c->tok_scores_cap * 8 + (c->scores_cap + c->scores_aux_cap) * 4 + c->tab_cap * 8;
   return n;
 }
 
@@ -2123,6 +2245,7 @@ extern "C" int infllm_ctx_append(infllm_ctx* c, const void* d_q, int64_t q_hs, i
   if (!c->initialized) INFLLM_TRY(lazy_init(c, s));
   INFLLM_TRY(order_behind_reset(c, s));
   INFLLM_TRY(poll_device_error(c, s));
+  if (c->h_tc_err && !c->err_pending && *(volatile int32_t*)c->h_tc_err) INFLLM_TRY(check_device_error(c, s));  // a one-launch token gave up
   c->failed = true;  // until the call has gone through
   if (c->seal_aside) {  // a call that gave up half-way left it so
     INFLLM_CUDA_OK(cudaStreamWaitEvent(s, c->ev_seal, 0));

@@ -1,0 +1,75 @@
+"""The one-launch decode token (token.cu) against the same tokens as separate kernels (which per-kernel timing asks
+for): the scores are summed in the same order, so the retrieved ids are equal, in order; outputs differ by the order in
+which partial results are added (probabilities and outputs are rounded to 16 bits: a few 2^-9 relative)."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+D, UNIT, N_INIT = 128, 128, 40
+
+
+def _memory(H, HKV, n_units, n_local, topk, dtype, ties):
+    from infllm_b200.attention import ContextManager, RotaryEmbeddingESM
+
+    g = torch.Generator().manual_seed(n_units + H)
+    pool = torch.randn((min(n_units, 64), 2, HKV, UNIT, D), generator=g).to(dtype)
+    units = pool.repeat((-(-n_units // pool.size(0)), 1, 1, 1, 1))[:n_units]
+    block_k = torch.randn((n_units, H * D), generator=g).to(dtype)
+    if ties:  # every third row is the same: equal scores, also at the cut
+        block_k[::3] = block_k[0]
+    rnd = lambda n: torch.randn((HKV, n, D), generator=g).to(dtype)  # noqa: E731
+    small = (rnd(N_INIT), rnd(N_INIT), rnd(n_local), rnd(n_local))
+    out = []
+    for apart in (False, True):
+        cm = ContextManager(RotaryEmbeddingESM(D, 1e6, 1.0), N_INIT, n_local, UNIT, 2 * topk, topk, 128, None, True, 2)
+        cm.profile(apart)
+        cm.load_synthetic(units, block_k, *small)
+        out.append(cm)
+    return out
+
+
+@pytest.mark.parametrize("H,HKV,n_units,n_local,topk,dtype,ties", [
+    (32, 8, 17, 1000, 16, torch.bfloat16, False),    # one unit more than a retrieval
+    (32, 8, 384, 513, 16, torch.bfloat16, True),     # as many scores as ranking threads
+    (32, 8, 385, 4096, 16, torch.float16, True),     # one more
+    (28, 4, 500, 700, 64, torch.bfloat16, True),     # the largest retrieval
+    (8, 1, 8460, 300, 32, torch.bfloat16, True),     # more scores than the ranking keeps in registers; one KV head
+    (8, 1, 8460, 300, 1, torch.bfloat16, False),
+    (32, 32, 300, 257, 8, torch.float16, False),     # one query head per KV head, four runs each
+    (7, 7, 40, 130, 3, torch.bfloat16, False),       # a width that is no multiple of 2048
+    (96, 48, 60, 200, 4, torch.bfloat16, False),     # the widest rows, three runs per KV head
+])
+def test_one_launch_equals_separate_kernels(H, HKV, n_units, n_local, topk, dtype, ties):
+    one, apart = _memory(H, HKV, n_units, n_local, topk, dtype, ties)
+    g = torch.Generator(device="cuda").manual_seed(5)
+    for i in range(UNIT + 3):  # past a sealing
+        q, k, v = (torch.randn((1, h, 1, D), generator=g, device="cuda").to(dtype) for h in (H, HKV, HKV))
+        a, b = one.append(q, k, v, q, k, v), apart.append(q, k, v, q, k, v)
+        if i % 16 == 0 or i > UNIT - 4:
+            assert one.last_topk() == apart.last_topk()
+            assert one.cached_blocks == apart.cached_blocks
+            assert (a.float() - b.float()).abs().max() <= 1e-2 * b.float().abs().max()
+    assert one.info()["num_blocks"] == n_units + 1
+    assert torch.equal(one.block_k_rows()[:n_units], apart.block_k_rows()[:n_units])
+    # the sealed unit's representative keys come from the accumulated scores: equal unless two tokens tie to 1e-6
+    assert (one.block_k_rows()[n_units] != apart.block_k_rows()[n_units]).float().mean() < 0.05
+
+
+def test_a_word_that_does_not_arrive_is_an_error():
+    """The error record that a token's bounded wait leaves (set here from the host) fails the next call."""
+    from infllm_b200 import _lib
+
+    one, _ = _memory(8, 2, 20, 200, 4, torch.bfloat16, False)
+    q, k, v = (torch.randn((1, h, 1, D), device="cuda").to(torch.bfloat16) for h in (8, 2, 2))
+    one.append(q, k, v, q, k, v)
+    torch.cuda.synchronize()
+    _lib.check(_lib.lib.infllm_device_error_set(1, 700))
+    with pytest.raises(_lib.InfLLMError):
+        for n in (200, 1, 1):  # a longer call carries the record to the host
+            qq, kk, vv = (torch.randn((1, h, n, D), device="cuda").to(torch.bfloat16) for h in (8, 2, 2))
+            one.append(qq, kk, vv, qq, kk, vv)
+            torch.cuda.synchronize()
+    for _ in range(2):  # and the memory goes on
+        one.append(q, k, v, q, k, v)
+    torch.cuda.synchronize()
