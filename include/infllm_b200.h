@@ -302,7 +302,10 @@ int infllm_device_store_reserve(int device, int64_t bytes);
 int infllm_device_store_release(int device);
 int infllm_device_store_info(int device, int64_t* total_bytes, int64_t* used_bytes);
 
-/* Validates the configuration (exc_block_size <= n_local, context_manager.py:219;
+/* Device memory of the cache: max_cached_block + look_depth * topk slots of one unit, and on top up to 256 MiB (no more
+ * than 1/128 of the free memory when the context is initialised) in which evicted units stay readable until their slots
+ * are needed.  The cache, its LRU order and the counters of hits, misses and evictions are those of max_cached_block.
+ * Validates the configuration (exc_block_size <= n_local, context_manager.py:219;
  * max_cached_block >= topk, context_manager.py:19 -> INFLLM_E_CAPACITY) and allocates nothing
  * large: buffers are created on the first append (context_manager.py:292-363). */
 int infllm_ctx_create(const infllm_config* cfg, infllm_ctx** out);

@@ -135,6 +135,54 @@ struct LruTable {
   }
 };
 
+// ------------------------------------------------------------------------------------- cache slots
+// The slots that nothing is using, in the order in which they will be taken: empty ones first, then the one that became
+// free longest ago.  A slot whose unit was evicted keeps its data until it is taken for something else, and the unit can be
+// claimed back meanwhile: a retrieval that returns to it costs no copy.
+struct SlotPool {
+  std::list<int> order;
+  std::vector<std::list<int>::iterator> at;  // per slot
+  std::vector<int32_t> holds;                // per slot: the unit whose data a free slot still has, -1 none
+  std::unordered_map<int32_t, int> kept;     // unit -> the free slot that has its data
+
+  void init(int n) {
+    order.clear();
+    kept.clear();
+    at.resize(n);
+    holds.assign(n, -1);
+    for (int i = 0; i < n; ++i) at[i] = order.insert(order.end(), i);
+  }
+  bool empty() const { return order.empty(); }
+  // a slot to write to; *lost is the unit whose data goes with it, or -1
+  int take(int32_t* lost) {
+    const int slot = order.front();
+    order.pop_front();
+    *lost = holds[slot];
+    if (*lost >= 0) kept.erase(*lost);
+    holds[slot] = -1;
+    return slot;
+  }
+  void give(int slot, int32_t unit) {
+    if (unit >= 0 && kept.emplace(unit, slot).second) {
+      holds[slot] = unit;
+      at[slot] = order.insert(order.end(), slot);
+    } else {
+      holds[slot] = -1;
+      at[slot] = order.insert(order.begin(), slot);
+    }
+  }
+  // the slot that still has the unit, no longer free; -1: none has
+  int claim(int32_t unit) {
+    auto it = kept.find(unit);
+    if (it == kept.end()) return -1;
+    const int slot = it->second;
+    kept.erase(it);
+    holds[slot] = -1;
+    order.erase(at[slot]);
+    return slot;
+  }
+};
+
 // --------------------------------------------------------------------------------------- context
 struct TokenBuffers {
   void* k_raw = nullptr;  // (H_kv, cap, D) un-rotated keys
@@ -196,7 +244,8 @@ struct infllm_ctx {
 
   // unit store
   void* cache = nullptr;  // (max_cached, 2, H_kv, bs, D)
-  std::vector<int> free_slots;
+  SlotPool free_slots;
+  int64_t n_slots = 0;
   std::vector<cudaEvent_t> slot_ev;   // per slot: behind the last look-ahead copy into it
   std::vector<char> slot_ev_used;
   std::unordered_map<int32_t, int> slot_of;
@@ -219,7 +268,6 @@ struct infllm_ctx {
     uint32_t seq = 0;          // != 0: the ids are in h_words and carry this number
     cudaEvent_t ev = nullptr;  // seq == 0: behind the ids
     int64_t serial = 0;        // the append call it belongs to
-    std::vector<int32_t> listed;  // units the device table showed in a cache slot when the token was launched
     std::vector<int> landing;     // the landing slot of every retrieval position at that time (-1: none)
   };
   static constexpr int kPendSlots = 4, kMaxOutstanding = 1;
@@ -543,9 +591,22 @@ int lazy_init(infllm_ctx* c, cudaStream_t s) {
   INFLLM_CUDA_OK(dev_malloc((void**)&c->part_o, (int64_t)c->max_parts * H * D * sizeof(float)));
   INFLLM_CUDA_OK(dev_malloc((void**)&c->part_lse, (int64_t)c->max_parts * H * sizeof(float)));
   INFLLM_CUDA_OK(dev_malloc((void**)&c->dec_logits, H * ((int64_t)g.n_local + 1) * sizeof(float)));
-  // max_cached_block slots hold the cache proper; topk more per look-ahead step hold the copies staged ahead
-  const int64_t n_slots = (int64_t)g.max_cached_block + (int64_t)c->look_depth * g.topk;
-  INFLLM_CUDA_OK(dev_malloc((void**)&c->cache, n_slots * c->unit_bytes));
+  // max_cached_block slots hold the cache proper; topk more per look-ahead step hold the copies staged ahead.  Past those,
+  // up to kKeepBytes (and no more than 1/128 of the free memory) let evicted units stay until their slots are needed: the
+  // cache and its LRU order are those of max_cached_block, but a unit that is retrieved again after its eviction does not
+  // cross PCIe again.  64K tokens of a 32-KV-head layer whose retrievals rotate through 128 units of 2 MiB:
+  // 102 -> 39 ms; a token over 1M tokens whose topic changes every 16 tokens: 88 -> 35 us.
+  int64_t n_slots = (int64_t)g.max_cached_block + (int64_t)c->look_depth * g.topk;
+  {
+    constexpr int64_t kKeepBytes = 256ll << 20;
+    size_t free_b = 0, total_b = 0;
+    INFLLM_CUDA_OK(cudaMemGetInfo(&free_b, &total_b));
+    const int64_t extra = std::min<int64_t>(kKeepBytes, (int64_t)(free_b / 128)) / c->unit_bytes;
+    if (extra > 0 && cudaMalloc(&c->cache, (n_slots + extra) * c->unit_bytes) == cudaSuccess) n_slots += extra;
+    else cudaGetLastError();
+  }
+  if (!c->cache) INFLLM_CUDA_OK(dev_malloc((void**)&c->cache, n_slots * c->unit_bytes));
+  c->n_slots = n_slots;
   INFLLM_CUDA_OK(cudaMemsetAsync(c->cache, 0, n_slots * c->unit_bytes, s));
   c->use_tc = D == 128 && g.block_size % 128 == 0 && !(g.debug_flags & 1);
   if (c->use_tc) {
@@ -564,8 +625,7 @@ int lazy_init(infllm_ctx* c, cudaStream_t s) {
     c->h_tc_err[0] = c->h_tc_err[1] = c->h_tc_err[2] = c->h_tc_err[3] = 0;
     INFLLM_CUDA_OK(cudaEventCreateWithFlags(&c->ev_err, cudaEventDisableTiming));
   }
-  c->free_slots.clear();
-  for (int i = (int)n_slots - 1; i >= 0; --i) c->free_slots.push_back(i);
+  c->free_slots.init((int)n_slots);
   c->slot_ev.assign(n_slots, nullptr);
   c->slot_ev_used.assign(n_slots, 0);
   c->slab_units = std::max<int64_t>(16, (128ll << 20) / c->unit_bytes);
@@ -809,6 +869,14 @@ int lookahead_launch(infllm_ctx* c, int64_t target, cudaStream_t s) {
   return INFLLM_OK;
 }
 
+// a free slot (there is one) to write to; the unit whose data it still had is at its place in the store from now on
+int take_slot(infllm_ctx* c) {
+  int32_t lost;
+  const int slot = c->free_slots.take(&lost);
+  if (lost >= 0 && c->table_valid) c->tab_updates[lost] = -1;
+  return slot;
+}
+
 // an event behind the copy just issued into a cache slot on the copy stream: whoever later writes the slot from
 // another stream waits for it (the copy may have been abandoned, never awaited, and still be in flight)
 int mark_slot_copy(infllm_ctx* c, void* slot_ptr) {
@@ -840,9 +908,14 @@ int lookahead_stage(infllm_ctx* c, int64_t target) {
       sf->second = std::max(sf->second, target);
       continue;
     }
-    if (c->free_slots.empty()) break;  // no spare slot: the unit is fetched at plan time instead
-    int slot = c->free_slots.back();
-    c->free_slots.pop_back();
+    const int kept = c->free_slots.claim(b);
+    if (kept >= 0) {  // evicted, but its slot has not been needed since
+      c->staged[b] = kept;
+      c->staged_for[b] = target;
+      continue;
+    }
+    if (c->free_slots.empty()) continue;  // no spare slot: the unit is fetched at plan time instead
+    const int slot = take_slot(c);
     c->staged[b] = slot;
     c->staged_for[b] = target;
     if (b >= c->d2h_synced_upto) {  // sealed recently: its copy-out must land in the store first
@@ -957,10 +1030,9 @@ int plan_and_refill(infllm_ctx* c, const std::vector<int32_t>& ids, int64_t eb, 
         c->staged[b] = it->second;
         c->staged_for[b] = wanted_by;
       } else {
-        c->free_slots.push_back(it->second);
+        c->free_slots.give(it->second, b);  // (a one-token attention goes on finding it there)
       }
       c->slot_of.erase(it);
-      if (track) c->tab_updates[b] = -1;
     }
   }
   c->counters.evictions += (int64_t)evicted.size();
@@ -970,11 +1042,26 @@ int plan_and_refill(infllm_ctx* c, const std::vector<int32_t>& ids, int64_t eb, 
   } else {
     c->lru.stamp(ids.data(), (int)ids.size(), 0.0);
   }
+  // units that were evicted and still are in their slots come back before any slot is taken for another
+  std::vector<int32_t> back;
+  for (int32_t b : ids) {
+    if (c->slot_of.count(b) || c->staged.count(b)) continue;
+    const int slot = c->free_slots.claim(b);
+    if (slot < 0) continue;
+    if (c->slot_ev_used[slot]) INFLLM_CUDA_OK(cudaStreamWaitEvent(s, c->slot_ev[slot], 0));  // an abandoned look-ahead copy
+    c->slot_of[b] = slot;
+    if (track) c->tab_updates[b] = slot;
+    back.push_back(b);
+  }
   bool late = false;
   std::vector<const void*> late_src;
   std::vector<void*> late_dst;
   for (int32_t b : ids) {
     if (c->slot_of.count(b)) {
+      if (std::find(back.begin(), back.end(), b) != back.end()) {
+        c->counters.cache_misses += 1;
+        continue;
+      }
       c->counters.cache_hits += 1;
       continue;
     }
@@ -1009,13 +1096,12 @@ int plan_and_refill(infllm_ctx* c, const std::vector<int32_t>& ids, int64_t eb, 
       auto victim = c->staged.begin();
       for (auto it2 = c->staged.begin(); it2 != c->staged.end(); ++it2)
         if (std::find(ids.begin(), ids.end(), it2->first) == ids.end()) { victim = it2; break; }
-      c->free_slots.push_back(victim->second);
+      c->free_slots.give(victim->second, -1);
       if (track) c->tab_updates[victim->first] = -1;
       c->staged_for.erase(victim->first);
       c->staged.erase(victim);
     }
-    int slot = c->free_slots.back();
-    c->free_slots.pop_back();
+    const int slot = take_slot(c);
     c->slot_of[b] = slot;
     if (mode == PLAN_DECODE_SYNC) c->tab_updates[b] = slot;
     const int64_t tok0 = (int64_t)g.n_init + (int64_t)b * g.block_size;  // the unit's first token
@@ -1064,7 +1150,7 @@ int plan_and_refill(infllm_ctx* c, const std::vector<int32_t>& ids, int64_t eb, 
   // ordered behind the unfinished ones on the side stream; no kernel reads them)
   for (auto it = c->staged.begin(); it != c->staged.end();) {
     if (c->staged_for[it->first] <= eb) {  // staged for this exec block (or an earlier one) and not taken
-      c->free_slots.push_back(it->second);
+      c->free_slots.give(it->second, it->first);
       c->staged_for.erase(it->first);
       it = c->staged.erase(it);
     } else {
@@ -1097,8 +1183,7 @@ int flush_table(infllm_ctx* c, cudaStream_t s, TokenParams* tok = nullptr) {
   c->landing_slots.resize(topk, -1);
   for (int i = 0; i < topk; ++i) {
     if (c->landing_slots[i] >= 0 || c->free_slots.empty()) continue;
-    const int slot = c->free_slots.back();
-    c->free_slots.pop_back();
+    const int slot = take_slot(c);
     // an abandoned look-ahead copy of an earlier prefill may still be on its way into this slot
     if (c->slot_ev_used[slot]) INFLLM_CUDA_OK(cudaStreamWaitEvent(s, c->slot_ev[slot], 0));
     c->landing_slots[i] = slot;
@@ -1119,6 +1204,14 @@ int flush_table(infllm_ctx* c, cudaStream_t s, TokenParams* tok = nullptr) {
     for (auto& kv : c->slot_of) {
       all[(size_t)kv.first] = slot_addr(kv.second);
       c->dev_table[kv.first] = kv.second;
+    }
+    if (!c->free_slots.kept.empty()) {  // the evicted ones too, once every look-ahead copy has landed
+      INFLLM_CUDA_OK(cudaEventRecord(c->ev_stage, c->copy_stream));
+      INFLLM_CUDA_OK(cudaStreamWaitEvent(s, c->ev_stage, 0));
+      for (auto& kv : c->free_slots.kept) {
+        all[(size_t)kv.first] = slot_addr(kv.second);
+        c->dev_table[kv.first] = kv.second;
+      }
     }
     if (c->d2h_recorded) INFLLM_CUDA_OK(cudaStreamWaitEvent(s, c->ev_d2h, 0));   // the store holds every sealed unit
     INFLLM_CUDA_OK(cudaMemcpyAsync(c->d_unit_ptrs, all.data(), all.size() * sizeof(unsigned long long),
@@ -1197,7 +1290,7 @@ int settle_one(infllm_ctx* c, cudaStream_t s) {
   // the units that token's attention did not find in a cache slot were read in place and sit in the landing slots
   c->settle_landing.assign(ids.size(), -1);
   for (size_t i = 0; i < ids.size(); ++i)
-    if (std::find(p.listed.begin(), p.listed.end(), ids[i]) == p.listed.end()) {
+    if (!c->dev_table.count(ids[i])) {  // (the table is as that token saw it: it changes with the next one)
       c->counters.inplace_units += 1;
       if (i < p.landing.size() && p.landing[i] >= 0 && c->landing_slots[i] == p.landing[i]) {
         c->settle_landing[i] = p.landing[i];
@@ -1623,7 +1716,7 @@ int append_sub(infllm_ctx* c, const char* q, int64_t q_hs, int64_t q_ts, const c
   if (L > 1) {  // units a previous one-token append fetched ahead are not wanted by a prefill's look-ahead
     for (auto it = c->staged.begin(); it != c->staged.end();) {
       if (c->staged_for[it->first] == INT64_MAX) {
-        c->free_slots.push_back(it->second);
+        c->free_slots.give(it->second, it->first);
         c->staged_for.erase(it->first);
         it = c->staged.erase(it);
       } else {
@@ -1632,7 +1725,7 @@ int append_sub(infllm_ctx* c, const char* q, int64_t q_hs, int64_t q_ts, const c
     }
     // the slots set aside for one-token attentions to deposit in go back to the pool
     for (int slot : c->landing_slots)
-      if (slot >= 0) c->free_slots.push_back(slot);
+      if (slot >= 0) c->free_slots.give(slot, -1);
     c->landing_slots.clear();
     c->landing_listed.clear();
     c->table_valid = false;
@@ -1701,8 +1794,6 @@ int append_sub(infllm_ctx* c, const char* q, int64_t q_hs, int64_t q_ts, const c
       pt.serial = c->call_serial;
       c->pend_count += 1;
       if (!one_launch) INFLLM_TRY(flush_table(c, s));
-      pt.listed.clear();
-      for (auto& kv : c->dev_table) pt.listed.push_back(kv.first);
       pt.landing = c->landing_slots;
     }
     // bit 1 of the flags turns the look-ahead off; a chunk's retrievals are fixed when it starts, so they need none
@@ -1982,8 +2073,7 @@ static int ctx_reset(infllm_ctx* c, bool wait) {
   c->table_valid = false;
   c->tab_updates.clear();
   c->dev_table.clear();
-  c->free_slots.clear();
-  for (int i = c->cfg.max_cached_block + c->look_depth * c->cfg.topk - 1; i >= 0; --i) c->free_slots.push_back(i);
+  c->free_slots.init((int)c->n_slots);
   c->staged.clear();
   c->staged_for.clear();
   for (auto& l : c->la) l.target = -1, l.launched = l.staged = false;
@@ -2112,7 +2202,7 @@ static int64_t ctx_device_bytes(const infllm_ctx* c) {
   int64_t n = 2 * c->pack_units * c->unit_bytes + c->tab_len * D * 4 + 2 * HKV * c->init_cap * D * c->esz;
   n += 2 * H * c->sub_max * D * c->esz + (c->sub_max / exc + 1) * c->width * 4 + H * exc * (D + 3) * 4;
   n += (int64_t)c->max_parts * H * (D + 1) * 4 + H * ((int64_t)g.n_local + 1) * 4;
-  n += ((int64_t)g.max_cached_block + (int64_t)c->look_depth * g.topk) * c->unit_bytes;
+  n += c->n_slots * c->unit_bytes;
   n += HKV * c->tb.cap * D * c->esz * 3 + H * c->tb.cap * 4 + c->block_k_cap * c->width * c->esz;
   n += (int64_t)c->tc_part_floats * 4 + (int64_t)c->tok_part_words * 8 + c->tok_scores_cap * 8 + (c->scores_cap + c->scores_aux_cap) * 4 + c->tab_cap * 8;
   return n;
@@ -2730,8 +2820,7 @@ extern "C" int infllm_ctx_load(infllm_ctx* c, const char* path, void* stream) {
   c->rope_origin = -1;  // the window is rotated anew by the next append
   // the cache comes back as the LRU table lists it (n_lru <= max_cached_block slots were checked above)
   for (auto& kv : lru) {
-    const int slot = c->free_slots.back();
-    c->free_slots.pop_back();
+    const int slot = take_slot(c);
     c->slot_of[kv.first] = slot;
     c->lru.set(kv.first, kv.second);
     INFLLM_CUDA_OK(cudaMemcpyAsync((char*)c->cache + (int64_t)slot * c->unit_bytes, c->host_unit(kv.first), c->unit_bytes,
