@@ -966,7 +966,8 @@ __global__ void __launch_bounds__(352, 1) attn_tc3_kernel(const __grid_constant_
     // Three ways out: a run of a split work item leaves its un-normalised partial; a stage of a multi-stage attention
     // leaves the state (acc, m, l); everything else is normalised.  A state that came in is folded in first.
     const int64_t srow = (int64_t)h * P.lq + qi;
-    float ws = 1.f, wp = 0.f, m_out = m_row, l_out = it >= 1 ? l_sum : 0.f;
+    // (the cubic exponential leaves 2^-126 of a masked key: a row that saw no key has the sum 0 by its maximum)
+    float ws = 1.f, wp = 0.f, m_out = m_row, l_out = it >= 1 && m_row != -INFINITY ? l_sum : 0.f;
     if (P.st_acc) {
       if (row_valid) {
         const float mp = P.st_m[srow], mm = fmaxf(mp, m_row), ms = mm == -INFINITY ? 0.f : mm;
