@@ -229,6 +229,13 @@ def dtype_code(dtype):
     raise TypeError(f"infllm_b200 kernels take bfloat16 or float16 activations, got {dtype}")
 
 
+def raw_stream(device):
+    """The current stream's handle as an int (without building a Stream object: 3 us of a token's 15 on the host)."""
+    import torch
+
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if device.index is None else device.index)
+
+
 def stream_ptr(device=None):
     import torch
 

@@ -187,7 +187,7 @@ class ContextManager:
 
     def _append_units(self, q, k, v, out, length):
         """One native call per unit (sequence, or head of a sequence); addresses by arithmetic, 2 bytes per element."""
-        append, stream = _lib.lib.infllm_ctx_append, torch.cuda.current_stream(q.device).cuda_stream
+        append, stream = _lib.lib.infllm_ctx_append, _lib.raw_stream(q.device)
         q_bs, q_hs, q_ts, _ = q.stride()
         k_bs, k_hs, k_ts, _ = k.stride()
         o_bs, o_hs, o_ts, _ = out.stride()

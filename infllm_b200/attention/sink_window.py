@@ -22,71 +22,88 @@ from .dot_production_attention import get_multi_stage_dot_production_attention
 from .rope import RotaryEmbeddingESM
 
 
-def _rows_aligned(t):
+_NATIVE = (torch.bfloat16, torch.float16)
+
+
+def _rows(t):
+    """A projection (B, L, heads * 128) with 16-byte aligned rows, copied if it has others."""
+    a, b, c = t.stride()
+    return t if c == 1 and (a | b) % 8 == 0 and t.data_ptr() % 16 == 0 else t.contiguous()
+
+
+def _cache_rows(t):
     a, b, c, d = t.stride()
     return d == 1 and (a | b | c) % 8 == 0 and t.data_ptr() % 16 == 0
 
 
-def _run_native(rope, q, k, v, past, n_local, n_init, stream_positions, use_cache):
-    """The call in libinfllm_b200 (infllm_sink_window_run): q (B, H, L, D), k and v (B, H_kv, L, D) views of the
-    projections; returns (o (B, L, H * D), cache or None)."""
-    batch, heads, len_q, dim = q.shape
-    kv = k.size(1)
-    if not _rows_aligned(q):
-        q = q.contiguous()
-    if not _rows_aligned(k) or k.stride() != v.stride() or not _rows_aligned(v):
+def _run_native(rope, q, k, v, heads, kv, past, n_local, n_init, stream_positions, use_cache):
+    """The call in libinfllm_b200 (infllm_sink_window_run) on the projections q (B, L, heads * 128) and k, v
+    (B, L, kv * 128); returns (o (B, L, heads * 128), cache or None), or None where the general path is needed."""
+    dim = 128
+    batch, len_q, _ = q.shape
+    q, k, v = _rows(q), _rows(k), _rows(v)
+    if k.stride() != v.stride():
         k, v = k.contiguous(), v.contiguous()
     pk = pv = None
     past_len, seen = 0, len_q
+    p_bs = p_hs = p_ts = 0
     if past is not None:
         pk, pv = past[0], past[1]
-        if not _rows_aligned(pk) or pk.stride() != pv.stride() or not _rows_aligned(pv):
+        if not _cache_rows(pk) or pk.stride() != pv.stride() or not _cache_rows(pv):
             pk, pv = pk.contiguous(), pv.contiguous()
         past_len = pk.size(2)
         seen += past[2]
+        p_bs, p_hs, p_ts, _ = pk.stride()
     total = past_len + len_q
-    cache = None
+    head = rows = 0
+    kept = ck_at = cv_at = None
+    device, dtype = q.device, q.dtype
     if use_cache:  # everything while the history is short, then [first n_init | last n_local]
         short = seen <= n_local + n_init
         head = total if short else min(n_init, total)
         rows = total if short else head + min(n_local, total)
-        if rows > total:  # the two parts of a short cache overlap: left to the general path
+        if rows > total:  # the two parts of a short cache overlap
             return None
-        kept = torch.empty((2, batch, kv, rows, dim), dtype=q.dtype, device=q.device)
-        cache = (kept[0], kept[1], seen)
-    out = torch.empty((batch, len_q, heads * dim), dtype=q.dtype, device=q.device)
-    cos, sin = rope._tables(max(min(total, len_q + n_local), n_local + n_init), q.device)
-    q_bs, q_hs, q_ts, _ = q.stride()
-    k_bs, k_hs, k_ts, _ = k.stride()
-    p_bs, p_hs, p_ts, _ = pk.stride() if past_len else (0, 0, 0, 0)
-    q_at, k_at, v_at, o_at = q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr()
+        kept = torch.empty((2, batch, kv, rows, dim), dtype=dtype, device=device)
+        ck_at = kept.data_ptr()
+        cv_at = ck_at + 2 * batch * kv * rows * dim
+    cos, sin = rope._tables(max(min(total, len_q + n_local), n_local + n_init), device)
+    q_bs, q_ts, _ = q.stride()
+    k_bs, k_ts, _ = k.stride()
+    q_at, k_at, v_at = q.data_ptr(), k.data_ptr(), v.data_ptr()
     pk_at, pv_at = (pk.data_ptr(), pv.data_ptr()) if past_len else (None, None)
-    ck_at, cv_at = (kept.data_ptr(), kept.data_ptr() + 2 * batch * kv * rows * dim) if cache is not None else (None, None)
-    if cache is None:
-        head = rows = 0
     # fields in the order of the structure
     a = _lib.SinkWindow(
-        q_at, k_at, v_at, pk_at, pv_at, ck_at, cv_at, o_at, None, cos.data_ptr(), sin.data_ptr(), q_hs, q_ts, k_hs, k_ts, p_hs,
+        q_at, k_at, v_at, pk_at, pv_at, ck_at, cv_at, None, None, cos.data_ptr(), sin.data_ptr(), dim, q_ts, dim, k_ts, p_hs,
         p_ts, dim, heads * dim, len_q, past_len, seen, head, rows, cos.size(0), 0, heads, kv, dim, n_local, n_init,
-        1 if stream_positions else 0, _lib.dtype_code(q.dtype), 0)
+        1 if stream_positions else 0, _lib.dtype_code(dtype), 0)
     ref = ctypes.byref(a)
     lib = _lib.lib
     n = lib.infllm_sink_window_scratch(ref)
-    scratch = torch.empty(max(n, 16), dtype=torch.uint8, device=q.device)
-    a.d_scratch, a.scratch_bytes = scratch.data_ptr(), n
-    stream = torch.cuda.current_stream(q.device).cuda_stream
+    n_out = batch * len_q * heads * dim
+    if len_q == 1:  # one allocation: the scratch of a token is of the output's order
+        both = torch.empty(n_out + (n >> 1), dtype=dtype, device=device)
+        out, o_at = both[:n_out].view(batch, 1, heads * dim), both.data_ptr()
+        a.d_scratch = o_at + 2 * n_out
+    else:
+        out = torch.empty((batch, len_q, heads * dim), dtype=dtype, device=device)
+        scratch = torch.empty(max(n, 16), dtype=torch.uint8, device=device)
+        o_at, a.d_scratch = out.data_ptr(), scratch.data_ptr()
+    a.scratch_bytes = n
+    a.d_out = o_at
+    stream = _lib.raw_stream(device)
     for i in range(batch):
         if i:  # 2 bytes per element
             a.d_q, a.d_k, a.d_v = q_at + 2 * i * q_bs, k_at + 2 * i * k_bs, v_at + 2 * i * k_bs
             a.d_out = o_at + 2 * i * len_q * heads * dim
             if past_len:
                 a.d_past_k, a.d_past_v = pk_at + 2 * i * p_bs, pv_at + 2 * i * p_bs
-            if cache is not None:
+            if use_cache:
                 a.d_cache_k, a.d_cache_v = ck_at + 2 * i * kv * rows * dim, cv_at + 2 * i * kv * rows * dim
         rc = lib.infllm_sink_window_run(ref, stream)
         if rc:
             _lib.check(rc)
-    return out, cache
+    return out, ((kept[0], kept[1], seen) if use_cache else None)
 
 
 def _sink_window_forward(n_local, n_init, fattn, stream_positions):
@@ -99,20 +116,22 @@ def _sink_window_forward(n_local, n_init, fattn, stream_positions):
         def heads(x, n, length):  # (B, L, n*D) -> (B, n, L, D)
             return x.view(batch, length, n, dim_head).permute(0, 2, 1, 3)
 
-        q = heads(project_q(query), num_heads, len_q)
-        k = heads(project_k(key_value), num_heads_kv, len_new)
-        v = heads(project_v(key_value), num_heads_kv, len_new)
+        q, k, v = project_q(query), project_k(key_value), project_v(key_value)
         # The library does the whole call for the rotary embedding it knows; another one's rotations, other head
         # sizes and self-made caches are put together below from the attention class.
-        if (type(position_bias) is RotaryEmbeddingESM and position_bias.dim == dim_head == 128 and len_q == len_new and len_q > 0
-                and q.is_cuda and q.dtype in (torch.bfloat16, torch.float16) and k.dtype == v.dtype == q.dtype
-                and num_heads % num_heads_kv == 0 and (past_key_value is None or (
+        if type(position_bias) is RotaryEmbeddingESM and position_bias.dim == dim_head == 128 and len_q == len_new and len_q > 0 \
+                and q.is_cuda and q.dtype in _NATIVE and k.dtype == v.dtype == q.dtype and num_heads % num_heads_kv == 0 \
+                and q.shape == (batch, len_q, num_heads * 128) and k.shape == v.shape == (batch, len_q, num_heads_kv * 128) \
+                and (past_key_value is None or (
                     past_key_value[0].dtype == past_key_value[1].dtype == q.dtype and past_key_value[0].is_cuda
-                    and past_key_value[0].shape == past_key_value[1].shape == (batch, num_heads_kv, past_key_value[0].size(2), 128)))):
-            done = _run_native(position_bias, q, k, v, past_key_value, n_local, n_init, stream_positions, use_cache)
+                    and past_key_value[0].shape == past_key_value[1].shape == (
+                        batch, num_heads_kv, past_key_value[0].size(2), 128))):
+            done = _run_native(position_bias, q, k, v, num_heads, num_heads_kv, past_key_value, n_local, n_init,
+                               stream_positions, use_cache)
             if done is not None:
                 o = attention_out(done[0])
                 return (o, done[1]) if use_cache else o
+        q, k, v = heads(q, num_heads, len_q), heads(k, num_heads_kv, len_new), heads(v, num_heads_kv, len_new)
         q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
         seen = len_new
         if past_key_value is not None:
