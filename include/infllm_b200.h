@@ -326,6 +326,13 @@ int infllm_ctx_append(infllm_ctx* ctx, const void* d_q, int64_t q_hs, int64_t q_
                       const void* d_k, int64_t k_hs, int64_t k_ts,
                       const void* d_v, int64_t v_hs, int64_t v_ts,
                       void* d_out, int64_t o_hs, int64_t o_ts, int64_t len, void* stream);
+/* The same call for n memories (sequences of a batch, or, with per_seq > 1, units of a sequence): unit u = b * per_seq + h
+ * reads q at b * q_bs + h * q_us and k, v at b * k_bs + h / k_group * k_us, and writes out at b * o_bs + h * o_us
+ * (elements).  One-token calls share kernel launches where the sizes allow it. */
+int infllm_ctx_append_units(infllm_ctx* const* ctx, int n, int per_seq, int k_group,
+                            const void* d_q, int64_t q_bs, int64_t q_us, int64_t q_hs, int64_t q_ts,
+                            const void* d_k, const void* d_v, int64_t k_bs, int64_t k_us, int64_t k_hs, int64_t k_ts,
+                            void* d_out, int64_t o_bs, int64_t o_us, int64_t o_hs, int64_t o_ts, int64_t len, void* stream);
 
 /* Introspection (what the reference keeps as Python attributes). */
 typedef struct infllm_ctx_info {

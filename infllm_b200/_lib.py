@@ -171,6 +171,8 @@ SIGNATURES = {
     "infllm_ctx_reset": (c_int, [c_void_p]),
     "infllm_ctx_append": (c_int, [c_void_p, c_void_p, c_int64, c_int64, c_void_p, c_int64, c_int64, c_void_p,
                                   c_int64, c_int64, c_void_p, c_int64, c_int64, c_int64, c_void_p]),
+    "infllm_ctx_append_units": (c_int, [c_void_p, c_int, c_int, c_int] + [c_void_p] + [c_int64] * 4 + [c_void_p] * 2 + [c_int64] * 4
+                                + [c_void_p] + [c_int64] * 5 + [c_void_p]),
     "infllm_ctx_get_info": (c_int, [c_void_p, POINTER(CtxInfo)]),
     "infllm_ctx_profile": (c_int, [c_void_p, c_int]),
     "infllm_ctx_get_profile": (c_int, [c_void_p, POINTER(c_double), POINTER(c_double), POINTER(c_int64)]),

@@ -93,6 +93,7 @@ class ContextManager:
             raise ValueError("chunk_topk_calc must hold at least one exec block")  # the reference divides by zero
         self.chunk_topk_calc = chunk_topk_calc
         self._ctx = []  # native contexts, one per unit
+        self._unit_array = None
 
     # -- native contexts
     def _init(self, q, k):
@@ -186,30 +187,28 @@ class ContextManager:
         return out
 
     def _append_units(self, q, k, v, out, length):
-        """One native call per unit (sequence, or head of a sequence); addresses by arithmetic, 2 bytes per element."""
-        append, stream = _lib.lib.infllm_ctx_append, _lib.raw_stream(q.device)
+        """One native call for all units (sequences, or heads of sequences)."""
+        stream = _lib.raw_stream(q.device)
         q_bs, q_hs, q_ts, _ = q.stride()
         k_bs, k_hs, k_ts, _ = k.stride()
         o_bs, o_hs, o_ts, _ = out.stride()
-        q_at, k_at, v_at, o_at = q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr()
-        rc = 0
-        if self.perhead:
-            heads, g = self.num_heads, self.num_heads // self.num_heads_kv
-            for i, ctx in enumerate(self._ctx):
-                b, h = divmod(i, heads)
-                kv = 2 * (b * k_bs + h // g * k_hs)
-                rc = append(ctx, q_at + 2 * (b * q_bs + h * q_hs), q_hs, q_ts, k_at + kv, k_hs, k_ts, v_at + kv, k_hs, k_ts,
-                            o_at + 2 * (b * o_bs + h * o_hs), o_hs, o_ts, length, stream)
-                if rc:
-                    break
+        n = len(self._ctx)
+        if n == 1:
+            rc = _lib.lib.infllm_ctx_append(self._ctx[0], q.data_ptr(), q_hs, q_ts, k.data_ptr(), k_hs, k_ts, v.data_ptr(), k_hs,
+                                            k_ts, out.data_ptr(), o_hs, o_ts, length, stream)
         else:
-            for b, ctx in enumerate(self._ctx):
-                rc = append(ctx, q_at + 2 * b * q_bs, q_hs, q_ts, k_at + 2 * b * k_bs, k_hs, k_ts, v_at + 2 * b * k_bs, k_hs,
-                            k_ts, o_at + 2 * b * o_bs, o_hs, o_ts, length, stream)
-                if rc:
-                    break
+            per_seq, group, us = (self.num_heads, self.num_heads // self.num_heads_kv, 1) if self.perhead else (1, 1, 0)
+            rc = _lib.lib.infllm_ctx_append_units(
+                self._units(), n, per_seq, group, q.data_ptr(), q_bs, us * q_hs, q_hs, q_ts, k.data_ptr(), v.data_ptr(), k_bs,
+                us * k_hs, k_hs, k_ts, out.data_ptr(), o_bs, us * o_hs, o_hs, o_ts, length, stream)
         if rc:
             _lib.check(rc)
+
+    def _units(self):
+        """The native contexts as an array."""
+        if self._unit_array is None or len(self._unit_array) != len(self._ctx):
+            self._unit_array = (ctypes.c_void_p * len(self._ctx))(*self._ctx)
+        return self._unit_array
 
     def size(self, *args, **kwargs):
         return self.length

@@ -1559,19 +1559,71 @@ int unit_score_update(infllm_ctx* c, const std::vector<int32_t>& ids, const char
   return INFLLM_OK;
 }
 
-// A one-token append as one launch: ingestion, retrieval, attention and merge (token.cu).  S is the token's absolute
-// index, `at` its slot in the token buffers; the ids go, marked, to pt.h_words.
-int token_whole(infllm_ctx* c, infllm_ctx::PendingToken& pt, int runs, const char* q, int64_t q_hs, const char* k, int64_t k_hs,
-                const char* v, int64_t v_hs, char* out, int64_t o_hs, int64_t at, int64_t S, cudaStream_t s) {
+// Room for L more tokens in the token buffers, the rows behind them and the rotations of the keys before them.
+int prepare_tokens(infllm_ctx* c, int64_t L, cudaStream_t s) {
+  const infllm_config& g = c->cfg;
+  const int64_t D = g.head_dim, HKV = g.n_kv_heads, T = c->length;
+  const int esz = c->esz;
+  INFLLM_TRY(ensure_tokens(c, L, s));
+  TokenBuffers& tb = c->tb;
+  const int64_t kv_hs = tb.cap * D, at = T - tb.t0;
+  if (c->use_tc) {
+    // a 128-row tile that ends the window may reach past the last ingested token: keep those rows finite.
+    // Rows are zeroed well ahead of the data so that token-by-token appends rarely pay for it.
+    if (tb.zero_upto < std::min<int64_t>(tb.cap, at + L + 128)) {
+      const int64_t upto = std::min<int64_t>(tb.cap, at + L + 128 + 4096), pad = upto - (at + L);
+      INFLLM_CUDA_OK(cudaMemset2DAsync((char*)tb.v + (at + L) * D * esz, kv_hs * esz, 0, pad * D * esz, HKV, s));
+      INFLLM_CUDA_OK(cudaMemset2DAsync((char*)tb.k_rot + (at + L) * D * esz, kv_hs * esz, 0, pad * D * esz, HKV, s));
+      INFLLM_CUDA_OK(cudaMemset2DAsync((char*)tb.k_raw + (at + L) * D * esz, kv_hs * esz, 0, pad * D * esz, HKV, s));
+      tb.zero_upto = upto;
+    }
+  }
+  // RoPE: keys keep the position (token - rope_origin) until the table would run out
+  const int64_t win0 = std::max<int64_t>(T - g.n_local, 0);  // oldest key any query of this call can see locally
+  if (c->rope_origin < 0 || T + L - c->rope_origin > c->tab_len || win0 < c->rope_origin) {
+    c->rope_origin = win0;
+    if (T > win0)
+      INFLLM_TRY(rope_apply_launch((char*)tb.k_raw + (win0 - tb.t0) * D * esz, kv_hs, D,
+                                   (char*)tb.k_rot + (win0 - tb.t0) * D * esz, kv_hs, D, (int)HKV, T - win0, (int)D,
+                                   c->cos_t, c->sin_t, c->tab_len, 0, 1, g.dtype, s));
+  }
+  return INFLLM_OK;
+}
+
+// One-token appends over more units than a retrieval takes run ahead of the host (see append_sub).
+bool token_runs_ahead(const infllm_ctx* c) {
+  const infllm_config& g = c->cfg;
+  return g.head_dim == 128 && c->num_blocks > g.topk && g.topk <= kMaxSeg - 4 && !(g.debug_flags & 16) && g.chunk_topk_calc == 0 &&
+         g.cache_strategy == INFLLM_CACHE_LRU;
+}
+
+// Where the sizes allow it such a token is one launch: its runs per KV head over `sms` SMs, or 0 (per-kernel timing wants
+// the kernels apart).
+int token_one_launch(const infllm_ctx* c, int sms) {
+  const infllm_config& g = c->cfg;
+  if (!token_runs_ahead(c) || !c->use_tc || c->prof || c->comm) return 0;
+  return token_runs(g.n_heads, g.n_kv_heads, g.head_dim, c->num_blocks, g.topk, g.block_size, sms);
+}
+
+// A one-token append as one launch: ingestion, retrieval, attention and merge (token.cu).  token_begin prepares it,
+// token_end is what follows it on the stream; several contexts' tokens may share the launch between the two.  The ids
+// go, marked, to the pending token's h_words.
+int token_begin(infllm_ctx* c, const char* q, int64_t q_hs, const char* k, int64_t k_hs, const char* v, int64_t v_hs, char* out,
+                int64_t o_hs, TokenParams& P, cudaStream_t s) {
   const infllm_config& g = c->cfg;
   TokenBuffers& tb = c->tb;
-  const int64_t D = g.head_dim, kv_hs = tb.cap * D, wsz = sizeof(unsigned long long);
+  const int64_t S = c->length;
+  INFLLM_TRY(prepare_tokens(c, 1, s));
+  const int64_t D = g.head_dim, kv_hs = tb.cap * D, wsz = sizeof(unsigned long long), at = S - tb.t0;
   const int esz = c->esz;
-  TokenParams P;
+  c->ingest_event_due = true;
+  // at most kMaxOutstanding tokens ahead of the cache: apply the older retrievals first
+  while (c->pend_count >= infllm_ctx::kMaxOutstanding) INFLLM_TRY(settle_one(c, s));
+  infllm_ctx::PendingToken& pt = c->pend[(c->pend_head + c->pend_count) % infllm_ctx::kPendSlots];
   P.n_upd = 0;
   INFLLM_TRY(flush_table(c, s, &P));
   if (!c->tok_ids) {
-    c->tok_part_words = (size_t)runs * g.n_heads * 129;
+    c->tok_part_words = (size_t)token_one_launch(c, c->tok_sms) * g.n_heads * 129;
     INFLLM_CUDA_OK(dev_malloc((void**)&c->tok_ids, g.topk * wsz));
     INFLLM_CUDA_OK(dev_malloc((void**)&c->tok_parts, c->tok_part_words * wsz));
     c->tok_restart = true;
@@ -1608,14 +1660,61 @@ int token_whole(infllm_ctx* c, infllm_ctx::PendingToken& pt, int runs, const cha
   P.rest_begin[0] = 0;
   for (int i = 0; i < 3; ++i) P.rest_begin[i + 1] = P.rest_begin[i] + (P.rest[i].len + 15) / 16;
   P.ptrs = c->d_unit_ptrs, P.landing_at = c->tab_cap, P.unit_bytes = c->unit_bytes, P.unit_len = g.block_size;
-  P.n_heads = g.n_heads, P.n_kv = g.n_kv_heads, P.group = g.n_heads / g.n_kv_heads, P.n_runs = runs;
+  P.n_heads = g.n_heads, P.n_kv = g.n_kv_heads, P.group = g.n_heads / g.n_kv_heads, P.n_runs = 0;
   P.scale_log2 = kLog2e / sqrtf((float)D);
   P.part_words = c->tok_parts, P.logits = c->dec_logits, P.logit_hs = (int64_t)g.n_local + 1;
   P.win_score = tb.score + (wlo - tb.t0), P.score_hs = tb.cap;
   P.out = out, P.o_hs = o_hs;
   P.seq = c->tok_seq;
   P.err = c->tc_err, P.err_host = c->h_tc_err;
-  return token_launch(P, g.dtype, s);
+  pt.serial = c->call_serial;
+  pt.landing = c->landing_slots;
+  c->pend_count += 1;
+  trace_mark(c, s, TR_ATTN_BEGIN, 0);
+  return INFLLM_OK;
+}
+
+// what the last kernel that reads a token's keys leaves behind: ev_attn; ev_attn_prev: the exec block's before
+int mark_attention(infllm_ctx* c, cudaStream_t s) {
+  std::swap(c->ev_attn, c->ev_attn_prev);
+  c->attn_prev_recorded = c->attn_recorded;
+  INFLLM_CUDA_OK(cudaEventRecord(c->ev_attn, s));
+  c->attn_recorded = true;
+  return INFLLM_OK;
+}
+
+// A token sealed units: a one-token attention finds a unit through the table of unit addresses.  The new units are listed
+// at their place in the store, which the copy-out must have reached first (once per block_size tokens).
+int list_new_units(infllm_ctx* c, int64_t first_new, cudaStream_t s) {
+  INFLLM_CUDA_OK(cudaStreamWaitEvent(s, c->ev_d2h, 0));
+  c->d2h_synced_upto = c->d2h_synced_upto_urgent = c->num_blocks;
+  for (int64_t b = first_new; b < c->num_blocks; ++b) c->tab_updates[(int32_t)b] = -1;
+  return INFLLM_OK;
+}
+
+int token_undo(infllm_ctx* c, int rc) {  // the launch failed: there will be no ids to wait for
+  c->pend_count -= 1;
+  return rc;
+}
+
+int token_end(infllm_ctx* c, cudaStream_t s) {
+  INFLLM_TRY(mark_attention(c, s));
+  trace_mark(c, s, TR_ATTN_END, 0);
+  const SealPlan sp = plan_seal(c, c->length + 1);
+  const int64_t first_new = c->num_blocks;
+  int n_cand = 0;
+  INFLLM_TRY(seal_offload(c, first_new, sp.n_new, c->frontier + sp.take, s));
+  trace_mark(c, s, TR_URGENT_END, 0);
+  {
+    HostTimer ht(&c->host_us[5]);
+    INFLLM_TRY(seal_apply(c, sp, -1, &n_cand, s));
+  }
+  trace_mark(c, s, TR_SEAL_END, 0);
+  if (sp.n_new > 0) INFLLM_TRY(list_new_units(c, first_new, s));
+  trace_mark(c, s, TR_REST_END, 0);
+  c->length += 1;
+  c->counters.exec_blocks += 1;
+  return INFLLM_OK;
 }
 
 // one internal call of at most sub_max tokens whose exec-block boundaries coincide with the caller's
@@ -1626,44 +1725,16 @@ int append_sub(infllm_ctx* c, const char* q, int64_t q_hs, int64_t q_ts, const c
   const int64_t D = g.head_dim, H = g.n_heads, HKV = g.n_kv_heads, bs = g.block_size;
   const int esz = c->esz;
   const int64_t T = c->length;
-  INFLLM_TRY(ensure_tokens(c, L, s));
+  INFLLM_TRY(prepare_tokens(c, L, s));
   TokenBuffers& tb = c->tb;
   const int64_t kv_hs = tb.cap * D;  // head stride of the token buffers, elements
   // ---- ingest the new tokens
   const int64_t at = T - tb.t0;
   const int64_t q_hs_s = c->sub_max * D;
-  if (c->use_tc) {
-    // a 128-row tile that ends the window may reach past the last ingested token: keep those rows finite.
-    // Rows are zeroed well ahead of the data so that token-by-token appends rarely pay for it.
-    if (tb.zero_upto < std::min<int64_t>(tb.cap, at + L + 128)) {
-      const int64_t upto = std::min<int64_t>(tb.cap, at + L + 128 + 4096), pad = upto - (at + L);
-      INFLLM_CUDA_OK(cudaMemset2DAsync((char*)tb.v + (at + L) * D * esz, kv_hs * esz, 0, pad * D * esz, HKV, s));
-      INFLLM_CUDA_OK(cudaMemset2DAsync((char*)tb.k_rot + (at + L) * D * esz, kv_hs * esz, 0, pad * D * esz, HKV, s));
-      INFLLM_CUDA_OK(cudaMemset2DAsync((char*)tb.k_raw + (at + L) * D * esz, kv_hs * esz, 0, pad * D * esz, HKV, s));
-      tb.zero_upto = upto;
-    }
-  }
-  // RoPE: keys keep the position (token - rope_origin) until the table would run out
   if (c->chunk_mode && c->call_off % ((int64_t)(g.chunk_topk_calc / g.exc_block_size) * g.exc_block_size) == 0) c->chunk_n0 = c->num_blocks;
   bool ranked = false;  // the first exec block's ids have been asked for
-  const int64_t win0 = std::max<int64_t>(T - g.n_local, 0);  // oldest key any query of this call can see locally
-  if (c->rope_origin < 0 || T + L - c->rope_origin > c->tab_len || win0 < c->rope_origin) {
-    c->rope_origin = win0;
-    if (T > win0)
-      INFLLM_TRY(rope_apply_launch((char*)tb.k_raw + (win0 - tb.t0) * D * esz, kv_hs, D,
-                                   (char*)tb.k_rot + (win0 - tb.t0) * D * esz, kv_hs, D, (int)HKV, T - win0, (int)D,
-                                   c->cos_t, c->sin_t, c->tab_len, 0, 1, g.dtype, s));
-  }
-  // One-token appends over more units than a retrieval takes run ahead of the host (see below); where the sizes allow it
-  // the whole token is one launch (per-kernel timing wants the kernels apart).
-  const bool run_ahead = L == 1 && D == 128 && c->num_blocks > g.topk && g.topk <= kMaxSeg - 4 && !(g.debug_flags & 16) &&
-                         g.chunk_topk_calc == 0 && g.cache_strategy == INFLLM_CACHE_LRU;
-  const int tok_runs = run_ahead && c->use_tc && !c->prof && !c->comm
-                           ? token_runs((int)H, (int)HKV, (int)D, c->num_blocks, g.topk, (int)bs, c->tok_sms) : 0;
-  const bool one_launch = tok_runs > 0;
-  if (one_launch) {
-    c->ingest_event_due = true;
-  } else if (L == 1) {
+  const bool run_ahead = L == 1 && token_runs_ahead(c);
+  if (L == 1) {
     // one token: copies, the three rotations, the query mean and the cleared score column in one launch
     INFLLM_TRY(ingest_token_launch(q, q_hs, k, k_hs, v, v_hs, c->q_loc, c->q_glb, q_hs_s, c->qbar,
                                    (char*)tb.k_raw + at * D * esz, (char*)tb.k_rot + at * D * esz,
@@ -1772,16 +1843,12 @@ int append_sub(infllm_ctx* c, const char* q, int64_t q_hs, int64_t q_ts, const c
       infllm_ctx::PendingToken& pt = c->pend[slot];
       d_ids_tok = c->d_topk_ring + (int64_t)slot * std::max(1, g.topk);
       pt.seq = 0;
-      if (one_launch) {
-        INFLLM_TRY(token_whole(c, pt, tok_runs, q, q_hs, k, k_hs, v, v_hs, out, o_hs, at, S, s));
-      } else {
+      {
         INFLLM_TRY(ensure_scores(c, c->num_blocks, s));
         ProfScope ps(c, s, INFLLM_PROF_TOPK, (double)c->num_blocks * c->width * c->esz);
         INFLLM_TRY(score_topk(c, c->num_blocks, c->qbar, c->scores, d_ids_tok, s, 0, g.topk, direct ? pt.h_ids : nullptr));
       }
-      if (one_launch) {
-        // the ranking threads write the ids, marked, into the pinned words
-      } else if (direct) {
+      if (direct) {
         // the ranking threads wrote the ids into the pinned words themselves; the event that tells the host so is
         // recorded behind the token's last kernel, so that nothing stands between the kernels of the chain
         token_ev = pt.ev;
@@ -1793,7 +1860,7 @@ int append_sub(infllm_ctx* c, const char* q, int64_t q_hs, int64_t q_ts, const c
       }
       pt.serial = c->call_serial;
       c->pend_count += 1;
-      if (!one_launch) INFLLM_TRY(flush_table(c, s));
+      INFLLM_TRY(flush_table(c, s));
       pt.landing = c->landing_slots;
     }
     // bit 1 of the flags turns the look-ahead off; a chunk's retrievals are fixed when it starts, so they need none
@@ -1819,9 +1886,7 @@ int append_sub(infllm_ctx* c, const char* q, int64_t q_hs, int64_t q_ts, const c
     const char* qglb_eb = (const char*)c->q_glb + st * D * esz;
     const bool decode_path = lq == 1 && D == 128;
     double local_pairs_eb = 0;
-    if (one_launch) {
-      // launched above
-    } else if (decode_path) {
+    if (decode_path) {
       // ---- one-token exec block: split-K decode over [visible window | global segments]
       const int64_t wlo = std::max<int64_t>(E - g.n_local, ks);  // window mask of the single query
       std::vector<KvSeg> segs;
@@ -1963,11 +2028,7 @@ int append_sub(infllm_ctx* c, const char* q, int64_t q_hs, int64_t q_ts, const c
       }
     }
     if (g.cache_strategy == INFLLM_CACHE_LRU_S && !ids.empty()) INFLLM_TRY(unit_score_update(c, ids, qglb_eb, lq, s));
-    // ev_attn: behind this exec block's attention; ev_attn_prev: behind the previous one's
-    std::swap(c->ev_attn, c->ev_attn_prev);
-    c->attn_prev_recorded = c->attn_recorded;
-    INFLLM_CUDA_OK(cudaEventRecord(c->ev_attn, s));
-    c->attn_recorded = true;
+    INFLLM_TRY(mark_attention(c, s));
     if (token_ev) INFLLM_CUDA_OK(cudaEventRecord(token_ev, s));
     delete ht_attn;
     trace_mark(c, s, TR_ATTN_END, eb);
@@ -2010,13 +2071,7 @@ int append_sub(infllm_ctx* c, const char* q, int64_t q_hs, int64_t q_ts, const c
       INFLLM_TRY(seal_apply(c, sp, more ? eb + 1 : -1, &n_cand, s));
     }
     trace_mark(c, s, TR_SEAL_END, eb);
-    if (L == 1 && sp.n_new > 0) {
-      // a one-token attention finds a unit through the table of unit addresses: the new units are listed at their
-      // place in the store, which the copy-out must have reached first (once per block_size tokens)
-      INFLLM_CUDA_OK(cudaStreamWaitEvent(s, c->ev_d2h, 0));
-      c->d2h_synced_upto = c->d2h_synced_upto_urgent = c->num_blocks;
-      for (int64_t b = first_new; b < c->num_blocks; ++b) c->tab_updates[(int32_t)b] = -1;
-    }
+    if (L == 1 && sp.n_new > 0) INFLLM_TRY(list_new_units(c, first_new, s));
     if (!decode_path) INFLLM_TRY(local_scores(c, s, st, ks, lq, lk, j_u, lk, 0.0));
     trace_mark(c, s, TR_REST_END, eb);
     if (more)  // behind every launch of this exec block: the host waits for the look-ahead here
@@ -2322,15 +2377,8 @@ extern "C" int infllm_ctx_create(const infllm_config* cfg, infllm_ctx** out) {
   return INFLLM_OK;
 }
 
-extern "C" int infllm_ctx_append(infllm_ctx* c, const void* d_q, int64_t q_hs, int64_t q_ts, const void* d_k,
-                                 int64_t k_hs, int64_t k_ts, const void* d_v, int64_t v_hs, int64_t v_ts, void* d_out,
-                                 int64_t o_hs, int64_t o_ts, int64_t len, void* stream) {
-  if (!c) return fail(INFLLM_E_BADARG, "ctx_append: null context");
-  if (len < 0 || (len > 0 && (!d_q || !d_k || !d_v || !d_out))) return fail(INFLLM_E_BADARG, "ctx_append: bad argument");
-  if (len == 0) return INFLLM_OK;
-  if ((o_hs % 2) || (o_ts % 2) || ((uintptr_t)d_out % 4))
-    return fail(INFLLM_E_BADARG, "ctx_append: output rows must be 4-byte aligned");
-  cudaStream_t s = (cudaStream_t)stream;
+// the start of an append: the checks, the context's order on stream s
+static int open_call(infllm_ctx* c, cudaStream_t s) {
   INFLLM_CUDA_OK(cudaSetDevice(c->cfg.device));
   if (!c->initialized) INFLLM_TRY(lazy_init(c, s));
   INFLLM_TRY(order_behind_reset(c, s));
@@ -2345,9 +2393,47 @@ extern "C" int infllm_ctx_append(infllm_ctx* c, const void* d_q, int64_t q_hs, i
   c->last_stream = s;
   c->trace_topk.clear();
   c->counters.exec_blocks = 0;
+  return INFLLM_OK;
+}
+
+// its end; a token that seals nothing ends with its attention, ev_attn
+static int close_call(infllm_ctx* c, int64_t len, int64_t units_before, cudaStream_t s) {
+  if (len > 1 || c->num_blocks != units_before) {
+    INFLLM_CUDA_OK(cudaEventRecord(c->ev_last, s));
+    c->last_recorded = true;
+  }
+  c->failed = false;
+  return INFLLM_OK;
+}
+
+static int check_append(infllm_ctx* const* ctx, int n, const void* d_q, const void* d_k, const void* d_v, const void* d_out,
+                        int64_t o_hs, int64_t o_ts, int64_t len) {
+  for (int i = 0; i < n; ++i)
+    if (!ctx[i]) return fail(INFLLM_E_BADARG, "ctx_append: null context");
+  if (len < 0 || (len > 0 && (!d_q || !d_k || !d_v || !d_out))) return fail(INFLLM_E_BADARG, "ctx_append: bad argument");
+  if (len > 0 && ((o_hs % 2) || (o_ts % 2) || ((uintptr_t)d_out % 4)))
+    return fail(INFLLM_E_BADARG, "ctx_append: output rows must be 4-byte aligned");
+  return INFLLM_OK;
+}
+
+extern "C" int infllm_ctx_append(infllm_ctx* c, const void* d_q, int64_t q_hs, int64_t q_ts, const void* d_k,
+                                 int64_t k_hs, int64_t k_ts, const void* d_v, int64_t v_hs, int64_t v_ts, void* d_out,
+                                 int64_t o_hs, int64_t o_ts, int64_t len, void* stream) {
+  INFLLM_TRY(check_append(&c, 1, d_q, d_k, d_v, d_out, o_hs, o_ts, len));
+  if (len == 0) return INFLLM_OK;
+  cudaStream_t s = (cudaStream_t)stream;
+  INFLLM_TRY(open_call(c, s));
   const int esz = c->esz;
   const int64_t units_before = c->num_blocks;
   c->chunk_mode = c->cfg.chunk_topk_calc > 0 && len > 1;  // context_manager.py:749
+  if (const int runs = len == 1 ? token_one_launch(c, c->tok_sms) : 0) {
+    TokenParams P;
+    INFLLM_TRY(token_begin(c, (const char*)d_q, q_hs, (const char*)d_k, k_hs, (const char*)d_v, v_hs, (char*)d_out, o_hs, P, s));
+    P.n_runs = runs;
+    if (const int rc = token_launch(&P, 1, c->cfg.dtype, s)) return token_undo(c, rc);
+    INFLLM_TRY(token_end(c, s));
+    return close_call(c, 1, units_before, s);
+  }
   for (int64_t off = 0; off < len; off += c->sub_max) {
     const int64_t n = std::min<int64_t>(c->sub_max, len - off);
     c->call_off = off;
@@ -2356,11 +2442,72 @@ extern "C" int infllm_ctx_append(infllm_ctx* c, const void* d_q, int64_t q_hs, i
                           o_ts, n, s));
   }
   if (c->use_tc && len > 64) INFLLM_TRY(send_device_error(c, s));  // read by the next call (or by get_info)
-  if (len > 1 || c->num_blocks != units_before) {  // a token that seals nothing ends with its attention: ev_attn
-    INFLLM_CUDA_OK(cudaEventRecord(c->ev_last, s));
-    c->last_recorded = true;
+  return close_call(c, len, units_before, s);
+}
+
+// The same for n memories, unit u = b * per_seq + h at b * (batch stride) + h * (unit stride), k_group units to a KV head.
+// Tokens that are one launch each share launches: alone a token at ordinary context lengths is a chain of latencies on a
+// chip that is mostly idle, and four of them side by side take little longer than one.  Four sequences of 28/4 heads over
+// 75 units: 75 us as four launches, 29.7 us as one.
+extern "C" int infllm_ctx_append_units(infllm_ctx* const* ctx, int n, int per_seq, int k_group, const void* d_q, int64_t q_bs,
+                                       int64_t q_us, int64_t q_hs, int64_t q_ts, const void* d_k, const void* d_v, int64_t k_bs,
+                                       int64_t k_us, int64_t k_hs, int64_t k_ts, void* d_out, int64_t o_bs, int64_t o_us,
+                                       int64_t o_hs, int64_t o_ts, int64_t len, void* stream) {
+  if (n < 0 || (n > 0 && !ctx) || per_seq < 1 || k_group < 1) return fail(INFLLM_E_BADARG, "ctx_append_units: bad argument");
+  INFLLM_TRY(check_append(ctx, n, d_q, d_k, d_v, d_out, o_hs, o_ts, len));
+  if (n == 0 || len == 0) return INFLLM_OK;
+  cudaStream_t s = (cudaStream_t)stream;
+  auto q_at = [&](int u) { return (const char*)d_q + (u / per_seq * q_bs + u % per_seq * q_us) * 2; };  // 2 bytes per element
+  auto kv_at = [&](int u) { return (u / per_seq * k_bs + u % per_seq / k_group * k_us) * 2; };
+  auto o_at = [&](int u) { return (char*)d_out + (u / per_seq * o_bs + u % per_seq * o_us) * 2; };
+  TokenParams P[kTokMaxBatch];
+  for (int u = 0; u < n;) {
+    infllm_ctx* c = ctx[u];
+    const int room = len == 1 && c->initialized ? std::min(n - u, token_batch_max(c->cfg.n_kv_heads, c->tok_sms)) : 1;
+    // the tokens that go together: as many in a row as take the one launch and are of one kind (a context may be there once)
+    auto joins = [&](int w) {
+      const infllm_ctx* o = ctx[w];
+      for (int x = u; x < w; ++x)
+        if (ctx[x] == o) return false;
+      return o->initialized && o->cfg.device == c->cfg.device && o->cfg.dtype == c->cfg.dtype &&
+             o->cfg.n_kv_heads == c->cfg.n_kv_heads && token_one_launch(o, o->tok_sms / room) > 0;
+    };
+    int m = 0;
+    while (m < room && joins(u + m)) ++m;
+    if (m < 2) {
+      INFLLM_TRY(infllm_ctx_append(c, q_at(u), q_hs, q_ts, (const char*)d_k + kv_at(u), k_hs, k_ts, (const char*)d_v + kv_at(u), k_hs,
+                                   k_ts, o_at(u), o_hs, o_ts, len, stream));
+      ++u;
+      continue;
+    }
+    int ready = 0, rc = INFLLM_OK;
+    for (; ready < m; ++ready) {
+      infllm_ctx* o = ctx[u + ready];
+      rc = open_call(o, s);
+      if (rc == INFLLM_OK) {
+        o->chunk_mode = false;
+        rc = token_begin(o, q_at(u + ready), q_hs, (const char*)d_k + kv_at(u + ready), k_hs, (const char*)d_v + kv_at(u + ready),
+                         k_hs, o_at(u + ready), o_hs, P[ready], s);
+      }
+      if (rc != INFLLM_OK) break;
+    }
+    // (those before one that failed still go: their contexts count on it)
+    for (int i = 0; i < ready; ++i) P[i].n_runs = token_one_launch(ctx[u + i], ctx[u + i]->tok_sms / ready);
+    if (ready > 0) {
+      if (const int lrc = token_launch(P, ready, c->cfg.dtype, s)) {
+        for (int i = 0; i < ready; ++i) token_undo(ctx[u + i], lrc);
+        return lrc;
+      }
+    }
+    for (int i = 0; i < ready; ++i) {
+      infllm_ctx* o = ctx[u + i];
+      const int64_t units_before = o->num_blocks;
+      INFLLM_TRY(token_end(o, s));
+      INFLLM_TRY(close_call(o, 1, units_before, s));
+    }
+    if (rc != INFLLM_OK) return rc;
+    u += ready;
   }
-  c->failed = false;
   return INFLLM_OK;
 }
 

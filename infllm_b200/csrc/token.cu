@@ -19,6 +19,10 @@
 // a cooperative launch (all of them are resident), and every wait is bounded: one that runs out leaves the error record
 // (device and pinned host copy) and the token's output is not written.
 //
+// Several contexts' tokens share a launch: the y index of a CTA is its context, whose runs are what its share of the SMs
+// gives.  More rounds per warp, but the latencies of the chain are paid once: four contexts of 28/4 heads take 27.9 us
+// side by side and 18.7 us each one after another.
+//
 // Bound: HBM (representative keys + K/V); at small sizes the chain prologue - rows - ranking - units - merge.  160 units of
 // 32/8 heads: 14.4 us inside the kernel (prologue 1.9, rows 1.6, window 2 beside the ranking, ids at 7.1, units at 9.5,
 // partials at 10.3, log-sum-exps at 12.5) where the five launches took 27; 8192 units: 24 us, of which 10 stream
@@ -177,8 +181,14 @@ __device__ __forceinline__ void token_rank(const TokenParams& P, unsigned long l
   }
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kTokThreads, 1) token_kernel(const __grid_constant__ TokenParams P) {
+template <int NB>
+struct TokenBatch {
+  TokenParams p[NB];
+};
+
+template <typename T, int NB>
+__global__ void __launch_bounds__(kTokThreads, 1) token_kernel(const __grid_constant__ TokenBatch<NB> B) {
+  const TokenParams& P = B.p[NB == 1 ? 0 : blockIdx.y];
   extern __shared__ __align__(16) unsigned char dyn[];
   // [0, width) fp32 query mean, then the warps' attention results; the ranking CTA keeps its candidates here
   float* sq = reinterpret_cast<float*>(dyn);
@@ -194,6 +204,7 @@ __global__ void __launch_bounds__(kTokThreads, 1) token_kernel(const __grid_cons
     token_rank(P, reinterpret_cast<unsigned long long*>(dyn));
     return;
   }
+  if (cta > n_cta) return;  // (a context of the batch with fewer CTAs than another)
   const int group = P.group;
   const bool qrow = g < group;
   const T* bk = (const T*)P.bk;
@@ -491,23 +502,33 @@ __global__ void __launch_bounds__(kTokThreads, 1) token_kernel(const __grid_cons
     num += __shfl_xor_sync(0xffffffffu, num, 4);
     if (o < o_hi && sub == 0) ((T*)P.out)[(int64_t)(hkv * group + h) * P.o_hs + decode_dim(o & 127)] = Act<T>::from_f(num);
   }
+#pragma unroll 1
+  for (int i0 = tid; i0 < n_add; i0 += 4 * kTokThreads) {
+    if (i0 != tid) {
 #pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    const int i = tid + e * kTokThreads;
-    if (i < n_add) {
-      const float* lg;
-      float* sc;
-      int h;
-      column(i, &lg, &sc, &h);
-      *sc = pre_s[e] + exp2f(pre_l[e] - s_lse[h]);
+      for (int e = 0; e < 4; ++e) {
+        const int i = i0 + e * kTokThreads;
+        if (i < n_add) {
+          const float* lg;
+          float* sc;
+          int h;
+          column(i, &lg, &sc, &h);
+          pre_l[e] = __ldcg(lg);
+          pre_s[e] = *sc;
+        }
+      }
     }
-  }
-  for (int i = tid + 4 * kTokThreads; i < n_add; i += kTokThreads) {
-    const float* lg;
-    float* sc;
-    int h;
-    column(i, &lg, &sc, &h);
-    *sc += exp2f(__ldcg(lg) - s_lse[h]);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int i = i0 + e * kTokThreads;
+      if (i < n_add) {
+        const float* lg;
+        float* sc;
+        int h;
+        column(i, &lg, &sc, &h);
+        *sc = pre_s[e] + exp2f(pre_l[e] - s_lse[h]);
+      }
+    }
   }
   if (run == 0 && tid < group)  // the new token's column starts here
     P.win_score[(int64_t)(hkv * group + tid) * P.score_hs + P.rest[0].len] = exp2f(sm_m[kTokWarps][tid] - s_lse[tid]);
@@ -526,11 +547,31 @@ int token_runs(int n_heads, int n_kv_heads, int head_dim, int64_t n_units, int t
   return std::min((sms - 1) / n_kv_heads, kTokMaxRuns);
 }
 
-int token_launch(const TokenParams& P, int dtype, cudaStream_t s) {
-  if (P.n_upd > kTokMaxUpdates || P.n_runs < 1 || P.n_runs > kTokMaxRuns) return fail(INFLLM_E_BADARG, "token: bad argument");
-  const size_t smem = token_smem(P.width, P.n);
+// Two runs per KV head at least: below that the CTAs' rounds of window and units are long enough for a launch of their own.
+int token_batch_max(int n_kv_heads, int sms) { return std::max(1, std::min(kTokMaxBatch, sms / (2 * n_kv_heads + 1))); }
+
+template <typename T, int NB>
+static int token_launch_batch(const TokenParams* P, int n, cudaLaunchConfig_t& cfg) {
+  TokenBatch<NB> B;
+  std::copy(P, P + n, B.p);
+  auto kern = token_kernel<T, NB>;
+  // (the opt-in holds for the current device only: asked for at every launch)
+  INFLLM_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes));
+  INFLLM_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, B));
+  return INFLLM_OK;
+}
+
+int token_launch(const TokenParams* P, int n, int dtype, cudaStream_t s) {
+  size_t smem = 0;
+  int ctas = 0;
+  for (int i = 0; i < n; ++i) {
+    if (P[i].n_upd > kTokMaxUpdates || P[i].n_runs < 1 || P[i].n_runs > kTokMaxRuns) return fail(INFLLM_E_BADARG, "token: bad argument");
+    smem = std::max(smem, token_smem(P[i].width, P[i].n));
+    ctas = std::max(ctas, P[i].n_runs * P[i].n_kv + 1);
+  }
+  if (n < 1 || n > kTokMaxBatch) return fail(INFLLM_E_BADARG, "token: %d contexts", n);
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(P.n_runs * P.n_kv + 1);
+  cfg.gridDim = dim3(ctas, n);
   cfg.blockDim = dim3(kTokThreads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
@@ -540,10 +581,13 @@ int token_launch(const TokenParams& P, int dtype, cudaStream_t s) {
   cfg.attrs = at;
   cfg.numAttrs = 1;
   INFLLM_DISPATCH_DTYPE(dtype, T, {
-    auto kern = token_kernel<T>;
-    // (the opt-in holds for the current device only: asked for at every launch)
-    INFLLM_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    INFLLM_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, P));
+    if (n == 1) {
+      INFLLM_TRY((token_launch_batch<T, 1>(P, n, cfg)));
+    } else if (n <= 4) {
+      INFLLM_TRY((token_launch_batch<T, 4>(P, n, cfg)));
+    } else {
+      INFLLM_TRY((token_launch_batch<T, kTokMaxBatch>(P, n, cfg)));
+    }
   });
   INFLLM_LAUNCH_OK("token_kernel");
   return INFLLM_OK;

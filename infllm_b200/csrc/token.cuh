@@ -1,4 +1,4 @@
-// Parameters of the one-launch decode token (token.cu).
+// Parameters of the one-launch decode token (token.cu), of one context memory or of several at once.
 #pragma once
 #include "common.cuh"
 
@@ -46,8 +46,13 @@ struct TokenParams {
   unsigned long long upd_val[kTokMaxUpdates];
 };
 
-// runs per KV head (0: these sizes are not for token_kernel)
+constexpr int kTokMaxBatch = 8;  // contexts of one launch: their parameters are 14 KB
+
+// runs per KV head over `sms` SMs (0: these sizes are not for token_kernel)
 int token_runs(int n_heads, int n_kv_heads, int head_dim, int64_t n_units, int topk, int block_size, int sms);
-int token_launch(const TokenParams& P, int dtype, cudaStream_t s);
+// how many contexts with that many KV heads share a launch on a device of `sms` SMs
+int token_batch_max(int n_kv_heads, int sms);
+// n contexts' tokens, each with the n_runs its share of the SMs gives it
+int token_launch(const TokenParams* P, int n, int dtype, cudaStream_t s);
 
 }  // namespace infllm
