@@ -11,6 +11,8 @@
 // from their cache slots, the sink from its own buffer and the overflow from the remainder buffer.
 // Sealed units are copied to a pinned host store on a side stream and come back into one of
 // max_cached_block cache slots with cudaMemcpyAsync when retrieval asks for them.
+#include <sys/mman.h>
+
 #include <algorithm>
 #include <chrono>
 #include <cstring>
@@ -198,6 +200,12 @@ struct TokenBuffers {
 
 using namespace infllm;
 
+struct HostSlab {
+  void* p = nullptr;
+  void* map = nullptr;  // the mapping it lies in; null: memory of cudaHostAlloc
+  size_t map_bytes = 0;
+};
+
 struct infllm_ctx {
   infllm_config cfg;
   int esz = 2;                 // bytes per activation element
@@ -290,8 +298,8 @@ struct infllm_ctx {
   bool tok_restart = false;  // a token gave up, or the numbers are used up: the words start again
   int64_t call_serial = 0;
   cudaStream_t last_stream = nullptr;  // stream of the last append (for calls that take none)
-  std::vector<void*> slabs;  // pinned host memory
-  std::future<void*> slab_future;  // the next slab, being pinned by a helper thread
+  std::vector<HostSlab> slabs;  // pinned host memory
+  std::future<HostSlab> slab_future;  // the next slab, being pinned by a helper thread
   bool slab_pending = false;
   int64_t slab_units = 0;
   LruTable lru{0};
@@ -390,7 +398,7 @@ struct infllm_ctx {
   std::vector<std::vector<int32_t>> trace_topk;
   infllm_ctx_info counters{};
 
-  char* host_unit(int64_t b) { return (char*)slabs[b / slab_units] + (b % slab_units) * unit_bytes; }
+  char* host_unit(int64_t b) { return (char*)slabs[b / slab_units].p + (b % slab_units) * unit_bytes; }
   // Device copy of the store.  The reference keeps sealed units on the host because its GPUs have tens of GB; with
   // 180 GB of HBM a copy of the first dev_cap units stays on the device as well, and a cache refill of such a unit is
   // a device-to-device copy instead of a trip over PCIe.  Nothing else changes: the cache, its LRU order and the host
@@ -740,34 +748,68 @@ int ensure_block_k(infllm_ctx* c, int64_t n, cudaStream_t s) {
   return INFLLM_OK;
 }
 
-// Pinning a slab takes tens of milliseconds; a helper thread does it ahead of need
-void* alloc_slab(int device, size_t bytes) {
-  void* p = nullptr;
-  if (cudaSetDevice(device) != cudaSuccess || cudaHostAlloc(&p, bytes, cudaHostAllocDefault) != cudaSuccess) {
-    cudaGetLastError();
-    return nullptr;
+// A slab of the host store.  Anonymous memory on huge pages, touched by a few threads and then registered, because what
+// stops a decode is the driver's lock: cudaHostAlloc of 128 MiB holds it for 59 to 88 ms, in which no thread launches
+// anything, the registration of 64 huge pages for 5 to 14 ms (touching: 7 ms beside the launches).  Helper threads do it
+// ahead of need.  37-token turns, whose 152 KB each fill a slab every 860 turns: 88 us with the slabs there and 175 us when
+// they came from cudaHostAlloc within the measurement.
+HostSlab alloc_slab(int device, size_t bytes) {
+  HostSlab h;
+  if (cudaSetDevice(device) != cudaSuccess) return h;
+  constexpr size_t kHuge = 2u << 20, kTouchThreads = 4;
+  const size_t room = (bytes + kHuge - 1) / kHuge * kHuge;
+  void* map = mmap(nullptr, room + kHuge, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
+  if (map != MAP_FAILED) {
+    char* p = (char*)(((uintptr_t)map + kHuge - 1) / kHuge * kHuge);
+    madvise(p, room, MADV_HUGEPAGE);  // (advice: ordinary pages do too)
+    madvise(p, room, MADV_DONTFORK);  // as for memory of cudaHostAlloc
+    std::vector<std::future<void>> touch;
+    for (size_t i = 0; i < kTouchThreads; ++i)
+      touch.push_back(std::async(std::launch::async, [=] {
+        const size_t per = (room / kHuge + kTouchThreads - 1) / kTouchThreads * kHuge;
+        for (size_t o = i * per; o < std::min(room, (i + 1) * per); o += 4096) *(volatile char*)(p + o) = 0;
+      }));
+    for (auto& t : touch) t.get();
+    void* dev = nullptr;
+    if (cudaHostRegister(p, bytes, cudaHostRegisterDefault) == cudaSuccess) {
+      if (cudaHostGetDevicePointer(&dev, p, 0) == cudaSuccess && dev == p) {  // kernels read units in place by this address
+        h.p = p, h.map = map, h.map_bytes = room + kHuge;
+        return h;
+      }
+      cudaHostUnregister(p);
+    }
+    munmap(map, room + kHuge);
   }
-  return p;
+  cudaGetLastError();
+  if (cudaHostAlloc(&h.p, bytes, cudaHostAllocDefault) != cudaSuccess) {
+    cudaGetLastError();
+    h.p = nullptr;
+  }
+  return h;
+}
+
+void free_slab(const HostSlab& h) {
+  if (!h.p) return;
+  if (!h.map) {
+    cudaFreeHost(h.p);
+    return;
+  }
+  cudaHostUnregister(h.p);
+  munmap(h.map, h.map_bytes);
 }
 
 int ensure_host_units(infllm_ctx* c, int64_t n) {
   const size_t bytes = (size_t)(c->slab_units * c->unit_bytes);
   while ((int64_t)c->slabs.size() * c->slab_units < n) {
-    void* p = nullptr;
+    HostSlab h;
     if (c->slab_pending) {
-      p = c->slab_future.get();
+      h = c->slab_future.get();
       c->slab_pending = false;
     }
-    if (!p) {
-      cudaError_t e = cudaHostAlloc(&p, bytes, cudaHostAllocDefault);
-      if (e == cudaErrorMemoryAllocation && idle_trim(0, 0, 0, true) > 0) {
-        cudaGetLastError();
-        e = cudaHostAlloc(&p, bytes, cudaHostAllocDefault);
-      }
-      if (e != cudaSuccess) return fail(INFLLM_E_NOMEM, "pinned host store: cudaHostAlloc of %lld bytes failed: %s",
-                                        (long long)bytes, cudaGetErrorString(e));
-    }
-    c->slabs.push_back(p);
+    if (!h.p) h = alloc_slab(c->cfg.device, bytes);
+    if (!h.p && idle_trim(0, 0, 0, true) > 0) h = alloc_slab(c->cfg.device, bytes);
+    if (!h.p) return fail(INFLLM_E_NOMEM, "pinned host store: no %lld bytes of page-locked memory", (long long)bytes);
+    c->slabs.push_back(h);
   }
   // once the last slab is half full, the next one is pinned in the background
   if (!c->slab_pending && n + c->slab_units / 2 > (int64_t)c->slabs.size() * c->slab_units) {
@@ -2201,12 +2243,11 @@ static void ctx_free(infllm_ctx* c) {
     cudaEventDestroy(c->ev_seal);
     cudaEventDestroy(c->ev_stage);
     if (c->slab_pending) {
-      void* p = c->slab_future.get();
-      if (p) cudaFreeHost(p);
+      free_slab(c->slab_future.get());
     }
     for (cudaEvent_t e : c->slot_ev)
       if (e) cudaEventDestroy(e);
-    for (void* p : c->slabs) cudaFreeHost(p);
+    for (const HostSlab& h : c->slabs) free_slab(h);
     release_dev_slabs(c);
     cudaStreamDestroy(c->copy_stream);
     cudaEventDestroy(c->ev_main);
