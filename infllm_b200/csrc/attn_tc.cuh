@@ -48,6 +48,7 @@ struct ColsumTcParams {
   int32_t q_row0, k_tok0, n_heads, group;
   int64_t lq, lk;
   int32_t accumulate, tiles_per_cta;
+  int32_t late_wait;  // nothing is read that the kernel before on the stream writes: it is waited for at the end only
   int32_t lo_add, hi_add;  // queries [j + lo_add, j + hi_add] see key j; kNoBound: no bound on that side
   const float* lse;
   float* score;
@@ -71,7 +72,7 @@ int attn_tc2_launch(const AttnTcParams& P, int dtype, cudaStream_t s);
 int colsum_tc_launch_maps(const CUtensorMap& map_q, const CUtensorMap& map_k, int q_row0, int k_tok0, int n_heads,
                           int n_kv_heads, int64_t lq, int64_t lk, int mask_mode, int64_t mask_offset,
                           int64_t mask_size, const float* lse, float* score, int64_t score_hs, int accumulate,
-                          int dtype, cudaStream_t s);
+                          bool late_wait, int dtype, cudaStream_t s);
 int colsum_tc_launch(const void* q, int64_t q_hs, int64_t q_ts, const void* k, int64_t k_hs, int64_t k_ts, int n_heads,
                      int n_kv_heads, int64_t lq, int64_t lk, int mask_mode, int64_t mask_offset, int64_t mask_size,
                      const float* lse, float* score, int64_t score_hs, int accumulate, int dtype, cudaStream_t s);

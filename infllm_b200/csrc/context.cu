@@ -46,8 +46,8 @@ int block_topk_launch(const void* bk, int64_t n, int width, const float* qbar, f
                       int32_t* out_ids_copy = nullptr);
 int seal_score_launch(const void* k, int64_t k_hs, int64_t k_ts, const float* score, int64_t score_hs, int64_t tok0, int n_new,
                       int first_new, int block_size, int repr_topk, int n_heads, int n_kv_heads, int head_dim, void* bk,
-                      const int32_t* rows, int n_old, const float* qbar, float* scores, const int32_t* err, int32_t* err_out,
-                      int dtype, cudaStream_t s);
+                      const int32_t* rows, int n_old, const float* qbar, float* scores, unsigned long long* words, uint32_t seq,
+                      const int32_t* err, int32_t* err_out, bool chain, int dtype, cudaStream_t s);
 bool seal_score_ok(int block_size, int head_dim, int64_t k_hs, int64_t k_ts, const void* k);
 int mail_words_launch(const int32_t* src, int32_t* dst, cudaStream_t s);
 int ingest_rows_launch(const void* q, int64_t q_hs, int64_t q_ts, const void* k, int64_t k_hs, int64_t k_ts, const void* v,
@@ -339,7 +339,9 @@ struct infllm_ctx {
   std::unordered_map<int32_t, int64_t> staged_for;  // staged unit -> latest exec block that wants it
   int32_t* h_spec = nullptr;        // pinned: look-ahead ids
   int32_t* h_cand_rows = nullptr;   // pinned: candidate unit ids
-  float* h_cand_scores = nullptr;   // pinned: their scores
+  float* h_cand_scores = nullptr;   // pinned: their scores, where they are summed over ranks
+  unsigned long long* h_cand_words = nullptr;  // pinned: elsewhere, {score, cand_seq} words, read as they arrive
+  uint32_t cand_seq = 0;
   float* d_cand_scores = nullptr;   // device side of the same mailbox
   int32_t* d_spec = nullptr;        // device side of the look-ahead id mailboxes, (look_depth + 1) x topk
   cudaStream_t mail_stream = nullptr;  // carries the small result copies to the host, off the main stream
@@ -360,20 +362,21 @@ struct infllm_ctx {
   int64_t d2h_synced_upto = 0;  // units below this id are known to be in the host store as far as copy_stream is concerned
 
   cudaStream_t copy_stream = nullptr, aux_stream = nullptr;
-  // Sealing and the ranking of the next exec block's candidates run beside the main stream, which goes on with the rest
-  // of the column sums; ev_seal is behind the last sealing (on whichever stream it ran), ev_urgent behind the sums it needs.
-  cudaStream_t seal_stream = nullptr;
-  cudaEvent_t ev_urgent = nullptr;
-  bool seal_aside = false;  // the last sealing ran on seal_stream: the main stream has not waited for it
   cudaEvent_t ev_main = nullptr, ev_copy = nullptr, ev_sync = nullptr, ev_attn = nullptr, ev_attn_prev = nullptr, ev_spec = nullptr,
               ev_cand = nullptr, ev_seal = nullptr, ev_stage = nullptr;
   bool attn_recorded = false, attn_prev_recorded = false, spec_recorded = false;
+  cudaEvent_t look_after = nullptr;  // what the look-ahead of the next exec blocks follows: the last sealing
+  cudaEvent_t free_after = nullptr;  // what last read the slots that the running exec block's plan has freed
+  int64_t plan_serial = 0;
+  std::vector<int64_t> slot_freed;   // per slot: the plan that freed it
+  int64_t copy_serial = 0, copy_waited = 0;  // look-ahead copies marked so far; those the caller's stream has waited for
+  std::vector<int64_t> slot_serial;  // per slot: the number of the last one into it
   cudaStream_t urgent_stream = nullptr;  // copies an exec block is waiting for, past the queue of staged copies
   // A reset waits for nothing: it marks where every stream of the context stands, and the next append orders all of
   // them behind those marks (order_behind_reset).
   cudaEvent_t ev_last = nullptr;  // behind the last kernel of an append on the caller's stream, where ev_attn is not
   bool last_recorded = false;
-  cudaEvent_t ev_side[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
+  cudaEvent_t ev_side[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
   bool reset_pending = false, reset_attn = false, reset_last = false;
   bool failed = false;  // an append gave up half-way: the context is not handed to anybody else afterwards
 
@@ -523,14 +526,12 @@ int lazy_init(infllm_ctx* c, cudaStream_t s) {
     int lo = 0, hi = 0;  // the look-ahead kernels are short and latency matters: highest priority
     INFLLM_CUDA_OK(cudaDeviceGetStreamPriorityRange(&lo, &hi));
     INFLLM_CUDA_OK(cudaStreamCreateWithPriority(&c->aux_stream, cudaStreamNonBlocking, hi));
-    INFLLM_CUDA_OK(cudaStreamCreateWithPriority(&c->seal_stream, cudaStreamNonBlocking, hi));
   }
   INFLLM_CUDA_OK(cudaEventCreateWithFlags(&c->ev_spec, cudaEventDisableTiming));
   INFLLM_CUDA_OK(cudaEventCreateWithFlags(&c->ev_cand, cudaEventDisableTiming));
   INFLLM_CUDA_OK(cudaEventCreateWithFlags(&c->ev_seal, cudaEventDisableTiming));
   INFLLM_CUDA_OK(cudaEventCreateWithFlags(&c->ev_stage, cudaEventDisableTiming));
   INFLLM_CUDA_OK(cudaEventCreateWithFlags(&c->ev_last, cudaEventDisableTiming));
-  INFLLM_CUDA_OK(cudaEventCreateWithFlags(&c->ev_urgent, cudaEventDisableTiming));
   for (auto& e : c->ev_side) INFLLM_CUDA_OK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
 
   const int64_t D = g.head_dim, H = g.n_heads, HKV = g.n_kv_heads;
@@ -589,6 +590,8 @@ int lazy_init(infllm_ctx* c, cudaStream_t s) {
   }
   INFLLM_CUDA_OK(cudaHostAlloc((void**)&c->h_cand_rows, c->cand_cap * sizeof(int32_t), cudaHostAllocDefault));
   INFLLM_CUDA_OK(cudaHostAlloc((void**)&c->h_cand_scores, c->cand_cap * sizeof(float), cudaHostAllocDefault));
+  INFLLM_CUDA_OK(cudaHostAlloc((void**)&c->h_cand_words, c->cand_cap * sizeof(unsigned long long), cudaHostAllocDefault));
+  memset(c->h_cand_words, 0, c->cand_cap * sizeof(unsigned long long));
   INFLLM_CUDA_OK(dev_malloc((void**)&c->d_cand_scores, c->cand_cap * sizeof(float)));
   INFLLM_CUDA_OK(dev_malloc((void**)&c->d_spec, (c->look_depth + 1) * std::max(1, g.topk) * sizeof(int32_t)));
   INFLLM_CUDA_OK(cudaStreamCreateWithFlags(&c->mail_stream, cudaStreamNonBlocking));
@@ -636,6 +639,8 @@ int lazy_init(infllm_ctx* c, cudaStream_t s) {
   c->free_slots.init((int)n_slots);
   c->slot_ev.assign(n_slots, nullptr);
   c->slot_ev_used.assign(n_slots, 0);
+  c->slot_freed.assign(n_slots, 0);
+  c->slot_serial.assign(n_slots, 0);
   c->slab_units = std::max<int64_t>(16, (128ll << 20) / c->unit_bytes);
   c->dev_cap = (int64_t)g.device_store_mb * (1ll << 20) / c->unit_bytes;  // device copy of the store, in units
   c->initialized = true;
@@ -647,7 +652,7 @@ int lazy_init(infllm_ctx* c, cudaStream_t s) {
 int order_behind_reset(infllm_ctx* c, cudaStream_t s) {
   if (!c->reset_pending) return INFLLM_OK;
   c->reset_pending = false;
-  cudaStream_t side[6] = {c->copy_stream, c->urgent_stream, c->aux_stream, c->d2h_stream, c->mail_stream, c->seal_stream};
+  cudaStream_t side[5] = {c->copy_stream, c->urgent_stream, c->aux_stream, c->d2h_stream, c->mail_stream};
   for (cudaEvent_t e : c->ev_side) INFLLM_CUDA_OK(cudaStreamWaitEvent(s, e, 0));
   if (c->reset_attn) INFLLM_CUDA_OK(cudaStreamWaitEvent(s, c->ev_attn, 0));
   if (c->reset_last) INFLLM_CUDA_OK(cudaStreamWaitEvent(s, c->ev_last, 0));
@@ -887,9 +892,8 @@ int lookahead_launch(infllm_ctx* c, int64_t target, cudaStream_t s) {
   la.n_spec = c->num_blocks;
   la.ids.clear();
   if (la.n_spec <= g.topk) return INFLLM_OK;  // every known unit is a candidate; nothing to rank
-  // ev_seal was recorded on s right after the last sealing (or after the query means at the start of the
-  // call): the look-ahead needs nothing that s enqueued later, in particular not the rest of the score pass
-  INFLLM_CUDA_OK(cudaStreamWaitEvent(c->aux_stream, c->ev_seal, 0));
+  // recorded on s behind the last exec block's sealing, or behind the query means at the start of the call
+  INFLLM_CUDA_OK(cudaStreamWaitEvent(c->aux_stream, c->look_after, 0));
   if (la.n_spec > c->scores_aux_cap) {
     int64_t cap = std::max<int64_t>(1024, c->scores_aux_cap);
     while (cap < la.n_spec) cap *= 2;
@@ -926,6 +930,7 @@ int mark_slot_copy(infllm_ctx* c, void* slot_ptr) {
   if (!c->slot_ev[slot]) INFLLM_CUDA_OK(cudaEventCreateWithFlags(&c->slot_ev[slot], cudaEventDisableTiming));
   INFLLM_CUDA_OK(cudaEventRecord(c->slot_ev[slot], c->copy_stream));
   c->slot_ev_used[slot] = 1;
+  c->slot_serial[slot] = ++c->copy_serial;
   return INFLLM_OK;
 }
 
@@ -972,7 +977,7 @@ int lookahead_stage(infllm_ctx* c, int64_t target) {
   }
   if (!src.empty()) {
     // the spare slots taken above may have held units that the previous exec block's attention read
-    if (c->attn_prev_recorded) INFLLM_CUDA_OK(cudaStreamWaitEvent(c->copy_stream, c->ev_attn_prev, 0));
+    if (c->free_after) INFLLM_CUDA_OK(cudaStreamWaitEvent(c->copy_stream, c->free_after, 0));
     trace_mark(c, c->copy_stream, TR_STAGE_BEGIN, target);  // behind the waits: the interval is copy time only
     // Units that have a device copy are gathered by the copy kernel (one launch for the batch); units that only the
     // pinned host store holds travel by one cudaMemcpyAsync each on the copy engine: a kernel that reads host memory
@@ -1003,6 +1008,28 @@ int lookahead_stage(infllm_ctx* c, int64_t target) {
   return INFLLM_OK;
 }
 
+// A word {value, seq} that a kernel writes to pinned memory, as soon as it is there - an event behind the kernel arrives 3 us
+// later.  Bounded: the kernels' own waits end after a second or two and leave the error record; the rest of the limit is
+// for work ahead of the kernel on its stream.
+int wait_word(infllm_ctx* c, const unsigned long long* p, uint32_t seq, uint32_t* value) {
+  const auto t0 = std::chrono::steady_clock::now();
+  for (unsigned turn = 1;; ++turn) {
+    const unsigned long long w = *(const volatile unsigned long long*)p;
+    if ((uint32_t)(w >> 32) == seq) {
+      *value = (uint32_t)w;
+      return INFLLM_OK;
+    }
+    for (int spin = 0; spin < 32; ++spin) __builtin_ia32_pause();
+    if (turn % 64) continue;
+    if (c->h_tc_err && *(volatile int32_t*)c->h_tc_err) INFLLM_TRY(check_device_error(c, c->last_stream));
+    if (turn % 4096) continue;
+    const cudaError_t e = cudaStreamQuery(c->last_stream);
+    if (e != cudaSuccess && e != cudaErrorNotReady) INFLLM_CUDA_OK(e);
+    if (std::chrono::steady_clock::now() - t0 > std::chrono::seconds(60))
+      return fail(INFLLM_E_TIMEOUT, "a result that a kernel sends to the host did not arrive");
+  }
+}
+
 // the candidates of the next exec block once n_now units exist: what its look-ahead found, then the units sealed since.
 // *n_old of the *n exist already; none when every unit is retrieved anyway (context_manager.py:370-371).
 int candidates_list(infllm_ctx* c, int64_t eb_next, int64_t n_now, int* n_old, int* n) {
@@ -1028,7 +1055,15 @@ int candidates_finish(infllm_ctx* c, int n_cand, std::vector<int32_t>* ids) {
     for (int64_t b = 0; b < c->num_blocks; ++b) ids->push_back((int32_t)b);
     return INFLLM_OK;
   }
-  INFLLM_CUDA_OK(cudaEventSynchronize(c->comm ? c->ev_cand : c->ev_seal));
+  if (c->comm) {
+    INFLLM_CUDA_OK(cudaEventSynchronize(c->ev_cand));
+  } else {
+    for (int i = 0; i < n_cand; ++i) {
+      uint32_t bits = 0;
+      INFLLM_TRY(wait_word(c, c->h_cand_words + i, c->cand_seq, &bits));
+      memcpy(c->h_cand_scores + i, &bits, sizeof(float));
+    }
+  }
   INFLLM_TRY(check_device_error(c, c->mail_stream));
   std::vector<int> order(n_cand);
   for (int i = 0; i < n_cand; ++i) order[i] = i;
@@ -1055,6 +1090,17 @@ int plan_and_refill(infllm_ctx* c, const std::vector<int32_t>& ids, int64_t eb, 
   const infllm_config& g = c->cfg;
   const bool track = mode != PLAN_PREFILL;
   if (!track) c->table_valid = false;
+  c->plan_serial += 1;
+  c->free_after = c->attn_recorded ? c->ev_attn : nullptr;
+  // s waits for the look-ahead copies into the slots it is about to read: for the last of them, they are all on one stream
+  int last_copy = -1;
+  auto needs_copy = [&](int slot) {
+    if (c->slot_ev_used[slot] && (last_copy < 0 || c->slot_serial[slot] > c->slot_serial[last_copy])) last_copy = slot;
+  };
+  auto give = [&](int slot, int32_t unit) {
+    c->free_slots.give(slot, unit);
+    c->slot_freed[slot] = c->plan_serial;
+  };
   std::vector<int32_t> evicted;
   c->lru.plan(ids.data(), (int)ids.size(), &evicted);
   for (int32_t b : evicted) {  // MemoryUnit.offload -> CudaCache.delete (context_manager.py:104-109)
@@ -1072,7 +1118,7 @@ int plan_and_refill(infllm_ctx* c, const std::vector<int32_t>& ids, int64_t eb, 
         c->staged[b] = it->second;
         c->staged_for[b] = wanted_by;
       } else {
-        c->free_slots.give(it->second, b);  // (a one-token attention goes on finding it there)
+        give(it->second, b);  // (a one-token attention goes on finding it there)
       }
       c->slot_of.erase(it);
     }
@@ -1090,12 +1136,12 @@ int plan_and_refill(infllm_ctx* c, const std::vector<int32_t>& ids, int64_t eb, 
     if (c->slot_of.count(b) || c->staged.count(b)) continue;
     const int slot = c->free_slots.claim(b);
     if (slot < 0) continue;
-    if (c->slot_ev_used[slot]) INFLLM_CUDA_OK(cudaStreamWaitEvent(s, c->slot_ev[slot], 0));  // an abandoned look-ahead copy
+    needs_copy(slot);  // an abandoned look-ahead copy
     c->slot_of[b] = slot;
     if (track) c->tab_updates[b] = slot;
     back.push_back(b);
   }
-  bool late = false;
+  bool late = false, late_attn = false;
   std::vector<const void*> late_src;
   std::vector<void*> late_dst;
   for (int32_t b : ids) {
@@ -1114,7 +1160,7 @@ int plan_and_refill(infllm_ctx* c, const std::vector<int32_t>& ids, int64_t eb, 
       if (track) c->tab_updates[b] = st->second;
       // s waits for THIS unit's copy: a unit sealed a moment ago can be staged for a later exec block and still be
       // retrieved by this one, so the event of "this exec block's batch" would not cover it
-      if (c->slot_ev_used[st->second]) INFLLM_CUDA_OK(cudaStreamWaitEvent(s, c->slot_ev[st->second], 0));
+      needs_copy(st->second);
       c->staged.erase(st);
       c->staged_for.erase(b);
       continue;
@@ -1138,7 +1184,7 @@ int plan_and_refill(infllm_ctx* c, const std::vector<int32_t>& ids, int64_t eb, 
       auto victim = c->staged.begin();
       for (auto it2 = c->staged.begin(); it2 != c->staged.end(); ++it2)
         if (std::find(ids.begin(), ids.end(), it2->first) == ids.end()) { victim = it2; break; }
-      c->free_slots.give(victim->second, -1);
+      give(victim->second, -1);
       if (track) c->tab_updates[victim->first] = -1;
       c->staged_for.erase(victim->first);
       c->staged.erase(victim);
@@ -1163,9 +1209,15 @@ int plan_and_refill(infllm_ctx* c, const std::vector<int32_t>& ids, int64_t eb, 
       continue;
     }
     if (mode == PLAN_DECODE_ASYNC) c->tab_updates[b] = slot;  // no landing slot was free: fetched like a waited-for refill
-    if (!late) {
-      // slots freed above may still be read by the previous exec block's attention
+    // The previous exec block may still be reading a slot that was freed above - one freed before has only been read by
+    // those before it - and a token any slot that its table of addresses names.
+    const bool busy = track || c->slot_freed[slot] == c->plan_serial;
+    if (busy && !late_attn) {
       if (c->attn_recorded) INFLLM_CUDA_OK(cudaStreamWaitEvent(c->urgent_stream, c->ev_attn, 0));
+      late_attn = true;
+    }
+    if (!late) {
+      if (!busy && c->attn_prev_recorded) INFLLM_CUDA_OK(cudaStreamWaitEvent(c->urgent_stream, c->ev_attn_prev, 0));
       late = true;
       trace_mark(c, c->urgent_stream, TR_LATE_BEGIN, eb);
     }
@@ -1192,12 +1244,16 @@ int plan_and_refill(infllm_ctx* c, const std::vector<int32_t>& ids, int64_t eb, 
   // ordered behind the unfinished ones on the side stream; no kernel reads them)
   for (auto it = c->staged.begin(); it != c->staged.end();) {
     if (c->staged_for[it->first] <= eb) {  // staged for this exec block (or an earlier one) and not taken
-      c->free_slots.give(it->second, it->first);
+      give(it->second, it->first);
       c->staged_for.erase(it->first);
       it = c->staged.erase(it);
     } else {
       ++it;
     }
+  }
+  if (last_copy >= 0 && c->slot_serial[last_copy] > c->copy_waited) {
+    INFLLM_CUDA_OK(cudaStreamWaitEvent(s, c->slot_ev[last_copy], 0));
+    c->copy_waited = c->slot_serial[last_copy];
   }
   if (!late_src.empty())
     INFLLM_TRY(stage_units_launch(late_src.data(), late_dst.data(), (int)late_src.size(), c->unit_bytes, c->urgent_stream));
@@ -1293,23 +1349,15 @@ int flush_table(infllm_ctx* c, cudaStream_t s, TokenParams* tok = nullptr) {
 }
 
 // The ids of a one-launch token, as its ranking threads write them: long before the token is through, so that the host
-// prepares the next one under its attention.  Bounded: the kernel's own waits end after a second or two and leave the
-// error record; the rest of the limit is for work ahead of the token on its stream.
+// prepares the next one under its attention.
 int wait_words(infllm_ctx* c, infllm_ctx::PendingToken& p) {
-  const int k = c->cfg.topk;
-  const auto t0 = std::chrono::steady_clock::now();
-  for (int i = 0; i < k;) {
-    const unsigned long long w = *(volatile unsigned long long*)(p.h_words + i);
-    if ((uint32_t)(w >> 32) == p.seq) {
-      p.h_ids[i++] = (int32_t)(uint32_t)w;
-      continue;
-    }
-    for (int spin = 0; spin < 64; ++spin) __builtin_ia32_pause();
-    if (*(volatile int32_t*)c->h_tc_err) INFLLM_TRY(check_device_error(c, c->last_stream));
-    if (std::chrono::steady_clock::now() - t0 > std::chrono::seconds(60)) {
+  for (int i = 0; i < c->cfg.topk; ++i) {
+    uint32_t id = 0;
+    if (const int rc = wait_word(c, p.h_words + i, p.seq, &id)) {
       c->tok_restart = true;
-      return fail(INFLLM_E_TIMEOUT, "the retrieved ids of a token did not arrive");
+      return rc;
     }
+    p.h_ids[i] = (int32_t)id;
   }
   return INFLLM_OK;
 }
@@ -1380,9 +1428,9 @@ SealPlan plan_seal(const infllm_ctx* c, int64_t end) {
 }
 
 // Sealing, and, with eb_next >= 0, the scores of exec block eb_next's candidates in the same launch: *n_cand of them, on
-// their way to the host with ev_seal behind them.  When there is a next exec block this runs on seal_stream: what it reads -
-// keys, and the scores of tokens that have left every later query's window - the main stream does not write again.
-int seal_apply(infllm_ctx* c, const SealPlan& sp, int64_t eb_next, int* n_cand, cudaStream_t s) {
+// their way to the host as words.  `behind_sums`: the last launch on s was the column sums of the tokens to be sealed;
+// *chained says whether this one was chained to it (launch_chained) and lets the next one start at once.
+int seal_apply(infllm_ctx* c, const SealPlan& sp, int64_t eb_next, int* n_cand, bool behind_sums, bool* chained, cudaStream_t s) {
   const infllm_config& g = c->cfg;
   TokenBuffers& tb = c->tb;
   const int64_t D = g.head_dim, HKV = g.n_kv_heads, bs = g.block_size;
@@ -1398,33 +1446,33 @@ int seal_apply(infllm_ctx* c, const SealPlan& sp, int64_t eb_next, int* n_cand, 
   }
   if (c->init_len == g.n_init) c->init_full = true;
   const int n_new = sp.n_new;
-  const bool aside = eb_next >= 0 && !c->comm, grow = n_new > 0 && c->num_blocks + n_new > c->block_k_cap;
-  if (c->seal_aside && (!aside || grow)) INFLLM_CUDA_OK(cudaStreamWaitEvent(s, c->ev_seal, 0));
+  const bool grow = n_new > 0 && c->num_blocks + n_new > c->block_k_cap;
   if (grow) INFLLM_TRY(ensure_block_k(c, c->num_blocks + n_new, s));
-  if (aside) {
-    INFLLM_CUDA_OK(cudaEventRecord(c->ev_urgent, s));
-    INFLLM_CUDA_OK(cudaStreamWaitEvent(c->seal_stream, c->ev_urgent, 0));
-    s = c->seal_stream;
-  }
-  c->seal_aside = aside;
+  *chained = false;
   int n_old = 0;
   *n_cand = 0;
   if (eb_next >= 0) INFLLM_TRY(candidates_list(c, eb_next, c->num_blocks + n_new, &n_old, n_cand));
   const float* qbar = *n_cand > 0 ? c->qbar + eb_next * c->width : nullptr;
   // the scores go straight to pinned memory, unless they are summed over ranks first
-  float* scores = c->comm ? c->d_cand_scores : c->h_cand_scores;
+  float* scores = c->comm ? c->d_cand_scores : nullptr;
+  unsigned long long* words = c->comm ? nullptr : c->h_cand_words;
+  if (qbar && ++c->cand_seq == 0) {  // the numbers are used up: no word carries one any more
+    memset(c->h_cand_words, 0, c->cand_cap * sizeof(unsigned long long));
+    c->cand_seq = 1;
+  }
   const int64_t tok0 = c->frontier - tb.t0;
   if (seal_score_ok((int)bs, (int)D, tb.cap * D, D, tb.k_raw)) {
+    *chained = behind_sums && n_new > 0 && eb_next >= 0 && !c->comm && !grow && sp.take == 0;
     if (n_new > 0 || qbar)
       INFLLM_TRY(seal_score_launch(tb.k_raw, tb.cap * D, D, tb.score, tb.cap, tok0, n_new, (int)c->num_blocks, (int)bs, g.repr_topk,
-                                   g.n_heads, g.n_kv_heads, (int)D, c->block_k, c->h_cand_rows, n_old, qbar, scores, c->tc_err,
-                                   qbar ? c->h_tc_err : nullptr, g.dtype, s));
+                                   g.n_heads, g.n_kv_heads, (int)D, c->block_k, c->h_cand_rows, n_old, qbar, scores, words, c->cand_seq,
+                                   c->tc_err, qbar ? c->h_tc_err : nullptr, *chained, g.dtype, s));
   } else {
     INFLLM_TRY(repr_select_launch(tb.k_raw, tb.cap * D, D, tb.score, tb.cap, tok0, n_new, (int)bs, g.repr_topk, g.n_heads,
                                   g.n_kv_heads, (int)D, (char*)c->block_k + c->num_blocks * c->width * c->esz, g.dtype, s));
     if (qbar)  // every candidate exists by now
       INFLLM_TRY(seal_score_launch(nullptr, 0, 0, nullptr, 0, 0, 0, 0, 1, 1, g.n_heads, g.n_kv_heads, (int)D, c->block_k, c->h_cand_rows,
-                                   *n_cand, qbar, scores, c->tc_err, c->h_tc_err, g.dtype, s));
+                                   *n_cand, qbar, scores, words, c->cand_seq, c->tc_err, c->h_tc_err, false, g.dtype, s));
   }
   trace_mark(c, s, TR_REPR_END, c->num_blocks);
   c->num_blocks += n_new;
@@ -1437,7 +1485,6 @@ int seal_apply(infllm_ctx* c, const SealPlan& sp, int64_t eb_next, int* n_cand, 
                                    c->mail_stream));
     INFLLM_CUDA_OK(cudaEventRecord(c->ev_cand, c->mail_stream));
   }
-  if (eb_next >= 0) INFLLM_CUDA_OK(cudaEventRecord(c->ev_seal, s));
   return INFLLM_OK;
 }
 
@@ -1554,7 +1601,7 @@ int seal_offload(infllm_ctx* c, int64_t first, int n_new, int64_t tok0, cudaStre
 // column sums of the local stage for the window keys [j_begin, j_end) (indices relative to the window start ks),
 // added into the score buffer; `work` is the FLOP count attributed to this launch
 int local_scores(infllm_ctx* c, cudaStream_t s, int64_t st, int64_t ks, int64_t lq, int64_t lk, int64_t j_begin,
-                 int64_t j_end, double work) {
+                 int64_t j_end, double work, bool late_wait = false) {
   if (j_end <= j_begin) return INFLLM_OK;
   const infllm_config& g = c->cfg;
   TokenBuffers& tb = c->tb;
@@ -1563,7 +1610,7 @@ int local_scores(infllm_ctx* c, cudaStream_t s, int64_t st, int64_t ks, int64_t 
   ProfScope ps(c, s, INFLLM_PROF_COLSUM, work);
   if (c->use_tc && lq > 1 && lq <= 512)
     return colsum_tc_launch_maps(c->m_qloc, c->m_krot, (int)st, (int)tok, (int)H, (int)HKV, lq, n, INFLLM_MASK_WINDOW,
-                                 off, g.n_local, c->lse, tb.score + tok, tb.cap, 1, g.dtype, s);
+                                 off, g.n_local, c->lse, tb.score + tok, tb.cap, 1, late_wait, g.dtype, s);
   return attn_colsum_launch((const char*)c->q_loc + st * D * c->esz, c->sub_max * D, D,
                             (char*)tb.k_rot + tok * D * c->esz, tb.cap * D, D, (int)H, (int)HKV, lq, n, (int)D,
                             INFLLM_MASK_WINDOW, off, g.n_local, c->lse, tb.score + tok, tb.cap, 1, g.dtype, s);
@@ -1716,7 +1763,7 @@ int token_begin(infllm_ctx* c, const char* q, int64_t q_hs, const char* k, int64
   return INFLLM_OK;
 }
 
-// what the last kernel that reads a token's keys leaves behind: ev_attn; ev_attn_prev: the exec block's before
+// behind the last kernel of an exec block that reads keys: ev_attn; ev_attn_prev: the exec block's before
 int mark_attention(infllm_ctx* c, cudaStream_t s) {
   std::swap(c->ev_attn, c->ev_attn_prev);
   c->attn_prev_recorded = c->attn_recorded;
@@ -1745,11 +1792,12 @@ int token_end(infllm_ctx* c, cudaStream_t s) {
   const SealPlan sp = plan_seal(c, c->length + 1);
   const int64_t first_new = c->num_blocks;
   int n_cand = 0;
+  bool chained = false;
   INFLLM_TRY(seal_offload(c, first_new, sp.n_new, c->frontier + sp.take, s));
   trace_mark(c, s, TR_URGENT_END, 0);
   {
     HostTimer ht(&c->host_us[5]);
-    INFLLM_TRY(seal_apply(c, sp, -1, &n_cand, s));
+    INFLLM_TRY(seal_apply(c, sp, -1, &n_cand, false, &chained, s));
   }
   trace_mark(c, s, TR_SEAL_END, 0);
   if (sp.n_new > 0) INFLLM_TRY(list_new_units(c, first_new, s));
@@ -1845,7 +1893,10 @@ int append_sub(infllm_ctx* c, const char* q, int64_t q_hs, int64_t q_ts, const c
   }
   std::vector<int32_t> ids;
   for (auto& l : c->la) l.target = -1, l.launched = l.staged = false;
-  if (L > 1) INFLLM_CUDA_OK(cudaEventRecord(c->ev_seal, s));  // the look-ahead's starting point; one token has none
+  if (L > 1) {  // the look-ahead's starting point; one token has none
+    INFLLM_CUDA_OK(cudaEventRecord(c->ev_seal, s));
+    c->look_after = c->ev_seal;
+  }
   std::vector<KvSeg> gsegs;
   int eb = 0, n_cand = 0;
   bool have_ids = false;  // the ids of this exec block were already ranked at the end of the previous one
@@ -2070,7 +2121,7 @@ int append_sub(infllm_ctx* c, const char* q, int64_t q_hs, int64_t q_ts, const c
       }
     }
     if (g.cache_strategy == INFLLM_CACHE_LRU_S && !ids.empty()) INFLLM_TRY(unit_score_update(c, ids, qglb_eb, lq, s));
-    INFLLM_TRY(mark_attention(c, s));
+    if (decode_path) INFLLM_TRY(mark_attention(c, s));
     if (token_ev) INFLLM_CUDA_OK(cudaEventRecord(token_ev, s));
     delete ht_attn;
     trace_mark(c, s, TR_ATTN_END, eb);
@@ -2101,6 +2152,7 @@ int append_sub(infllm_ctx* c, const char* q, int64_t q_hs, int64_t q_ts, const c
       INFLLM_TRY(local_scores(c, s, st, ks, lq, lk, 0, j_u, local_pairs_eb));
     }
     trace_mark(c, s, TR_URGENT_END, eb);
+    bool chained = false;
     auto stage = [&](int d) -> int {  // refill copies for exec block eb + d, once its look-ahead is back
       const int64_t tgt = eb + d;
       infllm_ctx::LookAhead& la = c->la[tgt % (c->look_depth + 1)];
@@ -2110,11 +2162,16 @@ int append_sub(infllm_ctx* c, const char* q, int64_t q_hs, int64_t q_ts, const c
     if (more) INFLLM_TRY(stage(1));  // the candidates contain its ids (back since the last exec block, as a rule)
     {
       HostTimer ht(&c->host_us[5]);
-      INFLLM_TRY(seal_apply(c, sp, more ? eb + 1 : -1, &n_cand, s));
+      INFLLM_TRY(seal_apply(c, sp, more ? eb + 1 : -1, &n_cand, c->use_tc && lq > 1 && lq <= 512 && j_u > 0, &chained, s));
     }
     trace_mark(c, s, TR_SEAL_END, eb);
     if (L == 1 && sp.n_new > 0) INFLLM_TRY(list_new_units(c, first_new, s));
-    if (!decode_path) INFLLM_TRY(local_scores(c, s, st, ks, lq, lk, j_u, lk, 0.0));
+    if (!decode_path) {
+      // The rest needs nothing of the sealing's: chained to it, it starts as soon as the sealing's CTAs have their places.
+      INFLLM_TRY(local_scores(c, s, st, ks, lq, lk, j_u, lk, 0.0, chained));
+      INFLLM_TRY(mark_attention(c, s));  // (an event between attention, sums and sealing would cost each of them its early start)
+      c->look_after = c->ev_attn;
+    }
     trace_mark(c, s, TR_REST_END, eb);
     if (more)  // behind every launch of this exec block: the host waits for the look-ahead here
       for (int d = 2; d <= c->look_depth; ++d) INFLLM_TRY(stage(d));
@@ -2138,13 +2195,13 @@ int append_sub(infllm_ctx* c, const char* q, int64_t q_hs, int64_t q_ts, const c
 static int ctx_reset(infllm_ctx* c, bool wait) {
   if (c->initialized) {
     INFLLM_CUDA_OK(cudaSetDevice(c->cfg.device));
-    cudaStream_t side[6] = {c->copy_stream, c->urgent_stream, c->aux_stream, c->d2h_stream, c->mail_stream, c->seal_stream};
+    cudaStream_t side[5] = {c->copy_stream, c->urgent_stream, c->aux_stream, c->d2h_stream, c->mail_stream};
     if (wait || !c->dev_slabs.empty()) {
       for (cudaStream_t s : side) INFLLM_CUDA_OK(cudaStreamSynchronize(s));
       if (c->attn_recorded) INFLLM_CUDA_OK(cudaEventSynchronize(c->ev_attn));
       if (c->last_recorded) INFLLM_CUDA_OK(cudaEventSynchronize(c->ev_last));
     } else {
-      for (int i = 0; i < 6; ++i) INFLLM_CUDA_OK(cudaEventRecord(c->ev_side[i], side[i]));
+      for (int i = 0; i < 5; ++i) INFLLM_CUDA_OK(cudaEventRecord(c->ev_side[i], side[i]));
       // (marks of an earlier reset that no append has followed still stand)
       c->reset_attn = c->attn_recorded || (c->reset_pending && c->reset_attn);
       c->reset_last = c->last_recorded || (c->reset_pending && c->reset_last);
@@ -2179,7 +2236,7 @@ static int ctx_reset(infllm_ctx* c, bool wait) {
   c->attn_recorded = false;
   c->attn_prev_recorded = false;
   c->spec_recorded = false;
-  c->seal_aside = false;
+  c->free_after = nullptr;
   c->last_recorded = false;
   c->counters = infllm_ctx_info{};
   return INFLLM_OK;
@@ -2223,12 +2280,11 @@ static void ctx_free(infllm_ctx* c) {
     }
     if (c->h_cand_rows) cudaFreeHost(c->h_cand_rows);
     if (c->h_cand_scores) cudaFreeHost(c->h_cand_scores);
+    if (c->h_cand_words) cudaFreeHost(c->h_cand_words);
     if (c->scores_aux) cudaFreeAsync(c->scores_aux, nullptr);
     if (c->tc_part) cudaFreeAsync(c->tc_part, nullptr);
     cudaStreamDestroy(c->aux_stream);
     cudaStreamDestroy(c->mail_stream);
-    cudaStreamDestroy(c->seal_stream);
-    cudaEventDestroy(c->ev_urgent);
     if (c->d_cand_scores) cudaFree(c->d_cand_scores);
     if (c->d_spec) cudaFree(c->d_spec);
     cudaStreamDestroy(c->d2h_stream);
@@ -2426,10 +2482,7 @@ static int open_call(infllm_ctx* c, cudaStream_t s) {
   INFLLM_TRY(poll_device_error(c, s));
   if (c->h_tc_err && !c->err_pending && *(volatile int32_t*)c->h_tc_err) INFLLM_TRY(check_device_error(c, s));  // a one-launch token gave up
   c->failed = true;  // until the call has gone through
-  if (c->seal_aside) {  // a call that gave up half-way left it so
-    INFLLM_CUDA_OK(cudaStreamWaitEvent(s, c->ev_seal, 0));
-    c->seal_aside = false;
-  }
+  if (s != c->last_stream) c->copy_waited = 0;
   c->call_serial += 1;
   c->last_stream = s;
   c->trace_topk.clear();

@@ -63,6 +63,7 @@ block_score_kernel(const T* __restrict__ bk, int64_t n, int width, const float* 
 // the same way.  Latency only: 5 us against 4.4 us for selection and 8.5 us for scoring as two launches of CTAs of
 // four and eight warps, which read a row in four rounds.
 constexpr int kSealThreads = 1024;
+constexpr int kSealRows = 4;   // listed rows per CTA (a CTA of its own for each took 20 SMs from the column sums that run beside)
 constexpr int kSealItems = 8;  // tokens per lane: units of up to 256 tokens
 struct RowList {
   int32_t rows[kMaxScoreRows];
@@ -74,17 +75,27 @@ struct SealArgs {
   T* bk;             // representative keys, row 0
   const float* qbar; // null: nothing is scored
   float* scores;
+  unsigned long long* words;  // not null: the scores go here instead, as {score, seq}
   const int32_t* err;
   int32_t* err_out;
   int64_t k_hs, k_ts, score_hs, tok0;
   int32_t n_new, first_new, n_old, block_size, repr_topk, group, n_heads, head_dim, width;
+  uint32_t seq;
 };
 template <typename T>
 __global__ void __launch_bounds__(kSealThreads)
 seal_score_kernel(const __grid_constant__ SealArgs<T> A, const __grid_constant__ RowList list) {
   __shared__ float s_dot[32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, b = blockIdx.x;
-  if (A.err_out && b == 0 && tid < 4) A.err_out[tid] = A.err[tid];
+  __shared__ int32_t s_err;
+  // Launched behind the column sums of the tokens that are sealed here (see launch_chained): the CTAs of units that exist
+  // already do not wait for them, and what follows may start at once.
+  chain_trigger();
+  if (b < A.n_new) chain_wait();
+  if (A.err_out && b == 0) {  // the error record goes ahead of the scores that tell the host to look at it
+    if (tid == 0) s_err = __ldcg(A.err);
+    if (tid < 4 && __ldcg(A.err) != 0) A.err_out[tid] = __ldcg(A.err + tid);
+  }
   float dot = 0.f;
   if (b < A.n_new) {
     const int vec = A.head_dim / 32;  // 2 or 4 elements of the head per lane
@@ -144,23 +155,44 @@ seal_score_kernel(const __grid_constant__ SealArgs<T> A, const __grid_constant__
         for (int e = 0; e < vec; ++e) dot = fmaf(Act<T>::to_f(o[e]), A.qbar[at + e], dot);
       }
     }
-  } else {
-    const T* row = A.bk + (int64_t)list.rows[b - A.n_new] * A.width;
-    for (int c = tid * 8; c < A.width; c += kSealThreads * 8) {
-      const uint4 raw = *reinterpret_cast<const uint4*>(row + c);
-      const T* x = reinterpret_cast<const T*>(&raw);
+  } else {  // kSealRows listed rows, eight warps to each
+    const int at = (b - A.n_new) * kSealRows + warp / (32 / kSealRows);
+    if (at < A.n_old) {
+      const T* row = A.bk + (int64_t)list.rows[at] * A.width;
+      for (int c = (tid % (kSealThreads / kSealRows)) * 8; c < A.width; c += kSealThreads / kSealRows * 8) {
+        const uint4 raw = *reinterpret_cast<const uint4*>(row + c);
+        const T* x = reinterpret_cast<const T*>(&raw);
 #pragma unroll
-      for (int e = 0; e < 8; ++e) dot = fmaf(Act<T>::to_f(x[e]), A.qbar[c + e], dot);
+        for (int e = 0; e < 8; ++e) dot = fmaf(Act<T>::to_f(x[e]), A.qbar[c + e], dot);
+      }
     }
   }
-  if (!A.qbar) return;
-  dot = warp_sum(dot);
-  if (lane == 0) s_dot[warp] = dot;
-  __syncthreads();
-  if (warp == 0) {
-    dot = warp_sum(s_dot[lane]);
-    if (lane == 0) A.scores[b < A.n_new ? A.n_old + b : b - A.n_new] = dot;
+  if (A.qbar) {
+    dot = warp_sum(dot);
+    if (lane == 0) s_dot[warp] = dot;
+    __syncthreads();
+    if (warp == 0) {
+      // lane i has warp i's sum: all 32 of a new unit, those of the lane's row of the list
+      dot = s_dot[lane];
+#pragma unroll
+      for (int o = 1; o < 32 / kSealRows; o <<= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+      int at = (b - A.n_new) * kSealRows + lane / (32 / kSealRows);
+      if (b < A.n_new) {
+#pragma unroll
+        for (int o = 32 / kSealRows; o < 32; o <<= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+        at = A.n_old + b;
+      }
+      if (b < A.n_new ? lane == 0 : lane % (32 / kSealRows) == 0 && at < A.n_old) {
+        if (A.words) {  // pinned memory: the host reads them as they arrive
+          if (A.err_out && b == 0 && s_err != 0) __threadfence_system();
+          *(volatile unsigned long long*)(A.words + at) = ((unsigned long long)A.seq << 32) | __float_as_uint(dot);
+        } else {
+          A.scores[at] = dot;
+        }
+      }
+    }
   }
+  if (b >= A.n_new) chain_wait();  // whoever follows this kernel follows the one before it too
 }
 
 __device__ __forceinline__ uint32_t float_key(float f) {
@@ -648,14 +680,14 @@ int topk_launch(const float* scores, int64_t n, int k, int id_base, int32_t* out
 // seals); see seal_score_kernel.
 int seal_score_launch(const void* k, int64_t k_hs, int64_t k_ts, const float* score, int64_t score_hs, int64_t tok0, int n_new,
                       int first_new, int block_size, int repr_topk, int n_heads, int n_kv_heads, int head_dim, void* bk,
-                      const int32_t* rows, int n_old, const float* qbar, float* scores, const int32_t* err, int32_t* err_out,
-                      int dtype, cudaStream_t s) {
+                      const int32_t* rows, int n_old, const float* qbar, float* scores, unsigned long long* words, uint32_t seq,
+                      const int32_t* err, int32_t* err_out, bool chain, int dtype, cudaStream_t s) {
   if (n_new > 0 && (repr_topk <= 0 || repr_topk > block_size))
     return fail(INFLLM_E_BADARG, "repr_select: repr_topk %d vs block_size %d", repr_topk, block_size);
   if (n_heads % n_kv_heads) return fail(INFLLM_E_BADARG, "repr_select: heads %d / kv heads %d", n_heads, n_kv_heads);
   INFLLM_DISPATCH_DTYPE(dtype, T, {
-    SealArgs<T> A{(const T*)k, score, (T*)bk, qbar, scores, err, err_out, k_hs, k_ts, score_hs, tok0, n_new, first_new, n_old,
-                  block_size, repr_topk, n_heads / n_kv_heads, n_heads, head_dim, n_heads * head_dim};
+    SealArgs<T> A{(const T*)k, score, (T*)bk, qbar, scores, words, err, err_out, k_hs, k_ts, score_hs, tok0, n_new, first_new, n_old,
+                  block_size, repr_topk, n_heads / n_kv_heads, n_heads, head_dim, n_heads * head_dim, seq};
     RowList list;
     for (int done = 0; done == 0 || done < n_old;) {
       const int m = qbar ? std::min(n_old - done, kMaxScoreRows) : 0;  // `rows` is a host array
@@ -663,10 +695,13 @@ int seal_score_launch(const void* k, int64_t k_hs, int64_t k_ts, const float* sc
       const int last = done + m >= n_old || !qbar;  // the new units go with the last part of the list
       A.n_new = last ? n_new : 0;
       A.n_old = m;
-      A.scores = scores + done;
+      A.scores = scores ? scores + done : nullptr;
+      A.words = words ? words + done : nullptr;
       A.err_out = last ? err_out : nullptr;
       if (A.n_new + m > 0) {
-        seal_score_kernel<T><<<A.n_new + m, kSealThreads, 0, s>>>(A, list);
+        const dim3 grid(A.n_new + (m + kSealRows - 1) / kSealRows);
+        if (chain) INFLLM_CUDA_OK(launch_chained(seal_score_kernel<T>, grid, dim3(kSealThreads), 0, s, A, list));
+        else seal_score_kernel<T><<<grid, kSealThreads, 0, s>>>(A, list);
         INFLLM_LAUNCH_OK("seal_score_kernel");
       }
       done += m;
@@ -691,7 +726,7 @@ int repr_select_launch(const void* k, int64_t k_hs, int64_t k_ts, const float* s
   if (n_heads % n_kv_heads) return fail(INFLLM_E_BADARG, "repr_select: heads %d / kv heads %d", n_heads, n_kv_heads);
   if (seal_score_ok(block_size, head_dim, k_hs, k_ts, k) && (uintptr_t)out % 8 == 0)
     return seal_score_launch(k, k_hs, k_ts, score, score_hs, tok0, n_new, 0, block_size, repr_topk, n_heads, n_kv_heads, head_dim,
-                             out, nullptr, 0, nullptr, nullptr, nullptr, nullptr, dtype, s);
+                             out, nullptr, 0, nullptr, nullptr, nullptr, 0, nullptr, nullptr, false, dtype, s);
   dim3 grid(n_new, n_heads);
   size_t smem = block_size * sizeof(float) + repr_topk * sizeof(int);
   INFLLM_DISPATCH_DTYPE(dtype, T, {
@@ -732,7 +767,7 @@ extern "C" int infllm_block_score_rows(const void* d_block_k, const int32_t* h_r
     return fail(INFLLM_E_BADARG, "block_score_rows: width %d must be a multiple of 8, at most 12288, rows 16-byte aligned", width);
   // (no new units: of the head counts only their product with head_dim, the width, matters)
   return seal_score_launch(nullptr, 0, 0, nullptr, 0, 0, 0, 0, 1, 1, 1, 1, width, const_cast<void*>(d_block_k), h_rows, n, d_qbar,
-                           d_scores, nullptr, nullptr, dtype, (cudaStream_t)stream);
+                           d_scores, nullptr, 0, nullptr, nullptr, false, dtype, (cudaStream_t)stream);
 }
 
 extern "C" int infllm_ptr_table_update(uint64_t* d_table, const int32_t* h_ids, const uint64_t* h_addrs, int n, void* stream) {
