@@ -38,6 +38,8 @@ int copy_rows_launch(const void* x, int64_t x_hs, int64_t x_ts, void* out, int64
                      int n_heads, int64_t len, int head_dim, cudaStream_t s);
 int pack_units_launch(const void* k, const void* v, int64_t hs, int64_t tok0, int n_new, int block_size, int n_kv_heads,
                       int head_dim, void* out, cudaStream_t s);
+int shift_tokens_launch(void* k_raw, void* k_rot, void* v, float* score, int row_bytes, int n_heads, int n_kv_heads, int64_t cap,
+                        int64_t off, int64_t live, int64_t pad0, int64_t pad1, cudaStream_t s);
 int stage_units_launch(const void* const* h_src, void* const* d_dst, int n, int64_t unit_bytes, cudaStream_t s);
 int qbar_launch(const void* q, int64_t q_hs, int64_t q_ts, int n_heads, int64_t len, int exc, int head_dim,
                 float* qbar, int64_t qbar_stride, int dtype, cudaStream_t s);
@@ -351,8 +353,8 @@ struct infllm_ctx {
 
   // sealed units leave through a packing buffer (two in rotation) and one copy per run of units
   void* pack_buf[2] = {nullptr, nullptr};
-  cudaEvent_t ev_pack[2] = {nullptr, nullptr};
-  bool pack_used[2] = {false, false};
+  cudaEvent_t ev_packed = nullptr;  // behind the last packing of sealed units: it reads the token buffers
+  bool packed_recorded = false;
   int pack_idx = 0, pack_units = 0;
   cudaStream_t d2h_stream = nullptr;
   cudaEvent_t ev_d2h = nullptr, ev_ingest = nullptr;
@@ -515,7 +517,6 @@ int lazy_init(infllm_ctx* c, cudaStream_t s) {
   c->pack_units = g.exc_block_size / g.block_size + 2;
   for (int i = 0; i < 2; ++i) {
     INFLLM_CUDA_OK(dev_malloc((void**)&c->pack_buf[i], (int64_t)c->pack_units * c->unit_bytes));
-    INFLLM_CUDA_OK(cudaEventCreateWithFlags(&c->ev_pack[i], cudaEventDisableTiming));
   }
   INFLLM_CUDA_OK(cudaEventCreateWithFlags(&c->ev_main, cudaEventDisableTiming));
   INFLLM_CUDA_OK(cudaEventCreateWithFlags(&c->ev_copy, cudaEventDisableTiming));
@@ -530,6 +531,7 @@ int lazy_init(infllm_ctx* c, cudaStream_t s) {
   INFLLM_CUDA_OK(cudaEventCreateWithFlags(&c->ev_spec, cudaEventDisableTiming));
   INFLLM_CUDA_OK(cudaEventCreateWithFlags(&c->ev_cand, cudaEventDisableTiming));
   INFLLM_CUDA_OK(cudaEventCreateWithFlags(&c->ev_seal, cudaEventDisableTiming));
+  INFLLM_CUDA_OK(cudaEventCreateWithFlags(&c->ev_packed, cudaEventDisableTiming));
   INFLLM_CUDA_OK(cudaEventCreateWithFlags(&c->ev_stage, cudaEventDisableTiming));
   INFLLM_CUDA_OK(cudaEventCreateWithFlags(&c->ev_last, cudaEventDisableTiming));
   for (auto& e : c->ev_side) INFLLM_CUDA_OK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
@@ -702,9 +704,19 @@ int ensure_tokens(infllm_ctx* c, int64_t add, cudaStream_t s) {
   const int64_t D = g.head_dim, H = g.n_heads, HKV = g.n_kv_heads;
   if (tb.cap > 0 && c->length + add - tb.t0 <= tb.cap) return INFLLM_OK;
   const int64_t live0 = c->frontier, live = c->length - c->frontier;
-  const int64_t need = live + add;
+  const int64_t need = live + add, off = live > 0 ? live0 - tb.t0 : 0;
+  if (need <= tb.cap && live <= off) {
+    // In place where the tokens that are left fit before those that are gone - the slack below sees to it for a prompt in
+    // calls of one size and for tokens one by one.  The packing of sealed units, on its own stream, reads what is overwritten.
+    if (c->packed_recorded) INFLLM_CUDA_OK(cudaStreamWaitEvent(s, c->ev_packed, 0));
+    const int64_t pad = std::min<int64_t>(tb.cap, need + 256);
+    INFLLM_TRY(shift_tokens_launch(tb.k_raw, tb.k_rot, tb.v, tb.score, (int)D * c->esz, (int)H, (int)HKV, tb.cap, off, live, need, pad, s));
+    tb.t0 = live0;
+    tb.zero_upto = pad;
+    return INFLLM_OK;
+  }
   TokenBuffers nb;
-  nb.cap = round_up(need + std::max<int64_t>(4096, g.n_local), 256);
+  nb.cap = round_up(need + std::max<int64_t>(4096, g.n_local + g.n_init + 4 * g.block_size), 256);
   nb.t0 = live0;
   INFLLM_CUDA_OK(dev_malloc_async((void**)&nb.k_raw, HKV * nb.cap * D * c->esz, s));
   INFLLM_CUDA_OK(dev_malloc_async((void**)&nb.k_rot, HKV * nb.cap * D * c->esz, s));
@@ -1574,6 +1586,10 @@ int seal_offload(infllm_ctx* c, int64_t first, int n_new, int64_t tok0, cudaStre
     c->pack_idx ^= 1;
     INFLLM_TRY(pack_units_launch(tb.k_raw, tb.v, tb.cap * D, tok0 + (int64_t)done * bs - tb.t0, n, (int)bs, (int)HKV,
                                  (int)D, c->pack_buf[r], c->d2h_stream));
+    if (done + n == n_new) {
+      INFLLM_CUDA_OK(cudaEventRecord(c->ev_packed, c->d2h_stream));
+      c->packed_recorded = true;
+    }
     for (int i = 0; i < n;) {  // runs that stay inside one slab of the store are contiguous on the host
       const int64_t b0 = first + done + i;
       const int run = (int)std::min<int64_t>(n - i, c->slab_units - b0 % c->slab_units);
@@ -2215,8 +2231,7 @@ static int ctx_reset(infllm_ctx* c, bool wait) {
   c->d2h_synced_upto_urgent = 0;
   release_dev_slabs(c);
   c->dev_cap = (int64_t)c->cfg.device_store_mb * (1ll << 20) / std::max<int64_t>(c->unit_bytes, 1);
-  c->d2h_recorded = false;
-  c->pack_used[0] = c->pack_used[1] = false;
+  c->d2h_recorded = c->packed_recorded = false;
   c->length = c->frontier = c->num_blocks = c->init_len = c->load_count = 0;
   c->init_full = false;
   c->rope_origin = -1;
@@ -2292,11 +2307,11 @@ static void ctx_free(infllm_ctx* c) {
     cudaEventDestroy(c->ev_ingest);
     for (int i = 0; i < 2; ++i) {
       if (c->pack_buf[i]) cudaFree(c->pack_buf[i]);
-      if (c->ev_pack[i]) cudaEventDestroy(c->ev_pack[i]);
     }
     cudaEventDestroy(c->ev_spec);
     cudaEventDestroy(c->ev_cand);
     cudaEventDestroy(c->ev_seal);
+    cudaEventDestroy(c->ev_packed);
     cudaEventDestroy(c->ev_stage);
     if (c->slab_pending) {
       free_slab(c->slab_future.get());

@@ -82,6 +82,33 @@ __global__ void copy_rows_kernel(const T* __restrict__ x, int64_t x_hs, int64_t 
       *reinterpret_cast<const uint4*>(x + h * x_hs + t * x_ts + c * 8);
 }
 
+// The live tokens of the token buffers move to the front: rows [off, off + live) of every KV head of the three key/value
+// buffers to [0, live) (off >= live: nothing overlaps), rows [pad0, pad1) become zero, and the same tokens of every head's
+// scores.  Rows are `row` 16-byte pieces, heads `cap` rows apart; plane blockIdx.y is a buffer's head, then a head's scores.
+// Bound: HBM.  4.6K tokens of 8 KV heads: four copies into new buffers and three memsets took 56 us, and the host 40 us.
+__global__ void __launch_bounds__(256) shift_tokens_kernel(uint4* k_raw, uint4* k_rot, uint4* v, float* score, int row, int hkv,
+                                                           int64_t cap, int64_t off, int64_t live, int64_t pad0, int64_t pad1) {
+  const int plane = blockIdx.y, step = gridDim.x * 256;
+  if (plane >= 3 * hkv) {
+    float* p = score + (int64_t)(plane - 3 * hkv) * cap;
+    for (int64_t i = blockIdx.x * 256 + threadIdx.x; i < live; i += step) p[i] = p[off + i];
+    return;
+  }
+  const int which = plane / hkv;
+  uint4* p = (which == 0 ? k_raw : which == 1 ? k_rot : v) + (int64_t)(plane - which * hkv) * cap * row;
+  const int64_t n = live * row, d = off * row;
+  for (int64_t i = blockIdx.x * 256 + threadIdx.x; i < n; i += 4 * step) {
+    uint4 x[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      if (i + e * step < n) x[e] = __ldcs(p + d + i + e * step);
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      if (i + e * step < n) p[i + e * step] = x[e];
+  }
+  for (int64_t i = pad0 * row + blockIdx.x * 256 + threadIdx.x; i < pad1 * row; i += step) p[i] = make_uint4(0, 0, 0, 0);
+}
+
 // mean over the rows of each exec block of the one-angle-rotated queries:
 // qbar[e, h*D + d] = mean_t q[h, e*exc + t, d]  (context_manager.py:373-375), fp32.
 template <typename T>
@@ -378,6 +405,17 @@ int copy_rows_launch(const void* x, int64_t x_hs, int64_t x_ts, void* out, int64
   copy_rows_kernel<__half><<<(unsigned)ceil_div(total, 256), 256, 0, s>>>(
       (const __half*)x, x_hs, x_ts, (__half*)out, o_hs, o_ts, n_heads, len, head_dim);
   INFLLM_LAUNCH_OK("copy_rows_kernel");
+  return INFLLM_OK;
+}
+
+int shift_tokens_launch(void* k_raw, void* k_rot, void* v, float* score, int row_bytes, int n_heads, int n_kv_heads, int64_t cap,
+                        int64_t off, int64_t live, int64_t pad0, int64_t pad1, cudaStream_t s) {
+  if (off < live || off + live > cap || pad0 < live || pad1 > cap || row_bytes % 16)
+    return fail(INFLLM_E_BADARG, "shift_tokens: %lld tokens from %lld of %lld", (long long)live, (long long)off, (long long)cap);
+  const dim3 grid((unsigned)std::max(1, 1184 / (3 * n_kv_heads)), 3 * n_kv_heads + n_heads);
+  shift_tokens_kernel<<<grid, 256, 0, s>>>((uint4*)k_raw, (uint4*)k_rot, (uint4*)v, score, row_bytes / 16, n_kv_heads, cap, off, live,
+                                           pad0, pad1);
+  INFLLM_LAUNCH_OK("shift_tokens_kernel");
   return INFLLM_OK;
 }
 
