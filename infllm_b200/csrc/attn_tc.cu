@@ -599,17 +599,103 @@ __global__ void __launch_bounds__(576, 1) attn_tc2_kernel(const __grid_constant_
 // four to eight tiles ahead (no change), all exponentials or half of them on the special-function unit (87, 86 us).
 // 83 us per exec block of the 128K prefill.
 namespace tc3 {
-constexpr int kQ = 0;
-constexpr int kK = kQ + 2 * kSubTileBytes;       // two stages
+constexpr int kQ = 0;                            // two stages
+constexpr int kK = kQ + 4 * kSubTileBytes;       // two stages
 constexpr int kV = kK + 4 * kSubTileBytes;       // two stages
 constexpr int kBar = kV + 4 * kSubTileBytes;
 constexpr int kXmax = kBar + 256;                // reference maxima of the 128 rows, for the epilogue's layout
 constexpr int kXsum = kXmax + 512;               // row sums of the 128 rows
-constexpr int kTotal = kXsum + 512;
+constexpr int kPlan = kXsum + 512;
+constexpr int kTotal = kPlan + 32 + kMaxSeg * 32;
 constexpr int kPolyEvery = 4;
-enum { T3_Q_FULL = 0, T3_Q_EMPTY, T3_K_FULL0, T3_K_FULL1, T3_K_EMPTY0, T3_K_EMPTY1, T3_V_FULL0, T3_V_FULL1, T3_V_EMPTY0,
-       T3_V_EMPTY1, T3_S_FULL0, T3_S_FULL1, T3_S_FULL2, T3_P_FULL0, T3_P_FULL1, T3_P_FULL2, T3_PV_DONE0, T3_PV_DONE1, T3_PV_DONE2,
-       T3_O_FULL, T3_N_BARS };
+enum { T3_Q_FULL0 = 0, T3_Q_FULL1, T3_Q_EMPTY0, T3_Q_EMPTY1, T3_K_FULL0, T3_K_FULL1, T3_K_EMPTY0, T3_K_EMPTY1, T3_V_FULL0, T3_V_FULL1,
+       T3_V_EMPTY0, T3_V_EMPTY1, T3_S_FULL0, T3_S_FULL1, T3_S_FULL2, T3_P_FULL0, T3_P_FULL1, T3_P_FULL2, T3_PV_DONE0, T3_PV_DONE1,
+       T3_PV_DONE2, T3_O_FULL, T3_N_BARS };
+// What a CTA does, worked out once, by one warp: the segments of its run that have tiles, in order.  Left to every role's own
+// loop over stages and segments, the 64-bit arithmetic for 20 segments took 8400 cycles before the first product of a run
+// and 6000 behind its last one, of 46000 for 12 tiles.
+struct Part {
+  int32_t n;           // key tiles
+  int32_t tok;         // token coordinate of the first
+  int32_t c3_k, c3_v;
+  int16_t map_k, map_v;
+  int32_t stage;       // bit 8: the stage's last part of this run
+  int32_t j;           // the first tile's first key within the stage
+  int32_t lim;         // the segment's last key within the stage
+};
+static_assert(sizeof(Part) == 32, "");
+struct Plan {
+  int32_t n_parts, n_tiles, pad[6];
+  Part part[kMaxSeg];
+};
+__device__ __forceinline__ int warp_scan(int v) {  // inclusive
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, v, o);
+    if (lane >= o) v += u;
+  }
+  return v;
+}
+// one warp; queries [i0, i1], run `split` of n_split.  kPer segments per lane: one for the usual numbers.
+template <int kPer>
+__device__ __forceinline__ void make_plan(const AttnTcParams& P, int64_t i0, int64_t i1, int split, Plan* plan) {
+  static_assert(kMaxStage == 2, "");
+  const int lane = threadIdx.x & 31, n_stage = P.n_stage, n_seg = P.stage[n_stage - 1].seg_end;
+  const int seg1 = n_stage > 1 ? P.stage[1].seg_begin : n_seg;  // the second stage's first
+  int64_t vlo[2] = {0, 0}, vhi[2] = {-1, -1};
+  visible_key_range(P.stage[0].mask_mode, P.stage[0].mask_offset, P.stage[0].mask_size, i0, i1, P.stage[0].lk, &vlo[0], &vhi[0]);
+  if (n_stage > 1)
+    visible_key_range(P.stage[1].mask_mode, P.stage[1].mask_offset, P.stage[1].mask_size, i0, i1, P.stage[1].lk, &vlo[1], &vhi[1]);
+  int len[kPer], j0[kPer], tf[kPer], n[kPer], first[kPer];
+  int keys = 0, base = 0, tiles = 0;  // keys of the segments before, of the first stage's; tiles
+#pragma unroll
+  for (int e = 0; e < kPer; ++e) {
+    const int sg = e * 32 + lane;
+    len[e] = sg < n_seg ? P.seg[sg].len : 0;
+    const int inc = warp_scan(len[e]);
+    j0[e] = keys + inc - len[e];
+    keys += __shfl_sync(0xffffffffu, inc, 31);
+    if (seg1 / 32 == e) base = __shfl_sync(0xffffffffu, j0[e], seg1 & 31);
+  }
+#pragma unroll
+  for (int e = 0; e < kPer; ++e) {
+    const int sg = e * 32 + lane, st = sg >= seg1;
+    if (st) j0[e] -= base;
+    const int64_t lo = st ? vlo[1] : vlo[0], hi = st ? vhi[1] : vhi[0];
+    int tl;
+    n[e] = 0;
+    if (sg < n_seg && lo <= hi && seg_tiles(lo, hi, j0[e], len[e], &tf[e], &tl)) n[e] = tl - tf[e] + 1;
+    const int inc = warp_scan(n[e]);
+    first[e] = tiles + inc - n[e];
+    tiles += __shfl_sync(0xffffffffu, inc, 31);
+  }
+  int g0 = 0, g1 = tiles;
+  if (P.n_split > 1) g0 = tiles * split / P.n_split, g1 = tiles * (split + 1) / P.n_split;
+  int at = 0, last[2] = {-1, -1};
+#pragma unroll
+  for (int e = 0; e < kPer; ++e) {
+    const int sg = e * 32 + lane, st = sg >= seg1;
+    const int a = first[e] > g0 ? first[e] : g0, b = first[e] + n[e] < g1 ? first[e] + n[e] : g1;
+    const unsigned has = __ballot_sync(0xffffffffu, a < b), has1 = __ballot_sync(0xffffffffu, a < b && st);
+    if (a < b) {
+      const TcSeg& G = P.seg[sg];
+      Part& R = plan->part[at + __popc(has & ((1u << lane) - 1u))];
+      const int t = tf[e] + a - first[e];
+      R.n = b - a, R.tok = G.tok0 + t * kTile, R.c3_k = G.c3_k, R.c3_v = G.c3_v, R.map_k = G.map_k, R.map_v = G.map_v;
+      R.stage = st, R.j = j0[e] + t * kTile, R.lim = j0[e] + len[e] - 1;
+    }
+    if (has != has1) last[0] = at + __popc(has & ~has1) - 1;  // (the first stage's parts come before the second's)
+    if (has1) last[1] = at + __popc(has) - 1;
+    at += __popc(has);
+  }
+  __syncwarp();
+  if (lane == 0) {
+    plan->n_parts = at, plan->n_tiles = g1 - g0;
+    if (last[0] >= 0) plan->part[last[0]].stage |= 256;
+    if (last[1] >= 0) plan->part[last[1]].stage |= 256;
+  }
+}
 }  // namespace tc3
 
 template <typename T>
@@ -632,17 +718,18 @@ __global__ void __launch_bounds__(352, 1) attn_tc3_kernel(const __grid_constant_
   const int rows_q = (int)((P.lq - i0) < kTile ? (P.lq - i0) : kTile);
   const int split = blockIdx.z;
 
-  // this CTA's run [g0, g1) of the work item's key tiles, numbered over all stages
-  int g0 = 0, g1 = 1 << 30;
-  if (P.n_split > 1) {
-    int n_total = 0;
-    for (int st = 0; st < P.n_stage; ++st) {
-      const TcStage& S = P.stage[st];
-      int64_t vis_lo, vis_hi;
-      visible_key_range(S.mask_mode, S.mask_offset, S.mask_size, i0, i0 + rows_q - 1, S.lk, &vis_lo, &vis_hi);
-      if (vis_lo <= vis_hi) n_total += stage_tiles(P, S, vis_lo, vis_hi);
+  if (warp == 10 && lane < P.n_stage) {  // the descriptors of the first loads are on their way while the run's parts are worked out
+    const TcStage& S = P.stage[lane];
+    tma_prefetch_map(&P.maps[S.map_q]);
+    if (S.seg_begin < S.seg_end) {
+      tma_prefetch_map(&P.maps[P.seg[S.seg_begin].map_k]);
+      tma_prefetch_map(&P.maps[P.seg[S.seg_begin].map_v]);
     }
-    g0 = (int)((int64_t)n_total * split / P.n_split), g1 = (int)((int64_t)n_total * (split + 1) / P.n_split);
+  }
+  tc3::Plan* plan = reinterpret_cast<tc3::Plan*>(smem + kPlan);
+  if (warp == 8) {  // the run's parts
+    if (P.stage[P.n_stage - 1].seg_end <= 32) make_plan<1>(P, i0, i0 + rows_q - 1, split, plan);
+    else make_plan<(kMaxSeg + 31) / 32>(P, i0, i0 + rows_q - 1, split, plan);
   }
 
   if (threadIdx.x == 0) {
@@ -669,7 +756,7 @@ __global__ void __launch_bounds__(352, 1) attn_tc3_kernel(const __grid_constant_
     // when the P V product of tile t-2 has run, late in the tile's cycle; asked for in tile order, K(t+1) queued
     // behind that wait and S(t+1) was not ready when the softmax warps came for it.
     if (lane == 0) {
-      int g = 0, it = 0, sidx = 0;
+      int it = 0, sidx = 0, stage = -1;
       bool ok = true;
       struct { int it, tok, c3, map; } pend = {-1, 0, 0, 0};  // the V tile that has not been asked for yet
       auto load_v = [&]() {
@@ -687,50 +774,38 @@ __global__ void __launch_bounds__(352, 1) attn_tc3_kernel(const __grid_constant_
         }
         pend.it = -1;
       };
-      for (int st = 0; st < P.n_stage && ok; ++st) {
-        const TcStage& S = P.stage[st];
-        int64_t vis_lo, vis_hi;
-        visible_key_range(S.mask_mode, S.mask_offset, S.mask_size, i0, i0 + rows_q - 1, S.lk, &vis_lo, &vis_hi);
-        if (vis_lo > vis_hi) continue;
-        const int n_st = stage_tiles(P, S, vis_lo, vis_hi);
-        if ((g > g0 ? g : g0) >= (g + n_st < g1 ? g + n_st : g1)) {  // none of this run's tiles
-          g += n_st;
-          continue;
+      const int n_parts = plan->n_parts;
+      for (int p = 0; p < n_parts && ok; ++p) {
+        const Part R = plan->part[p];
+        if ((R.stage & 255) != stage) {  // the stage's queries; the buffer was the stage's before the last one's
+          stage = R.stage & 255;
+          const TcStage& S = P.stage[stage];
+          const int qb = sidx & 1;
+          if (sidx >= 2) ok = wait_or_abort(bar(T3_Q_EMPTY0 + qb), ((sidx >> 1) - 1) & 1, abort_flag, P.err, 600);
+          if (!ok) break;
+          const uint32_t dq = sQ + qb * 2 * kSubTileBytes;
+          mbar_expect_tx(bar(T3_Q_FULL0 + qb), 2 * kSubTileBytes);
+          tma_load_3d(dq, &P.maps[S.map_q], bar(T3_Q_FULL0 + qb), 0, S.q_row0 + (int)i0, h);
+          tma_load_3d(dq + kSubTileBytes, &P.maps[S.map_q], bar(T3_Q_FULL0 + qb), 64, S.q_row0 + (int)i0, h);
+          ++sidx;
         }
-        if (sidx >= 1) ok = wait_or_abort(bar(T3_Q_EMPTY), (sidx - 1) & 1, abort_flag, P.err, 600);
-        if (!ok) break;
-        mbar_expect_tx(bar(T3_Q_FULL), 2 * kSubTileBytes);
-        tma_load_3d(sQ, &P.maps[S.map_q], bar(T3_Q_FULL), 0, S.q_row0 + (int)i0, h);
-        tma_load_3d(sQ + kSubTileBytes, &P.maps[S.map_q], bar(T3_Q_FULL), 64, S.q_row0 + (int)i0, h);
-        ++sidx;
-        int64_t seg_j0 = 0;
-        for (int sg = S.seg_begin; sg < S.seg_end && ok; ++sg) {
-          const TcSeg& G = P.seg[sg];
-          int tf, tl;
-          if (seg_tiles(vis_lo, vis_hi, seg_j0, G.len, &tf, &tl)) {
-            const int skip = g0 > g ? g0 - g : 0;  // tiles of earlier runs
-            for (int t = tf + skip; t <= tl && ok; ++t) {
-              if (g + t - tf >= g1) break;
-              const int b = it & 1, tok = G.tok0 + t * kTile;
-              if (it >= 2) ok = wait_or_abort(bar(T3_K_EMPTY0 + b), ((it >> 1) - 1) & 1, abort_flag, P.err, 601);
-              if (!ok) break;
-              const uint32_t dk = sK + b * 2 * kSubTileBytes;
-              mbar_expect_tx(bar(T3_K_FULL0 + b), 2 * kSubTileBytes);
-              if (G.c3_k < 0) {
-                tma_load_3d(dk, &P.maps[G.map_k], bar(T3_K_FULL0 + b), 0, tok, hkv);
-                tma_load_3d(dk + kSubTileBytes, &P.maps[G.map_k], bar(T3_K_FULL0 + b), 64, tok, hkv);
-              } else {
-                tma_load_4d(dk, &P.maps[G.map_k], bar(T3_K_FULL0 + b), 0, tok, hkv, G.c3_k);
-                tma_load_4d(dk + kSubTileBytes, &P.maps[G.map_k], bar(T3_K_FULL0 + b), 64, tok, hkv, G.c3_k);
-              }
-              if (pend.it >= 0) load_v();
-              if (!ok) break;
-              pend.it = it, pend.tok = tok, pend.c3 = G.c3_v, pend.map = G.map_v;
-              ++it;
-            }
-            g += tl - tf + 1;
+        for (int t = 0; t < R.n && ok; ++t) {
+          const int b = it & 1, tok = R.tok + t * kTile;
+          if (it >= 2) ok = wait_or_abort(bar(T3_K_EMPTY0 + b), ((it >> 1) - 1) & 1, abort_flag, P.err, 601);
+          if (!ok) break;
+          const uint32_t dk = sK + b * 2 * kSubTileBytes;
+          mbar_expect_tx(bar(T3_K_FULL0 + b), 2 * kSubTileBytes);
+          if (R.c3_k < 0) {
+            tma_load_3d(dk, &P.maps[R.map_k], bar(T3_K_FULL0 + b), 0, tok, hkv);
+            tma_load_3d(dk + kSubTileBytes, &P.maps[R.map_k], bar(T3_K_FULL0 + b), 64, tok, hkv);
+          } else {
+            tma_load_4d(dk, &P.maps[R.map_k], bar(T3_K_FULL0 + b), 0, tok, hkv, R.c3_k);
+            tma_load_4d(dk + kSubTileBytes, &P.maps[R.map_k], bar(T3_K_FULL0 + b), 64, tok, hkv, R.c3_k);
           }
-          seg_j0 += G.len;
+          if (pend.it >= 0) load_v();
+          if (!ok) break;
+          pend.it = it, pend.tok = tok, pend.c3 = R.c3_v, pend.map = R.map_v;
+          ++it;
         }
       }
       if (ok && pend.it >= 0) load_v();
@@ -750,41 +825,38 @@ __global__ void __launch_bounds__(352, 1) attn_tc3_kernel(const __grid_constant_
     // before - S of tile t+2 may overwrite its buffer only when P V of tile t has read P from it - is now the
     // wait for that product's commit.
     if (lane == 0) {
-      int nt[kMaxStage], n_act = 0, n = 0, g = 0;  // this run's tiles per stage that has any, in order
-      for (int st = 0; st < P.n_stage; ++st) {
-        const TcStage& S = P.stage[st];
-        int64_t vis_lo, vis_hi;
-        visible_key_range(S.mask_mode, S.mask_offset, S.mask_size, i0, i0 + rows_q - 1, S.lk, &vis_lo, &vis_hi);
-        if (vis_lo > vis_hi) continue;
-        const int n_st = stage_tiles(P, S, vis_lo, vis_hi);
-        const int c = (g + n_st < g1 ? g + n_st : g1) - (g > g0 ? g : g0);
-        g += n_st;
-        if (c > 0) nt[n_act++] = c, n += c;
-      }
+      const int n = plan->n_tiles;
       bool ok = true;
       if (warp == 10) {
-        const uint64_t qd0 = make_sdesc(sQ, 16, 1024);
+        const uint64_t qd0[2] = {make_sdesc(sQ, 16, 1024), make_sdesc(sQ + 2 * kSubTileBytes, 16, 1024)};
         const uint64_t kd0[2] = {make_sdesc(sK, 16, 1024), make_sdesc(sK + 2 * kSubTileBytes, 16, 1024)};
-        int sq = 0, tq = 0;
-        for (int iq = 0; iq < n && ok; ++iq) {
-          const int b = iq & 1;
-          if (tq == 0) ok = wait_or_abort(bar(T3_Q_FULL), sq & 1, abort_flag, P.err, 610);
-          if (ok) ok = wait_or_abort(bar(T3_K_FULL0 + b), (iq >> 1) & 1, abort_flag, P.err, 611);
-          const int b3 = iq % 3;  // S/P buffer: free once the P V product of tile iq-3 has read P from it
-          if (ok && iq >= 3) ok = wait_or_abort(bar(T3_PV_DONE0 + b3), ((iq / 3) - 1) & 1, abort_flag, P.err, 614);
-          if (!ok) break;
-          tc_fence_after();
+        const int n_parts = plan->n_parts;
+        int iq = 0, sq = 0;
+        bool q_due = true;
+        for (int p = 0; p < n_parts && ok; ++p) {
+          const int np = plan->part[p].n, last = plan->part[p].stage & 256;
+          for (int t = 0; t < np && ok; ++t, ++iq) {
+            const int b = iq & 1, qb = sq & 1;
+            if (q_due) ok = wait_or_abort(bar(T3_Q_FULL0 + qb), (sq >> 1) & 1, abort_flag, P.err, 610);
+            q_due = false;
+            if (ok) ok = wait_or_abort(bar(T3_K_FULL0 + b), (iq >> 1) & 1, abort_flag, P.err, 611);
+            const int b3 = iq % 3;  // S/P buffer: free once the P V product of tile iq-3 has read P from it
+            if (ok && iq >= 3) ok = wait_or_abort(bar(T3_PV_DONE0 + b3), ((iq / 3) - 1) & 1, abort_flag, P.err, 614);
+            if (!ok) break;
+            tc_fence_after();
+            const uint64_t qd = sq & 1 ? qd0[1] : qd0[0], kd = b ? kd0[1] : kd0[0];
 #pragma unroll
-          for (int ks = 0; ks < 8; ++ks) {
-            const uint64_t off = (uint64_t)(((ks >> 2) * kSubTileBytes + (ks & 3) * 32) >> 4);
-            mma_ss(tmem + b3 * 128, qd0 + off, kd0[b] + off, idesc_qk, ks > 0);
-          }
-          tc_commit(bar(T3_S_FULL0 + b3));
-          tc_commit(bar(T3_K_EMPTY0 + b));
-          if (++tq == nt[sq]) {
-            tc_commit(bar(T3_Q_EMPTY));  // the last product that reads this stage's Q tile
-            ++sq;
-            tq = 0;
+            for (int ks = 0; ks < 8; ++ks) {
+              const uint64_t off = (uint64_t)(((ks >> 2) * kSubTileBytes + (ks & 3) * 32) >> 4);
+              mma_ss(tmem + b3 * 128, qd + off, kd + off, idesc_qk, ks > 0);
+            }
+            tc_commit(bar(T3_S_FULL0 + b3));
+            tc_commit(bar(T3_K_EMPTY0 + b));
+            if (last && t == np - 1) {
+              tc_commit(bar(T3_Q_EMPTY0 + qb));  // the last product that reads this stage's Q tile
+              ++sq;
+              q_due = true;
+            }
           }
         }
       } else {
@@ -820,34 +892,32 @@ __global__ void __launch_bounds__(352, 1) attn_tc3_kernel(const __grid_constant_
     const int64_t qrow[2] = {i0 + rbase, i0 + rbase + 8};
     const bool valid[2] = {qrow[0] < P.lq, qrow[1] < P.lq};
     float m_ref[2] = {-INFINITY, -INFINITY}, l_part[2] = {0.f, 0.f};
-    int g = 0, it = 0;
+    int it = 0, stage = -1;
     bool ok = true;
-    for (int st = 0; st < P.n_stage && ok; ++st) {
-      const TcStage& S = P.stage[st];
-      int64_t vis_lo, vis_hi;
-      visible_key_range(S.mask_mode, S.mask_offset, S.mask_size, i0, i0 + rows_q - 1, S.lk, &vis_lo, &vis_hi);
-      if (vis_lo > vis_hi) continue;
-      int64_t jlo[2], jhi[2];  // keys of this stage visible to this thread's two query rows
+    int jlo[2] = {0, 0}, jhi[2] = {0, 0};  // keys of the stage visible to this thread's two query rows
+    const int n_parts = plan->n_parts;
+    for (int p = 0; p < n_parts && ok; ++p) {
+      const Part R = plan->part[p];
+      if ((R.stage & 255) != stage) {
+        stage = R.stage & 255;
+        const TcStage& S = P.stage[stage];
+        auto clamp = [](int64_t v) { return (int)(v < -(1 << 30) ? -(1 << 30) : v > (1 << 30) ? (1 << 30) : v); };
 #pragma unroll
-      for (int r = 0; r < 2; ++r) {
-        jlo[r] = 0, jhi[r] = S.lk - 1;
-        if (S.mask_mode == INFLLM_MASK_WINDOW) {
-          jlo[r] = qrow[r] + S.mask_offset - S.mask_size + 1;
-          jhi[r] = qrow[r] + S.mask_offset;
-        } else if (S.mask_mode == INFLLM_MASK_COMPLEMENT) {
-          jhi[r] = qrow[r] + S.mask_offset - S.mask_size;
+        for (int r = 0; r < 2; ++r) {
+          int64_t lo = 0, hi = S.lk - 1;
+          // rows past the last query are not masked, so that whole tiles stay whole: nothing of them is written
+          if (valid[r] && S.mask_mode == INFLLM_MASK_WINDOW) {
+            lo = qrow[r] + S.mask_offset - S.mask_size + 1;
+            hi = qrow[r] + S.mask_offset;
+          } else if (valid[r] && S.mask_mode == INFLLM_MASK_COMPLEMENT) {
+            hi = qrow[r] + S.mask_offset - S.mask_size;
+          }
+          jlo[r] = clamp(lo), jhi[r] = clamp(hi);
         }
-        // rows past the last query are not masked, so that whole tiles stay whole: nothing of them is written
-        if (!valid[r]) jhi[r] = S.lk - 1, jlo[r] = 0;
       }
-      int64_t seg_j0 = 0;
-      for (int sg = S.seg_begin; sg < S.seg_end && ok; ++sg) {
-        const TcSeg& G = P.seg[sg];
-        int tf, tl;
-        if (seg_tiles(vis_lo, vis_hi, seg_j0, G.len, &tf, &tl)) {
-          const int skip = g0 > g ? g0 - g : 0;
-          for (int t = tf + skip; t <= tl && ok; ++t, ++it) {
-            if (g + t - tf >= g1) break;
+      {
+        {
+          for (int t = 0; t < R.n && ok; ++t, ++it) {
             const int b3 = it % 3;
             const uint32_t tS = tmem + b3 * 128 + lane_base;
             ok = __all_sync(0xffffffffu, wait_or_abort(bar(T3_S_FULL0 + b3), (it / 3) & 1, abort_flag, P.err, 620));
@@ -856,14 +926,12 @@ __global__ void __launch_bounds__(352, 1) attn_tc3_kernel(const __grid_constant_
             float s[64];
             tmem_ld_16x256b_x16(tS, reinterpret_cast<uint32_t*>(s));
             tmem_wait_ld();
-            const int64_t jt = seg_j0 + (int64_t)t * kTile;
-            const int64_t lim = seg_j0 + G.len - 1;  // last key of the segment
+            const int jt = R.j + t * kTile;
             int c_lo[2], c_hi[2];
 #pragma unroll
             for (int r = 0; r < 2; ++r) {
-              const int64_t a = jlo[r] > jt ? jlo[r] : jt, e = jhi[r] < lim ? jhi[r] : lim;
-              c_lo[r] = (int)(a - jt);
-              c_hi[r] = (int)((e - jt) > (kTile - 1) ? (kTile - 1) : (e - jt));
+              c_lo[r] = jlo[r] - jt;
+              c_hi[r] = (jhi[r] < R.lim ? jhi[r] : R.lim) - jt;
             }
             if (!(c_lo[0] <= 0 && c_hi[0] >= kTile - 1 && c_lo[1] <= 0 && c_hi[1] >= kTile - 1)) {
 #pragma unroll
@@ -940,9 +1008,7 @@ __global__ void __launch_bounds__(352, 1) attn_tc3_kernel(const __grid_constant_
             __syncwarp();
             if (lane == 0) mbar_arrive(bar(T3_P_FULL0 + b3));  // per warp: 256 arrivals on one word took turns
           }
-          g += tl - tf + 1;
         }
-        seg_j0 += G.len;
       }
     }
     // ---- epilogue: row sums and reference maxima go through shared memory to the thread-per-row layout, in which
