@@ -1050,46 +1050,77 @@ __global__ void __launch_bounds__(352, 1) attn_tc3_kernel(const __grid_constant_
       const bool raw = P.part_acc != nullptr;
       const int64_t prow = (int64_t)split * P.n_heads * P.lq + srow;
       const float inv = l_out > 0.f ? 1.f / l_out : 0.f;
-      T* orow = raw ? nullptr : (T*)P.out + (int64_t)h * P.o_hs + qi * P.o_ts + col0;
+      // (loops that stay rolled: this runs once, and what it waits for is its instructions)
+      if (!P.st_acc && (!raw || rows_q <= 64)) {
+        T* orow = raw ? nullptr : (T*)P.out + (int64_t)h * P.o_hs + qi * P.o_ts + col0;
+#pragma unroll 1
+        for (int c = 0; c < 64; c += 32) {
+          uint32_t o[32];
+          if (it >= 1) {
+            tmem_ld32(tO + row_base + col0 + c, o);
+            tmem_wait_ld();
+          } else {
 #pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        uint32_t o[32];
-        if (it >= 1) {
-          tmem_ld32(tO + row_base + col0 + c * 32, o);
-          tmem_wait_ld();
-        } else {
-#pragma unroll
-          for (int k = 0; k < 32; ++k) o[k] = 0;
-        }
-        if (row_valid) {
-          if (P.st_acc) {
-            const float4* sp = reinterpret_cast<const float4*>(P.st_acc + srow * 128 + col0 + c * 32);
-#pragma unroll
-            for (int k = 0; k < 32; k += 4) {
-              const float4 v = sp[k >> 2];
-              o[k] = __float_as_uint(fmaf(wp, v.x, ws * __uint_as_float(o[k])));
-              o[k + 1] = __float_as_uint(fmaf(wp, v.y, ws * __uint_as_float(o[k + 1])));
-              o[k + 2] = __float_as_uint(fmaf(wp, v.z, ws * __uint_as_float(o[k + 2])));
-              o[k + 3] = __float_as_uint(fmaf(wp, v.w, ws * __uint_as_float(o[k + 3])));
-            }
+            for (int k = 0; k < 32; ++k) o[k] = 0;
           }
-          if (raw) {
-            uint4* ap = reinterpret_cast<uint4*>(P.part_acc + prow * 128 + col0 + c * 32);
+          if (row_valid && raw) {
+            uint4* ap = reinterpret_cast<uint4*>(P.part_acc + prow * 128 + col0 + c);
 #pragma unroll
             for (int k = 0; k < 32; k += 4) ap[k >> 2] = make_uint4(o[k], o[k + 1], o[k + 2], o[k + 3]);
-          } else {
+          } else if (row_valid) {
 #pragma unroll
             for (int k = 0; k < 32; k += 8) {
               uint4 v;
               uint32_t* pv = reinterpret_cast<uint32_t*>(&v);
 #pragma unroll
               for (int e = 0; e < 4; ++e) {
-                typename Act<T>::T2 v2 = Act<T>::from_f2(__uint_as_float(o[k + 2 * e]) * inv,
-                                                         __uint_as_float(o[k + 2 * e + 1]) * inv);
+                typename Act<T>::T2 v2 = Act<T>::from_f2(__uint_as_float(o[k + 2 * e]) * inv, __uint_as_float(o[k + 2 * e + 1]) * inv);
                 pv[e] = *reinterpret_cast<uint32_t*>(&v2);
               }
-              *reinterpret_cast<uint4*>(orow + c * 32 + k) = v;
+              *reinterpret_cast<uint4*>(orow + c + k) = v;
             }
+          }
+        }
+      } else if (i0 + quad * 32 < P.lq) {
+        // fp32 in or out, for more than a few rows: the warp's 32 rows by 64 columns go through shared memory (the operand buffers, which nothing reads
+        // any more), so that half a warp has 64 columns of a row and touches every 32-byte sector once
+        constexpr int kPitch = 68;  // floats; 16-byte pieces of eight neighbouring rows are in 32 different banks
+        float* stage = reinterpret_cast<float*>(smem) + warp * 32 * kPitch;
+#pragma unroll 1
+        for (int c = 0; c < 64; c += 32) {
+          uint32_t o[32];
+          if (it >= 1) {
+            tmem_ld32(tO + row_base + col0 + c, o);
+            tmem_wait_ld();
+          } else {
+#pragma unroll
+            for (int k = 0; k < 32; ++k) o[k] = 0;
+          }
+          uint4* w = reinterpret_cast<uint4*>(stage + lane * kPitch + c);
+#pragma unroll
+          for (int k = 0; k < 32; k += 4) w[k >> 2] = make_uint4(o[k], o[k + 1], o[k + 2], o[k + 3]);
+        }
+        __syncwarp();
+        const int cl = (lane & 15) * 4;
+        const int64_t row0 = i0 + quad * 32, srow0 = (int64_t)h * P.lq + row0, prow0 = (int64_t)split * P.n_heads * P.lq + srow0;
+        const float nrm = raw ? 1.f : inv;
+#pragma unroll 4
+        for (int k = 0; k < 16; ++k) {
+          const int rr = 2 * k + (lane >> 4);
+          const float f = __shfl_sync(0xffffffffu, ws * nrm, rr), fp = __shfl_sync(0xffffffffu, wp * nrm, rr);
+          if (row0 + rr >= P.lq) continue;
+          float4 v = *reinterpret_cast<const float4*>(stage + rr * kPitch + cl);
+          v = make_float4(v.x * f, v.y * f, v.z * f, v.w * f);
+          if (P.st_acc) {
+            const float4 x = *reinterpret_cast<const float4*>(P.st_acc + (srow0 + rr) * 128 + col0 + cl);
+            v = make_float4(fmaf(fp, x.x, v.x), fmaf(fp, x.y, v.y), fmaf(fp, x.z, v.z), fmaf(fp, x.w, v.w));
+          }
+          if (raw) {
+            *reinterpret_cast<float4*>(P.part_acc + (prow0 + rr) * 128 + col0 + cl) = v;
+          } else {
+            typename Act<T>::T2 v01 = Act<T>::from_f2(v.x, v.y), v23 = Act<T>::from_f2(v.z, v.w);
+            *reinterpret_cast<uint2*>((T*)P.out + (int64_t)h * P.o_hs + (row0 + rr) * P.o_ts + col0 + cl) =
+                make_uint2(*reinterpret_cast<uint32_t*>(&v01), *reinterpret_cast<uint32_t*>(&v23));
           }
         }
       }
