@@ -1425,20 +1425,21 @@ __global__ void __launch_bounds__(colsum_smem::kThreads, 1) colsum_tc_kernel(con
                   c_hi = vi_hi - t * kTile < q_end ? vi_hi - t * kTile : q_end;
         // a query row without any visible key has lse = -inf; it cannot see this key either, so it is masked
         const bool full = __all_sync(0xffffffffu, c_lo <= 0 && c_hi >= kTile - 1);
+        const int last = q_end < kTile - 1 ? q_end >> 5 : 3;  // the last 32 columns with queries at all
         const float* ls = s_lse + t * kTile;
         const float2 sc2 = make_float2(P.scale_log2, P.scale_log2);
         float2 acc[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
 #pragma unroll 1
-        for (int cc = 0; cc < 4; ++cc) {
+        for (int cc = 0; cc <= last; ++cc) {
           float sc[32];
           tmem_ld32(tS + cc * 32, reinterpret_cast<uint32_t*>(sc));
           tmem_wait_ld();
-          if (cc == 3) {  // everything is in registers: the buffer can be overwritten
+          if (cc == last) {  // everything is in registers: the buffer can be overwritten
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(bar(FR + part));
           }
-          if (full) {
+          if (full || __all_sync(0xffffffffu, c_lo <= cc * 32 && c_hi >= cc * 32 + 31)) {
 #pragma unroll
             for (int c = 0; c < 32; c += 4) {
               const float4 l4 = *reinterpret_cast<const float4*>(ls + cc * 32 + c);  // negated
@@ -1447,7 +1448,7 @@ __global__ void __launch_bounds__(colsum_smem::kThreads, 1) colsum_tc_kernel(con
               acc[0] = fadd2(acc[0], make_float2(ex2_approx(a0.x), ex2_approx(a0.y)));
               acc[1] = fadd2(acc[1], (c & 4) ? ex2_poly2<4>(a1) : make_float2(ex2_approx(a1.x), ex2_approx(a1.y)));
             }
-          } else {
+          } else if (__any_sync(0xffffffffu, c_lo <= cc * 32 + 31 && c_hi >= cc * 32)) {
 #pragma unroll
             for (int c = 0; c < 32; ++c) {
               const float pv = ex2_approx(fmaf(sc[c], P.scale_log2, ls[cc * 32 + c]));
