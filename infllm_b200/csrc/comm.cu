@@ -448,7 +448,7 @@ int ingest_token_launch(const void* q, int64_t q_hs, const void* k, int64_t k_hs
                         int dtype, cudaStream_t s, int32_t* clear);
 int block_topk_launch(const void* bk, int64_t n, int width, const float* qbar, float* scores, int k, int id_base,
                       int32_t* out_ids, float* out_scores, int dtype, cudaStream_t s, unsigned int* ticket,
-                      int32_t* out_ids_copy = nullptr);
+                      int32_t* out_ids_copy = nullptr, uint32_t seq = 0);
 }  // namespace infllm
 
 __global__ void stamp_kernel(unsigned long long* p) {

@@ -45,7 +45,7 @@ int qbar_launch(const void* q, int64_t q_hs, int64_t q_ts, int n_heads, int64_t 
                 float* qbar, int64_t qbar_stride, int dtype, cudaStream_t s);
 int block_topk_launch(const void* bk, int64_t n, int width, const float* qbar, float* scores, int k, int id_base,
                       int32_t* out_ids, float* out_scores, int dtype, cudaStream_t s, unsigned int* ticket,
-                      int32_t* out_ids_copy = nullptr);
+                      int32_t* out_ids_copy = nullptr, uint32_t seq = 0);
 int seal_score_launch(const void* k, int64_t k_hs, int64_t k_ts, const float* score, int64_t score_hs, int64_t tok0, int n_new,
                       int first_new, int block_size, int repr_topk, int n_heads, int n_kv_heads, int head_dim, void* bk,
                       const int32_t* rows, int n_old, const float* qbar, float* scores, unsigned long long* words, uint32_t seq,
@@ -248,7 +248,8 @@ struct infllm_ctx {
   int32_t* d_topk = nullptr; // (topk)
   infllm_comm* comm = nullptr;  // KV-head-group sharding: the retrieval scores are summed over the ranks
   unsigned int* tickets = nullptr;  // "last CTA" counters of the fused scoring kernel: [0] main stream, [1] look-ahead stream
-  int32_t* h_topk = nullptr; // pinned
+  int32_t* h_topk = nullptr; // pinned; {id, topk_seq} words where the ranking kernel writes them itself
+  uint32_t topk_seq = 0;
   float *part_o = nullptr, *part_lse = nullptr, *dec_logits = nullptr;
   int max_parts = 0;
 
@@ -581,8 +582,8 @@ int lazy_init(infllm_ctx* c, cudaStream_t s) {
   INFLLM_CUDA_OK(cudaDeviceGetAttribute(&c->tok_sms, cudaDevAttrMultiProcessorCount, g.device));
   INFLLM_CUDA_OK(dev_malloc((void**)&c->tickets, 2 * sizeof(unsigned int)));
   INFLLM_CUDA_OK(cudaMemsetAsync(c->tickets, 0, 2 * sizeof(unsigned int), s));
-  INFLLM_CUDA_OK(cudaHostAlloc((void**)&c->h_topk, std::max(1, g.topk) * sizeof(int32_t),
-                               cudaHostAllocDefault));
+  INFLLM_CUDA_OK(cudaHostAlloc((void**)&c->h_topk, std::max(1, g.topk) * sizeof(unsigned long long), cudaHostAllocDefault));
+  memset(c->h_topk, 0, std::max(1, g.topk) * sizeof(unsigned long long));
   INFLLM_CUDA_OK(cudaHostAlloc((void**)&c->h_spec, std::max(1, g.topk) * sizeof(int32_t), cudaHostAllocDefault));
   c->cand_cap = g.topk + (c->look_depth + 1) * (g.exc_block_size / g.block_size + 2) + 4;
   for (auto& l : c->la) {
@@ -850,15 +851,37 @@ int ensure_scores(infllm_ctx* c, int64_t n, cudaStream_t s) {
 // this context holds a slice of the heads) the scores are summed over the ranks between the two halves, so that
 // every rank ranks the same numbers.  `which` picks the communicator of the stream (0 main, 1 look-ahead).
 int score_topk(infllm_ctx* c, int64_t n, const float* qbar, float* scores, int32_t* d_ids, cudaStream_t s, int which,
-               int k = 0, int32_t* ids_copy = nullptr) {
+               int k = 0, int32_t* ids_copy = nullptr, uint32_t seq = 0) {
   const infllm_config& g = c->cfg;
   if (k <= 0) k = g.topk;
   if (!c->comm)
     return block_topk_launch(c->block_k, n, (int)c->width, qbar, scores, k, 0, d_ids, nullptr, g.dtype, s,
-                             c->tickets + which, ids_copy);
+                             c->tickets + which, ids_copy, seq);
   INFLLM_TRY(block_score_launch(c->block_k, n, (int)c->width, qbar, scores, g.dtype, s));
   INFLLM_TRY(comm_allreduce_sum(c->comm, which, scores, (size_t)n, s));
   return topk_launch(scores, n, k, 0, d_ids, nullptr, s);
+}
+
+// A word {value, seq} that a kernel writes to pinned memory, as soon as it is there - an event behind the kernel arrives 3 us
+// later.  Bounded: the kernels' own waits end after a second or two and leave the error record; the rest of the limit is
+// for work ahead of the kernel on its stream.
+int wait_word(infllm_ctx* c, const unsigned long long* p, uint32_t seq, uint32_t* value) {
+  const auto t0 = std::chrono::steady_clock::now();
+  for (unsigned turn = 1;; ++turn) {
+    const unsigned long long w = *(const volatile unsigned long long*)p;
+    if ((uint32_t)(w >> 32) == seq) {
+      *value = (uint32_t)w;
+      return INFLLM_OK;
+    }
+    for (int spin = 0; spin < 32; ++spin) __builtin_ia32_pause();
+    if (turn % 64) continue;
+    if (c->h_tc_err && *(volatile int32_t*)c->h_tc_err) INFLLM_TRY(check_device_error(c, c->last_stream));
+    if (turn % 4096) continue;
+    const cudaError_t e = cudaStreamQuery(c->last_stream);
+    if (e != cudaSuccess && e != cudaErrorNotReady) INFLLM_CUDA_OK(e);
+    if (std::chrono::steady_clock::now() - t0 > std::chrono::seconds(60))
+      return fail(INFLLM_E_TIMEOUT, "a result that a kernel sends to the host did not arrive");
+  }
 }
 
 // the scorer's one-launch form can write the ids into pinned host words itself (no copy, which would queue behind the
@@ -872,10 +895,17 @@ int retrieve_launch(infllm_ctx* c, int eb_in_call, int64_t n, cudaStream_t s) {
   const bool direct = ids_direct(c, n);
   {
     ProfScope ps(c, s, INFLLM_PROF_TOPK, (double)n * c->width * c->esz);
-    INFLLM_TRY(score_topk(c, n, c->qbar + (int64_t)eb_in_call * c->width, c->scores, c->d_topk, s, 0, 0, direct ? c->h_topk : nullptr));
+    if (direct && ++c->topk_seq == 0) {  // the numbers are used up: no word carries one any more
+      memset(c->h_topk, 0, g.topk * sizeof(unsigned long long));
+      c->topk_seq = 1;
+    }
+    INFLLM_TRY(score_topk(c, n, c->qbar + (int64_t)eb_in_call * c->width, c->scores, c->d_topk, s, 0, 0, direct ? c->h_topk : nullptr,
+                          c->topk_seq));
   }
-  if (!direct) INFLLM_CUDA_OK(cudaMemcpyAsync(c->h_topk, c->d_topk, g.topk * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-  INFLLM_CUDA_OK(cudaEventRecord(c->ev_sync, s));
+  if (!direct) {
+    INFLLM_CUDA_OK(cudaMemcpyAsync(c->h_topk, c->d_topk, g.topk * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+    INFLLM_CUDA_OK(cudaEventRecord(c->ev_sync, s));
+  }
   return INFLLM_OK;
 }
 
@@ -888,8 +918,19 @@ int retrieve_now(infllm_ctx* c, int eb_in_call, std::vector<int32_t>* ids, cudaS
     return INFLLM_OK;
   }
   if (!launched) INFLLM_TRY(retrieve_launch(c, eb_in_call, n, s));
-  INFLLM_CUDA_OK(cudaEventSynchronize(c->ev_sync));  // the ids decide the cache plan (context_manager.py:163)
-  ids->assign(c->h_topk, c->h_topk + g.topk);
+  // the ids decide the cache plan (context_manager.py:163)
+  if (ids_direct(c, n)) {
+    for (int i = 0; i < g.topk; ++i) {
+      uint32_t id = 0;
+      INFLLM_TRY(wait_word(c, reinterpret_cast<unsigned long long*>(c->h_topk) + i, c->topk_seq, &id));
+      ids->push_back((int32_t)id);
+    }
+  } else {
+    INFLLM_CUDA_OK(cudaEventSynchronize(c->ev_sync));
+    // (a number of an earlier call may have been among the low halves: the words start again)
+    ids->assign(c->h_topk, c->h_topk + g.topk);
+    memset(c->h_topk, 0, g.topk * sizeof(unsigned long long));
+  }
   return INFLLM_OK;
 }
 
@@ -1018,28 +1059,6 @@ int lookahead_stage(infllm_ctx* c, int64_t target) {
   }
   if (!src.empty()) trace_mark(c, c->copy_stream, TR_STAGE_END, target);
   return INFLLM_OK;
-}
-
-// A word {value, seq} that a kernel writes to pinned memory, as soon as it is there - an event behind the kernel arrives 3 us
-// later.  Bounded: the kernels' own waits end after a second or two and leave the error record; the rest of the limit is
-// for work ahead of the kernel on its stream.
-int wait_word(infllm_ctx* c, const unsigned long long* p, uint32_t seq, uint32_t* value) {
-  const auto t0 = std::chrono::steady_clock::now();
-  for (unsigned turn = 1;; ++turn) {
-    const unsigned long long w = *(const volatile unsigned long long*)p;
-    if ((uint32_t)(w >> 32) == seq) {
-      *value = (uint32_t)w;
-      return INFLLM_OK;
-    }
-    for (int spin = 0; spin < 32; ++spin) __builtin_ia32_pause();
-    if (turn % 64) continue;
-    if (c->h_tc_err && *(volatile int32_t*)c->h_tc_err) INFLLM_TRY(check_device_error(c, c->last_stream));
-    if (turn % 4096) continue;
-    const cudaError_t e = cudaStreamQuery(c->last_stream);
-    if (e != cudaSuccess && e != cudaErrorNotReady) INFLLM_CUDA_OK(e);
-    if (std::chrono::steady_clock::now() - t0 > std::chrono::seconds(60))
-      return fail(INFLLM_E_TIMEOUT, "a result that a kernel sends to the host did not arrive");
-  }
 }
 
 // the candidates of the next exec block once n_now units exist: what its look-ahead found, then the units sealed since.
