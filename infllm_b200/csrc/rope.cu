@@ -83,8 +83,8 @@ __global__ void copy_rows_kernel(const T* __restrict__ x, int64_t x_hs, int64_t 
 }
 
 // The live tokens of the token buffers move to the front: rows [off, off + live) of every KV head of the three key/value
-// buffers to [0, live) (off >= live: nothing overlaps), rows [pad0, pad1) become zero, and the same tokens of every head's
-// scores.  Rows are `row` 16-byte pieces, heads `cap` rows apart; plane blockIdx.y is a buffer's head, then a head's scores.
+// buffers to [0, live) (off >= live: nothing overlaps), and the same tokens of every head's scores; rows [pad0, pad1) become
+// zero, in a launch of their own because they may be among the rows that are moved.  Rows are `row` 16-byte pieces, heads `cap` rows apart; plane blockIdx.y is a buffer's head, then a head's scores.
 // Bound: HBM.  4.6K tokens of 8 KV heads: four copies into new buffers and three memsets took 56 us, and the host 40 us.
 __global__ void __launch_bounds__(256) shift_tokens_kernel(uint4* k_raw, uint4* k_rot, uint4* v, float* score, int row, int hkv,
                                                            int64_t cap, int64_t off, int64_t live, int64_t pad0, int64_t pad1) {
@@ -413,9 +413,17 @@ int shift_tokens_launch(void* k_raw, void* k_rot, void* v, float* score, int row
   if (off < live || off + live > cap || pad0 < live || pad1 > cap || row_bytes % 16)
     return fail(INFLLM_E_BADARG, "shift_tokens: %lld tokens from %lld of %lld", (long long)live, (long long)off, (long long)cap);
   const dim3 grid((unsigned)std::max(1, 1184 / (3 * n_kv_heads)), 3 * n_kv_heads + n_heads);
-  shift_tokens_kernel<<<grid, 256, 0, s>>>((uint4*)k_raw, (uint4*)k_rot, (uint4*)v, score, row_bytes / 16, n_kv_heads, cap, off, live,
-                                           pad0, pad1);
-  INFLLM_LAUNCH_OK("shift_tokens_kernel");
+  auto run = [&](dim3 grid, int64_t from, int64_t n, int64_t p0, int64_t p1) {
+    shift_tokens_kernel<<<grid, 256, 0, s>>>((uint4*)k_raw, (uint4*)k_rot, (uint4*)v, score, row_bytes / 16, n_kv_heads, cap, from, n, p0, p1);
+  };
+  if (live > 0) {
+    run(grid, off, live, 0, 0);
+    INFLLM_LAUNCH_OK("shift_tokens_kernel");
+  }
+  if (pad0 < pad1) {
+    run(dim3(8, 3 * n_kv_heads), 0, 0, pad0, pad1);
+    INFLLM_LAUNCH_OK("shift_tokens_kernel");
+  }
   return INFLLM_OK;
 }
 
