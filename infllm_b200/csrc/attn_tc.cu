@@ -1151,6 +1151,7 @@ __global__ void attn_tc_combine_kernel(const float* __restrict__ acc, const floa
                                        T* __restrict__ out, int64_t o_hs, int64_t o_ts, float* __restrict__ lse,
                                        const float* st_acc, const float* st_m, const float* st_l, float* new_acc,
                                        float* new_m, float* new_l) {
+  chain_enter();
   const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);  // h * lq + i
   if (row >= (int64_t)n_heads * lq) return;
   const int lane = threadIdx.x & 31;
@@ -1554,8 +1555,8 @@ int attn_tc_combine_launch(const float* acc, const float* m, const float* l, int
   const int64_t rows = (int64_t)n_heads * lq;
   const int threads = rows >= 4096 ? 256 : 64;  // few rows: spread over the SMs
   INFLLM_DISPATCH_DTYPE(dtype, T, {
-    attn_tc_combine_kernel<T><<<(unsigned)ceil_div(rows, threads / 32), threads, 0, s>>>(
-        acc, m, l, n_split, n_heads, lq, (T*)out, o_hs, o_ts, lse, st_acc, st_m, st_l, new_acc, new_m, new_l);
+    INFLLM_CUDA_OK(launch_chained(attn_tc_combine_kernel<T>, dim3((unsigned)ceil_div(rows, threads / 32)), dim3(threads), 0, s, acc, m,
+                                  l, n_split, n_heads, lq, (T*)out, o_hs, o_ts, lse, st_acc, st_m, st_l, new_acc, new_m, new_l));
   });
   INFLLM_LAUNCH_OK("attn_tc_combine_kernel");
   return INFLLM_OK;
