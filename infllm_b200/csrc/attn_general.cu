@@ -478,7 +478,7 @@ static int stage_tc(const void* d_q, int64_t q_hs, int64_t q_ts, const void* d_k
   INFLLM_TRY(encode_rows_map(&P.maps[1], dtype, d_k, lk, n_kv_heads, k_hs, k_ts));
   INFLLM_TRY(encode_rows_map(&P.maps[2], dtype, d_v, lk, n_kv_heads, k_hs, k_ts));
   INFLLM_TRY(tc_get_error_ptr(&P.err));
-  P.n_stage = 1; P.n_heads = n_heads; P.n_kv_heads = n_kv_heads; P.lq = lq;
+  P.n_stage = 1; P.n_heads = n_heads; P.n_kv_heads = n_kv_heads; P.lq = lq; P.exact = 1;
   P.scale_log2 = kLog2e / sqrtf(128.f);
   P.stage[0] = {0, 0, mask_mode, 0, 1, 0, mask_offset, mask_size, lk};
   P.seg[0] = {1, 2, 0, -1, -1, (int32_t)lk};

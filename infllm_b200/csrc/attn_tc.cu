@@ -75,12 +75,14 @@ __device__ __forceinline__ float2 fadd2(float2 a, float2 b) {
 
 // exp2 of a pair on the FMA and integer pipes (the special-function unit does 16 per clock per SM, which bounds the
 // softmax when every exponential goes there): x = n + f with n the nearest integer (magic-number rounding) and f in
-// [-0.5, 0.5], 2^f by a polynomial whose relative error was minimised over that interval (weighted least squares on
-// Chebyshev points), n added into the exponent.  Cubic: 7.5e-5, a twentieth of the rounding of a 16-bit P; quartic:
-// 2.6e-6, for sums that stay fp32.
+// [-0.5, 0.5], 2^f by a polynomial whose relative error was minimised over that interval (least squares on Chebyshev
+// points), n added into the exponent.  Arguments below -126, those of masked keys too, give 2^-126.
+//   cubic    7.5e-5: a twentieth of the rounding of a bf16 P, a third to a sixth of that of an fp16 P
+//   quartic  2.6e-6
+//   quintic  2e-7 as evaluated in fp32, which is what ex2.approx has: where exp2f was
 template <int kDegree>
 __device__ __forceinline__ float2 ex2_poly2(float2 x) {
-  static_assert(kDegree == 3 || kDegree == 4, "");
+  static_assert(kDegree >= 3 && kDegree <= 5, "");
   x.x = fmaxf(x.x, -126.f);
   x.y = fmaxf(x.y, -126.f);
   const float2 magic = make_float2(12582912.f, 12582912.f), neg_magic = make_float2(-12582912.f, -12582912.f);
@@ -93,11 +95,17 @@ __device__ __forceinline__ float2 ex2_poly2(float2 x) {
     p = ffma2(f.x, f.y, c2(0.05517167f), c2(0.24261113f));
     p = ffma2(p.x, p.y, f, c2(0.69326097f));
     p = ffma2(p.x, p.y, f, c2(0.99992806f));
-  } else {
+  } else if (kDegree == 4) {
     p = ffma2(f.x, f.y, c2(0.0095701022f), c2(0.055917859f));
     p = ffma2(p.x, p.y, f, c2(0.24024744f));
     p = ffma2(p.x, p.y, f, c2(0.69312179f));
     p = ffma2(p.x, p.y, f, c2(0.99999928f));
+  } else {
+    p = ffma2(f.x, f.y, c2(0.00132669706f), c2(0.00967545994f));
+    p = ffma2(p.x, p.y, f, c2(0.0555074252f));
+    p = ffma2(p.x, p.y, f, c2(0.240221217f));
+    p = ffma2(p.x, p.y, f, c2(0.693146944f));
+    p = ffma2(p.x, p.y, f, c2(1.00000012f));
   }
   return make_float2(__int_as_float(__float_as_int(p.x) + (__float_as_int(t.x) << 23)),
                      __int_as_float(__float_as_int(p.y) + (__float_as_int(t.y) << 23)));
@@ -587,7 +595,8 @@ __global__ void __launch_bounds__(576, 1) attn_tc2_kernel(const __grid_constant_
 // producer, and one issuing thread per product (one thread for both was the longest serial chain of a tile).
 // The softmax warps read S in the 16-lane shape: warps w and w+4 share a TMEM lane quarter and take 16 of its rows
 // each with all 128 key columns, a row is spread over the four threads of a quad, so a row maximum is two shuffles
-// and no thread waits for another warp.  Every fourth pair of exponentials is a cubic on the FMA pipe.  The producer
+// and no thread waits for another warp.  Every fourth pair of exponentials is a polynomial on the FMA pipe: a
+// cubic in a memory's exec blocks, a quintic (kExact) where the work was the shape-generic kernel's before, with exp2f.  The producer
 // asks for K one tile ahead of V (the V buffer frees late in a tile's cycle and K(t+1) queued behind that wait).
 // What the clock stamps of one CTA say (cycles per 128-key tile, 131072-token prefill): the period is 2100-2200 and
 // it is the softmax warps' (1700 of work, 400 of waits and loop); S is ready 2000 cycles before they come for it; a
@@ -598,7 +607,7 @@ __global__ void __launch_bounds__(576, 1) attn_tc2_kernel(const __grid_constant_
 // asking TMEM for the next tile's scores before this tile's exponentials (111 us), an L2 prefetch of the key tiles
 // four to eight tiles ahead (no change), all exponentials or half of them on the special-function unit (87, 86 us).
 // 70 to 74 us per exec block of the 128K prefill (83 before the run's parts were listed once, the epilogue rolled and the
-// exponentials every fourth pair a cubic).  A CTA's cycles there: 7500 to the first tile's scores, 54 tiles of 2000, 3400
+// exponentials every fourth pair on the FMA pipe).  A CTA's cycles there: 7500 to the first tile's scores, 54 tiles of 2000, 3400
 // behind the last; a run of 12 tiles: 34000 in all.
 namespace tc3 {
 constexpr int kQ = 0;                            // two stages
@@ -700,7 +709,7 @@ __device__ __forceinline__ void make_plan(const AttnTcParams& P, int64_t i0, int
 }
 }  // namespace tc3
 
-template <typename T>
+template <typename T, bool kExact>
 __global__ void __launch_bounds__(352, 1) attn_tc3_kernel(const __grid_constant__ AttnTcParams P) {
   using namespace tc3;
   extern __shared__ unsigned char smem_raw[];
@@ -980,7 +989,7 @@ __global__ void __launch_bounds__(352, 1) attn_tc3_kernel(const __grid_constant_
               const float2 a = ffma2(s[2 * k], s[2 * k + 1], sc2, nm2[r]);
               float2 p;
               if ((k % kPolyEvery) == kPolyEvery - 1) {
-                p = ex2_poly2<3>(a);  // one pair in kPolyEvery off the special-function unit
+                p = ex2_poly2<kExact ? 5 : 3>(a);  // one pair in kPolyEvery off the special-function unit
               } else {
                 p = make_float2(ex2_approx(a.x), ex2_approx(a.y));
               }
@@ -1034,7 +1043,7 @@ __global__ void __launch_bounds__(352, 1) attn_tc3_kernel(const __grid_constant_
     // Three ways out: a run of a split work item leaves its un-normalised partial; a stage of a multi-stage attention
     // leaves the state (acc, m, l); everything else is normalised.  A state that came in is folded in first.
     const int64_t srow = (int64_t)h * P.lq + qi;
-    // (the cubic exponential leaves 2^-126 of a masked key: a row that saw no key has the sum 0 by its maximum)
+    // (the polynomial leaves 2^-126 of a masked key: a row that saw no key has the sum 0 by its maximum)
     float ws = 1.f, wp = 0.f, m_out = m_row, l_out = it >= 1 && m_row != -INFINITY ? l_sum : 0.f;
     if (P.st_acc) {
       if (row_valid) {
@@ -1196,7 +1205,7 @@ __global__ void attn_tc_combine_kernel(const float* __restrict__ acc, const floa
 // four of the sixteen compute warps of its own, which turn it into sum_q exp2(s - lse_q).  A key tile is loaded once
 // per head and a query tile once per CTA, which keeps the L2 traffic an order of magnitude below one load per pair.
 // Bound: 16384 exponentials per pair, 768 cycles of the special-function unit with every fourth pair of them as a
-// quartic on the FMA pipe, and the product, 514; a pair takes 1150.  512 queries x 32 heads over 4608 keys: 30.7 us.
+// quartic on the FMA pipe (a quintic, kExact, for the short calls), and the product, 514; a pair takes 1150.  512 queries x 32 heads over 4608 keys: 30.7 us.
 // (37.6 us with one issuing thread and all sixteen warps on one buffer at a time, whose exponentials were two at a
 // time in fp16: 1.4e-3 off in a sum, now 1e-6.)
 namespace colsum_smem {
@@ -1231,7 +1240,7 @@ __device__ __forceinline__ void colsum_q_tiles(const ColsumTcParams& P, int j0, 
   *tl = lo <= hi ? hi / kTile : -1;
 }
 
-template <typename T>
+template <typename T, bool kExact>
 __global__ void __launch_bounds__(colsum_smem::kThreads, 1) colsum_tc_kernel(const __grid_constant__ ColsumTcParams P) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -1449,7 +1458,7 @@ __global__ void __launch_bounds__(colsum_smem::kThreads, 1) colsum_tc_kernel(con
               const float2 a0 = ffma2(sc[c], sc[c + 1], sc2, make_float2(l4.x, l4.y));
               const float2 a1 = ffma2(sc[c + 2], sc[c + 3], sc2, make_float2(l4.z, l4.w));
               acc[0] = fadd2(acc[0], make_float2(ex2_approx(a0.x), ex2_approx(a0.y)));
-              acc[1] = fadd2(acc[1], (c & 4) ? ex2_poly2<4>(a1) : make_float2(ex2_approx(a1.x), ex2_approx(a1.y)));
+              acc[1] = fadd2(acc[1], (c & 4) ? ex2_poly2<kExact ? 5 : 4>(a1) : make_float2(ex2_approx(a1.x), ex2_approx(a1.y)));
             }
           } else if (__any_sync(0xffffffffu, c_lo <= cc * 32 + 31 && c_hi >= cc * 32)) {
 #pragma unroll
@@ -1579,7 +1588,7 @@ int attn_tc3_launch(const AttnTcParams& P, int dtype, cudaStream_t s) {
   dim3 grid((unsigned)ceil_div(P.lq, kTile), P.n_heads, P.n_split);
   const size_t smem = tc3::kTotal + 1024;
   INFLLM_DISPATCH_DTYPE(dtype, T, {
-    auto kern = attn_tc3_kernel<T>;
+    auto kern = P.exact ? attn_tc3_kernel<T, true> : attn_tc3_kernel<T, false>;
     // the opt-in holds for the current device only, and a process may drive several: asked for at every launch
     INFLLM_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     kern<<<grid, 352, smem, s>>>(P);
@@ -1646,7 +1655,7 @@ int colsum_tc_launch_maps(const CUtensorMap& map_q, const CUtensorMap& map_k, in
   dim3 grid((unsigned)ceil_div(n_tiles, per), n_heads);
   const size_t smem = colsum_smem::kTotal + 1024;
   INFLLM_DISPATCH_DTYPE(dtype, T, {
-    auto kern = colsum_tc_kernel<T>;
+    auto kern = lq <= kExactQueries ? colsum_tc_kernel<T, true> : colsum_tc_kernel<T, false>;
     // the opt-in holds for the current device only, and a process may drive several: asked for at every launch
     INFLLM_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     INFLLM_CUDA_OK(launch_chained(kern, grid, dim3(colsum_smem::kThreads), smem, s, P));

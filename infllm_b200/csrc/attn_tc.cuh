@@ -7,6 +7,9 @@ namespace infllm {
 
 constexpr int kTcMaxMaps = 12;
 constexpr int kTile = 128;
+// Exec blocks of up to this many queries, like every stage of the multi-stage class and the sink + window types, used to
+// be the shape-generic kernels', with exp2f; they keep its precision.  Larger ones have had the cubic all along.
+constexpr int kExactQueries = 64;
 
 struct TcSeg {
   int16_t map_k, map_v;  // indices into AttnTcParams::maps
@@ -35,7 +38,8 @@ struct AttnTcParams {
   // The key tiles of a work item are cut into n_split runs; with n_split > 1 every run writes an un-normalised
   // partial (acc, m, l) and attn_tc_combine merges them.  With n_split == 1 the one-head kernel writes its state here
   // instead of out / lse when part_acc is set, and folds in the state st_* when that is set (it may be the same memory).
-  int32_t n_split, pad2;
+  int32_t n_split;
+  int32_t exact;    // exponentials to fp32's precision throughout (see kExactQueries)
   float* part_acc;  // (n_split, H, lq, 128)
   float* part_m;    // (n_split, H, lq)
   float* part_l;    // (n_split, H, lq)

@@ -216,6 +216,7 @@ extern "C" int infllm_sink_window_run(const infllm_sink_window* args, void* stre
   INFLLM_TRY(encode_rows_map(&A.maps[1], a.dtype, P.k_rot, p.rows_w, a.n_kv_heads, p.rows_w * 128, 128));
   INFLLM_TRY(encode_rows_map(&A.maps[2], a.dtype, v_base, p.rows_w, a.n_kv_heads, v_hs, 128));
   INFLLM_TRY(tc_get_error_ptr(&A.err));
+  A.exact = 1;
   A.n_stage = 1; A.n_heads = a.n_heads; A.n_kv_heads = a.n_kv_heads; A.lq = a.len_q;
   A.out = a.d_out; A.o_hs = a.o_hs; A.o_ts = a.o_ts; A.scale_log2 = kLog2e / sqrtf(128.f);
   A.stage[0] = {0, 0, INFLLM_MASK_WINDOW, 0, 1, 0, p.lw - a.len_q, a.n_local, p.lw};
