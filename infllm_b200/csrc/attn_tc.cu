@@ -966,11 +966,12 @@ __global__ void __launch_bounds__(352, 1) attn_tc3_kernel(const __grid_constant_
               float mx = fmaxf(mxa[r], mxb[r]);
               mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
               mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2)) * P.scale_log2;
-              // lazy rescaling: the reference maximum only moves when the row maximum grew by more than 2^8
+              // lazy rescaling: the reference maximum only moves when the row maximum grew by more than 2^8 - or, kExact, at
+              // all, so that the largest probabilities of a row are the ones that a 16-bit P holds without a rounding
               if (mx > m_ref[r]) {
                 if (m_ref[r] == -INFINITY) {
                   m_ref[r] = mx;  // nothing accumulated for this row yet
-                } else if (mx - m_ref[r] > 8.f) {
+                } else if (mx - m_ref[r] > (kExact ? 0.f : 8.f)) {
                   alpha[r] = ex2_approx(m_ref[r] - mx);
                   l_part[r] *= alpha[r];
                   m_ref[r] = mx;
