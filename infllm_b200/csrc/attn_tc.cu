@@ -66,6 +66,12 @@ __device__ __forceinline__ float2 ffma2(float a0, float a1, float2 b, float2 c) 
       : "=f"(d.x), "=f"(d.y) : "f"(a0), "f"(a1), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
   return d;
 }
+__device__ __forceinline__ float2 fmul2(float2 a, float2 b) {
+  float2 d;
+  asm("{ .reg .b64 ra, rb, rd; mov.b64 ra, {%2,%3}; mov.b64 rb, {%4,%5}; mul.rn.f32x2 rd, ra, rb; mov.b64 {%0,%1}, rd; }"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
 __device__ __forceinline__ float2 fadd2(float2 a, float2 b) {
   float2 d;
   asm("{ .reg .b64 ra, rb, rd; mov.b64 ra, {%2,%3}; mov.b64 rb, {%4,%5}; add.rn.f32x2 rd, ra, rb; mov.b64 {%0,%1}, rd; }"
@@ -76,15 +82,20 @@ __device__ __forceinline__ float2 fadd2(float2 a, float2 b) {
 // exp2 of a pair on the FMA and integer pipes (the special-function unit does 16 per clock per SM, which bounds the
 // softmax when every exponential goes there): x = n + f with n the nearest integer (magic-number rounding) and f in
 // [-0.5, 0.5], 2^f by a polynomial whose relative error was minimised over that interval (least squares on Chebyshev
-// points), n added into the exponent.  Arguments below -126, those of masked keys too, give 2^-126.
+// points), times 2^n.  A NaN stays one; arguments below -126, those of masked keys too, give 2^-126.
 //   cubic    7.5e-5: a twentieth of the rounding of a bf16 P, a third to a sixth of that of an fp16 P
 //   quartic  2.6e-6
 //   quintic  2e-7 as evaluated in fp32, which is what ex2.approx has: where exp2f was
+__device__ __forceinline__ float max_nan(float a, float b) {
+  float d;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(d) : "f"(a), "f"(b));
+  return d;
+}
 template <int kDegree>
 __device__ __forceinline__ float2 ex2_poly2(float2 x) {
   static_assert(kDegree >= 3 && kDegree <= 5, "");
-  x.x = fmaxf(x.x, -126.f);
-  x.y = fmaxf(x.y, -126.f);
+  x.x = max_nan(x.x, -126.f);
+  x.y = max_nan(x.y, -126.f);
   const float2 magic = make_float2(12582912.f, 12582912.f), neg_magic = make_float2(-12582912.f, -12582912.f);
   const float2 t = fadd2(x, magic);
   const float2 n = fadd2(t, neg_magic);
@@ -107,8 +118,9 @@ __device__ __forceinline__ float2 ex2_poly2(float2 x) {
     p = ffma2(p.x, p.y, f, c2(0.693146944f));
     p = ffma2(p.x, p.y, f, c2(1.00000012f));
   }
-  return make_float2(__int_as_float(__float_as_int(p.x) + (__float_as_int(t.x) << 23)),
-                     __int_as_float(__float_as_int(p.y) + (__float_as_int(t.y) << 23)));
+  // a product, not an addition to the exponent's bits: that would make a number of a NaN
+  return fmul2(p, make_float2(__int_as_float((__float_as_int(t.x) << 23) + 0x3f800000),
+                              __int_as_float((__float_as_int(t.y) << 23) + 0x3f800000)));
 }
 
 // two exponentials per special-function instruction: exp2 of a pair of fp32 arguments evaluated in fp16

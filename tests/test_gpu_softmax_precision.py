@@ -98,3 +98,37 @@ def test_the_largest_probability_is_exact(where, dtype):
         z = _logits(qr[0], kr[0, :, at:at + 1], G)[..., 0] * log2e
         others = torch.full((L,), n_local + units * 128 + n_init + L - 1.0, device="cuda", dtype=torch.float64)
         _check_the_largest(out, z, others, val[:, 0].repeat_interleave(G, 0), 50)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_a_nan_is_seen(dtype):
+    """A NaN in one key reaches every query that sees it, whatever the key's place in a tile; one in a query reaches the
+    scores of the keys that it sees."""
+    from infllm_b200.attention import get_multi_stage_dot_production_attention
+
+    H, HKV, lq, lk = 4, 2, 160, 300
+    g = torch.Generator(device="cuda").manual_seed(4)
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda").to(dtype)  # noqa: E731
+    q, k, v = rnd(1, H, lq, D), rnd(1, HKV, lk, D), rnd(1, HKV, lk, D)
+
+    def run(q, k):
+        att = get_multi_stage_dot_production_attention(True)[0](q.shape, q.dtype, q.device)
+        att.append(q, k, v, end=True, sliding_window=200, get_score=True)
+        out, score = att.get_result()
+        return out[0], score[0][0]
+
+    for j in list(range(16)) + [lk - 1]:
+        bad = k.clone()
+        bad[0, 1, j, 5] = float("nan")
+        out, _ = run(q, bad)
+        i = torch.arange(lq, device="cuda") + lk - lq
+        sees = (i >= j) & (i - j < 200)
+        assert out[2:, sees].isnan().all() and not out[2:, ~sees].isnan().any() and not out[:2].isnan().any(), j
+    for i in list(range(8)) + [lq - 1]:
+        bad = q.clone()
+        bad[0, 3, i, 7] = float("nan")
+        _, score = run(bad, k)
+        j = torch.arange(lk, device="cuda")
+        d = i + lk - lq - j
+        sees = (d >= 0) & (d < 200)
+        assert score[3, sees].isnan().all() and not score[3, ~sees].isnan().any() and not score[:3].isnan().any(), i
