@@ -2231,15 +2231,18 @@ static int ctx_reset(infllm_ctx* c, bool wait) {
   if (c->initialized) {
     INFLLM_CUDA_OK(cudaSetDevice(c->cfg.device));
     cudaStream_t side[5] = {c->copy_stream, c->urgent_stream, c->aux_stream, c->d2h_stream, c->mail_stream};
+    // (marks of an earlier reset that no append has followed still stand)
+    const bool attn = c->attn_recorded || (c->reset_pending && c->reset_attn), last = c->last_recorded || (c->reset_pending && c->reset_last);
+    if (c->failed) INFLLM_CUDA_OK(cudaDeviceSynchronize());  // what a call that gave up half-way left behind has no mark
     if (wait || !c->dev_slabs.empty()) {
       for (cudaStream_t s : side) INFLLM_CUDA_OK(cudaStreamSynchronize(s));
-      if (c->attn_recorded) INFLLM_CUDA_OK(cudaEventSynchronize(c->ev_attn));
-      if (c->last_recorded) INFLLM_CUDA_OK(cudaEventSynchronize(c->ev_last));
+      if (attn) INFLLM_CUDA_OK(cudaEventSynchronize(c->ev_attn));
+      if (last) INFLLM_CUDA_OK(cudaEventSynchronize(c->ev_last));
+      c->reset_attn = c->reset_last = false;
     } else {
       for (int i = 0; i < 5; ++i) INFLLM_CUDA_OK(cudaEventRecord(c->ev_side[i], side[i]));
-      // (marks of an earlier reset that no append has followed still stand)
-      c->reset_attn = c->attn_recorded || (c->reset_pending && c->reset_attn);
-      c->reset_last = c->last_recorded || (c->reset_pending && c->reset_last);
+      c->reset_attn = attn;
+      c->reset_last = last;
     }
     c->reset_pending = true;
   }

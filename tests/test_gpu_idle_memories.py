@@ -70,3 +70,42 @@ def test_idle_memories_are_bounded_by_their_shape_and_given_back():
     release_idle_memories()
     torch.cuda.synchronize()
     assert torch.cuda.mem_get_info()[0] > held
+
+
+@pytest.mark.parametrize("dropped", [True, False])
+def test_a_new_store_waits_for_the_old_memorys_last_token(dropped):
+    """The last token of a memory reads its units in place from the host store and is still queued when the memory is
+    dropped (or reset) and other units are loaded into the same slabs: its output is that of its own units."""
+    from infllm_b200.attention import ContextManager, RotaryEmbeddingESM, release_idle_memories
+
+    n_units, n_init, n_local = 40, 64, 256
+    g = torch.Generator().manual_seed(6)
+    rnd = lambda *s: torch.randn(s, generator=g).to(torch.bfloat16)  # noqa: E731
+    block_k = rnd(n_units, H * D)
+    small = [rnd(HKV, n, D) for n in (n_init, n_init, n_local, n_local)]
+    units = [rnd(n_units, 2, HKV, 128, D) for _ in range(2)]
+    q, k, v = _tokens(1, 7)
+    make = lambda: ContextManager(RotaryEmbeddingESM(D, 1e6, 1.0), n_init, n_local, 128, 8, 8, 256, None, True, 2)  # noqa: E731
+
+    def run(behind_work):
+        cm = make()
+        cm.load_synthetic(units[0], block_k, *small)
+        if behind_work:
+            torch.cuda._sleep(400_000_000)  # about 0.2 s
+        out = cm.append(q, k, v, q, k, v)
+        if not behind_work:
+            torch.cuda.synchronize()
+        if dropped:
+            del cm
+            cm = make()
+        else:
+            cm.reset()
+        cm.load_synthetic(units[1], block_k, *small)
+        torch.cuda.synchronize()
+        return out, cm.append(q, k, v, q, k, v)
+
+    torch.cuda.synchronize()
+    release_idle_memories()
+    want, got = run(False), run(True)
+    assert not torch.equal(want[0], want[1])
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
