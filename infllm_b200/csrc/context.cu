@@ -863,10 +863,11 @@ int score_topk(infllm_ctx* c, int64_t n, const float* qbar, float* scores, int32
 }
 
 // A word {value, seq} that a kernel writes to pinned memory, as soon as it is there - an event behind the kernel arrives 3 us
-// later.  Bounded: the kernels' own waits end after a second or two and leave the error record; the rest of the limit is
-// for work ahead of the kernel on its stream.
-int wait_word(infllm_ctx* c, const unsigned long long* p, uint32_t seq, uint32_t* value) {
-  const auto t0 = std::chrono::steady_clock::now();
+// later.  `behind`: an event behind that kernel; without one it is the last work of the caller's stream.  No limit of its own:
+// the kernels' waits are bounded and leave the error record, and a word that is not there when its kernel is through will not
+// come - whereas what is ahead of the kernel on the caller's stream may take as long as it likes.
+int wait_word(infllm_ctx* c, const unsigned long long* p, uint32_t seq, uint32_t* value, cudaEvent_t behind = nullptr) {
+  bool through = false;
   for (unsigned turn = 1;; ++turn) {
     const unsigned long long w = *(const volatile unsigned long long*)p;
     if ((uint32_t)(w >> 32) == seq) {
@@ -874,13 +875,14 @@ int wait_word(infllm_ctx* c, const unsigned long long* p, uint32_t seq, uint32_t
       return INFLLM_OK;
     }
     for (int spin = 0; spin < 32; ++spin) __builtin_ia32_pause();
-    if (turn % 64) continue;
+    if (turn % 64 && !through) continue;
     if (c->h_tc_err && *(volatile int32_t*)c->h_tc_err) INFLLM_TRY(check_device_error(c, c->last_stream));
+    if (through) return fail(INFLLM_E_TIMEOUT, "a result that a kernel sends to the host did not arrive");
     if (turn % 4096) continue;
-    const cudaError_t e = cudaStreamQuery(c->last_stream);
-    if (e != cudaSuccess && e != cudaErrorNotReady) INFLLM_CUDA_OK(e);
-    if (std::chrono::steady_clock::now() - t0 > std::chrono::seconds(60))
-      return fail(INFLLM_E_TIMEOUT, "a result that a kernel sends to the host did not arrive");
+    const cudaError_t e = behind ? cudaEventQuery(behind) : cudaStreamQuery(c->last_stream);
+    if (e == cudaErrorNotReady) cudaGetLastError();  // (not an error of ours)
+    else if (e != cudaSuccess) INFLLM_CUDA_OK(e);
+    through = e == cudaSuccess;  // one more look: it may have come just before
   }
 }
 
@@ -1384,13 +1386,29 @@ int flush_table(infllm_ctx* c, cudaStream_t s, TokenParams* tok = nullptr) {
 int wait_words(infllm_ctx* c, infllm_ctx::PendingToken& p) {
   for (int i = 0; i < c->cfg.topk; ++i) {
     uint32_t id = 0;
-    if (const int rc = wait_word(c, p.h_words + i, p.seq, &id)) {
-      c->tok_restart = true;
-      return rc;
-    }
+    INFLLM_TRY(wait_word(c, p.h_words + i, p.seq, &id, c->attn_recorded ? c->ev_attn : nullptr));
     p.h_ids[i] = (int32_t)id;
   }
   return INFLLM_OK;
+}
+
+// A one-launch token gave up and its ids will not come: nothing of its retrieval reaches the cache.  What it may have left in
+// the landing slots belongs to no unit, and the words start again, behind whatever of it is still running.
+void drop_oldest(infllm_ctx* c) {
+  if (c->attn_recorded) cudaEventSynchronize(c->ev_attn);
+  c->pend_head = (c->pend_head + 1) % infllm_ctx::kPendSlots;
+  c->pend_count -= 1;
+  c->table_valid = false;
+  c->tok_restart = true;
+}
+void drop_lost_tokens(infllm_ctx* c) {
+  if (c->pend_count <= 0 || !c->attn_recorded || cudaEventSynchronize(c->ev_attn) != cudaSuccess) return;
+  for (; c->pend_count > 0; drop_oldest(c)) {
+    const infllm_ctx::PendingToken& p = c->pend[c->pend_head];
+    int there = 0;
+    for (int i = 0; i < c->cfg.topk && p.seq != 0; ++i) there += (uint32_t)(*(volatile unsigned long long*)(p.h_words + i) >> 32) == p.seq;
+    if (p.seq == 0 || there == c->cfg.topk) return;
+  }
 }
 
 // Apply the oldest pending retrieval of a one-token append to the cache: wait for its ids (they left the device
@@ -1402,7 +1420,10 @@ int settle_one(infllm_ctx* c, cudaStream_t s) {
   {
     HostTimer ht(&c->host_us[0]);
     if (p.seq != 0) {
-      INFLLM_TRY(wait_words(c, p));
+      if (const int rc = wait_words(c, p)) {
+        drop_oldest(c);
+        return rc;
+      }
     } else {
       INFLLM_CUDA_OK(cudaEventSynchronize(p.ev));
     }
@@ -1790,6 +1811,7 @@ int token_begin(infllm_ctx* c, const char* q, int64_t q_hs, const char* k, int64
   P.win_score = tb.score + (wlo - tb.t0), P.score_hs = tb.cap;
   P.out = out, P.o_hs = o_hs;
   P.seq = c->tok_seq;
+  P.spin = (g.debug_flags & 128) && c->tok_seq % 16 == 0 ? 0 : kTokSpin;
   P.err = c->tc_err, P.err_host = c->h_tc_err;
   pt.serial = c->call_serial;
   pt.landing = c->landing_slots;
@@ -2516,8 +2538,12 @@ static int open_call(infllm_ctx* c, cudaStream_t s) {
   INFLLM_CUDA_OK(cudaSetDevice(c->cfg.device));
   if (!c->initialized) INFLLM_TRY(lazy_init(c, s));
   INFLLM_TRY(order_behind_reset(c, s));
-  INFLLM_TRY(poll_device_error(c, s));
-  if (c->h_tc_err && !c->err_pending && *(volatile int32_t*)c->h_tc_err) INFLLM_TRY(check_device_error(c, s));  // a one-launch token gave up
+  int rc = poll_device_error(c, s);
+  if (rc == INFLLM_OK && c->h_tc_err && !c->err_pending && *(volatile int32_t*)c->h_tc_err) rc = check_device_error(c, s);
+  if (rc != INFLLM_OK) {  // a one-launch token may have given up
+    drop_lost_tokens(c);
+    return rc;
+  }
   c->failed = true;  // until the call has gone through
   if (s != c->last_stream) c->copy_waited = 0;
   c->call_serial += 1;

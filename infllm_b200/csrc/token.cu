@@ -17,7 +17,7 @@
 // arrival: the reader polls the words it needs.  (With a ticket counter, the last CTA ranking, and counters that the CTAs
 // meet at, each exchange is a fence, an atomic, a poll and a load one after another.)  The CTAs wait for one another, hence
 // a cooperative launch (all of them are resident), and every wait is bounded: one that runs out leaves the error record
-// (device and pinned host copy) and the token's output is not written.
+// (device and pinned host copy), and the outputs that it was for are not written.
 //
 // Several contexts' tokens share a launch: the y index of a CTA is its context, whose runs are what its share of the SMs
 // gives.  More rounds per warp, but the latencies of the chain are paid once: four contexts of 28/4 heads take 27.9 us
@@ -41,7 +41,6 @@ constexpr int kTokMaxRuns = 160;
 constexpr int kTokMaxK = 64;
 constexpr int kTokMaxUnits = 16384;
 constexpr int kTokScan = 22;    // scores a ranking thread keeps in registers: 8448 of them in one round
-constexpr uint32_t kTokSpin = 1u << 22;
 
 __device__ __forceinline__ unsigned long long ld_word(const unsigned long long* p) {
   unsigned long long v;
@@ -79,7 +78,7 @@ __device__ __noinline__ void token_gave_up(int32_t* err, int32_t* err_host, int 
 // a word once it carries this token's number (v: what was read of it already); false: the bound ran out
 __device__ __forceinline__ bool poll_word(const unsigned long long* p, unsigned long long& v, const TokenParams& P, int where) {
   for (uint32_t i = 0; (uint32_t)(v >> 32) != P.seq; v = ld_word(p)) {
-    if (++i > kTokSpin) {
+    if (++i > P.spin) {
       token_gave_up(P.err, P.err_host, where);
       return false;
     }
@@ -362,7 +361,7 @@ __global__ void __launch_bounds__(kTokThreads, 1) token_kernel(const __grid_cons
         cur = u;
         unsigned long long w = ld_word_acquire(P.id_words + u);
         for (uint32_t i = 0; (uint32_t)(w >> 32) != P.seq; w = ld_word_acquire(P.id_words + u)) {
-          if (++i > kTokSpin) {
+          if (++i > P.spin) {
             ok = false;
             break;
           }
@@ -500,7 +499,7 @@ __global__ void __launch_bounds__(kTokThreads, 1) token_kernel(const __grid_cons
     num += __shfl_xor_sync(0xffffffffu, num, 1);
     num += __shfl_xor_sync(0xffffffffu, num, 2);
     num += __shfl_xor_sync(0xffffffffu, num, 4);
-    if (o < o_hi && sub == 0) ((T*)P.out)[(int64_t)(hkv * group + h) * P.o_hs + decode_dim(o & 127)] = Act<T>::from_f(num);
+    if (__all_sync(0xffffffffu, ok) && o < o_hi && sub == 0) ((T*)P.out)[(int64_t)(hkv * group + h) * P.o_hs + decode_dim(o & 127)] = Act<T>::from_f(num);
   }
 #pragma unroll 1
   for (int i0 = tid; i0 < n_add; i0 += 4 * kTokThreads) {

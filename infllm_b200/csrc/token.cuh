@@ -5,6 +5,7 @@
 namespace infllm {
 
 constexpr int kTokMaxUpdates = 96;  // changes of the table of unit addresses that travel with a token
+constexpr uint32_t kTokSpin = 1u << 22;  // polls after which a wait gives up: a second or two
 constexpr int kTokErrTimeout = 1;   // code of the error record: a bounded wait ran out (700 ids, 701 partials, 702 scores)
 
 struct TokenParams {
@@ -31,7 +32,8 @@ struct TokenParams {
   int32_t rest_begin[4];  // first 16-key group of each
   unsigned long long* ptrs;  // table of unit addresses; the landing slots of the k_top positions from landing_at on
   int64_t landing_at, unit_bytes;
-  int32_t unit_len, n_heads, n_kv, group, n_runs, pad;
+  int32_t unit_len, n_heads, n_kv, group, n_runs;
+  uint32_t spin;  // kTokSpin
   float scale_log2;
   unsigned long long* part_words;  // (n_runs, n_heads, 129): a run's normalised outputs and their log-sum-exp
   float* logits;                   // (n_heads, logit_hs)

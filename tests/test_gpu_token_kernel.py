@@ -73,3 +73,36 @@ def test_a_word_that_does_not_arrive_is_an_error():
     for _ in range(2):  # and the memory goes on
         one.append(q, k, v, q, k, v)
     torch.cuda.synchronize()
+
+
+def test_a_token_that_gives_up_is_one_error(monkeypatch):
+    """The waits inside the sixteenth token give up at once: one of the calls that follow reports it, promptly, and the
+    memory goes on as one that never lost a retrieval (the token itself was ingested)."""
+    import time
+
+    from infllm_b200 import _lib
+    from infllm_b200.attention import context_manager as cmod
+
+    want, _ = _memory(8, 2, 60, 300, 4, torch.bfloat16, False)
+    monkeypatch.setattr(cmod, "TEST_OVERRIDES", {"debug_flags": 128})
+    got, _ = _memory(8, 2, 60, 300, 4, torch.bfloat16, False)
+    g = torch.Generator(device="cuda").manual_seed(6)
+    errors = 0
+    for i in range(28):
+        q, k, v = (torch.randn((1, h, 1, D), generator=g, device="cuda").to(torch.bfloat16) for h in (8, 2, 2))
+        b = want.append(q, k, v, q, k, v)
+        t0 = time.perf_counter()
+        try:
+            a = got.append(q, k, v, q, k, v)
+        except _lib.InfLLMError:
+            errors += 1
+            a = got.append(q, k, v, q, k, v)
+        if i == 17:
+            assert errors == 1
+        torch.cuda.synchronize()
+        assert time.perf_counter() - t0 < 5
+        if i != 15:  # the one that gave up
+            assert torch.equal(a, b), i
+            if i % 4 == 0:
+                assert got.last_topk() == want.last_topk()
+    assert errors == 1 and got.info()["length"] == want.info()["length"]
