@@ -278,6 +278,7 @@ typedef struct infllm_config {
                            *     context_manager.py:57-71), not by the copy kernel
                            *  8: the two-heads-per-CTA tcgen05 attention kernel whatever the head count
                            * 16: one-token appends wait for the retrieved ids before launching the attention
+                           * 64: the 16th one-launch token asks for a grid that the device refuses
                            * 128: the waits inside every 16th one-launch token give up at once */
   int32_t look_depth;     /* exec blocks ranked and staged ahead of the running one; 0 = default (2), at most 8; the
                            * cache gets that many times topk spare slots */

@@ -1378,7 +1378,9 @@ int flush_table(infllm_ctx* c, cudaStream_t s, TokenParams* tok = nullptr) {
     std::copy(vals.begin(), vals.end(), tok->upd_val);
     return INFLLM_OK;
   }
-  return ptr_table_update_launch(c->d_unit_ptrs, ids.data(), vals.data(), (int)ids.size(), s);
+  const int rc = ptr_table_update_launch(c->d_unit_ptrs, ids.data(), vals.data(), (int)ids.size(), s);
+  if (rc != INFLLM_OK) c->table_valid = false;
+  return rc;
 }
 
 // The ids of a one-launch token, as its ranking threads write them: long before the token is through, so that the host
@@ -1765,8 +1767,6 @@ int token_begin(infllm_ctx* c, const char* q, int64_t q_hs, const char* k, int64
   // at most kMaxOutstanding tokens ahead of the cache: apply the older retrievals first
   while (c->pend_count >= infllm_ctx::kMaxOutstanding) INFLLM_TRY(settle_one(c, s));
   infllm_ctx::PendingToken& pt = c->pend[(c->pend_head + c->pend_count) % infllm_ctx::kPendSlots];
-  P.n_upd = 0;
-  INFLLM_TRY(flush_table(c, s, &P));
   if (!c->tok_ids) {
     c->tok_part_words = (size_t)token_one_launch(c, c->tok_sms) * g.n_heads * 129;
     INFLLM_CUDA_OK(dev_malloc((void**)&c->tok_ids, g.topk * wsz));
@@ -1789,6 +1789,8 @@ int token_begin(infllm_ctx* c, const char* q, int64_t q_hs, const char* k, int64
     c->tok_seq = 0;
     c->tok_restart = false;
   }
+  P.n_upd = 0;
+  INFLLM_TRY(flush_table(c, s, &P));  // the last thing that can fail: its changes travel with the launch (token_undo)
   pt.seq = ++c->tok_seq;
   if (c->tok_seq == UINT32_MAX) c->tok_restart = true;  // 0 marks "not a one-launch token"
   P.q = q, P.k = k, P.v = v, P.q_hs = q_hs, P.k_hs = k_hs, P.v_hs = v_hs;
@@ -1811,6 +1813,7 @@ int token_begin(infllm_ctx* c, const char* q, int64_t q_hs, const char* k, int64
   P.win_score = tb.score + (wlo - tb.t0), P.score_hs = tb.cap;
   P.out = out, P.o_hs = o_hs;
   P.seq = c->tok_seq;
+  P.too_large = (g.debug_flags & 64) && c->tok_seq == 16;
   P.spin = (g.debug_flags & 128) && c->tok_seq % 16 == 0 ? 0 : kTokSpin;
   P.err = c->tc_err, P.err_host = c->h_tc_err;
   pt.serial = c->call_serial;
@@ -1838,9 +1841,12 @@ int list_new_units(infllm_ctx* c, int64_t first_new, cudaStream_t s) {
   return INFLLM_OK;
 }
 
-int token_undo(infllm_ctx* c, int rc) {  // the launch failed: there will be no ids to wait for
+// The launch failed: there will be no ids to wait for, and the changes of the table of unit addresses have not arrived.
+// Where it was refused because the process may not use an SM for every CTA, tokens are separate kernels from here on.
+void token_undo(infllm_ctx* c, int rc) {
   c->pend_count -= 1;
-  return rc;
+  c->table_valid = false;
+  if (rc == INFLLM_E_UNSUPPORTED) c->tok_sms = 0;
 }
 
 int token_end(infllm_ctx* c, cudaStream_t s) {
@@ -2587,9 +2593,13 @@ extern "C" int infllm_ctx_append(infllm_ctx* c, const void* d_q, int64_t q_hs, i
     TokenParams P;
     INFLLM_TRY(token_begin(c, (const char*)d_q, q_hs, (const char*)d_k, k_hs, (const char*)d_v, v_hs, (char*)d_out, o_hs, P, s));
     P.n_runs = runs;
-    if (const int rc = token_launch(&P, 1, c->cfg.dtype, s)) return token_undo(c, rc);
-    INFLLM_TRY(token_end(c, s));
-    return close_call(c, 1, units_before, s);
+    const int rc = token_launch(&P, 1, c->cfg.dtype, s);
+    if (rc == INFLLM_OK) {
+      INFLLM_TRY(token_end(c, s));
+      return close_call(c, 1, units_before, s);
+    }
+    token_undo(c, rc);
+    if (rc != INFLLM_E_UNSUPPORTED) return rc;
   }
   for (int64_t off = 0; off < len; off += c->sub_max) {
     const int64_t n = std::min<int64_t>(c->sub_max, len - off);
@@ -2653,7 +2663,8 @@ extern "C" int infllm_ctx_append_units(infllm_ctx* const* ctx, int n, int per_se
     if (ready > 0) {
       if (const int lrc = token_launch(P, ready, c->cfg.dtype, s)) {
         for (int i = 0; i < ready; ++i) token_undo(ctx[u + i], lrc);
-        return lrc;
+        if (lrc != INFLLM_E_UNSUPPORTED) return lrc;
+        continue;  // the same contexts again, as separate kernels
       }
     }
     for (int i = 0; i < ready; ++i) {

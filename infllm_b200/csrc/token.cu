@@ -541,7 +541,7 @@ static size_t token_smem(int width, int n) {
 // (64 of 16384 units, as in block_score_topk_kernel), 8 query heads per KV head.
 int token_runs(int n_heads, int n_kv_heads, int head_dim, int64_t n_units, int topk, int block_size, int sms) {
   const int width = n_heads * head_dim;
-  if (head_dim != 128 || n_heads / n_kv_heads > kMaxGroup || width > 12288 || n_units > kTokMaxUnits || topk > kTokMaxK || block_size % 8)
+  if (sms <= n_kv_heads || head_dim != 128 || n_heads / n_kv_heads > kMaxGroup || width > 12288 || n_units > kTokMaxUnits || topk > kTokMaxK || block_size % 8)
     return 0;
   return std::min((sms - 1) / n_kv_heads, kTokMaxRuns);
 }
@@ -556,7 +556,12 @@ static int token_launch_batch(const TokenParams* P, int n, cudaLaunchConfig_t& c
   auto kern = token_kernel<T, NB>;
   // (the opt-in holds for the current device only: asked for at every launch)
   INFLLM_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes));
-  INFLLM_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, B));
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, B);
+  if (e == cudaErrorCooperativeLaunchTooLarge) {
+    cudaGetLastError();
+    return fail(INFLLM_E_UNSUPPORTED, "token: a grid of %u x %u CTAs that is not resident at once", cfg.gridDim.x, cfg.gridDim.y);
+  }
+  INFLLM_CUDA_OK(e);
   return INFLLM_OK;
 }
 
@@ -566,7 +571,7 @@ int token_launch(const TokenParams* P, int n, int dtype, cudaStream_t s) {
   for (int i = 0; i < n; ++i) {
     if (P[i].n_upd > kTokMaxUpdates || P[i].n_runs < 1 || P[i].n_runs > kTokMaxRuns) return fail(INFLLM_E_BADARG, "token: bad argument");
     smem = std::max(smem, token_smem(P[i].width, P[i].n));
-    ctas = std::max(ctas, P[i].n_runs * P[i].n_kv + 1);
+    ctas = std::max(ctas, P[i].n_runs * P[i].n_kv + 1 + (P[i].too_large ? 4096 : 0));
   }
   if (n < 1 || n > kTokMaxBatch) return fail(INFLLM_E_BADARG, "token: %d contexts", n);
   cudaLaunchConfig_t cfg = {};

@@ -42,6 +42,7 @@ struct TokenParams {
   int64_t score_hs;
   void* out;
   int64_t o_hs;
+  int32_t too_large;  // (for tests) a grid that no device can hold: the launch is refused
   uint32_t seq;  // number of this token among those that have used these words; never 0
   int32_t *err, *err_host;
   int32_t upd_id[kTokMaxUpdates];
@@ -54,7 +55,8 @@ constexpr int kTokMaxBatch = 8;  // contexts of one launch: their parameters are
 int token_runs(int n_heads, int n_kv_heads, int head_dim, int64_t n_units, int topk, int block_size, int sms);
 // how many contexts with that many KV heads share a launch on a device of `sms` SMs
 int token_batch_max(int n_kv_heads, int sms);
-// n contexts' tokens, each with the n_runs its share of the SMs gives it
+// n contexts' tokens, each with the n_runs its share of the SMs gives it; INFLLM_E_UNSUPPORTED: the CTAs cannot all be
+// resident where this process runs
 int token_launch(const TokenParams* P, int n, int dtype, cudaStream_t s);
 
 }  // namespace infllm

@@ -106,3 +106,30 @@ def test_a_token_that_gives_up_is_one_error(monkeypatch):
             if i % 4 == 0:
                 assert got.last_topk() == want.last_topk()
     assert errors == 1 and got.info()["length"] == want.info()["length"]
+
+
+@pytest.mark.parametrize("batch", [1, 3])
+def test_a_launch_that_is_refused_leaves_nothing_behind(monkeypatch, batch):
+    """The sixteenth token's grid is larger than the device: the runtime refuses it, that token and those behind it are
+    separate kernels, and what the refused launch should have told the table of unit addresses is not lost."""
+    from infllm_b200.attention import ContextManager, RotaryEmbeddingESM
+    from infllm_b200.attention import context_manager as cmod
+
+    H, HKV, topk, n = 8, 2, 6, 20 + 30 * UNIT + 256
+    make = lambda: ContextManager(RotaryEmbeddingESM(D, 1e6, 1.0), 20, 256, UNIT, topk, topk, 128, None, True, 2)  # noqa: E731
+    g = torch.Generator(device="cuda").manual_seed(7)
+    rnd = lambda n: [torch.randn((batch, h, n, D), generator=g, device="cuda").to(torch.bfloat16) for h in (H, HKV, HKV)]  # noqa: E731
+    q, k, v = rnd(n)
+    want = make()
+    want.append(q, k, v, q, k, v)
+    monkeypatch.setattr(cmod, "TEST_OVERRIDES", {"debug_flags": 64})
+    got = make()
+    got.append(q, k, v, q, k, v)
+    for i in range(40):
+        q, k, v = rnd(1)
+        a, b = got.append(q, k, v, q, k, v), want.append(q, k, v, q, k, v)
+        assert (a.float() - b.float()).abs().max() <= 1e-2 * b.float().abs().max(), i
+        if i in (15, 16, 39):
+            for u in range(batch):
+                assert got.last_topk(u) == want.last_topk(u)
+    assert got.cached_blocks == want.cached_blocks
