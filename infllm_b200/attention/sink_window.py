@@ -80,15 +80,11 @@ def _run_native(rope, q, k, v, heads, kv, past, n_local, n_init, stream_position
     ref = ctypes.byref(a)
     lib = _lib.lib
     n = lib.infllm_sink_window_scratch(ref)
-    n_out = batch * len_q * heads * dim
-    if len_q == 1:  # one allocation: the scratch of a token is of the output's order
-        both = torch.empty(n_out + (n >> 1), dtype=dtype, device=device)
-        out, o_at = both[:n_out].view(batch, 1, heads * dim), both.data_ptr()
-        a.d_scratch = o_at + 2 * n_out
-    else:
-        out = torch.empty((batch, len_q, heads * dim), dtype=dtype, device=device)
-        scratch = torch.empty(max(n, 16), dtype=torch.uint8, device=device)
-        o_at, a.d_scratch = out.data_ptr(), scratch.data_ptr()
+    # (allocations of their own: the output, or a view of it, may outlive the call by far, and the scratch is a thousand times
+    # a token's output)
+    out = torch.empty((batch, len_q, heads * dim), dtype=dtype, device=device)
+    scratch = torch.empty(max(n, 16), dtype=torch.uint8, device=device)
+    o_at, a.d_scratch = out.data_ptr(), scratch.data_ptr()
     a.scratch_bytes = n
     a.d_out = o_at
     stream = _lib.raw_stream(device)

@@ -41,3 +41,18 @@ def test_call_equals_the_composition(kind, h, hkv, batch, n_local, n_init, lens)
     o = forward(None, x, x, ropes[0], False, past[0], *proj, d, h, hkv)
     w = forward(None, x, x, ropes[1], False, past[1], *proj, d, h, hkv)
     assert (o.float() - w.float()).abs().max() <= 2e-2 * w.float().abs().max()
+
+
+@pytest.mark.parametrize("n", [1, 2, 70])
+def test_an_output_holds_no_more_memory_than_itself(n):
+    """attention_out may hand its input on, and a program may keep every token's output."""
+    from infllm_b200.attention import ATTN_FORWRAD, RotaryEmbeddingESM
+
+    h, hkv, d = 8, 2, 128
+    forward = ATTN_FORWRAD["infinite-lm"](n_local=256, n_init=64, fattn=True)
+    proj = (lambda x: x[..., :h * d], lambda x: x[..., h * d:(h + hkv) * d], lambda x: x[..., (h + hkv) * d:], lambda o: o)
+    past = None
+    for length in (700, n):
+        x = torch.randn((1, length, (h + 2 * hkv) * d), device="cuda").to(torch.bfloat16)
+        o, past = forward(None, x, x, RotaryEmbeddingESM(d, 1e6, 1.0), True, past, *proj, d, h, hkv)
+    assert o.untyped_storage().nbytes() == n * h * d * 2
