@@ -290,7 +290,11 @@ typedef struct infllm_config {
                            * > 0: up to this many MiB of the store's first units are ALSO kept in device memory taken
                            * from the pool of infllm_device_store_reserve, and a refill of such a unit is a
                            * device-to-device copy.  The cache, its LRU order and the host store are unchanged. */
-  int32_t reserved[2];    /* zero */
+  int32_t keep_evicted_mb; /* device memory in which evicted units stay readable until the room is needed, past the slots
+                           * of max_cached_block and of the look-ahead.  0 (default): as many units as 8 * max_cached_block,
+                           * at most 1/1024 of the device's memory per context, 1/32 of it over all contexts and 1/128 of
+                           * what is free; > 0: this many MiB; < 0: none */
+  int32_t reserved;       /* zero */
 } infllm_config;
 
 /* Device copy of the store: one pool per device, shared by every context of the process whose configuration asks
@@ -304,9 +308,8 @@ int infllm_device_store_reserve(int device, int64_t bytes);
 int infllm_device_store_release(int device);
 int infllm_device_store_info(int device, int64_t* total_bytes, int64_t* used_bytes);
 
-/* Device memory of the cache: max_cached_block + look_depth * topk slots of one unit, and on top up to 256 MiB (no more
- * than 1/128 of the free memory when the context is initialised) in which evicted units stay readable until their slots
- * are needed.  The cache, its LRU order and the counters of hits, misses and evictions are those of max_cached_block.
+/* Device memory of the cache: max_cached_block + look_depth * topk slots of one unit, and on top what keep_evicted_mb
+ * says, in which evicted units stay readable until their slots are needed.  The cache, its LRU order and the counters of hits, misses and evictions are those of max_cached_block.
  * Validates the configuration (exc_block_size <= n_local, context_manager.py:219;
  * max_cached_block >= topk, context_manager.py:19 -> INFLLM_E_CAPACITY) and allocates nothing
  * large: buffers are created on the first append (context_manager.py:292-363). */

@@ -39,7 +39,7 @@ class Config(ctypes.Structure):
         ("score_decay", c_double), ("rope_base", c_float), ("rope_scale", c_float),
         ("device", c_int32), ("shard_rank", c_int32), ("shard_world", c_int32),
         ("debug_flags", c_int32), ("look_depth", c_int32), ("chunk_topk_calc", c_int32), ("device_store_mb", c_int32),
-        ("reserved", c_int32 * 2),
+        ("keep_evicted_mb", c_int32), ("reserved", c_int32),
     ]
 
 

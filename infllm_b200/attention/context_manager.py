@@ -58,14 +58,19 @@ class ContextManager:
 
     `device_store_mb` (not in the reference; default 0) keeps up to that many MiB of this memory's sealed units in
     device memory as well, taken from the pool of device_store_reserve(): refills of those units are
-    device-to-device copies.  With 0 every refill comes from the pinned host store, as in the reference."""
+    device-to-device copies.  With 0 every refill comes from the pinned host store, as in the reference.
+
+    `keep_evicted_mb` (not in the reference): device memory in which evicted units stay readable until the room is
+    needed.  0 (default): up to 8 * max_cached_block units within 1/1024 of the device's memory per memory and 1/32 over
+    all of them; negative: none.  What is cached, evicted and retrieved does not depend on it."""
 
     def __init__(self, position_embedding, n_init, n_local, block_size, max_cached_block, topk, exc_block_size,
                  score_decay: Optional[float] = None, fattn: bool = False, repr_topk: int = 1,
                  cache_strategy="lru", chunk_topk_calc: Optional[int] = None, async_global_stream: bool = False,
                  pin_memory: bool = False, faiss: bool = False, perhead: bool = False, head_group_comm=None,
-                 device_store_mb: int = 0):
+                 device_store_mb: int = 0, keep_evicted_mb: int = 0):
         self.length = 0
+        self.keep_evicted_mb = int(keep_evicted_mb)
         self.device_store_mb = int(device_store_mb)
         self.head_group_comm = head_group_comm  # HeadGroupComm: the heads given to append() are this rank's slice
         self.position_embedding = position_embedding
@@ -118,6 +123,7 @@ class ContextManager:
         if self.chunk_topk_calc is not None:
             cfg.chunk_topk_calc = int(self.chunk_topk_calc)  # context_manager.py:749-770
         cfg.device_store_mb = int(self.device_store_mb)
+        cfg.keep_evicted_mb = int(self.keep_evicted_mb)
         for name, value in TEST_OVERRIDES.items():  # empty outside the test-suite
             setattr(cfg, name, int(value))
         for _ in range(self.num_units):

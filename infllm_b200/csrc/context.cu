@@ -257,6 +257,7 @@ struct infllm_ctx {
   void* cache = nullptr;  // (max_cached, 2, H_kv, bs, D)
   SlotPool free_slots;
   int64_t n_slots = 0;
+  int64_t kept_bytes = 0;  // of the device's budget for evicted units (reserve_kept_slots)
   std::vector<cudaEvent_t> slot_ev;   // per slot: behind the last look-ahead copy into it
   std::vector<char> slot_ev_used;
   std::unordered_map<int32_t, int> slot_of;
@@ -494,6 +495,42 @@ cudaError_t dev_malloc_async(void** p, size_t n, cudaStream_t s) {
   return e;
 }
 
+// How many slots of a context may hold evicted units.  Memory that the configuration does not name, so there is a rule for
+// it: no more than kKeepFactor times the cache that was asked for, no more than 1/32 of a budget that all live contexts of
+// the device share, 1/32 of its memory (a model of 32 layers then has a share for each: 179 MiB on a device of 179 GiB), and
+// no more than 1/128 of what is free.  keep_evicted_mb says otherwise: that many MiB, or, negative, none.  What it is worth
+// ends where a working set does not fit.  Tokens of 32/8 heads over 4096 units of 512 KiB that walk round a set of units, topk
+// 16 at a time, max_cached_block 32: sets of 128 (half of what is kept) and of 256 units 24.6 us a token and nothing over
+// PCIe, of 320 and of 1024 (three times) 203 us and 8 MiB; with none kept 203 us and 8 MiB from 64 units on.
+constexpr int64_t kKeepFactor = 8, kKeepShare = 32;
+struct KeptBytes {
+  std::mutex mu;
+  int64_t bytes = 0;
+};
+KeptBytes g_kept[64];
+void count_kept(const infllm_ctx* c, int64_t bytes) {
+  if (c->cfg.device < 0 || c->cfg.device >= 64) return;
+  std::lock_guard<std::mutex> lk(g_kept[c->cfg.device].mu);
+  g_kept[c->cfg.device].bytes += bytes;
+}
+int64_t reserve_kept_slots(infllm_ctx* c) {
+  const infllm_config& g = c->cfg;
+  size_t free_b = 0, total_b = 0;
+  count_kept(c, -c->kept_bytes);  // (an initialisation that failed and is tried again)
+  c->kept_bytes = 0;
+  if (g.keep_evicted_mb < 0 || g.device < 0 || g.device >= 64 || cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return 0;
+  int64_t extra = ((int64_t)g.keep_evicted_mb << 20) / c->unit_bytes;
+  std::lock_guard<std::mutex> lk(g_kept[g.device].mu);
+  if (g.keep_evicted_mb == 0) {
+    const int64_t budget = (int64_t)total_b / 32, share = std::min<int64_t>(budget / kKeepShare, budget - g_kept[g.device].bytes);
+    extra = std::min<int64_t>(kKeepFactor * g.max_cached_block, std::min<int64_t>(share, (int64_t)free_b / 128) / c->unit_bytes);
+    if (extra <= 0) return 0;
+    c->kept_bytes = extra * c->unit_bytes;
+    g_kept[g.device].bytes += c->kept_bytes;
+  }
+  return extra;
+}
+
 int lazy_init(infllm_ctx* c, cudaStream_t s) {
   const infllm_config& g = c->cfg;
   // keep freed device memory in the pool: the token buffers are re-created at every compaction
@@ -605,19 +642,20 @@ int lazy_init(infllm_ctx* c, cudaStream_t s) {
   INFLLM_CUDA_OK(dev_malloc((void**)&c->part_o, (int64_t)c->max_parts * H * D * sizeof(float)));
   INFLLM_CUDA_OK(dev_malloc((void**)&c->part_lse, (int64_t)c->max_parts * H * sizeof(float)));
   INFLLM_CUDA_OK(dev_malloc((void**)&c->dec_logits, H * ((int64_t)g.n_local + 1) * sizeof(float)));
-  // max_cached_block slots hold the cache proper; topk more per look-ahead step hold the copies staged ahead.  Past those,
-  // up to kKeepBytes (and no more than 1/128 of the free memory) let evicted units stay until their slots are needed: the
-  // cache and its LRU order are those of max_cached_block, but a unit that is retrieved again after its eviction does not
-  // cross PCIe again.  64K tokens of a 32-KV-head layer whose retrievals rotate through 128 units of 2 MiB:
-  // 102 -> 39 ms; a token over 1M tokens whose topic changes every 16 tokens: 88 -> 35 us.
+  // max_cached_block slots hold the cache proper; topk more per look-ahead step hold the copies staged ahead.  In those past
+  // them evicted units stay until the slots are needed: the cache and its LRU order are those of max_cached_block, but a unit
+  // that is retrieved again soon after its eviction does not cross PCIe again.
   int64_t n_slots = (int64_t)g.max_cached_block + (int64_t)c->look_depth * g.topk;
-  {
-    constexpr int64_t kKeepBytes = 256ll << 20;
-    size_t free_b = 0, total_b = 0;
-    INFLLM_CUDA_OK(cudaMemGetInfo(&free_b, &total_b));
-    const int64_t extra = std::min<int64_t>(kKeepBytes, (int64_t)(free_b / 128)) / c->unit_bytes;
-    if (extra > 0 && cudaMalloc(&c->cache, (n_slots + extra) * c->unit_bytes) == cudaSuccess) n_slots += extra;
-    else cudaGetLastError();
+  const int64_t extra = reserve_kept_slots(c);
+  if (extra > 0) {
+    if (cudaMalloc(&c->cache, (n_slots + extra) * c->unit_bytes) == cudaSuccess) {
+      n_slots += extra;
+    } else {
+      cudaGetLastError();
+      c->cache = nullptr;
+      count_kept(c, -c->kept_bytes);
+      c->kept_bytes = 0;
+    }
   }
   if (!c->cache) INFLLM_CUDA_OK(dev_malloc((void**)&c->cache, n_slots * c->unit_bytes));
   c->n_slots = n_slots;
@@ -2312,7 +2350,9 @@ extern "C" int infllm_ctx_reset(infllm_ctx* c) {
   return ctx_reset(c, false);
 }
 
-static void ctx_free(infllm_ctx* c) {
+// (an idle context's share of the budget is counted as its memory is: with the idle ones)
+static void ctx_free(infllm_ctx* c, bool idle) {
+  if (!idle) count_kept(c, -c->kept_bytes);
   if (c->initialized) {
     cudaSetDevice(c->cfg.device);
     cudaDeviceSynchronize();
@@ -2441,7 +2481,7 @@ static int idle_trim(int64_t dev, int64_t host, int64_t dev_limit, bool all) {
   }
   int cur = -1;
   if (!gone.empty()) cudaGetDevice(&cur);
-  for (infllm_ctx* c : gone) ctx_free(c);
+  for (infllm_ctx* c : gone) ctx_free(c, true);
   if (cur >= 0) cudaSetDevice(cur);
   return (int)gone.size();
 }
@@ -2476,6 +2516,7 @@ extern "C" int infllm_ctx_destroy(infllm_ctx* c) {
       c->marks.clear();
       for (int i = 0; i < INFLLM_PROF_SLOTS; ++i) c->prof_ms[i] = c->prof_work[i] = 0, c->prof_launches[i] = 0;
       for (double& us : c->host_us) us = 0;
+      count_kept(c, -c->kept_bytes);
       idle_trim(dev, host, limit, false);
       std::lock_guard<std::mutex> lk(p.mu);
       p.list.push_back({c, dev, host});
@@ -2484,7 +2525,7 @@ extern "C" int infllm_ctx_destroy(infllm_ctx* c) {
     }
     cudaSetDevice(cur);
   }
-  if (!keep) ctx_free(c);
+  if (!keep) ctx_free(c, false);
   return INFLLM_OK;
 }
 
@@ -2522,6 +2563,7 @@ extern "C" int infllm_ctx_create(const infllm_config* cfg, infllm_ctx** out) {
         *out = it->c;
         p.dev_bytes -= it->dev_bytes;
         p.host_bytes -= it->host_bytes;
+        count_kept(*out, (*out)->kept_bytes);
         p.list.erase(std::next(it).base());
         return INFLLM_OK;
       }

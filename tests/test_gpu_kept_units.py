@@ -14,7 +14,7 @@ H, D, UNIT, N_INIT, N_LOCAL, TOPK = 16, 128, 128, 64, 256, 16
 def test_retrievals_that_outgrow_the_slots():
     from infllm_b200.attention import ContextManager, RotaryEmbeddingESM
 
-    n_units = 640  # units of 1 MiB: 256 of them fit past the cache's own slots
+    n_units = 640  # units of 1 MiB: 128 of them, eight times the cache, fit past its own slots
     g = torch.Generator(device="cuda").manual_seed(1)
     rnd = lambda *s: torch.randn(s, generator=g, device="cuda").to(torch.bfloat16)  # noqa: E731
     units, block_k = rnd(n_units, 2, H, UNIT, D), rnd(n_units, H * D)
