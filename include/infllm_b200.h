@@ -315,9 +315,9 @@ int infllm_device_store_info(int device, int64_t* total_bytes, int64_t* used_byt
  * large: buffers are created on the first append (context_manager.py:292-363). */
 int infllm_ctx_create(const infllm_config* cfg, infllm_ctx** out);
 /* infllm_ctx_destroy forgets the tokens and keeps the context's workspaces (device buffers, pinned host slabs, streams)
- * for the next infllm_ctx_create with an equal configuration: at most 256 contexts, 16 GiB of pinned memory and
- * 16 GiB of device memory (no more than a quarter of what is free), the oldest are freed first.
- * infllm_ctx_release_idle frees all of them. */
+ * for the next infllm_ctx_create with an equal configuration: at most 256 contexts, 16 GiB of pinned memory and, per
+ * device, 1/8 of its memory (no more than a quarter of what would be free without them); the oldest are freed first.
+ * Allocations of the library that fail free them; for the program's own there is infllm_ctx_release_idle. */
 int infllm_ctx_destroy(infllm_ctx* ctx);
 int infllm_ctx_release_idle(void);
 /* Forget every token but keep the allocations (device buffers, pinned host store). */

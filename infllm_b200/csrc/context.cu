@@ -417,7 +417,7 @@ struct infllm_ctx {
   const char* unit_src(int64_t b) { return dev_resident(b) ? dev_unit(b) : host_unit(b); }
 };
 
-static int idle_trim(int64_t dev, int64_t host, int64_t dev_limit, bool all);
+static int idle_release();
 
 namespace {
 
@@ -480,7 +480,7 @@ int free_buffers(TokenBuffers& tb, cudaStream_t s) {
 // Device memory that idle contexts hold is given up before an allocation fails.
 cudaError_t dev_malloc(void** p, size_t n) {
   cudaError_t e = cudaMalloc(p, n);
-  if (e == cudaErrorMemoryAllocation && idle_trim(0, 0, 0, true) > 0) {
+  if (e == cudaErrorMemoryAllocation && idle_release() > 0) {
     cudaGetLastError();
     e = cudaMalloc(p, n);
   }
@@ -488,7 +488,7 @@ cudaError_t dev_malloc(void** p, size_t n) {
 }
 cudaError_t dev_malloc_async(void** p, size_t n, cudaStream_t s) {
   cudaError_t e = cudaMallocAsync(p, n, s);
-  if (e == cudaErrorMemoryAllocation && idle_trim(0, 0, 0, true) > 0) {
+  if (e == cudaErrorMemoryAllocation && idle_release() > 0) {
     cudaGetLastError();
     e = cudaMallocAsync(p, n, s);
   }
@@ -863,7 +863,7 @@ int ensure_host_units(infllm_ctx* c, int64_t n) {
       c->slab_pending = false;
     }
     if (!h.p) h = alloc_slab(c->cfg.device, bytes);
-    if (!h.p && idle_trim(0, 0, 0, true) > 0) h = alloc_slab(c->cfg.device, bytes);
+    if (!h.p && idle_release() > 0) h = alloc_slab(c->cfg.device, bytes);
     if (!h.p) return fail(INFLLM_E_NOMEM, "pinned host store: no %lld bytes of page-locked memory", (long long)bytes);
     c->slabs.push_back(h);
   }
@@ -2431,13 +2431,15 @@ static void ctx_free(infllm_ctx* c, bool idle) {
 // layer) would pay for its workspaces again: some twenty device allocations and as many frees, five streams, and a
 // slab of page-locked host memory, which alone costs 50 ms and more.  A destroyed context therefore becomes idle, its
 // tokens forgotten, and infllm_ctx_create hands it out again for an equal configuration.  Measured: an 8192-token prompt
-// into a new memory 140 -> 4.8 ms, a 32768-token prompt 217 -> 13 ms.  The bounds: at most kIdleContexts contexts, kIdleBytes of device memory (and no more than a
-// quarter of what is free on the device) and kIdleBytes of pinned host memory; past them the oldest are freed.
-// infllm_ctx_release_idle frees all of them, and an allocation of the library that fails does so before it tries
-// again.  The list is behind a mutex; the streams' order is kept by the marks of ctx_reset, whichever stream the next
-// owner appends on.
+// into a new memory 140 -> 4.8 ms, a 32768-token prompt 217 -> 13 ms; 32 memories of
+// 32/8 heads, 8192 tokens each, dropped at once and started again: 45 ms a round, 180 to 390 ms where nine of them did not fit.
+// The bounds: at most kIdleContexts contexts; per device 1/8 of its memory, and no more than a quarter of what would be free
+// without them; kIdleHostBytes of pinned host memory.  Past them the oldest are freed.  infllm_ctx_release_idle frees all of
+// them, and an allocation of the library that fails does so before it tries again (other allocators do not know of them).
+// The list is behind a mutex; the streams' order is kept by the marks of ctx_reset, whichever stream the next owner appends on.
 constexpr size_t kIdleContexts = 256;
-constexpr int64_t kIdleBytes = 16ll << 30;
+constexpr int64_t kIdleHostBytes = 16ll << 30;
+constexpr int kIdleDevices = 64;
 
 struct IdleContext {
   infllm_ctx* c;
@@ -2446,7 +2448,7 @@ struct IdleContext {
 struct IdlePool {
   std::mutex mu;
   std::list<IdleContext> list;  // oldest first
-  int64_t dev_bytes = 0, host_bytes = 0;
+  int64_t dev_bytes[kIdleDevices] = {}, host_bytes = 0;
 };
 static IdlePool& idle_pool() {
   static IdlePool* p = new IdlePool();  // never destroyed: the CUDA runtime may be gone when static objects are
@@ -2465,48 +2467,77 @@ static int64_t ctx_device_bytes(const infllm_ctx* c) {
   return n;
 }
 
-// frees the oldest idle contexts until the pool's bounds hold with `dev` and `host` bytes more (all: every context)
-static int idle_trim(int64_t dev, int64_t host, int64_t dev_limit, bool all) {
-  std::vector<infllm_ctx*> gone;
-  {
-    IdlePool& p = idle_pool();
-    std::lock_guard<std::mutex> lk(p.mu);
-    while (!p.list.empty() && (all || p.list.size() >= kIdleContexts || p.dev_bytes + dev > dev_limit ||
-                               p.host_bytes + host > kIdleBytes)) {
-      p.dev_bytes -= p.list.front().dev_bytes;
-      p.host_bytes -= p.list.front().host_bytes;
-      gone.push_back(p.list.front().c);
-      p.list.pop_front();
-    }
-  }
+// takes an idle context out of the list (under the lock)
+static std::list<IdleContext>::iterator idle_take(IdlePool& p, std::list<IdleContext>::iterator it) {
+  p.dev_bytes[it->c->cfg.device] -= it->dev_bytes;
+  p.host_bytes -= it->host_bytes;
+  return p.list.erase(it);
+}
+
+static void idle_free(const std::vector<infllm_ctx*>& gone) {
   int cur = -1;
   if (!gone.empty()) cudaGetDevice(&cur);
   for (infllm_ctx* c : gone) ctx_free(c, true);
   if (cur >= 0) cudaSetDevice(cur);
+}
+
+// Adds a context, and frees the oldest ones until the bounds hold; dev_limit is its device's.
+static void idle_add(infllm_ctx* c, int64_t dev, int64_t host, int64_t dev_limit) {
+  std::vector<infllm_ctx*> gone;
+  {
+    IdlePool& p = idle_pool();
+    std::lock_guard<std::mutex> lk(p.mu);
+    const int d = c->cfg.device;
+    for (auto it = p.list.begin(); it != p.list.end();) {
+      const bool over = p.list.size() >= kIdleContexts || p.host_bytes + host > kIdleHostBytes;
+      if (over || (it->c->cfg.device == d && p.dev_bytes[d] + dev > dev_limit)) {
+        gone.push_back(it->c);
+        it = idle_take(p, it);
+      } else {
+        ++it;
+      }
+    }
+    p.list.push_back({c, dev, host});
+    p.dev_bytes[d] += dev;
+    p.host_bytes += host;
+  }
+  idle_free(gone);
+}
+
+// Frees every idle context; how many there were.
+static int idle_release() {
+  std::vector<infllm_ctx*> gone;
+  {
+    IdlePool& p = idle_pool();
+    std::lock_guard<std::mutex> lk(p.mu);
+    for (auto it = p.list.begin(); it != p.list.end(); it = idle_take(p, it)) gone.push_back(it->c);
+  }
+  idle_free(gone);
   return (int)gone.size();
 }
 
 extern "C" int infllm_ctx_release_idle(void) {
-  idle_trim(0, 0, kIdleBytes, true);
+  idle_release();
   return INFLLM_OK;
 }
 
 extern "C" int infllm_ctx_destroy(infllm_ctx* c) {
   if (!c) return INFLLM_OK;
-  bool keep = c->initialized && !c->failed;
+  const int d = c->cfg.device;
+  bool keep = c->initialized && !c->failed && d >= 0 && d < kIdleDevices;
   if (keep) {
     int cur = 0;
     cudaGetDevice(&cur);
     const int64_t dev = ctx_device_bytes(c), host = (int64_t)c->slabs.size() * c->slab_units * c->unit_bytes;
     size_t free_b = 0, total_b = 0;
-    keep = cudaSetDevice(c->cfg.device) == cudaSuccess && cudaMemGetInfo(&free_b, &total_b) == cudaSuccess;
-    IdlePool& p = idle_pool();
+    keep = cudaSetDevice(d) == cudaSuccess && cudaMemGetInfo(&free_b, &total_b) == cudaSuccess;
     int64_t limit = 0;
     if (keep) {
+      IdlePool& p = idle_pool();
       std::lock_guard<std::mutex> lk(p.mu);
-      limit = std::min<int64_t>(kIdleBytes, ((int64_t)free_b + p.dev_bytes + dev) / 4);
+      limit = std::min<int64_t>((int64_t)total_b / 8, ((int64_t)free_b + p.dev_bytes[d] + dev) / 4);
     }
-    keep = keep && dev <= limit && host <= kIdleBytes && ctx_reset(c, false) == INFLLM_OK;
+    keep = keep && dev <= limit && host <= kIdleHostBytes && ctx_reset(c, false) == INFLLM_OK;
     if (keep) {
       c->comm = nullptr;
       c->prof = c->trace_on = false;
@@ -2517,11 +2548,7 @@ extern "C" int infllm_ctx_destroy(infllm_ctx* c) {
       for (int i = 0; i < INFLLM_PROF_SLOTS; ++i) c->prof_ms[i] = c->prof_work[i] = 0, c->prof_launches[i] = 0;
       for (double& us : c->host_us) us = 0;
       count_kept(c, -c->kept_bytes);
-      idle_trim(dev, host, limit, false);
-      std::lock_guard<std::mutex> lk(p.mu);
-      p.list.push_back({c, dev, host});
-      p.dev_bytes += dev;
-      p.host_bytes += host;
+      idle_add(c, dev, host, limit);
     }
     cudaSetDevice(cur);
   }
@@ -2561,10 +2588,8 @@ extern "C" int infllm_ctx_create(const infllm_config* cfg, infllm_ctx** out) {
     for (auto it = p.list.rbegin(); it != p.list.rend(); ++it)
       if (memcmp(&it->c->cfg, &use, sizeof(use)) == 0) {  // the one that became idle last: its memory is warm
         *out = it->c;
-        p.dev_bytes -= it->dev_bytes;
-        p.host_bytes -= it->host_bytes;
         count_kept(*out, (*out)->kept_bytes);
-        p.list.erase(std::next(it).base());
+        idle_take(p, std::next(it).base());
         return INFLLM_OK;
       }
   }

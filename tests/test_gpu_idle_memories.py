@@ -109,3 +109,34 @@ def test_a_new_store_waits_for_the_old_memorys_last_token(dropped):
     want, got = run(False), run(True)
     assert not torch.equal(want[0], want[1])
     assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+
+
+def test_a_whole_models_memories_are_dropped_and_taken_up_again():
+    """32 layers of 32/8 heads, exec blocks of 512, window 4096, dropped at once and started again twice: every one of them
+    stays, and the next prompt allocates nothing."""
+    from infllm_b200.attention import ContextManager, RotaryEmbeddingESM, release_idle_memories
+
+    h, hkv, n = 32, 8, 5000
+    g = torch.Generator(device="cuda").manual_seed(8)
+    q, k, v = (torch.randn((1, x, n, D), generator=g, device="cuda").to(torch.bfloat16) for x in (h, hkv, hkv))
+    rope = RotaryEmbeddingESM(D, 1e6, 1.0)
+
+    def model():
+        layers = [ContextManager(rope, 128, 4096, 128, 32, 16, 512, None, True, 4) for _ in range(32)]
+        outs = [m.append(q, k, v, q, k, v)[0, 0, -1, 0].item() for m in layers]
+        torch.cuda.synchronize()
+        return layers, outs, torch.cuda.mem_get_info()[0]
+
+    torch.cuda.synchronize()
+    release_idle_memories()
+    layers, want, live = model()
+    for _ in range(2):
+        del layers
+        torch.cuda.synchronize()
+        assert torch.cuda.mem_get_info()[0] <= live + (256 << 20)  # (one of them is 600 MiB)
+        layers, outs, now = model()
+        assert outs == want and now >= live - (64 << 20)
+    del layers
+    release_idle_memories()
+    torch.cuda.synchronize()
+    assert torch.cuda.mem_get_info()[0] > live + 32 * (400 << 20)
