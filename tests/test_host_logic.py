@@ -226,3 +226,20 @@ def test_shard_refill_argument_checks_and_foreign_ids_need_no_device():
         assert L.lib.infllm_shard_refill(ctypes.byref(cs), ids, 4, None) == L.E_BADARG
     finally:
         L.lib.infllm_lru_destroy(lru)
+
+
+@pytest.mark.parametrize("heads", [1, 7, 8, 32, 64, 74, 75, 148, 149])
+@pytest.mark.parametrize("lq", [2, 128, 129, 512])
+def test_attention_runs_fill_one_wave_and_hold_a_tile_each(heads, lq):
+    """The runs of key tiles that a stage is cut into (told by its scratch: 130 floats per run and row)."""
+    items = -(-lq // 128) * heads
+    for tiles in (1, 2, 3, 7, 8, 15, 36, 60, 500):
+        if lq <= 128 and tiles == 1:
+            continue  # the shape-generic kernel's
+        floats = _lib().lib.infllm_attn_stage_scratch(heads, 1, lq, tiles * 128 - 5, 128)
+        runs, rest = divmod(floats, 130 * heads * lq)
+        assert rest == 0
+        runs = max(runs, 1)
+        assert runs == 1 or runs * items <= 148 and runs <= min(tiles, 32)
+        if tiles >= 36 and items <= 64:
+            assert runs > 1
