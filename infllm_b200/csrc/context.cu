@@ -819,13 +819,21 @@ HostSlab alloc_slab(int device, size_t bytes) {
     char* p = (char*)(((uintptr_t)map + kHuge - 1) / kHuge * kHuge);
     madvise(p, room, MADV_HUGEPAGE);  // (advice: ordinary pages do too)
     madvise(p, room, MADV_DONTFORK);  // as for memory of cudaHostAlloc
-    std::vector<std::future<void>> touch;
-    for (size_t i = 0; i < kTouchThreads; ++i)
-      touch.push_back(std::async(std::launch::async, [=] {
-        const size_t per = (room / kHuge + kTouchThreads - 1) / kTouchThreads * kHuge;
-        for (size_t o = i * per; o < std::min(room, (i + 1) * per); o += 4096) *(volatile char*)(p + o) = 0;
-      }));
-    for (auto& t : touch) t.get();
+    auto touch = [=](size_t i) {
+      const size_t per = (room / kHuge + kTouchThreads - 1) / kTouchThreads * kHuge;
+      for (size_t o = i * per; o < std::min(room, (i + 1) * per); o += 4096) *(volatile char*)(p + o) = 0;
+    };
+    std::future<void> helper[kTouchThreads];
+    for (size_t i = 1; i < kTouchThreads; ++i) {
+      try {
+        helper[i] = std::async(std::launch::async, touch, i);
+      } catch (const std::exception&) {  // no thread to be had
+      }
+    }
+    for (size_t i = 0; i < kTouchThreads; ++i) {
+      if (helper[i].valid()) helper[i].get();
+      else touch(i);
+    }
     void* dev = nullptr;
     if (cudaHostRegister(p, bytes, cudaHostRegisterDefault) == cudaSuccess) {
       if (cudaHostGetDevicePointer(&dev, p, 0) == cudaSuccess && dev == p) {  // kernels read units in place by this address
@@ -869,8 +877,11 @@ int ensure_host_units(infllm_ctx* c, int64_t n) {
   }
   // once the last slab is half full, the next one is pinned in the background
   if (!c->slab_pending && n + c->slab_units / 2 > (int64_t)c->slabs.size() * c->slab_units) {
-    c->slab_future = std::async(std::launch::async, alloc_slab, c->cfg.device, bytes);
-    c->slab_pending = true;
+    try {
+      c->slab_future = std::async(std::launch::async, alloc_slab, c->cfg.device, bytes);
+      c->slab_pending = true;
+    } catch (const std::exception&) {  // no thread to be had: it is pinned when it is needed
+    }
   }
   return INFLLM_OK;
 }
