@@ -2539,6 +2539,11 @@ extern "C" int infllm_ctx_destroy(infllm_ctx* c) {
   if (keep) {
     int cur = 0;
     cudaGetDevice(&cur);
+    if (c->slab_pending) {  // its helper thread may not outlive the caller's interest: the process may be about to end
+      const HostSlab h = c->slab_future.get();
+      c->slab_pending = false;
+      if (h.p) c->slabs.push_back(h);
+    }
     const int64_t dev = ctx_device_bytes(c), host = (int64_t)c->slabs.size() * c->slab_units * c->unit_bytes;
     size_t free_b = 0, total_b = 0;
     keep = cudaSetDevice(d) == cudaSuccess && cudaMemGetInfo(&free_b, &total_b) == cudaSuccess;

@@ -66,3 +66,17 @@ def test_a_process_that_can_start_no_thread(tmp_path):
     """, LD_PRELOAD=str(lib))
     refused, units, equal = out.split()[-3:]
     assert int(refused) >= 4 and int(units) == 40 and equal == "True"
+
+
+def test_no_thread_outlives_its_memory():
+    out = _run("""
+        cm, _ = memory(20)
+        torch.cuda.synchronize()
+        del cm
+        before = len(os.listdir("/proc/self/task"))
+        cm, out = memory(33)
+        del cm
+        print(before, len(os.listdir("/proc/self/task")))
+    """)
+    before, after = map(int, out.split()[-2:])
+    assert after <= before
