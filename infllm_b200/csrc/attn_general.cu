@@ -396,26 +396,25 @@ int launch_colsum(const void* q, int64_t q_hs, int64_t q_ts, const void* k, int6
 }
 
 // out = acc / l: HBM-bound, four columns per thread (8 MB in and 4 MB out at 512 queries x 32 heads: 11 us with one CTA
-// per row, 3.2 us like this)
-template <typename T>
+// per row, 3.2 us like this); one column where the head size or the alignment of acc or out does not allow it
+template <typename T, int kCols>
 __global__ void __launch_bounds__(256)
 attn_finalize_kernel(const float* __restrict__ acc, const float* __restrict__ m, const float* __restrict__ l,
                      T* __restrict__ out, int64_t o_hs, int64_t o_ts, float* __restrict__ lse, int64_t rows, int64_t lq,
-                     int head_dim, int vec) {
-  const int per_row = head_dim / 4;
+                     int head_dim) {
+  const int per_row = head_dim / kCols;
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, row = idx / per_row;  // row = h * lq + i
   if (row >= rows) return;
-  const int d = (int)(idx - row * per_row) * 4;
+  const int d = (int)(idx - row * per_row) * kCols;
   const int64_t h = row / lq, i = row - h * lq;
   const float lv = l[row], inv = lv > 0.f ? 1.f / lv : 0.f;
-  const float2 a = *reinterpret_cast<const float2*>(acc + row * head_dim + d),
-               b = *reinterpret_cast<const float2*>(acc + row * head_dim + d + 2);
   T* o = out + h * o_hs + i * o_ts + d;
-  const typename Act<T>::T2 v01 = Act<T>::from_f2(a.x * inv, a.y * inv), v23 = Act<T>::from_f2(b.x * inv, b.y * inv);
-  if (vec) {
+  if (kCols == 4) {
+    const float4 a = *reinterpret_cast<const float4*>(acc + row * head_dim + d);
+    const typename Act<T>::T2 v01 = Act<T>::from_f2(a.x * inv, a.y * inv), v23 = Act<T>::from_f2(a.z * inv, a.w * inv);
     *reinterpret_cast<uint2*>(o) = make_uint2(*reinterpret_cast<const uint32_t*>(&v01), *reinterpret_cast<const uint32_t*>(&v23));
-  } else {  // rows that are not 8-byte aligned
-    o[0] = v01.x, o[1] = v01.y, o[2] = v23.x, o[3] = v23.y;
+  } else {
+    *o = Act<T>::from_f(acc[row * head_dim + d] * inv);
   }
   if (lse && d == 0) lse[row] = lv > 0.f ? m[row] + log2f(lv) : -INFINITY;
 }
@@ -602,13 +601,13 @@ extern "C" int infllm_attn_finalize(const float* d_acc, const float* d_m, const 
                                     void* stream) {
   using namespace infllm;
   if (!d_acc || !d_m || !d_l || !d_out) return fail(INFLLM_E_BADARG, "attn_finalize: null pointer");
-  if (head_dim <= 0 || head_dim % 4) return fail(INFLLM_E_BADARG, "attn_finalize: head_dim %d", head_dim);
-  const int vec = (uintptr_t)d_out % 8 == 0 && o_hs % 4 == 0 && o_ts % 4 == 0;
-  if (lq <= 0) return INFLLM_OK;
+  if (lq <= 0 || n_heads <= 0 || head_dim <= 0) return INFLLM_OK;
+  const bool four = head_dim % 4 == 0 && (uintptr_t)d_acc % 16 == 0 && (uintptr_t)d_out % 8 == 0 && o_hs % 4 == 0 && o_ts % 4 == 0;
+  const int64_t rows = (int64_t)n_heads * lq;
   INFLLM_DISPATCH_DTYPE(dtype, T, {
-    const int64_t rows = (int64_t)n_heads * lq;
-    attn_finalize_kernel<T><<<(unsigned)ceil_div(rows * (head_dim / 4), 256), 256, 0, (cudaStream_t)stream>>>(
-        d_acc, d_m, d_l, (T*)d_out, o_hs, o_ts, d_lse, rows, lq, head_dim, vec);
+    auto kern = four ? attn_finalize_kernel<T, 4> : attn_finalize_kernel<T, 1>;
+    kern<<<(unsigned)ceil_div(rows * (head_dim / (four ? 4 : 1)), 256), 256, 0, (cudaStream_t)stream>>>(
+        d_acc, d_m, d_l, (T*)d_out, o_hs, o_ts, d_lse, rows, lq, head_dim);
   });
   INFLLM_LAUNCH_OK("attn_finalize_kernel");
   return INFLLM_OK;
