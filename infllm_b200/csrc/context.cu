@@ -2133,7 +2133,8 @@ int append_sub(infllm_ctx* c, const char* q, int64_t q_hs, int64_t q_ts, const c
       for (int64_t i = 0; i < lq; ++i) local_pairs += (double)std::min<int64_t>(S + i + 1, g.n_local);
       for (auto& sgm : gsegs) all_glk += sgm.len;
       local_pairs_eb = local_pairs;
-      const bool tc_now = c->use_tc && lq > 1 && gsegs.size() + 1 <= (size_t)kMaxSeg;
+      // (the tcgen05 kernel writes 16 bytes at a time, the caller's rows need not allow it)
+      const bool tc_now = c->use_tc && lq > 1 && gsegs.size() + 1 <= (size_t)kMaxSeg && tc_rows_ok(out_eb, o_hs, o_ts);
       if (tc_now) {
         AttnTcParams TP{};
         TP.maps[0] = c->m_qloc; TP.maps[1] = c->m_qglb; TP.maps[2] = c->m_krot; TP.maps[3] = c->m_kraw;
