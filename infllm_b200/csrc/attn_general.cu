@@ -461,7 +461,7 @@ namespace infllm {
 //                short as one tile, with at most one tile of queries, before that one is the cheaper.
 enum StageKernel { STAGE_GENERIC, STAGE_ONE, STAGE_TC };
 static StageKernel stage_kernel(int n_heads, int n_kv_heads, int64_t lq, int64_t lk, int head_dim) {
-  if (head_dim != 128 || n_heads % n_kv_heads || lk <= 0 || lk > INT32_MAX) return STAGE_GENERIC;
+  if (head_dim != 128 || n_heads % n_kv_heads || lk <= 0 || lk > (1 << 30)) return STAGE_GENERIC;  // (keys are counted in 32 bits)
   if (lq == 1 && n_heads / n_kv_heads <= 8) return STAGE_ONE;
   if (lk > kTile || lq > kTile) return STAGE_TC;
   return STAGE_GENERIC;
