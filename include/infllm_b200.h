@@ -276,7 +276,7 @@ typedef struct infllm_config {
                            *  4: refills from a device copy of the store by one cudaMemcpyAsync per unit as well
                            *     (refills from the pinned host store always are, like MemoryUnit.load,
                            *     context_manager.py:57-71), not by the copy kernel
-                           *  8: the two-heads-per-CTA tcgen05 attention kernel whatever the head count
+                           *  8: nothing any more
                            * 16: one-token appends wait for the retrieved ids before launching the attention
                            * 64: the 16th one-launch token asks for a grid that the device refuses
                            * 128: the waits inside every 16th one-launch token give up at once */

@@ -36,7 +36,7 @@ struct AttnTcParams {
   float scale_log2;
   int* err;
   // The key tiles of a work item are cut into n_split runs; with n_split > 1 every run writes an un-normalised
-  // partial (acc, m, l) and attn_tc_combine merges them.  With n_split == 1 the one-head kernel writes its state here
+  // partial (acc, m, l) and attn_tc_combine merges them.  With n_split == 1 the kernel writes its state here
   // instead of out / lse when part_acc is set, and folds in the state st_* when that is set (it may be the same memory).
   int32_t n_split;
   int32_t exact;    // exponentials to fp32's precision throughout (see kExactQueries)
@@ -71,8 +71,6 @@ int attn_tc3_splits(int64_t lq, int n_heads, int64_t keys);
 int attn_tc_combine_launch(const float* acc, const float* m, const float* l, int n_split, int n_heads, int64_t lq, void* out,
                            int64_t o_hs, int64_t o_ts, float* lse, const float* st_acc, const float* st_m,
                            const float* st_l, float* new_acc, float* new_m, float* new_l, int dtype, cudaStream_t s);
-// two query heads of one KV head per CTA (needs an even number of query heads per KV head)
-int attn_tc2_launch(const AttnTcParams& P, int dtype, cudaStream_t s);
 int colsum_tc_launch_maps(const CUtensorMap& map_q, const CUtensorMap& map_k, int q_row0, int k_tok0, int n_heads,
                           int n_kv_heads, int64_t lq, int64_t lk, int mask_mode, int64_t mask_offset,
                           int64_t mask_size, const float* lse, float* score, int64_t score_hs, int accumulate,

@@ -319,7 +319,7 @@ struct infllm_ctx {
   int32_t* h_tc_err = nullptr;   // pinned, 4 words
   cudaEvent_t ev_err = nullptr;  // behind the last copy of the record
   bool err_pending = false;
-  float* tc_part = nullptr;  // partial results of the two-head attention kernel's key-tile runs
+  float* tc_part = nullptr;  // partial results of the attention's key-tile runs
   size_t tc_part_floats = 0;
 
   // look-ahead retrieval inside one append: while exec block t runs, the top-k of t+1 over the units known
@@ -334,14 +334,11 @@ struct infllm_ctx {
     std::vector<int32_t> ids;
     int32_t* h_ids = nullptr;  // pinned: ids written by the device
     cudaEvent_t ev = nullptr;
-    cudaEvent_t ev_staged = nullptr;  // on the copy stream, behind the copies staged for this exec block
-    bool staged_recorded = false;
   };
   static constexpr int kMaxLookDepth = 8;
   int look_depth = 2;                             // exec blocks ranked ahead (cfg.look_depth overrides)
   LookAhead la[kMaxLookDepth + 1];
   std::unordered_map<int32_t, int64_t> staged_for;  // staged unit -> latest exec block that wants it
-  int32_t* h_spec = nullptr;        // pinned: look-ahead ids
   int32_t* h_cand_rows = nullptr;   // pinned: candidate unit ids
   float* h_cand_scores = nullptr;   // pinned: their scores, where they are summed over ranks
   unsigned long long* h_cand_words = nullptr;  // pinned: elsewhere, {score, cand_seq} words, read as they arrive
@@ -351,7 +348,6 @@ struct infllm_ctx {
   cudaStream_t mail_stream = nullptr;  // carries the small result copies to the host, off the main stream
   int cand_cap = 0;
   std::unordered_map<int32_t, int> staged;  // unit -> slot holding a prefetched copy
-  bool staged_pending = false;              // staged copies issued since the last wait on them
 
   // sealed units leave through a packing buffer (two in rotation) and one copy per run of units
   void* pack_buf[2] = {nullptr, nullptr};
@@ -621,12 +617,10 @@ int lazy_init(infllm_ctx* c, cudaStream_t s) {
   INFLLM_CUDA_OK(cudaMemsetAsync(c->tickets, 0, 2 * sizeof(unsigned int), s));
   INFLLM_CUDA_OK(cudaHostAlloc((void**)&c->h_topk, std::max(1, g.topk) * sizeof(unsigned long long), cudaHostAllocDefault));
   memset(c->h_topk, 0, std::max(1, g.topk) * sizeof(unsigned long long));
-  INFLLM_CUDA_OK(cudaHostAlloc((void**)&c->h_spec, std::max(1, g.topk) * sizeof(int32_t), cudaHostAllocDefault));
   c->cand_cap = g.topk + (c->look_depth + 1) * (g.exc_block_size / g.block_size + 2) + 4;
   for (auto& l : c->la) {
     INFLLM_CUDA_OK(cudaHostAlloc((void**)&l.h_ids, std::max(1, g.topk) * sizeof(int32_t), cudaHostAllocDefault));
     INFLLM_CUDA_OK(cudaEventCreateWithFlags(&l.ev, cudaEventDisableTiming));
-    INFLLM_CUDA_OK(cudaEventCreateWithFlags(&l.ev_staged, cudaEventDisableTiming));
   }
   INFLLM_CUDA_OK(cudaHostAlloc((void**)&c->h_cand_rows, c->cand_cap * sizeof(int32_t), cudaHostAllocDefault));
   INFLLM_CUDA_OK(cudaHostAlloc((void**)&c->h_cand_scores, c->cand_cap * sizeof(float), cudaHostAllocDefault));
@@ -635,9 +629,6 @@ int lazy_init(infllm_ctx* c, cudaStream_t s) {
   INFLLM_CUDA_OK(dev_malloc((void**)&c->d_cand_scores, c->cand_cap * sizeof(float)));
   INFLLM_CUDA_OK(dev_malloc((void**)&c->d_spec, (c->look_depth + 1) * std::max(1, g.topk) * sizeof(int32_t)));
   INFLLM_CUDA_OK(cudaStreamCreateWithFlags(&c->mail_stream, cudaStreamNonBlocking));
-  // decode partials: window + units + sink + overflow, each segment may add one ragged chunk
-  int64_t dec_keys = (int64_t)g.n_local + (int64_t)g.topk * g.block_size + g.n_init + g.block_size + g.exc_block_size;
-  (void)dec_keys;
   c->max_parts = 2 * 148;  // the decode attention launches at most two CTAs per SM, one partial each
   INFLLM_CUDA_OK(dev_malloc((void**)&c->part_o, (int64_t)c->max_parts * H * D * sizeof(float)));
   INFLLM_CUDA_OK(dev_malloc((void**)&c->part_lse, (int64_t)c->max_parts * H * sizeof(float)));
@@ -992,7 +983,6 @@ int lookahead_launch(infllm_ctx* c, int64_t target, cudaStream_t s) {
   la.target = target;
   la.launched = true;
   la.staged = false;
-  la.staged_recorded = false;
   la.n_spec = c->num_blocks;
   la.ids.clear();
   if (la.n_spec <= g.topk) return INFLLM_OK;  // every known unit is a candidate; nothing to rank
@@ -1077,7 +1067,6 @@ int lookahead_stage(infllm_ctx* c, int64_t target) {
     dst.push_back((char*)c->cache + (int64_t)slot * c->unit_bytes);
     on_device.push_back(c->dev_resident(b));
     if (!c->dev_resident(b)) c->counters.h2d_bytes += c->unit_bytes;
-    c->staged_pending = true;
   }
   if (!src.empty()) {
     // the spare slots taken above may have held units that the previous exec block's attention read
@@ -1101,12 +1090,6 @@ int lookahead_stage(infllm_ctx* c, int64_t target) {
     }
     if (!ksrc.empty()) INFLLM_TRY(stage_units_launch(ksrc.data(), kdst.data(), (int)ksrc.size(), c->unit_bytes, c->copy_stream));
     for (size_t i = 0; i < src.size(); ++i) INFLLM_TRY(mark_slot_copy(c, dst[i]));
-  }
-  if (c->staged_pending) {
-    INFLLM_CUDA_OK(cudaEventRecord(c->ev_stage, c->copy_stream));
-    // the exec block this batch is for waits for this event only, not for batches staged later for later blocks
-    INFLLM_CUDA_OK(cudaEventRecord(la.ev_staged, c->copy_stream));
-    la.staged_recorded = true;
   }
   if (!src.empty()) trace_mark(c, c->copy_stream, TR_STAGE_END, target);
   return INFLLM_OK;
@@ -1344,7 +1327,6 @@ int plan_and_refill(infllm_ctx* c, const std::vector<int32_t>& ids, int64_t eb, 
     INFLLM_CUDA_OK(cudaEventRecord(c->ev_copy, c->urgent_stream));
     INFLLM_CUDA_OK(cudaStreamWaitEvent(s, c->ev_copy, 0));
   }
-  if (c->staged.empty()) c->staged_pending = false;
   return INFLLM_OK;
 }
 
@@ -2159,11 +2141,8 @@ int append_sub(infllm_ctx* c, const char* q, int64_t q_hs, int64_t q_ts, const c
         TP.stage[1].lk = (int64_t)all_glk; TP.stage[1].seg_begin = 1; TP.stage[1].seg_end = ns;
         ProfScope ps(c, s, INFLLM_PROF_ATTN, 4.0 * D * H * (local_pairs + (double)lq * all_glk));
         // One CTA per (128-query tile, head); few queries or few heads on this GPU (a short call, a KV-head-group shard)
-        // leave most SMs idle that way, and the key tiles are cut into runs until the grid fills them.  Flag bit 3
-        // forces the kernel that takes two heads of a KV head per CTA.
-        const bool two = (H / HKV) % 2 == 0 && (g.debug_flags & 8);
-        const int items = (int)((lq + 127) / 128) * (int)(H / 2);
-        TP.n_split = two ? std::max(1, std::min(8, 148 / items)) : attn_tc3_splits(lq, (int)H, lk + (int64_t)all_glk);
+        // leave most SMs idle that way, and the key tiles are cut into runs until the grid fills them.
+        TP.n_split = attn_tc3_splits(lq, (int)H, lk + (int64_t)all_glk);
         const size_t need = TP.n_split > 1 ? (size_t)TP.n_split * H * lq * (128 + 2) : 0;
         if (need > c->tc_part_floats) {
           if (c->tc_part) INFLLM_CUDA_OK(cudaFreeAsync(c->tc_part, s));
@@ -2177,14 +2156,10 @@ int append_sub(infllm_ctx* c, const char* q, int64_t q_hs, int64_t q_ts, const c
           TP.part_m = c->tc_part + (size_t)TP.n_split * H * lq * 128;
           TP.part_l = TP.part_m + (size_t)TP.n_split * H * lq;
         }
-        if (two) {
-          INFLLM_TRY(attn_tc2_launch(TP, g.dtype, s));
-        } else {
-          INFLLM_TRY(attn_tc3_launch(TP, g.dtype, s));
-          if (TP.n_split > 1)
-            INFLLM_TRY(attn_tc_combine_launch(TP.part_acc, TP.part_m, TP.part_l, TP.n_split, (int)H, lq, out_eb, o_hs, o_ts,
-                                              c->lse, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, g.dtype, s));
-        }
+        INFLLM_TRY(attn_tc3_launch(TP, g.dtype, s));
+        if (TP.n_split > 1)
+          INFLLM_TRY(attn_tc_combine_launch(TP.part_acc, TP.part_m, TP.part_l, TP.n_split, (int)H, lq, out_eb, o_hs, o_ts,
+                                            c->lse, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, g.dtype, s));
       } else {
       AttnParams P{};
       P.n_heads = (int)H; P.n_kv_heads = (int)HKV; P.lq = lq; P.first = 1;
@@ -2346,7 +2321,6 @@ static int ctx_reset(infllm_ctx* c, bool wait) {
   c->staged.clear();
   c->staged_for.clear();
   for (auto& l : c->la) l.target = -1, l.launched = l.staged = false;
-  c->staged_pending = false;
   c->trace_topk.clear();
   c->attn_recorded = false;
   c->attn_prev_recorded = false;
@@ -2389,11 +2363,9 @@ static void ctx_free(infllm_ctx* c, bool idle) {
     if (c->h_topk) cudaFreeHost(c->h_topk);
     if (c->h_tc_err) cudaFreeHost(c->h_tc_err);
     if (c->ev_err) cudaEventDestroy(c->ev_err);
-    if (c->h_spec) cudaFreeHost(c->h_spec);
     for (auto& l : c->la) {
       if (l.h_ids) cudaFreeHost(l.h_ids);
       if (l.ev) cudaEventDestroy(l.ev);
-      if (l.ev_staged) cudaEventDestroy(l.ev_staged);
     }
     if (c->h_cand_rows) cudaFreeHost(c->h_cand_rows);
     if (c->h_cand_scores) cudaFreeHost(c->h_cand_scores);

@@ -17,7 +17,7 @@
 namespace infllm {
 
 constexpr int kScoreWarps = 8;
-constexpr int kMaxScoreRows = 512;  // candidate rows per launch of block_score_rows_kernel
+constexpr int kMaxScoreRows = 512;  // listed rows per launch of seal_score_kernel
 
 template <typename T>
 __global__ void __launch_bounds__(kScoreWarps * 32)
