@@ -446,7 +446,7 @@ def measured_peaks():
 
 def run_ours(args, rank, world, local_rank, device_store_mb=0, light=False):
     """The prefill workload.  device_store_mb = 0 (the headline): sealed units live in the pinned host store only and
-    every cache refill is a cudaMemcpyAsync over PCIe on a side stream, as in the reference.  > 0: the variant that
+    a refill of a unit that no slot holds any more is a cudaMemcpyAsync over PCIe on a side stream.  > 0: the variant that
     also keeps a device copy of the store (refills are device-to-device copies).  `light` skips the end-to-end pass,
     the overlap trace and the CPU sample."""
     import torch.distributed as dist
@@ -546,7 +546,8 @@ def run_ours(args, rank, world, local_rank, device_store_mb=0, light=False):
                              "in 8192-token calls, exec 512, n_init 128, n_local 4096, unit 128, topk 16, repr_topk 4, "
                              f"max_cached {CFG['max_cached']}, lru; 64 planted units", l2="inputs (1 GiB of hidden states per step) exceed L2",
                     replicas=world // groups,
-                    store="pinned host store; every cache refill is a 512 KiB cudaMemcpyAsync over PCIe on a side stream",
+                    store="pinned host store; evicted units stay readable in spare slots until those are needed, a refill of any "
+                          "other unit is a 512 KiB cudaMemcpyAsync over PCIe on a side stream",
                     parallelism=(f"kv-head groups x{groups}: one layer over all GPUs, retrieval scores and output "
                                  "projection all-reduced (NCCL)") if groups > 1 else f"dp{world}: one layer replica per GPU"),
         e2e=dict(value=e2e, unit="tokens/s", h2d_bytes_per_step=int(hidden.numel() * 2),
@@ -627,7 +628,8 @@ def make_decode_memory(dev, rope, seed):
 
 def run_decode(args, rank, world, local_rank, device_store_mb=0):
     """The decode workload on one GPU per rank.  device_store_mb = 0 (the headline): the 8192 units of a layer live in
-    the pinned host store and every cache refill crosses PCIe.  > 0: the variant with a device copy of the store."""
+    the pinned host store, and a retrieved unit that no slot holds crosses PCIe.  > 0: the variant with a device copy
+    of the store."""
     import torch.distributed as dist
 
     from infllm_b200 import _lib
@@ -713,8 +715,8 @@ def run_decode(args, rank, world, local_rank, device_store_mb=0):
         ms = timed(step_device, args.steps)
         launches = _lib.lib.infllm_launch_count() - l0
         info1 = [cm.info() for cm in cms]
-        # the kernels' own durations: the same K steps once more with CUDA events around the scoring and the
-        # attention of every token.  Kept out of `value`'s region: four event records per 50 us token cost 14 us of it
+        # the same K steps once more as separate kernels (per-kernel timing takes a token apart), with CUDA events around
+        # the scoring and the attention of every token
         for cm in cms:
             cm.profile(True)
             cm.get_profile()
@@ -730,7 +732,8 @@ def run_decode(args, rank, world, local_rank, device_store_mb=0):
     us = 1e3 * ms / per_layer
     topk_ms, topk_bytes, topk_n = prof["topk"]
     dec_ms, dec_bytes, dec_n = prof["decode"]
-    achieved = topk_bytes / (topk_ms / 1e3) / 1e9 if topk_ms > 0 else None
+    token_bytes = topk_bytes / max(topk_n, 1) + dec_bytes / max(dec_n, 1)
+    achieved = token_bytes / us / 1e3 if dec_n else None
     hits = sum(y["cache_hits"] - x["cache_hits"] for x, y in zip(info0, info1))
     misses = sum(y["cache_misses"] - x["cache_misses"] for x, y in zip(info0, info1))
     cold = DEC["units"] * n_layers >= 16384
@@ -748,12 +751,14 @@ def run_decode(args, rank, world, local_rank, device_store_mb=0):
         e2e=dict(value=1e3 * ms_e2e / per_layer, unit="us/token", h2d_bytes_per_step=int((H + 2 * HKV) * D * 2 * n_layers),
                  d2h_bytes_per_step=int(H * D * 2 * n_layers)),
         gpu_launches=int(launches),
-        roofline=dict(bound="hbm", kernel="block_score_topk_kernel (unit scoring + top-k)", achieved=achieved,
-                      peak=hbm_peak, unit="GB/s", frac=(achieved / hbm_peak if achieved else None), traffic=None,
-                      peak_source=f"hbm_gbs of {which}", launches=int(topk_n),
-                      us_per_launch=1e3 * topk_ms / max(topk_n, 1), bytes_per_launch=topk_bytes / max(topk_n, 1),
-                      timed_in="a second pass of the same K steps with CUDA events around the kernel on its stream",
-                      us_per_token_with_events=1e3 * ms_events / per_layer),
+        roofline=dict(bound="hbm", kernel="token_kernel (scoring, top-k, attention and merge of a token, one launch)",
+                      achieved=achieved, peak=hbm_peak, unit="GB/s", frac=(achieved / hbm_peak if achieved else None),
+                      traffic=None, peak_source=f"hbm_gbs of {which}", launches=per_layer, us_per_launch=us,
+                      bytes_per_launch=token_bytes, timed_in="the timed region: the time from one token to the next"),
+        scoring_apart=dict(kernel="block_score_topk_kernel", achieved_gbs=(topk_bytes / (topk_ms / 1e3) / 1e9 if topk_ms > 0 else None),
+                           us_per_launch=1e3 * topk_ms / max(topk_n, 1), bytes_per_launch=topk_bytes / max(topk_n, 1),
+                           timed_in="a second pass of the same K steps as separate kernels, with CUDA events around them",
+                           us_per_token_with_events=1e3 * ms_events / per_layer),
         kernels={k: dict(ms=v[0], launches=v[2], work=v[1]) for k, v in prof.items()},
         decode_attention=dict(kernels="attn_decode_kernel + lse_merge_kernel",
                               achieved_gbs=(dec_bytes / (dec_ms / 1e3) / 1e9 if dec_ms > 0 else None),
@@ -800,8 +805,8 @@ def run_thrash(args, rank, world, local_rank):
     """Cache-thrash stress: a Qwen-1.5-7B-shaped layer (32 query / 32 KV heads), 524288 tokens = 4096 memory units of
     2 MiB, topk 16, repr_topk 8, exec blocks of 256, and a cache of exactly one retrieval (max_cached_block 16: the
     configuration's literal 8 cannot hold a retrieval and is refused, as the reference asserts).  Consecutive exec
-    blocks retrieve disjoint groups of units, so every exec block evicts the whole cache and refills it from the
-    pinned host store: 32 MiB over PCIe per 256 tokens."""
+    blocks retrieve disjoint groups of units, so every exec block evicts the whole cache and takes up another 16 units:
+    from the slots that keep evicted units, where they still are, else from the pinned host store, 2 MiB over PCIe each."""
     from infllm_b200 import _lib
     from infllm_b200.attention import ContextManager, RotaryEmbeddingESM
 
@@ -888,8 +893,9 @@ def run_thrash(args, rank, world, local_rank):
                              f"8192-token calls, exec 256, n_local 4096, unit 128 (2 MiB), topk 16, repr_topk 8, "
                              f"max_cached 16; {G} unit groups, exec block t retrieves group t % {G}",
                     literal_max_cached_8=("refused: " + refused) if refused else "NOT refused",
-                    l2="16 units x 2 MiB refilled per exec block exceed nothing by themselves; the 4 GiB of q/k/v per "
-                       "131072 tokens do", replicas=world),
+                    l2="the 4 GiB of q/k/v per 131072 tokens exceed L2",
+                    kept="the groups' 128 units fit into the slots that keep evicted units: each exec block evicts 16 units "
+                         "and takes 16 others up, most of them without a copy", replicas=world),
         gpu_launches=int(launches),
         store=dict(misses_per_exec_block=info["cache_misses"] / max(n_eb, 1), evictions_per_exec_block=info["evictions"] / max(n_eb, 1),
                    h2d_bytes_per_exec_block=info["h2d_bytes"] / max(n_eb, 1), h2d_late_bytes=info["h2d_late_bytes"],
@@ -959,8 +965,8 @@ def sharded_decode_selfcheck(rank, world, dev, mailbox_on=True, tokens=48):
 def head_groups_selfcheck(rank, world, dev, comm, tokens=16384):
     """Untimed: a `tokens`-token prompt through one layer sharded by KV-head groups over all ranks, and on rank 0 also
     through the whole layer.  Per exec block: the retrieved unit sets, and the outputs (within 2 % of their range) for
-    as long as the two runs have retrieved the same units.  The two runs do not use the same attention kernel (few
-    heads per GPU take the two-heads-per-CTA kernel), so their accumulated local scores differ in the last bits and a
+    as long as the two runs have retrieved the same units.  Few heads per GPU have their key tiles cut
+    into runs that are merged, so the accumulated local scores of the two differ in the last bits and a
     representative key can be built from another of several tied tokens; from then on the retrievals may differ
     legitimately.  ok = every exec block before the first difference agrees in its outputs (that prefix holds at least
     the exec blocks that retrieve every unit there is) and the retrieved sets overlap by 80 % or more over the prompt."""
