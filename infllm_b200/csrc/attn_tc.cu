@@ -144,7 +144,7 @@ __device__ __forceinline__ bool seg_tiles(int64_t vis_lo, int64_t vis_hi, int64_
 // each with all 128 key columns, a row is spread over the four threads of a quad, so a row maximum is two shuffles
 // and no thread waits for another warp.  Every fourth pair of exponentials is a polynomial on the FMA pipe.  The producer
 // asks for K one tile ahead of V (the V buffer frees late in a tile's cycle and K(t+1) queued behind that wait).
-// kExact, where the work used to be the shape-generic kernel's: that polynomial is as good as exp2f, and the reference
+// kExact (see kExactQueries): that polynomial is as good as exp2f, and the reference
 // maximum of a row follows its maximum, so that the largest probabilities have no rounding (2 to 6 % less error of an
 // output against 64 bits); whenever a row's maximum grows, O is scaled.  13001 tokens of sink + window attention: 1.25 ms,
 // 1.12 without.
@@ -756,7 +756,7 @@ __global__ void attn_tc_combine_kernel(const float* __restrict__ acc, const floa
 // four of the sixteen compute warps of its own, which turn it into sum_q exp2(s - lse_q).  A key tile is loaded once
 // per head and a query tile once per CTA, which keeps the L2 traffic an order of magnitude below one load per pair.
 // Bound: 16384 exponentials per pair, 768 cycles of the special-function unit with every fourth pair of them as a
-// quartic on the FMA pipe (a quintic, kExact, for the short calls), and the product, 514; a pair takes 1150.  512 queries x 32 heads over 4608 keys: 30.7 us.
+// quartic on the FMA pipe (a quintic, kExact, for exec blocks of one query tile), and the product, 514; a pair takes 1150.  512 queries x 32 heads over 4608 keys: 30.7 us.
 // (37.6 us with one issuing thread and all sixteen warps on one buffer at a time, whose exponentials were two at a
 // time in fp16: 1.4e-3 off in a sum, now 1e-6.)
 namespace colsum_smem {

@@ -2123,7 +2123,7 @@ int append_sub(infllm_ctx* c, const char* q, int64_t q_hs, int64_t q_ts, const c
         TP.maps[4] = c->m_v; TP.maps[5] = c->m_cache; TP.maps[6] = c->m_initk; TP.maps[7] = c->m_initv;
         TP.n_stage = 2; TP.n_heads = (int)H; TP.n_kv_heads = (int)HKV; TP.lq = lq;
         TP.out = out_eb; TP.o_hs = o_hs; TP.o_ts = o_ts; TP.lse = c->lse;
-        TP.scale_log2 = kLog2e / sqrtf((float)D); TP.err = c->tc_err; TP.exact = lq <= kExactQueries;
+        TP.scale_log2 = kLog2e / sqrtf((float)D); TP.err = c->tc_err;
         TP.stage[0].map_q = 0; TP.stage[0].q_row0 = (int)st; TP.stage[0].mask_mode = INFLLM_MASK_WINDOW;
         TP.stage[0].mask_offset = lk - lq; TP.stage[0].mask_size = g.n_local; TP.stage[0].lk = lk;
         TP.stage[0].seg_begin = 0; TP.stage[0].seg_end = 1;
@@ -2143,6 +2143,7 @@ int append_sub(infllm_ctx* c, const char* q, int64_t q_hs, int64_t q_ts, const c
         // One CTA per (128-query tile, head); few queries or few heads on this GPU (a short call, a KV-head-group shard)
         // leave most SMs idle that way, and the key tiles are cut into runs until the grid fills them.
         TP.n_split = attn_tc3_splits(lq, (int)H, lk + (int64_t)all_glk);
+        TP.exact = lq <= kExactQueries;
         const size_t need = TP.n_split > 1 ? (size_t)TP.n_split * H * lq * (128 + 2) : 0;
         if (need > c->tc_part_floats) {
           if (c->tc_part) INFLLM_CUDA_OK(cudaFreeAsync(c->tc_part, s));
