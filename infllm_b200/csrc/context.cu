@@ -1133,7 +1133,9 @@ int candidates_finish(infllm_ctx* c, int n_cand, std::vector<int32_t>* ids) {
   std::vector<int> order(n_cand);
   for (int i = 0; i < n_cand; ++i) order[i] = i;
   const int32_t* rows = c->h_cand_rows;
-  const float* sc = c->h_cand_scores;
+  float* sc = c->h_cand_scores;
+  for (int i = 0; i < n_cand; ++i)
+    if (!(sc[i] == sc[i])) sc[i] = -INFINITY;  // NaN ranks with -inf, as on the device (and an order it is not)
   std::sort(order.begin(), order.end(), [&](int a, int b) {
     if (sc[a] != sc[b]) return sc[a] > sc[b];
     return rows[a] < rows[b];
