@@ -473,9 +473,10 @@ static int stage_tc(const void* d_q, int64_t q_hs, int64_t q_ts, const void* d_k
                     float* scratch, int64_t scratch_floats, void* out, int64_t o_hs, int64_t o_ts, float* lse, int dtype,
                     cudaStream_t s) {
   AttnTcParams P{};
-  INFLLM_TRY(encode_rows_map(&P.maps[0], dtype, d_q, lq, n_heads, q_hs, q_ts));
-  INFLLM_TRY(encode_rows_map(&P.maps[1], dtype, d_k, lk, n_kv_heads, k_hs, k_ts));
-  INFLLM_TRY(encode_rows_map(&P.maps[2], dtype, d_v, lk, n_kv_heads, k_hs, k_ts));
+  const bool pair = attn_tc3_pairs(lq, n_heads, n_kv_heads);
+  INFLLM_TRY(encode_rows_map(&P.maps[0], dtype, d_q, lq, n_heads, q_hs, q_ts, kBoxTile));
+  INFLLM_TRY(encode_rows_map(&P.maps[1], dtype, d_k, lk, n_kv_heads, k_hs, k_ts, box_k(pair)));
+  INFLLM_TRY(encode_rows_map(&P.maps[2], dtype, d_v, lk, n_kv_heads, k_hs, k_ts, box_v(pair)));
   INFLLM_TRY(tc_get_error_ptr(&P.err));
   P.n_stage = 1; P.n_heads = n_heads; P.n_kv_heads = n_kv_heads; P.lq = lq; P.exact = 1;
   P.scale_log2 = kLog2e / sqrtf(128.f);

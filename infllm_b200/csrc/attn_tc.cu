@@ -3,11 +3,11 @@
 // attn_tc3_kernel   one 128-query tile of one head per CTA, all stages of an exec block fused:
 //                   local window stage (window-relative rotated q/k, causal window mask) and global
 //                   stage (one-angle q; retrieved units in their cache slots, init sink, overflow),
-//                   jointly normalised.  Warp-specialised: 8 softmax warps (16 query rows each, a row spread over
-//                   the four threads of a quad), 1 TMA producer warp, two issuing threads (S = Q K^T and
-//                   O += P V).  S accumulates in TMEM (three buffers), P is written back over its S columns and
-//                   feeds the P V product from TMEM, O stays in TMEM for the whole tile with lazy rescaling; K/V
-//                   tiles are double buffered.  Where the grid leaves SMs idle the key tiles are cut into runs.
+//                   jointly normalised.  Two CTAs of a cluster share the key tiles (cta_group::2).  Warp-specialised: two
+//                   teams of four softmax warps (a thread per query row, key tiles in turn), 1 TMA producer warp, two
+//                   issuing warps (S = Q K^T and O += P V).  S accumulates in TMEM (three buffers), P is written back over
+//                   its S columns and feeds the P V product from TMEM, O stays in TMEM for the whole tile with lazy
+//                   rescaling.  Where the grid leaves SMs idle the key tiles are cut into runs.
 // colsum_tc_kernel  per-key score pass: S^T = K Q^T with keys as TMEM lanes; a CTA keeps one head's query tiles
 //                   resident and streams a run of key tiles through a TMA ring and four TMEM buffers; four
 //                   threads per key sum exp2(s - lse) over the queries that see it.
@@ -44,6 +44,11 @@ __device__ __forceinline__ bool wait_or_abort(uint32_t bar, uint32_t parity, vol
   *abort_flag = 1;
   record_error(err, kErrWaitTimeout, where);
   return false;
+}
+
+// the same for a whole (converged) warp, whose lanes go on or give up together
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* err, int where) {
+  return __all_sync(0xffffffffu, wait_or_abort(bar, parity, abort_flag, err, where));
 }
 
 __device__ __forceinline__ float ex2_approx(float x) {
@@ -136,42 +141,46 @@ __device__ __forceinline__ bool seg_tiles(int64_t vis_lo, int64_t vis_hi, int64_
 
 // ------------------------------------------------------------------------------------------------
 // attn_tc3_kernel: one 128-query tile of one head per CTA; P never touches shared memory.  P = exp2(S - m) goes back
-// into the TMEM columns of its S buffer as packed 16-bit pairs and is the A operand of the P V product from there
-// (a key tile moves 160 KB through shared memory: Q, K, V operand reads and the TMA fill of K and V), and there are
-// three S/P buffers in TMEM, so that S runs a tile ahead of the softmax.  Eleven warps: eight softmax warps, the TMA
-// producer, and one issuing thread per product (one thread for both was the longest serial chain of a tile).
-// The softmax warps read S in the 16-lane shape: warps w and w+4 share a TMEM lane quarter and take 16 of its rows
-// each with all 128 key columns, a row is spread over the four threads of a quad, so a row maximum is two shuffles
-// and no thread waits for another warp.  Every fourth pair of exponentials is a polynomial on the FMA pipe.  The producer
-// asks for K one tile ahead of V (the V buffer frees late in a tile's cycle and K(t+1) queued behind that wait).
+// into the TMEM columns of its S buffer as packed 16-bit pairs and is the A operand of the P V product from there, and there are
+// three S/P buffers in TMEM.
+// Pairs of CTAs (attn_tc3_pairs: where a KV head's query tiles, over all its query heads, come out even): the products are
+// cta_group::2, 256 rows of two CTAs by 128 keys, and a CTA fetches and holds half of every K and V tile.  That halves the
+// bytes from L2 to shared memory (a lone CTA's 64 KB a tile take 1600 cycles at 40 bytes per clock and SM) and leaves room for
+// four tiles in flight; the same code without pairs takes 78 us where pairs take 70.  Two query heads of a KV head make a pair, so
+// that both see the same keys; two tiles of one head where there is only one.
+// The softmax is two teams of four warps with the key tiles in turn, a thread per query row: no exchange within a row, and one
+// team's maximum and waits under the other's exponentials.  With all eight warps on one tile at a time (a row over four threads)
+// a tile took 2000 cycles, 1700 of them theirs.  One pair of exponentials in eight is a polynomial on the FMA pipe: none to a
+// quarter make no difference to the time.
+// Issuers and producer are whole warps of which one lane issues: eight products in 120 cycles instead of 600, and one load per
+// tile and operand (both 64-dimension halves in one box) instead of four at about 390 cycles each, which was 1570 per tile
+// whatever their size.  The producer asks for K one tile ahead of V.
 // kExact (see kExactQueries): that polynomial is as good as exp2f, and the reference
 // maximum of a row follows its maximum, so that the largest probabilities have no rounding (2 to 6 % less error of an
-// output against 64 bits); whenever a row's maximum grows, O is scaled.  13001 tokens of sink + window attention: 1.25 ms,
-// 1.12 without.
-// What the clock stamps of one CTA say (cycles per 128-key tile, 131072-token prefill): the period is 2000 (2100-2200 when
-// the rest of these stamps was taken) and it is the softmax warps' (1700 of work, 400 of waits and loop); S is ready 2000
-// cycles before they come for it; a K or V tile takes 900-1000 cycles from request to arrival, which is also what the loads
-// alone allow (a CTA whose softmax does nothing and whose P V products are left out still needs 1600 per tile: four 16 KB
-// boxes at about 40 bytes per clock and SM from L2).  Tried and not kept: a second softmax team on alternate tiles with its
-// own S buffer and accumulator (the chain S -> softmax -> P V -> next S of one team is as long as two tiles; 94 us),
-// asking TMEM for the next tile's scores before this tile's exponentials (111 us), an L2 prefetch of the key tiles
-// four to eight tiles ahead (no change), all exponentials or half of them on the special-function unit (87, 86 us).
-// 70 to 74 us per exec block of the 128K prefill (83 before the run's parts were listed once and the epilogue rolled).  A
-// CTA's cycles there: 7500 to the first tile's scores, 54 tiles of 2000, 3400 behind the last; a run of 12 tiles: 34000 in
-// all.
+// output against 64 bits); whenever a row's maximum grows, O is scaled.
+// What bounds it (clock stamps, cycles per 128-key tile): a period of 1600 at 1.75 GHz, a third of the way round of an S/P buffer:
+// product and commit 700, maximum 480, the other team's maximum 400, exponentials 1500, to the issuer 250, P V and back 800;
+// the tensor pipe needs 1024.  Per exec block of 32/8 heads, 512 queries by 4608 + 2688 keys: 64.3 us, 71.8 before (kExact: 70.6,
+// 84.6); 256 queries of 32/32 heads in two runs 45.5, 47.6; 4096 queries by 8192 keys, kExact, 306, 355.
+// Tried and not kept: four warps to half a tile's keys each, two tiles at once (70.5: more warps at the same pipes); the 64
+// score columns that a later tile needs first kept in registers, so that their buffer frees early (70.3); one issuer for both
+// products (72.3); three teams.
 namespace tc3 {
+constexpr int kBufs = 3;                         // S/P buffers in TMEM
 constexpr int kQ = 0;                            // two stages
-constexpr int kK = kQ + 4 * kSubTileBytes;       // two stages
-constexpr int kV = kK + 4 * kSubTileBytes;       // two stages
+constexpr int kK = kQ + 4 * kSubTileBytes;       // two stages of a tile, or four of a CTA's half of one
+constexpr int kV = kK + 4 * kSubTileBytes;       // the same
 constexpr int kBar = kV + 4 * kSubTileBytes;
-constexpr int kXmax = kBar + 256;                // reference maxima of the 128 rows, for the epilogue's layout
-constexpr int kXsum = kXmax + 512;               // row sums of the 128 rows
-constexpr int kPlan = kXsum + 512;
+constexpr int kTmax = kBar + 512;                // the rows' maxima in the last four tiles
+constexpr int kXmax = kTmax + 4 * 512;           // per team: the reference its row sums stand at
+constexpr int kXsum = kXmax + 2 * 512;           // per team: row sums
+constexpr int kPlan = kXsum + 2 * 512;
 constexpr int kTotal = kPlan + 32 + kMaxSeg * 32;
-constexpr int kPolyEvery = 4;
-enum { T3_Q_FULL0 = 0, T3_Q_FULL1, T3_Q_EMPTY0, T3_Q_EMPTY1, T3_K_FULL0, T3_K_FULL1, T3_K_EMPTY0, T3_K_EMPTY1, T3_V_FULL0, T3_V_FULL1,
-       T3_V_EMPTY0, T3_V_EMPTY1, T3_S_FULL0, T3_S_FULL1, T3_S_FULL2, T3_P_FULL0, T3_P_FULL1, T3_P_FULL2, T3_PV_DONE0, T3_PV_DONE1,
-       T3_PV_DONE2, T3_O_FULL, T3_N_BARS };
+constexpr int kPolyEvery = 8;
+enum { T3_Q_FULL0 = 0, T3_Q_EMPTY0 = 2, T3_K_FULL0 = 4, T3_K_EMPTY0 = 8, T3_V_FULL0 = 12, T3_V_EMPTY0 = 16, T3_S_FULL0 = 20,
+       T3_P_FULL0 = 23, T3_PV_DONE0 = 26, T3_MAX0 = 29, T3_O_FULL = 45, T3_N_BARS };
+constexpr int kWarpTma = 8, kWarpPv = 9, kWarpQk = 10;  // behind the eight softmax warps
+constexpr int kThreads = 11 * 32;
 // What a CTA does, worked out once, by one warp: the segments of its run that have tiles, in order.  Left to every role's own
 // loop over stages and segments, the 64-bit arithmetic for 20 segments took 8400 cycles before the first product of a run
 // and 6000 behind its last one, of 46000 for 12 tiles.
@@ -257,11 +266,54 @@ __device__ __forceinline__ void make_plan(const AttnTcParams& P, int64_t i0, int
     if (last[1] >= 0) plan->part[last[1]].stage |= 256;
   }
 }
+// exponentials of 32 columns of a row, packed; sums into rs
+template <typename T, bool kExact>
+__device__ __forceinline__ void exp_chunk(const float2* a, float2* rs, uint32_t* pk) {
+#pragma unroll
+  for (int k = 0; k < 16; ++k) {
+    float2 p;
+    if (k % kPolyEvery == kPolyEvery - 1) {
+      p = ex2_poly2<kExact ? 5 : 3>(a[k]);  // one pair in kPolyEvery off the special-function unit
+    } else {
+      p = make_float2(ex2_approx(a[k].x), ex2_approx(a[k].y));
+    }
+    rs[k & 3] = fadd2(rs[k & 3], p);
+    typename Act<T>::T2 v = Act<T>::from_f2(p.x, p.y);
+    pk[k] = *reinterpret_cast<uint32_t*>(&v);
+  }
+}
+// 32 columns of scores into exponents; what they were loaded into may be loaded into again behind it
+__device__ __forceinline__ void arg_chunk(const float* s, float sc, float neg_m, float2* a) {
+  const float2 sc2 = make_float2(sc, sc), nm2 = make_float2(neg_m, neg_m);
+#pragma unroll
+  for (int k = 0; k < 16; ++k) {
+    a[k] = ffma2(s[2 * k], s[2 * k + 1], sc2, nm2);
+    asm volatile("" : "+f"(a[k].x), "+f"(a[k].y));
+  }
+}
+// a row's reference maximum behind a tile whose maximum is m_tile.  Lazy: it only moves when the maximum grew by more than
+// 2^8 - or, kExact, at all, so that the largest probabilities of a row are the ones that a 16-bit P holds without a rounding
+template <bool kExact>
+__device__ __forceinline__ float next_ref(float m, float m_tile) {
+  return m_tile - m > (kExact ? 0.f : 8.f) ? m_tile : m;  // (from -inf: any number)
+}
+__device__ __forceinline__ void max_chunk(const float* s, float* mx) {
+#pragma unroll
+  for (int i = 0; i < 32; i += 8) {
+    mx[0] = fmax3(mx[0], s[i], s[i + 1]);
+    mx[1] = fmax3(mx[1], s[i + 2], s[i + 3]);
+    mx[2] = fmax3(mx[2], s[i + 4], s[i + 5]);
+    mx[3] = fmax3(mx[3], s[i + 6], s[i + 7]);
+  }
+}
 }  // namespace tc3
 
-template <typename T, bool kExact>
-__global__ void __launch_bounds__(352, 1) attn_tc3_kernel(const __grid_constant__ AttnTcParams P) {
+template <typename T, bool kExact, bool kPair>
+__global__ void __launch_bounds__(tc3::kThreads, 1) attn_tc3_kernel(const __grid_constant__ AttnTcParams P) {
   using namespace tc3;
+  constexpr int kStages = kPair ? 4 : 2;
+  constexpr int kCtas = kPair ? 2 : 1;
+  constexpr int kShare = 2 * kSubTileBytes / kCtas;  // bytes of a K or V tile that a CTA holds
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const uint32_t s_base = smem_u32(smem);
@@ -269,17 +321,23 @@ __global__ void __launch_bounds__(352, 1) attn_tc3_kernel(const __grid_constant_
   const uint32_t bars = s_base + kBar;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + kBar + T3_N_BARS * 8);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + kBar + T3_N_BARS * 8 + 8);
+  float* tmax = reinterpret_cast<float*>(smem + kTmax);
   float* xmax = reinterpret_cast<float*>(smem + kXmax);
   float* xsum = reinterpret_cast<float*>(smem + kXsum);
   auto bar = [&](int i) { return bars + 8u * (uint32_t)i; };
+  const int rank = kPair ? (int)(blockIdx.x & 1) : 0;
+  // the barriers that count both CTAs' loads and probabilities are those of the first
+  auto lead_bar = [&](int i) { return kPair ? cluster_map(bar(i), 0) : bar(i); };
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int h = blockIdx.y, hkv = h / (P.n_heads / P.n_kv_heads);
-  const int64_t i0 = (int64_t)blockIdx.x * kTile;
+  // work items of a KV head: (query tile, head), the heads of a tile side by side; a pair of CTAs takes two in a row
+  const int group = P.n_heads / P.n_kv_heads, hkv = blockIdx.y;
+  const int qt = (int)blockIdx.x / group, h = hkv * group + (int)blockIdx.x % group;
+  const int64_t i0 = (int64_t)qt * kTile;
   const int rows_q = (int)((P.lq - i0) < kTile ? (P.lq - i0) : kTile);
   const int split = blockIdx.z;
 
-  if (warp == 10 && lane < P.n_stage) {  // the descriptors of the first loads are on their way while the run's parts are worked out
+  if (warp == kWarpQk && lane < P.n_stage) {  // the descriptors of the first loads are on their way while the run's parts are worked out
     const TcStage& S = P.stage[lane];
     tma_prefetch_map(&P.maps[S.map_q]);
     if (S.seg_begin < S.seg_end) {
@@ -288,309 +346,321 @@ __global__ void __launch_bounds__(352, 1) attn_tc3_kernel(const __grid_constant_
     }
   }
   tc3::Plan* plan = reinterpret_cast<tc3::Plan*>(smem + kPlan);
-  if (warp == 8) {  // the run's parts
-    if (P.stage[P.n_stage - 1].seg_end <= 32) make_plan<1>(P, i0, i0 + rows_q - 1, split, plan);
-    else make_plan<(kMaxSeg + 31) / 32>(P, i0, i0 + rows_q - 1, split, plan);
+  if (warp == kWarpTma) {  // the run's parts, of all queries of the pair
+    const int64_t u0 = kPair ? (int64_t)((int)(blockIdx.x & ~1u) / group) * kTile : i0;
+    const int64_t u1 = kPair ? (int64_t)((int)(blockIdx.x | 1u) / group + 1) * kTile : i0 + kTile;
+    const int64_t last = (u1 < P.lq ? u1 : P.lq) - 1;
+    if (P.stage[P.n_stage - 1].seg_end <= 32) make_plan<1>(P, u0, last, split, plan);
+    else make_plan<(kMaxSeg + 31) / 32>(P, u0, last, split, plan);
   }
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < T3_N_BARS; ++i) mbar_init(bar(i), (i >= T3_P_FULL0 && i <= T3_P_FULL2) ? 8u : 1u);
+    for (int i = 0; i < T3_N_BARS; ++i) mbar_init(bar(i), i >= T3_P_FULL0 && i < T3_P_FULL0 + kBufs ? 4u * kCtas : 1u);
     *abort_flag = 0;
     mbar_fence_init();
   }
-  if (warp == 9) {
-    tmem_alloc(smem_u32(tmem_slot), 512);
-    tmem_relinquish();
+  if (warp == kWarpPv) {
+    tmem_alloc<kPair>(smem_u32(tmem_slot), 512);
+    tmem_relinquish<kPair>();
   }
   tc_fence_before();
   __syncthreads();
+  if (kPair) cluster_sync();  // the other CTA's barriers stand before anything is signalled on them
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   const uint32_t tO = tmem + 384;  // three S/P buffers at columns [0,128), [128,256), [256,384)
   constexpr bool kBf16 = !std::is_same<T, __half>::value;
-  constexpr uint32_t idesc_qk = make_idesc(kBf16, 128, 128, false);
-  constexpr uint32_t idesc_pv = make_idesc(kBf16, 128, 128, true);
+  constexpr uint32_t idesc_qk = make_idesc(kBf16, 128 * kCtas, 128, false);
+  constexpr uint32_t idesc_pv = make_idesc(kBf16, 128 * kCtas, 128, true);
 
-  if (warp == 8) {
+  if (warp == kWarpTma) {
     // ======================================================================== TMA producer
-    // K runs one tile ahead of V: the buffer of K(t+1) is free as soon as S(t-1) has been formed, that of V(t) only
-    // when the P V product of tile t-2 has run, late in the tile's cycle; asked for in tile order, K(t+1) queued
-    // behind that wait and S(t+1) was not ready when the softmax warps came for it.
-    if (lane == 0) {
-      int it = 0, sidx = 0, stage = -1;
-      bool ok = true;
-      struct { int it, tok, c3, map; } pend = {-1, 0, 0, 0};  // the V tile that has not been asked for yet
-      auto load_v = [&]() {
-        const int b = pend.it & 1;
-        if (pend.it >= 2) ok = wait_or_abort(bar(T3_V_EMPTY0 + b), ((pend.it >> 1) - 1) & 1, abort_flag, P.err, 602);
-        if (!ok) return;
-        const uint32_t dv = sV + b * 2 * kSubTileBytes;
-        mbar_expect_tx(bar(T3_V_FULL0 + b), 2 * kSubTileBytes);
-        if (pend.c3 < 0) {
-          tma_load_3d(dv, &P.maps[pend.map], bar(T3_V_FULL0 + b), 0, pend.tok, hkv);
-          tma_load_3d(dv + kSubTileBytes, &P.maps[pend.map], bar(T3_V_FULL0 + b), 64, pend.tok, hkv);
-        } else {
-          tma_load_4d(dv, &P.maps[pend.map], bar(T3_V_FULL0 + b), 0, pend.tok, hkv, pend.c3);
-          tma_load_4d(dv + kSubTileBytes, &P.maps[pend.map], bar(T3_V_FULL0 + b), 64, pend.tok, hkv, pend.c3);
-        }
-        pend.it = -1;
-      };
-      const int n_parts = plan->n_parts;
-      for (int p = 0; p < n_parts && ok; ++p) {
-        const Part R = plan->part[p];
-        if ((R.stage & 255) != stage) {  // the stage's queries; the buffer was the stage's before the last one's
-          stage = R.stage & 255;
-          const TcStage& S = P.stage[stage];
-          const int qb = sidx & 1;
-          if (sidx >= 2) ok = wait_or_abort(bar(T3_Q_EMPTY0 + qb), ((sidx >> 1) - 1) & 1, abort_flag, P.err, 600);
-          if (!ok) break;
-          const uint32_t dq = sQ + qb * 2 * kSubTileBytes;
-          mbar_expect_tx(bar(T3_Q_FULL0 + qb), 2 * kSubTileBytes);
-          tma_load_3d(dq, &P.maps[S.map_q], bar(T3_Q_FULL0 + qb), 0, S.q_row0 + (int)i0, h);
-          tma_load_3d(dq + kSubTileBytes, &P.maps[S.map_q], bar(T3_Q_FULL0 + qb), 64, S.q_row0 + (int)i0, h);
-          ++sidx;
-        }
-        for (int t = 0; t < R.n && ok; ++t) {
-          const int b = it & 1, tok = R.tok + t * kTile;
-          if (it >= 2) ok = wait_or_abort(bar(T3_K_EMPTY0 + b), ((it >> 1) - 1) & 1, abort_flag, P.err, 601);
-          if (!ok) break;
-          const uint32_t dk = sK + b * 2 * kSubTileBytes;
-          mbar_expect_tx(bar(T3_K_FULL0 + b), 2 * kSubTileBytes);
-          if (R.c3_k < 0) {
-            tma_load_3d(dk, &P.maps[R.map_k], bar(T3_K_FULL0 + b), 0, tok, hkv);
-            tma_load_3d(dk + kSubTileBytes, &P.maps[R.map_k], bar(T3_K_FULL0 + b), 64, tok, hkv);
-          } else {
-            tma_load_4d(dk, &P.maps[R.map_k], bar(T3_K_FULL0 + b), 0, tok, hkv, R.c3_k);
-            tma_load_4d(dk + kSubTileBytes, &P.maps[R.map_k], bar(T3_K_FULL0 + b), 64, tok, hkv, R.c3_k);
-          }
-          if (pend.it >= 0) load_v();
-          if (!ok) break;
-          pend.it = it, pend.tok = tok, pend.c3 = R.c3_v, pend.map = R.map_v;
-          ++it;
-        }
+    // K runs one tile ahead of V: the buffer of K is free as soon as its S has been formed, that of V only
+    // when its P V product has run, late in the tile's cycle; asked for in tile order, K queued
+    // behind that wait and the next S was not ready when the softmax warps came for it.
+    // Of a pair, each CTA fetches its own queries, 64 of a tile's keys and half of the values' dimensions.
+    // One load per tile and operand, asked for by one lane of a warp whose lanes stay together: four loads a tile from a
+    // thread of its own took 1570 cycles a tile whatever their size, and nothing could be faster than that.
+    const bool lead = elect_one();
+    int it = 0, sidx = 0, stage = -1;
+    bool ok = true;
+    struct { int it, tok, c3, map; } pend = {-1, 0, 0, 0};  // the V tile that has not been asked for yet
+    auto load_v = [&]() {
+      const int b = pend.it % kStages;
+      if (pend.it >= kStages) ok = warp_wait(bar(T3_V_EMPTY0 + b), ((pend.it / kStages) - 1) & 1, abort_flag, P.err, 602);
+      if (!ok) return;
+      if (lead) {
+        const uint32_t dv = sV + b * kShare, fb = lead_bar(T3_V_FULL0 + b);
+        if (rank == 0) mbar_expect_tx(bar(T3_V_FULL0 + b), 2 * kSubTileBytes);
+        if (pend.c3 < 0) tma_load_4d<kPair>(dv, &P.maps[pend.map], fb, 0, pend.tok, rank, hkv);
+        else tma_load_5d<kPair>(dv, &P.maps[pend.map], fb, 0, pend.tok, rank, hkv, pend.c3);
       }
-      if (ok && pend.it >= 0) load_v();
-      if (!ok) {
-        // give loads that are still in flight a bounded chance to land before the CTA's memory goes away
-        for (int b = 0; b < 2; ++b) {
-          for (uint32_t i = 0; i < 4096 && !mbar_try_wait(bar(T3_K_FULL0 + b), 0) && !mbar_try_wait(bar(T3_K_FULL0 + b), 1); ++i) __nanosleep(64);
-          for (uint32_t i = 0; i < 4096 && !mbar_try_wait(bar(T3_V_FULL0 + b), 0) && !mbar_try_wait(bar(T3_V_FULL0 + b), 1); ++i) __nanosleep(64);
+      __syncwarp();
+      pend.it = -1;
+    };
+    const int n_parts = plan->n_parts;
+    for (int p = 0; p < n_parts && ok; ++p) {
+      const Part R = plan->part[p];
+      if ((R.stage & 255) != stage) {  // the stage's queries; the buffer was the stage's before the last one's
+        stage = R.stage & 255;
+        const TcStage& S = P.stage[stage];
+        const int qb = sidx & 1;
+        if (sidx >= 2) ok = warp_wait(bar(T3_Q_EMPTY0 + qb), ((sidx >> 1) - 1) & 1, abort_flag, P.err, 600);
+        if (!ok) break;
+        if (lead) {
+          const uint32_t dq = sQ + qb * 2 * kSubTileBytes, fb = lead_bar(T3_Q_FULL0 + qb);
+          if (rank == 0) mbar_expect_tx(bar(T3_Q_FULL0 + qb), 2 * kSubTileBytes * kCtas);
+          tma_load_4d<kPair>(dq, &P.maps[S.map_q], fb, 0, S.q_row0 + (int)i0, 0, h);
         }
+        __syncwarp();
+        ++sidx;
+      }
+      for (int t = 0; t < R.n && ok; ++t) {
+        const int b = it % kStages, tok = R.tok + t * kTile;
+        if (it >= kStages) ok = warp_wait(bar(T3_K_EMPTY0 + b), ((it / kStages) - 1) & 1, abort_flag, P.err, 601);
+        if (!ok) break;
+        if (lead) {
+          const uint32_t dk = sK + b * kShare, fb = lead_bar(T3_K_FULL0 + b);
+          if (rank == 0) mbar_expect_tx(bar(T3_K_FULL0 + b), 2 * kSubTileBytes);
+          if (R.c3_k < 0) tma_load_4d<kPair>(dk, &P.maps[R.map_k], fb, 0, tok + 64 * rank, 0, hkv);
+          else tma_load_5d<kPair>(dk, &P.maps[R.map_k], fb, 0, tok + 64 * rank, 0, hkv, R.c3_k);
+        }
+        __syncwarp();
+        if (pend.it >= 0) load_v();
+        if (!ok) break;
+        pend.it = it, pend.tok = tok, pend.c3 = R.c3_v, pend.map = R.map_v;
+        ++it;
       }
     }
-  } else if (warp == 9 || warp == 10) {
+    if (ok && pend.it >= 0) load_v();
+    if (!ok && lane == 0) {
+      // give loads that are still in flight a bounded chance to land before the CTA's memory goes away
+      for (int b = 0; b < kStages && rank == 0; ++b) {
+        for (uint32_t i = 0; i < 4096 && !mbar_try_wait(bar(T3_K_FULL0 + b), 0) && !mbar_try_wait(bar(T3_K_FULL0 + b), 1); ++i) __nanosleep(64);
+        for (uint32_t i = 0; i < 4096 && !mbar_try_wait(bar(T3_V_FULL0 + b), 0) && !mbar_try_wait(bar(T3_V_FULL0 + b), 1); ++i) __nanosleep(64);
+      }
+      for (uint32_t i = 0; i < 4096 && rank != 0; ++i) __nanosleep(256);  // its loads are counted in the first CTA
+    }
+  } else if (warp == kWarpPv || warp == kWarpQk) {
     // ========================================================================== MMA issuers
-    // Two threads: warp 10 issues S = Q K^T, warp 9 issues O += P V.  One thread doing both was the longest serial
+    // Two threads: one issues S = Q K^T, one O += P V.  One thread doing both was the longest serial
     // chain of a key tile (waits, 16 products that each hold the thread while the pipe is busy, commits: about
     // 2500 cycles); apart they take about 1100 each and the softmax sets the pace.  What the tensor pipe ordered
-    // before - S of tile t+2 may overwrite its buffer only when P V of tile t has read P from it - is now the
-    // wait for that product's commit.
-    if (lane == 0) {
+    // before - S of tile t+3 may overwrite its buffer only when P V of tile t has read P from it - is
+    // the wait for that product's commit.  Of a pair, the first CTA's issue for both.
+    if (rank == 0) {
+      const bool lead = elect_one();
       const int n = plan->n_tiles;
       bool ok = true;
-      if (warp == 10) {
+      if (warp == kWarpQk) {
         const uint64_t qd0[2] = {make_sdesc(sQ, 16, 1024), make_sdesc(sQ + 2 * kSubTileBytes, 16, 1024)};
-        const uint64_t kd0[2] = {make_sdesc(sK, 16, 1024), make_sdesc(sK + 2 * kSubTileBytes, 16, 1024)};
+        const uint64_t kd0 = make_sdesc(sK, 16, 1024);
         const int n_parts = plan->n_parts;
         int iq = 0, sq = 0;
         bool q_due = true;
         for (int p = 0; p < n_parts && ok; ++p) {
           const int np = plan->part[p].n, last = plan->part[p].stage & 256;
           for (int t = 0; t < np && ok; ++t, ++iq) {
-            const int b = iq & 1, qb = sq & 1;
-            if (q_due) ok = wait_or_abort(bar(T3_Q_FULL0 + qb), (sq >> 1) & 1, abort_flag, P.err, 610);
+            const int b = iq % kStages, qb = sq & 1;
+            if (q_due) ok = warp_wait(bar(T3_Q_FULL0 + qb), (sq >> 1) & 1, abort_flag, P.err, 610);
             q_due = false;
-            if (ok) ok = wait_or_abort(bar(T3_K_FULL0 + b), (iq >> 1) & 1, abort_flag, P.err, 611);
-            const int b3 = iq % 3;  // S/P buffer: free once the P V product of tile iq-3 has read P from it
-            if (ok && iq >= 3) ok = wait_or_abort(bar(T3_PV_DONE0 + b3), ((iq / 3) - 1) & 1, abort_flag, P.err, 614);
+            if (ok) ok = warp_wait(bar(T3_K_FULL0 + b), (iq / kStages) & 1, abort_flag, P.err, 611);
+            const int b3 = iq % kBufs;  // S/P buffer: free once the P V product of tile iq-3 has read P from it
+            if (ok && iq >= kBufs) ok = warp_wait(bar(T3_PV_DONE0 + b3), ((iq / kBufs) - 1) & 1, abort_flag, P.err, 614);
             if (!ok) break;
             tc_fence_after();
-            const uint64_t qd = sq & 1 ? qd0[1] : qd0[0], kd = b ? kd0[1] : kd0[0];
+            const uint64_t qd = sq & 1 ? qd0[1] : qd0[0], kd = kd0 + (uint64_t)(b * kShare >> 4);
+            if (lead) {
 #pragma unroll
             for (int ks = 0; ks < 8; ++ks) {
-              const uint64_t off = (uint64_t)(((ks >> 2) * kSubTileBytes + (ks & 3) * 32) >> 4);
-              mma_ss(tmem + b3 * 128, qd + off, kd + off, idesc_qk, ks > 0);
+              const uint64_t qo = (uint64_t)(((ks >> 2) * kSubTileBytes + (ks & 3) * 32) >> 4);
+              const uint64_t ko = (uint64_t)(((ks >> 2) * (kShare / 2) + (ks & 3) * 32) >> 4);
+              mma_ss<kPair>(tmem + b3 * 128, qd + qo, kd + ko, idesc_qk, ks > 0);
             }
-            tc_commit(bar(T3_S_FULL0 + b3));
-            tc_commit(bar(T3_K_EMPTY0 + b));
+            tc_commit<kPair>(bar(T3_S_FULL0 + b3));
+            tc_commit<kPair>(bar(T3_K_EMPTY0 + b));
             if (last && t == np - 1) {
-              tc_commit(bar(T3_Q_EMPTY0 + qb));  // the last product that reads this stage's Q tile
+              tc_commit<kPair>(bar(T3_Q_EMPTY0 + qb));  // the last product that reads this stage's Q tile
+            }
+            }
+            if (last && t == np - 1) {
               ++sq;
               q_due = true;
             }
+            __syncwarp();
           }
         }
       } else {
-        const uint64_t vd0[2] = {make_sdesc(sV, kSubTileBytes, 1024), make_sdesc(sV + 2 * kSubTileBytes, kSubTileBytes, 1024)};
+        const uint64_t vd0 = make_sdesc(sV, kSubTileBytes, 1024);
         for (int ip = 0; ip < n && ok; ++ip) {
-          const int b = ip & 1;
-          const int b3 = ip % 3;
-          ok = wait_or_abort(bar(T3_P_FULL0 + b3), (ip / 3) & 1, abort_flag, P.err, 612);
-          ok = ok && wait_or_abort(bar(T3_V_FULL0 + b), (ip >> 1) & 1, abort_flag, P.err, 613);
+          const int b = ip % kStages, b3 = ip % kBufs;
+          ok = warp_wait(bar(T3_V_FULL0 + b), (ip / kStages) & 1, abort_flag, P.err, 613);
+          ok = ok && warp_wait(bar(T3_P_FULL0 + b3), (ip / kBufs) & 1, abort_flag, P.err, 612);
           if (!ok) break;
           tc_fence_after();
+          const uint64_t vd = vd0 + (uint64_t)(b * kShare >> 4);
+          if (lead) {
 #pragma unroll
           for (int ks = 0; ks < 8; ++ks) {
-            // A = P from TMEM: keys 0-63 in the buffer's columns [0,32), keys 64-127 in [64,96)
-            const uint32_t a_t = tmem + b3 * 128 + 8 * ks;
-            mma_ts(tO, a_t, vd0[b] + (uint64_t)((ks * 2048) >> 4), idesc_pv, (ip > 0) || (ks > 0));
+            // A = P from TMEM, in the buffer's columns [0,64)
+            mma_ts<kPair>(tO, tmem + b3 * 128 + 8 * ks, vd + (uint64_t)((ks * 2048) >> 4), idesc_pv, (ip > 0) || (ks > 0));
           }
-          tc_commit(bar(T3_V_EMPTY0 + b));
-          tc_commit(bar(T3_PV_DONE0 + b3));
+          tc_commit<kPair>(bar(T3_V_EMPTY0 + b));
+          tc_commit<kPair>(bar(T3_PV_DONE0 + b3));
+          }
+          __syncwarp();
         }
-        if (ok) tc_commit(bar(T3_O_FULL));
+        if (ok && lead) tc_commit<kPair>(bar(T3_O_FULL));
       }
     }
   } else if (warp < 8) {
     // ===================================================================== softmax / epilogue
-    // Eight warps: warps w and w+4 share a TMEM lane quarter and take 16 of its query rows each, with all 128 key
-    // columns of those rows: the 16x256b load spreads a row over the four threads of a quad, so a row maximum is two
-    // shuffles and no thread waits for another warp.  A thread holds rows r and r+8, two columns of every block of 8.
-    const int quad = warp & 3, rh = warp >> 2;
-    const int rbase = quad * 32 + rh * 16 + (lane >> 2);
-    const int cq = 2 * (lane & 3);
-    const uint32_t lane_base = ((uint32_t)(quad * 32 + rh * 16)) << 16;
-    const int64_t qrow[2] = {i0 + rbase, i0 + rbase + 8};
-    const bool valid[2] = {qrow[0] < P.lq, qrow[1] < P.lq};
-    float m_ref[2] = {-INFINITY, -INFINITY}, l_part[2] = {0.f, 0.f};
-    int it = 0, stage = -1;
+    // Two teams of four warps take the key tiles in turn: a thread has a query row (its TMEM lane) and all 128 keys of
+    // it, so that nothing is exchanged within a row.  What one team waits for - scores from TMEM, the maximum, the way
+    // of P into TMEM - is covered by the other's exponentials.  There is one O and so one reference maximum per row; it follows
+    // from the tiles' maxima, in order, and every thread works it out for itself from those of its own tiles and those that
+    // the other team leaves in shared memory (tmax, a barrier per tile and quarter of the rows).
+    const int quad = warp & 3, team = warp >> 2, row = quad * 32 + lane;
+    const uint32_t lane_base = ((uint32_t)(quad * 32)) << 16;
+    const int64_t qi = i0 + row;
+    const bool row_valid = qi < P.lq;
+    const uint32_t p_full = lead_bar(T3_P_FULL0);
+    float m_ref = -INFINITY, l_part = 0.f;  // the reference behind this team's last tile, and its sum relative to it
+    int it0 = 0, stage = -1;
     bool ok = true;
-    int jlo[2] = {0, 0}, jhi[2] = {0, 0};  // keys of the stage visible to this thread's two query rows
-    const int n_parts = plan->n_parts;
+    int jlo = 0, jhi = 0;  // keys of the stage visible to this thread's query row
+    const int n_parts = plan->n_parts, n_tiles = plan->n_tiles;
     for (int p = 0; p < n_parts && ok; ++p) {
       const Part R = plan->part[p];
       if ((R.stage & 255) != stage) {
         stage = R.stage & 255;
         const TcStage& S = P.stage[stage];
         auto clamp = [](int64_t v) { return (int)(v < -(1 << 30) ? -(1 << 30) : v > (1 << 30) ? (1 << 30) : v); };
-#pragma unroll
-        for (int r = 0; r < 2; ++r) {
-          int64_t lo = 0, hi = S.lk - 1;
-          // rows past the last query are not masked, so that whole tiles stay whole: nothing of them is written
-          if (valid[r] && S.mask_mode == INFLLM_MASK_WINDOW) {
-            lo = qrow[r] + S.mask_offset - S.mask_size + 1;
-            hi = qrow[r] + S.mask_offset;
-          } else if (valid[r] && S.mask_mode == INFLLM_MASK_COMPLEMENT) {
-            hi = qrow[r] + S.mask_offset - S.mask_size;
-          }
-          jlo[r] = clamp(lo), jhi[r] = clamp(hi);
+        int64_t lo = 0, hi = S.lk - 1;
+        // rows past the last query are not masked, so that whole tiles stay whole: nothing of them is written
+        if (row_valid && S.mask_mode == INFLLM_MASK_WINDOW) {
+          lo = qi + S.mask_offset - S.mask_size + 1;
+          hi = qi + S.mask_offset;
+        } else if (row_valid && S.mask_mode == INFLLM_MASK_COMPLEMENT) {
+          hi = qi + S.mask_offset - S.mask_size;
         }
+        jlo = clamp(lo), jhi = clamp(hi);
       }
-      {
+      const int j_hi = jhi < R.lim ? jhi : R.lim;
+      for (int t = (team + it0) & 1; t < R.n && ok; t += 2) {
+        const int it = it0 + t, b3 = it % kBufs;
+        const uint32_t tS = tmem + b3 * 128 + lane_base;
+        ok = warp_wait(bar(T3_S_FULL0 + b3), (it / kBufs) & 1, abort_flag, P.err, 620);
+        if (!ok) break;
+        tc_fence_after();
+        const int c_lo = jlo - R.j - t * kTile, c_hi = j_hi - R.j - t * kTile;
+        if (!__all_sync(0xffffffffu, c_lo <= 0 && c_hi >= kTile - 1)) {
+          // a tile at an edge: what a row does not see is taken out of the scores where they are
+#pragma unroll 1
+          for (int c = 0; c < kTile; c += 32) {
+            uint32_t u[32];
+            tmem_ld32(tS + c, u);
+            tmem_wait_ld32(u);
+            const int lo = c_lo - c, hi = c_hi - c;
+#pragma unroll
+            for (int i = 0; i < 32; ++i) u[i] = i >= lo && i <= hi ? u[i] : 0xff800000u;
+            tmem_st32(tS + c, u);
+          }
+          tmem_wait_st();
+        }
+        float sa[32], mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+        uint32_t* ua = reinterpret_cast<uint32_t*>(sa);
         {
-          for (int t = 0; t < R.n && ok; ++t, ++it) {
-            const int b3 = it % 3;
-            const uint32_t tS = tmem + b3 * 128 + lane_base;
-            ok = __all_sync(0xffffffffu, wait_or_abort(bar(T3_S_FULL0 + b3), (it / 3) & 1, abort_flag, P.err, 620));
-            if (!ok) break;
-            tc_fence_after();
-            float s[64];
-            tmem_ld_16x256b_x16(tS, reinterpret_cast<uint32_t*>(s));
-            tmem_wait_ld();
-            const int jt = R.j + t * kTile;
-            int c_lo[2], c_hi[2];
+          float b[32];
+          uint32_t* ub = reinterpret_cast<uint32_t*>(b);
+          tmem_ld32(tS + 32, ub);
+          tmem_ld32(tS + 64, ua);
+          tmem_wait_ld32(ub);
+          tmem_wait_ld32(ua);
+          max_chunk(b, mx);
+          tmem_ld32(tS + 96, ub);
+          max_chunk(sa, mx);
+          tmem_ld32(tS, ua);
+          tmem_wait_ld32(ub);
+          tmem_wait_ld32(ua);
+          max_chunk(b, mx);
+          max_chunk(sa, mx);
+        }
+        const float m_tile = fmaxf(fmax3(mx[0], mx[1], mx[2]), mx[3]) * P.scale_log2;
+        float m_prev = m_ref;
+        if (it > 0) {
+          ok = warp_wait(bar(T3_MAX0 + ((it - 1) & 3) * 4 + quad), ((it - 1) >> 2) & 1, abort_flag, P.err, 621);
+          if (!ok) break;
+          m_prev = next_ref<kExact>(m_prev, tmax[((it - 1) & 3) * kTile + row]);
+        }
+        // (left behind the look at the other team's: a place is taken again by the tile after the next but one, whose team has
+        // then seen that it was read)
+        tmax[(it & 3) * kTile + row] = m_tile;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(T3_MAX0 + (it & 3) * 4 + quad));
+        const float m_new = next_ref<kExact>(m_prev, m_tile);
+        const bool resc = __any_sync(0xffffffffu, m_new != m_prev && m_prev != -INFINITY) && it >= 1;
+        const float alpha = m_prev == -INFINITY ? 1.f : ex2_approx(m_prev - m_new);
+        if (m_new != m_ref) {
+          l_part *= ex2_approx(m_ref - m_new);
+          m_ref = m_new;
+        }
+        const float neg_m = m_new == -INFINITY ? 0.f : -m_new;
+        float2 rs[4] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+        // P, packed, takes the place of the scores that have been read: 16 columns for 32.  (Rolled: the fetch of code is what
+        // unrolled loops wait for.)
+#pragma unroll 1
+        for (int c = 0; c < 4; ++c) {
+          float2 e[16];
+          uint32_t pk[16];
+          arg_chunk(sa, P.scale_log2, neg_m, e);
+          if (c < 3) tmem_ld32(tS + 32 * c + 32, ua);
+          exp_chunk<T, kExact>(e, rs, pk);
+          tmem_st16(tS + 16 * c, pk);
+          tmem_wait_ld32(ua);
+        }
+        const float2 r = fadd2(fadd2(rs[0], rs[1]), fadd2(rs[2], rs[3]));
+        l_part += r.x + r.y;
+        if (resc) {
+          // O holds the products up to tile it-1: wait for the last of them, then scale this warp's 32 rows
+          ok = warp_wait(bar(T3_PV_DONE0 + ((it - 1) % kBufs)), ((it - 1) / kBufs) & 1, abort_flag, P.err, 622);
+          if (!ok) break;
+          tc_fence_after();
+#pragma unroll 1
+          for (int c = 0; c < 128; c += 32) {
+            uint32_t o[32];
+            tmem_ld32(tO + lane_base + c, o);
+            tmem_wait_ld32(o);
 #pragma unroll
-            for (int r = 0; r < 2; ++r) {
-              c_lo[r] = jlo[r] - jt;
-              c_hi[r] = (jhi[r] < R.lim ? jhi[r] : R.lim) - jt;
-            }
-            if (!(c_lo[0] <= 0 && c_hi[0] >= kTile - 1 && c_lo[1] <= 0 && c_hi[1] >= kTile - 1)) {
-#pragma unroll
-              for (int i = 0; i < 64; ++i) {
-                const int col = 8 * (i >> 2) + cq + (i & 1), r = (i >> 1) & 1;
-                s[i] = (col >= c_lo[r] && col <= c_hi[r]) ? s[i] : -INFINITY;
-              }
-            }
-            float mxa[2] = {-INFINITY, -INFINITY}, mxb[2] = {-INFINITY, -INFINITY};
-#pragma unroll
-            for (int j = 0; j < 16; j += 2) {
-              mxa[0] = fmax3(mxa[0], s[4 * j], s[4 * j + 1]);
-              mxa[1] = fmax3(mxa[1], s[4 * j + 2], s[4 * j + 3]);
-              mxb[0] = fmax3(mxb[0], s[4 * j + 4], s[4 * j + 5]);
-              mxb[1] = fmax3(mxb[1], s[4 * j + 6], s[4 * j + 7]);
-            }
-            float alpha[2] = {1.f, 1.f}, neg_m[2];
-            bool resc = false;
-#pragma unroll
-            for (int r = 0; r < 2; ++r) {
-              float mx = fmaxf(mxa[r], mxb[r]);
-              mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-              mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2)) * P.scale_log2;
-              // lazy rescaling: the reference maximum only moves when the row maximum grew by more than 2^8 - or, kExact, at
-              // all, so that the largest probabilities of a row are the ones that a 16-bit P holds without a rounding
-              if (mx > m_ref[r]) {
-                if (m_ref[r] == -INFINITY) {
-                  m_ref[r] = mx;  // nothing accumulated for this row yet
-                } else if (mx - m_ref[r] > (kExact ? 0.f : 8.f)) {
-                  alpha[r] = ex2_approx(m_ref[r] - mx);
-                  l_part[r] *= alpha[r];
-                  m_ref[r] = mx;
-                  resc = true;
-                }
-              }
-              neg_m[r] = m_ref[r] == -INFINITY ? 0.f : -m_ref[r];
-            }
-            uint32_t pk[32];
-            float2 rs[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-            const float2 sc2 = make_float2(P.scale_log2, P.scale_log2);
-            const float2 nm2[2] = {make_float2(neg_m[0], neg_m[0]), make_float2(neg_m[1], neg_m[1])};
-#pragma unroll
-            for (int k = 0; k < 32; ++k) {  // pair k: block k/2, row k%2 - which is where the 16x128b store wants it
-              const int r = k & 1;
-              const float2 a = ffma2(s[2 * k], s[2 * k + 1], sc2, nm2[r]);
-              float2 p;
-              if ((k % kPolyEvery) == kPolyEvery - 1) {
-                p = ex2_poly2<kExact ? 5 : 3>(a);  // one pair in kPolyEvery off the special-function unit
-              } else {
-                p = make_float2(ex2_approx(a.x), ex2_approx(a.y));
-              }
-              rs[r] = fadd2(rs[r], p);
-              typename Act<T>::T2 v = Act<T>::from_f2(p.x, p.y);
-              pk[k] = *reinterpret_cast<uint32_t*>(&v);
-            }
-            l_part[0] += rs[0].x + rs[0].y;
-            l_part[1] += rs[1].x + rs[1].y;
-            if (__any_sync(0xffffffffu, resc) && it >= 1) {
-              // O holds the products up to tile it-1: wait for the last of them, then scale this warp's 16 rows
-              ok = __all_sync(0xffffffffu, wait_or_abort(bar(T3_PV_DONE0 + ((it - 1) % 3)), ((it - 1) / 3) & 1, abort_flag,
-                                                         P.err, 622));
-              if (!ok) break;
-              tc_fence_after();
-              uint32_t o[64];
-              tmem_ld_16x256b_x16(tO + lane_base, o);
-              tmem_wait_ld();
-#pragma unroll
-              for (int i = 0; i < 64; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha[(i >> 1) & 1]);
-              tmem_st_16x256b_x16(tO + lane_base, o);
-            }
-            // P, packed, over the first 64 columns of the S buffer: column c holds keys 2c, 2c+1
-            tmem_st_16x128b_x16(tS, pk);
-            tmem_wait_st();
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(bar(T3_P_FULL0 + b3));  // per warp: 256 arrivals on one word took turns
+            for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+            tmem_st32(tO + lane_base + c, o);
           }
         }
+        tmem_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) {  // per warp: arrivals on one word take turns
+          if (kPair) mbar_arrive_cluster(p_full + 8u * (uint32_t)b3);
+          else mbar_arrive(p_full + 8u * (uint32_t)b3);
+        }
       }
+      it0 += R.n;
     }
-    // ---- epilogue: row sums and reference maxima go through shared memory to the thread-per-row layout, in which
-    // each warp writes 64 output columns of 32 rows
-#pragma unroll
-    for (int r = 0; r < 2; ++r) {
-      float l = l_part[r];
-      l += __shfl_xor_sync(0xffffffffu, l, 1);
-      l += __shfl_xor_sync(0xffffffffu, l, 2);
-      if ((lane & 3) == 0) {
-        xsum[rbase + 8 * r] = l;
-        xmax[rbase + 8 * r] = m_ref[r];
-      }
-    }
+    // ---- epilogue: the teams' row sums come together; then every warp of the first two teams writes 64 output columns of
+    // 32 rows
+    xsum[team * kTile + row] = l_part;
+    xmax[team * kTile + row] = m_ref;
     asm volatile("bar.sync 1, 256;" ::: "memory");
-    const int half = warp >> 2, row = quad * 32 + lane, col0 = half * 64;
-    const int64_t qi = i0 + row;
-    const bool row_valid = qi < P.lq;
-    const uint32_t row_base = ((uint32_t)(quad * 32)) << 16;
-    const float l_sum = xsum[row], m_row = xmax[row];
+    const int half = team, col0 = half * 64;
+    const uint32_t row_base = lane_base;
+    const int it = n_tiles;
+    const float m_row = it >= 1 ? xmax[((it - 1) & 1) * kTile + row] : -INFINITY;
+    float l_sum = 0.f;
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const float m = xmax[e * kTile + row], l = xsum[e * kTile + row];
+      l_sum += m == m_row ? l : l * ex2_approx(m - m_row);
+    }
     // Three ways out: a run of a split work item leaves its un-normalised partial; a stage of a multi-stage attention
     // leaves the state (acc, m, l); everything else is normalised.  A state that came in is folded in first.
     const int64_t srow = (int64_t)h * P.lq + qi;
@@ -606,7 +676,7 @@ __global__ void __launch_bounds__(352, 1) attn_tc3_kernel(const __grid_constant_
       }
       asm volatile("bar.sync 1, 256;" ::: "memory");  // both halves of a row have read (m, l): they may be overwritten
     }
-    if (ok && it >= 1) ok = __all_sync(0xffffffffu, wait_or_abort(bar(T3_O_FULL), 0, abort_flag, P.err, 624));
+    if (ok && it >= 1) ok = warp_wait(bar(T3_O_FULL), 0, abort_flag, P.err, 624);
     if (ok) {
       tc_fence_after();
       const bool raw = P.part_acc != nullptr;
@@ -699,7 +769,8 @@ __global__ void __launch_bounds__(352, 1) attn_tc3_kernel(const __grid_constant_
   // ---- teardown
   tc_fence_before();
   __syncthreads();
-  if (warp == 9) tmem_dealloc(tmem, 512);
+  if (kPair) cluster_sync();  // nothing is signalled in a CTA that has gone
+  if (warp == kWarpPv) tmem_dealloc<kPair>(tmem, 512);
 }
 
 // Merge of n_split partials (acc, m, l) per row, and of a state that came in (st_*, may be null): the sum of
@@ -834,13 +905,11 @@ __global__ void __launch_bounds__(colsum_smem::kThreads, 1) colsum_tc_kernel(con
   const bool any = q_last >= q_first;
   auto load_q = [&](int t) {
     mbar_expect_tx(bar(QF + t), 2 * kSubTileBytes);
-    tma_load_3d(sQ + t * 2 * kSubTileBytes, &P.map_q, bar(QF + t), 0, P.q_row0 + t * kTile, h);
-    tma_load_3d(sQ + t * 2 * kSubTileBytes + kSubTileBytes, &P.map_q, bar(QF + t), 64, P.q_row0 + t * kTile, h);
+    tma_load_4d(sQ + t * 2 * kSubTileBytes, &P.map_q, bar(QF + t), 0, P.q_row0 + t * kTile, 0, h);
   };
   auto load_k = [&](int b, int j0) {
     mbar_expect_tx(bar(KF + b), 2 * kSubTileBytes);
-    tma_load_3d(sK + b * 2 * kSubTileBytes, &P.map_k, bar(KF + b), 0, P.k_tok0 + j0, hkv);
-    tma_load_3d(sK + b * 2 * kSubTileBytes + kSubTileBytes, &P.map_k, bar(KF + b), 64, P.k_tok0 + j0, hkv);
+    tma_load_4d(sK + b * 2 * kSubTileBytes, &P.map_k, bar(KF + b), 0, P.k_tok0 + j0, 0, hkv);
   };
   if (warp == 16 && lane == 0) {
     for (int i = 0; i < 2; ++i) {
@@ -981,7 +1050,7 @@ __global__ void __launch_bounds__(colsum_smem::kThreads, 1) colsum_tc_kernel(con
       float total = 0.f;
       for (int t = tf; t <= tl && ok; ++t, ++step) {
         if ((step % NB) != part) continue;
-        ok = __all_sync(0xffffffffu, wait_or_abort(bar(SF + part), (step / NB) & 1, abort_flag, P.err, 414));
+        ok = warp_wait(bar(SF + part), (step / NB) & 1, abort_flag, P.err, 414);
         if (!ok) break;
         tc_fence_after();
         const int q_end = (int)P.lq - 1 - t * kTile, c_lo = vi_lo - t * kTile,
@@ -1083,12 +1152,13 @@ int encode_tensor_map(CUtensorMap* map, int dtype, const void* base, int rank, c
   return INFLLM_OK;
 }
 
-// rows of `D`=128 elements: (D, rows, heads) view of a (heads, rows, D) tensor with element strides hs / ts
-int encode_rows_map(CUtensorMap* map, int dtype, const void* base, int64_t rows, int64_t heads, int64_t hs, int64_t ts) {
-  uint64_t dims[3] = {128, (uint64_t)rows, (uint64_t)heads};
-  uint64_t strides[2] = {(uint64_t)ts * 2, (uint64_t)hs * 2};
-  uint32_t box[3] = {64, 128, 1};
-  return encode_tensor_map(map, dtype, base, 3, dims, strides, box);
+// rows of 128 elements as (64, rows, 2, heads): a box of `box_rows` rows and one or both halves of the dimensions lands as
+// one or two 128-byte-swizzled tiles, one behind the other
+int encode_rows_map(CUtensorMap* map, int dtype, const void* base, int64_t rows, int64_t heads, int64_t hs, int64_t ts, TcBox bx) {
+  uint64_t dims[4] = {64, (uint64_t)rows, 2, (uint64_t)heads};
+  uint64_t strides[3] = {(uint64_t)ts * 2, 128, (uint64_t)hs * 2};
+  uint32_t box[4] = {64, bx.rows, bx.halves, 1};
+  return encode_tensor_map(map, dtype, base, 4, dims, strides, box);
 }
 
 bool tc_rows_ok(const void* base, int64_t hs, int64_t ts) {
@@ -1137,17 +1207,31 @@ int attn_tc3_splits(int64_t lq, int n_heads, int64_t keys) {
   return best;
 }
 
+bool attn_tc3_pairs(int64_t lq, int n_heads, int n_kv_heads) { return ceil_div(lq, kTile) * (n_heads / n_kv_heads) % 2 == 0; }
+
 int attn_tc3_launch(const AttnTcParams& P, int dtype, cudaStream_t s) {
   if (P.lq <= 0) return INFLLM_OK;
   if (P.n_split < 1 || (P.n_split > 1 && (!P.part_acc || !P.part_m || !P.part_l || P.st_acc)))
     return fail(INFLLM_E_BADARG, "attn_tc3: split %d without partial buffers", P.n_split);
-  dim3 grid((unsigned)ceil_div(P.lq, kTile), P.n_heads, P.n_split);
+  const int items = (int)ceil_div(P.lq, kTile) * (P.n_heads / P.n_kv_heads);
+  const bool pair = attn_tc3_pairs(P.lq, P.n_heads, P.n_kv_heads);
   const size_t smem = tc3::kTotal + 1024;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)items, P.n_kv_heads, P.n_split);
+  cfg.blockDim = dim3(tc3::kThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = 2, at[0].val.clusterDim.y = 1, at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = pair ? 1 : 0;
   INFLLM_DISPATCH_DTYPE(dtype, T, {
-    auto kern = P.exact ? attn_tc3_kernel<T, true> : attn_tc3_kernel<T, false>;
+    auto kern = pair ? (P.exact ? attn_tc3_kernel<T, true, true> : attn_tc3_kernel<T, false, true>)
+                     : (P.exact ? attn_tc3_kernel<T, true, false> : attn_tc3_kernel<T, false, false>);
     // the opt-in holds for the current device only, and a process may drive several: asked for at every launch
     INFLLM_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kern<<<grid, 352, smem, s>>>(P);
+    INFLLM_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, P));
   });
   INFLLM_LAUNCH_OK("attn_tc3_kernel");
   return INFLLM_OK;
@@ -1195,8 +1279,8 @@ int colsum_tc_launch(const void* q, int64_t q_hs, int64_t q_ts, const void* k, i
                      int n_kv_heads, int64_t lq, int64_t lk, int mask_mode, int64_t mask_offset, int64_t mask_size,
                      const float* lse, float* score, int64_t score_hs, int accumulate, int dtype, cudaStream_t s) {
   CUtensorMap mq, mk;
-  INFLLM_TRY(encode_rows_map(&mq, dtype, q, lq, n_heads, q_hs, q_ts));
-  INFLLM_TRY(encode_rows_map(&mk, dtype, k, lk, n_kv_heads, k_hs, k_ts));
+  INFLLM_TRY(encode_rows_map(&mq, dtype, q, lq, n_heads, q_hs, q_ts, kBoxTile));
+  INFLLM_TRY(encode_rows_map(&mk, dtype, k, lk, n_kv_heads, k_hs, k_ts, kBoxTile));
   return colsum_tc_launch_maps(mq, mk, 0, 0, n_heads, n_kv_heads, lq, lk, mask_mode, mask_offset, mask_size, lse, score,
                                score_hs, accumulate, false, dtype, s);
 }

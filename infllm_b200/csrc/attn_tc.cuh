@@ -7,6 +7,14 @@ namespace infllm {
 
 constexpr int kTcMaxMaps = 12;
 constexpr int kTile = 128;
+// boxes of the tensor maps: rows, and halves of the 128 dimensions
+struct TcBox {
+  uint32_t rows, halves;
+};
+constexpr TcBox kBoxTile = {kTile, 2};  // a whole tile: queries, and keys and values of a CTA that works alone
+constexpr TcBox kBoxPairK = {kTile / 2, 2}, kBoxPairV = {kTile, 1};  // a CTA's share of a pair's keys and values
+constexpr TcBox box_k(bool pair) { return pair ? kBoxPairK : kBoxTile; }
+constexpr TcBox box_v(bool pair) { return pair ? kBoxPairV : kBoxTile; }
 // Exec blocks of up to one tile of queries are attended to in fp32's precision throughout, like every stage of the
 // multi-stage class and the sink + window types.  Up to 64 queries they used to be the shape-generic kernel's, which does;
 // up to 128 their key tiles are cut into runs, and where a row is one key's for the most part it matters which tiles share
@@ -18,7 +26,7 @@ constexpr int kExactQueries = kTile;
 struct TcSeg {
   int16_t map_k, map_v;  // indices into AttnTcParams::maps
   int32_t tok0;          // token coordinate of the segment's first key
-  int32_t c3_k, c3_v;    // 4th coordinate for rank-4 maps (cache slots), -1 for rank-3 maps
+  int32_t c3_k, c3_v;    // 5th coordinate for rank-5 maps (cache slots), -1 for rank-4 maps
   int32_t len;
 };
 
@@ -66,12 +74,15 @@ struct ColsumTcParams {
 };
 
 
-int encode_rows_map(CUtensorMap* map, int dtype, const void* base, int64_t rows, int64_t heads, int64_t hs, int64_t ts);
+int encode_rows_map(CUtensorMap* map, int dtype, const void* base, int64_t rows, int64_t heads, int64_t hs, int64_t ts,
+                    TcBox box);
 bool tc_rows_ok(const void* base, int64_t hs, int64_t ts);
 int tc_get_error_ptr(int** p);
 // one CTA per (128-query tile, head)
 int attn_tc3_launch(const AttnTcParams& P, int dtype, cudaStream_t s);
 int attn_tc3_splits(int64_t lq, int n_heads, int64_t keys);
+// whether a launch of these sizes runs in pairs of CTAs: its maps of keys and values have the boxes of one
+bool attn_tc3_pairs(int64_t lq, int n_heads, int n_kv_heads);
 int attn_tc_combine_launch(const float* acc, const float* m, const float* l, int n_split, int n_heads, int64_t lq, void* out,
                            int64_t o_hs, int64_t o_ts, float* lse, const float* st_acc, const float* st_m,
                            const float* st_l, float* new_acc, float* new_m, float* new_l, int dtype, cudaStream_t s);

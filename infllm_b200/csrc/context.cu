@@ -311,7 +311,10 @@ struct infllm_ctx {
   // tensor-core path: tensor maps of the buffers the kernels read through TMA
   bool use_tc = false;
   int64_t init_cap = 0;  // rows allocated for the sink buffers (at least one 128-row tile)
-  CUtensorMap m_qloc, m_qglb, m_krot, m_kraw, m_v, m_cache, m_initk, m_initv;
+  CUtensorMap m_qloc, m_qglb;
+  struct KvMaps {
+    CUtensorMap krot, kraw, v, cache_k, cache_v, initk, initv;
+  } m_kv[2];  // with the boxes of CTAs that work alone and in pairs (attn_tc3_pairs)
   int* tc_err = nullptr;
   // The tensor-core kernels record a bounded wait that ran out in a device-side record; a copy of it travels to
   // h_tc_err with the candidate scores of every exec block and at the end of every call, and the host reads it
@@ -653,16 +656,19 @@ int lazy_init(infllm_ctx* c, cudaStream_t s) {
   INFLLM_CUDA_OK(cudaMemsetAsync(c->cache, 0, n_slots * c->unit_bytes, s));
   c->use_tc = D == 128 && g.block_size % 128 == 0 && !(g.debug_flags & 1);
   if (c->use_tc) {
-    INFLLM_TRY(encode_rows_map(&c->m_qloc, g.dtype, c->q_loc, c->sub_max, H, c->sub_max * D, D));
-    INFLLM_TRY(encode_rows_map(&c->m_qglb, g.dtype, c->q_glb, c->sub_max, H, c->sub_max * D, D));
-    INFLLM_TRY(encode_rows_map(&c->m_initk, g.dtype, c->init_k, c->init_cap, HKV, c->init_cap * D, D));
-    INFLLM_TRY(encode_rows_map(&c->m_initv, g.dtype, c->init_v, c->init_cap, HKV, c->init_cap * D, D));
-    // cache slots as (D, block_size, H_kv, 2 * slots): the last index is slot * 2 + (0 keys | 1 values)
-    uint64_t dims[4] = {128, (uint64_t)g.block_size, (uint64_t)HKV, 2ull * (uint64_t)n_slots};
-    uint64_t strides[3] = {(uint64_t)(D * c->esz), (uint64_t)(g.block_size * D * c->esz),
-                           (uint64_t)(c->unit_bytes / 2)};
-    uint32_t box[4] = {64, 128, 1, 1};
-    INFLLM_TRY(encode_tensor_map(&c->m_cache, g.dtype, c->cache, 4, dims, strides, box));
+    INFLLM_TRY(encode_rows_map(&c->m_qloc, g.dtype, c->q_loc, c->sub_max, H, c->sub_max * D, D, kBoxTile));
+    INFLLM_TRY(encode_rows_map(&c->m_qglb, g.dtype, c->q_glb, c->sub_max, H, c->sub_max * D, D, kBoxTile));
+    // cache slots as (64, block_size, 2, H_kv, 2 * slots): the last index is slot * 2 + (0 keys | 1 values)
+    uint64_t dims[5] = {64, (uint64_t)g.block_size, 2, (uint64_t)HKV, 2ull * (uint64_t)n_slots};
+    uint64_t strides[4] = {(uint64_t)(D * c->esz), 128, (uint64_t)(g.block_size * D * c->esz), (uint64_t)(c->unit_bytes / 2)};
+    for (int pair = 0; pair < 2; ++pair) {
+      infllm_ctx::KvMaps& m = c->m_kv[pair];
+      INFLLM_TRY(encode_rows_map(&m.initk, g.dtype, c->init_k, c->init_cap, HKV, c->init_cap * D, D, box_k(pair)));
+      INFLLM_TRY(encode_rows_map(&m.initv, g.dtype, c->init_v, c->init_cap, HKV, c->init_cap * D, D, box_v(pair)));
+      uint32_t bk[5] = {64, box_k(pair).rows, box_k(pair).halves, 1, 1}, bv[5] = {64, box_v(pair).rows, box_v(pair).halves, 1, 1};
+      INFLLM_TRY(encode_tensor_map(&m.cache_k, g.dtype, c->cache, 5, dims, strides, bk));
+      INFLLM_TRY(encode_tensor_map(&m.cache_v, g.dtype, c->cache, 5, dims, strides, bv));
+    }
     INFLLM_TRY(tc_get_error_ptr(&c->tc_err));
     INFLLM_CUDA_OK(cudaHostAlloc((void**)&c->h_tc_err, 4 * sizeof(int32_t), cudaHostAllocDefault));
     c->h_tc_err[0] = c->h_tc_err[1] = c->h_tc_err[2] = c->h_tc_err[3] = 0;
@@ -771,9 +777,12 @@ int ensure_tokens(infllm_ctx* c, int64_t add, cudaStream_t s) {
   }
   c->tb = nb;
   if (c->use_tc) {
-    INFLLM_TRY(encode_rows_map(&c->m_krot, g.dtype, nb.k_rot, nb.cap, HKV, nb.cap * D, D));
-    INFLLM_TRY(encode_rows_map(&c->m_kraw, g.dtype, nb.k_raw, nb.cap, HKV, nb.cap * D, D));
-    INFLLM_TRY(encode_rows_map(&c->m_v, g.dtype, nb.v, nb.cap, HKV, nb.cap * D, D));
+    for (int pair = 0; pair < 2; ++pair) {
+      infllm_ctx::KvMaps& m = c->m_kv[pair];
+      INFLLM_TRY(encode_rows_map(&m.krot, g.dtype, nb.k_rot, nb.cap, HKV, nb.cap * D, D, box_k(pair)));
+      INFLLM_TRY(encode_rows_map(&m.kraw, g.dtype, nb.k_raw, nb.cap, HKV, nb.cap * D, D, box_k(pair)));
+      INFLLM_TRY(encode_rows_map(&m.v, g.dtype, nb.v, nb.cap, HKV, nb.cap * D, D, box_v(pair)));
+    }
   }
   return INFLLM_OK;
 }
@@ -1700,7 +1709,7 @@ int local_scores(infllm_ctx* c, cudaStream_t s, int64_t st, int64_t ks, int64_t 
   const int64_t n = j_end - j_begin, tok = ks - tb.t0 + j_begin, off = (lk - lq) - j_begin;
   ProfScope ps(c, s, INFLLM_PROF_COLSUM, work);
   if (c->use_tc && lq > 1 && lq <= 512)
-    return colsum_tc_launch_maps(c->m_qloc, c->m_krot, (int)st, (int)tok, (int)H, (int)HKV, lq, n, INFLLM_MASK_WINDOW,
+    return colsum_tc_launch_maps(c->m_qloc, c->m_kv[0].krot, (int)st, (int)tok, (int)H, (int)HKV, lq, n, INFLLM_MASK_WINDOW,
                                  off, g.n_local, c->lse, tb.score + tok, tb.cap, 1, late_wait, g.dtype, s);
   return attn_colsum_launch((const char*)c->q_loc + st * D * c->esz, c->sub_max * D, D,
                             (char*)tb.k_rot + tok * D * c->esz, tb.cap * D, D, (int)H, (int)HKV, lq, n, (int)D,
@@ -2121,8 +2130,9 @@ int append_sub(infllm_ctx* c, const char* q, int64_t q_hs, int64_t q_ts, const c
       const bool tc_now = c->use_tc && lq > 1 && gsegs.size() + 1 <= (size_t)kMaxSeg && tc_rows_ok(out_eb, o_hs, o_ts);
       if (tc_now) {
         AttnTcParams TP{};
-        TP.maps[0] = c->m_qloc; TP.maps[1] = c->m_qglb; TP.maps[2] = c->m_krot; TP.maps[3] = c->m_kraw;
-        TP.maps[4] = c->m_v; TP.maps[5] = c->m_cache; TP.maps[6] = c->m_initk; TP.maps[7] = c->m_initv;
+        const infllm_ctx::KvMaps& m = c->m_kv[attn_tc3_pairs(lq, (int)H, (int)HKV)];
+        TP.maps[0] = c->m_qloc; TP.maps[1] = c->m_qglb; TP.maps[2] = m.krot; TP.maps[3] = m.kraw; TP.maps[4] = m.v;
+        TP.maps[5] = m.cache_k; TP.maps[6] = m.cache_v; TP.maps[7] = m.initk; TP.maps[8] = m.initv;
         TP.n_stage = 2; TP.n_heads = (int)H; TP.n_kv_heads = (int)HKV; TP.lq = lq;
         TP.out = out_eb; TP.o_hs = o_hs; TP.o_ts = o_ts; TP.lse = c->lse;
         TP.scale_log2 = kLog2e / sqrtf((float)D); TP.err = c->tc_err;
@@ -2135,9 +2145,9 @@ int append_sub(infllm_ctx* c, const char* q, int64_t q_hs, int64_t q_ts, const c
         // (query, key) pair visible (context_manager.py:437); the stage is therefore unmasked.
         for (int32_t b : ids) {
           const int slot = c->slot_of[b];
-          TP.seg[ns++] = {5, 5, 0, slot * 2, slot * 2 + 1, (int32_t)bs};
+          TP.seg[ns++] = {5, 6, 0, slot * 2, slot * 2 + 1, (int32_t)bs};
         }
-        if (c->init_len > 0) TP.seg[ns++] = {6, 7, 0, -1, -1, (int32_t)c->init_len};
+        if (c->init_len > 0) TP.seg[ns++] = {7, 8, 0, -1, -1, (int32_t)c->init_len};
         if (ovf > 0) TP.seg[ns++] = {3, 4, (int32_t)(c->frontier - tb.t0), -1, -1, (int32_t)ovf};
         TP.stage[1].map_q = 1; TP.stage[1].q_row0 = (int)st; TP.stage[1].mask_mode = INFLLM_MASK_NONE;
         TP.stage[1].lk = (int64_t)all_glk; TP.stage[1].seg_begin = 1; TP.stage[1].seg_end = ns;

@@ -212,9 +212,10 @@ extern "C" int infllm_sink_window_run(const infllm_sink_window* args, void* stre
     return lse_merge_launch(part, plse, n, a.n_heads, 128, a.d_out, a.o_hs, nullptr, a.dtype, s, nullptr, 0, nullptr, 0, nullptr);
   }
   AttnTcParams A{};
-  INFLLM_TRY(encode_rows_map(&A.maps[0], a.dtype, P.q_loc, a.len_q, a.n_heads, a.len_q * 128, 128));
-  INFLLM_TRY(encode_rows_map(&A.maps[1], a.dtype, P.k_rot, p.rows_w, a.n_kv_heads, p.rows_w * 128, 128));
-  INFLLM_TRY(encode_rows_map(&A.maps[2], a.dtype, v_base, p.rows_w, a.n_kv_heads, v_hs, 128));
+  const bool pair = attn_tc3_pairs(a.len_q, a.n_heads, a.n_kv_heads);
+  INFLLM_TRY(encode_rows_map(&A.maps[0], a.dtype, P.q_loc, a.len_q, a.n_heads, a.len_q * 128, 128, kBoxTile));
+  INFLLM_TRY(encode_rows_map(&A.maps[1], a.dtype, P.k_rot, p.rows_w, a.n_kv_heads, p.rows_w * 128, 128, box_k(pair)));
+  INFLLM_TRY(encode_rows_map(&A.maps[2], a.dtype, v_base, p.rows_w, a.n_kv_heads, v_hs, 128, box_v(pair)));
   INFLLM_TRY(tc_get_error_ptr(&A.err));
   A.exact = 1;
   A.n_stage = 1; A.n_heads = a.n_heads; A.n_kv_heads = a.n_kv_heads; A.lq = a.len_q;
@@ -222,9 +223,9 @@ extern "C" int infllm_sink_window_run(const infllm_sink_window* args, void* stre
   A.stage[0] = {0, 0, INFLLM_MASK_WINDOW, 0, 1, 0, p.lw - a.len_q, a.n_local, p.lw};
   A.seg[0] = {1, 2, 0, -1, -1, (int32_t)p.lw};
   if (p.n_snk > 0) {
-    INFLLM_TRY(encode_rows_map(&A.maps[3], a.dtype, P.q_snk, a.len_q, a.n_heads, a.len_q * 128, 128));
-    INFLLM_TRY(encode_rows_map(&A.maps[4], a.dtype, P.snk_k, p.n_snk, a.n_kv_heads, p.n_snk * 128, 128));
-    INFLLM_TRY(encode_rows_map(&A.maps[5], a.dtype, P.snk_v, p.n_snk, a.n_kv_heads, p.n_snk * 128, 128));
+    INFLLM_TRY(encode_rows_map(&A.maps[3], a.dtype, P.q_snk, a.len_q, a.n_heads, a.len_q * 128, 128, kBoxTile));
+    INFLLM_TRY(encode_rows_map(&A.maps[4], a.dtype, P.snk_k, p.n_snk, a.n_kv_heads, p.n_snk * 128, 128, box_k(pair)));
+    INFLLM_TRY(encode_rows_map(&A.maps[5], a.dtype, P.snk_v, p.n_snk, a.n_kv_heads, p.n_snk * 128, 128, box_v(pair)));
     A.stage[1] = {3, 0, INFLLM_MASK_COMPLEMENT, 1, 2, 0, snk_off, a.n_local, p.n_snk};
     A.seg[1] = {4, 5, 0, -1, -1, (int32_t)p.n_snk};
     A.n_stage = 2;
