@@ -827,14 +827,16 @@ __global__ void attn_tc_combine_kernel(const float* __restrict__ acc, const floa
 // four of the sixteen compute warps of its own, which turn it into sum_q exp2(s - lse_q).  A key tile is loaded once
 // per head and a query tile once per CTA, which keeps the L2 traffic an order of magnitude below one load per pair.
 // Bound: 16384 exponentials per pair, 768 cycles of the special-function unit with every fourth pair of them as a
-// quartic on the FMA pipe (a quintic, kExact, for exec blocks of one query tile), and the product, 514; a pair takes 1150.  512 queries x 32 heads over 4608 keys: 30.7 us.
-// (37.6 us with one issuing thread and all sixteen warps on one buffer at a time, whose exponentials were two at a
-// time in fp16: 1.4e-3 off in a sum, now 1e-6.)
+// quartic on the FMA pipe (a quintic, kExact, for exec blocks of one query tile), and the product, 514; a pair takes 1330 (the
+// special-function unit is busy for 54 % of the time, the schedulers for 56 %: what is waited for is latencies, and the
+// log-sum-exps out of shared memory share a queue with the exponentials).  512 queries x 32 heads over 4608 keys: 29.6 us, 37
+// over 4133: 10.8 (issued by lone threads: 30.2, 12.1).  Products of 64 queries, two buffers per group: 34.9 (half as many
+// columns are not half a product); two groups with two buffers each: 36.2.
 namespace colsum_smem {
 constexpr int kQTiles = 4;                     // resident query tiles
 constexpr int kMaxKeyTiles = 10;               // key tiles per CTA
 constexpr int kBufs = 4;                       // TMEM accumulators in flight
-constexpr int kIssuers = 2;                    // threads that issue products (a divisor of kBufs)
+constexpr int kIssuers = 2;                    // warps that issue products (a divisor of kBufs)
 constexpr int kThreads = (16 + 1 + kIssuers) * 32;
 constexpr int kQ = 0;
 constexpr int kK = kQ + kQTiles * 2 * kSubTileBytes;   // two stages
@@ -989,12 +991,13 @@ __global__ void __launch_bounds__(colsum_smem::kThreads, 1) colsum_tc_kernel(con
     }
   } else if (warp > 16) {
     // ====================================================================================== MMA issuers
-    // Two threads take the products in turn.  A product keeps the pipe busy for 514 cycles and the thread that issues
-    // it for 1385 (waits that are already over cost 200 cycles each, the eight instructions leave at the pipe's pace,
-    // then the commit): one thread for all of them was what the whole kernel waited for.  A TMEM buffer always has the
-    // same issuer, which therefore never gets a whole turn ahead of the buffer's phases.
-    if (lane == 0 && any) {
+    // Two warps take the products in turn, one lane of each issues (see attn_tc3_kernel); a thread of its own took 1385 cycles
+    // for a product, of which the pipe is busy for 514.  A TMEM buffer always has the same issuer, which therefore never
+    // gets a whole turn ahead of the buffer's phases.
+    if (any) {
       const int me = warp - 17;
+      const bool lead = elect_one();
+      const uint64_t kd0 = make_sdesc(sK, 16, 1024), qd0 = make_sdesc(sQ, 16, 1024);
       bool ok = true;
       int n = 0, step = 0, q_there = 0;
       for (int kt = kt0; kt < kt1 && ok; ++kt) {
@@ -1004,26 +1007,29 @@ __global__ void __launch_bounds__(colsum_smem::kThreads, 1) colsum_tc_kernel(con
         colsum_q_tiles(P, j0, keys, &tf, &tl);
         if (tl < tf) continue;
         const int kb = n & 1;
-        ok = wait_or_abort(bar(KF + kb), (n >> 1) & 1, abort_flag, P.err, 412);
-        const uint32_t kt_s = sK + kb * 2 * kSubTileBytes;
+        ok = warp_wait(bar(KF + kb), (n >> 1) & 1, abort_flag, P.err, 412);
         for (int t = tf; t <= tl && ok; ++t, ++step) {
           const int b = step % NB;
           if (b % colsum_smem::kIssuers != me) continue;
-          if (step >= NB) ok = wait_or_abort(bar(FR + b), ((step / NB) - 1) & 1, abort_flag, P.err, 413);
-          if (ok && !(q_there >> t & 1)) ok = wait_or_abort(bar(QF + t), 0, abort_flag, P.err, 411);
+          if (!(q_there >> t & 1)) ok = warp_wait(bar(QF + t), 0, abort_flag, P.err, 411);
           q_there |= 1 << t;
+          if (ok && step >= NB) ok = warp_wait(bar(FR + b), ((step / NB) - 1) & 1, abort_flag, P.err, 413);
           if (!ok) break;
           tc_fence_after();
-          const uint64_t ad = make_sdesc(kt_s, 16, 1024), bd = make_sdesc(sQ + t * 2 * kSubTileBytes, 16, 1024);
+          const uint64_t ad = kd0 + (uint64_t)(kb * 2 * kSubTileBytes >> 4), bd = qd0 + (uint64_t)(t * 2 * kSubTileBytes >> 4);
+          if (lead) {
 #pragma unroll
-          for (int ks = 0; ks < 8; ++ks) {
-            // S^T = K Q^T: keys are the M rows (TMEM lanes), queries the N columns
-            const uint64_t off = (uint64_t)(((ks >> 2) * kSubTileBytes + (ks & 3) * 32) >> 4);
-            mma_ss(tmem + b * 128, ad + off, bd + off, idesc, ks > 0);
+            for (int ks = 0; ks < 8; ++ks) {
+              // S^T = K Q^T: keys are the M rows (TMEM lanes), queries the N columns
+              const uint64_t off = (uint64_t)(((ks >> 2) * kSubTileBytes + (ks & 3) * 32) >> 4);
+              mma_ss(tmem + b * 128, ad + off, bd + off, idesc, ks > 0);
+            }
+            tc_commit(bar(SF + b));
           }
-          tc_commit(bar(SF + b));
+          __syncwarp();
         }
-        if (ok) tc_commit(bar(KE + kb));  // this thread's products with this key tile have been issued
+        if (ok && lead) tc_commit(bar(KE + kb));  // this warp's products with this key tile have been issued
+        __syncwarp();
         ++n;
       }
     }
