@@ -367,6 +367,7 @@ __global__ void __launch_bounds__(tc3::kThreads, 1) attn_tc3_kernel(const __grid
   __syncthreads();
   if (kPair) cluster_sync();  // the other CTA's barriers stand before anything is signalled on them
   tc_fence_after();
+  chain_wait();  // up to here nothing has been read or written that the kernel before on the stream has to do with
   const uint32_t tmem = *tmem_slot;
   const uint32_t tO = tmem + 384;  // three S/P buffers at columns [0,128), [128,256), [256,384)
   constexpr bool kBf16 = !std::is_same<T, __half>::value;
@@ -1227,11 +1228,13 @@ int attn_tc3_launch(const AttnTcParams& P, int dtype, cudaStream_t s) {
   cfg.blockDim = dim3(tc3::kThreads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = 2, at[0].val.clusterDim.y = 1, at[0].val.clusterDim.z = 1;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = 2, at[1].val.clusterDim.y = 1, at[1].val.clusterDim.z = 1;
   cfg.attrs = at;
-  cfg.numAttrs = pair ? 1 : 0;
+  cfg.numAttrs = pair ? 2 : 1;
   INFLLM_DISPATCH_DTYPE(dtype, T, {
     auto kern = pair ? (P.exact ? attn_tc3_kernel<T, true, true> : attn_tc3_kernel<T, false, true>)
                      : (P.exact ? attn_tc3_kernel<T, true, false> : attn_tc3_kernel<T, false, false>);
