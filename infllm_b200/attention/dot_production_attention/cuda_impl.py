@@ -53,29 +53,48 @@ class CudaMultiStageDotProductionAttention:
             k, v = k.contiguous(), v.contiguous()
         # (the strides of dimensions of one element are arbitrary, also behind contiguous())
         k_hs, k_ts = (k.stride(1) if hkv > 1 else max(lk, 1) * d), (k.stride(2) if lk > 1 else d)
-        stream = _lib.stream_ptr(self.device)
+        # addresses of a batch element's parts by arithmetic: a view of each cost 2 us, more than the whole launch
+        stream = _lib.raw_stream(self.device)
         lib, f32 = _lib.lib, torch.float32
         if get_score:
             self._scored.append(len(self._stages))
+        rows = h * lq
         if self._state is None and not end:
-            self._state = (torch.empty((b, h, lq, d), dtype=f32, device=self.device),
-                           torch.empty((2, b, h, lq), dtype=f32, device=self.device))
-        lse = None
+            self._state = torch.empty(b * rows * (d + 2), dtype=f32, device=self.device)
+        lse_at = None
         if end:
             self.ret = torch.empty(self.q_shape, dtype=self.dtype, device=self.device)
             lse = torch.empty((b, h, lq), dtype=f32, device=self.device) if self._scored else None
+            lse_at = lse.data_ptr() if lse is not None else None
         n_scratch = lib.infllm_attn_stage_scratch(h, hkv, lq, lk, d)
         scratch = torch.empty(n_scratch, dtype=f32, device=self.device) if n_scratch > 0 else None
-        out = self.ret
+        scratch_at = None if scratch is None else scratch.data_ptr()
+        q_at, q_bs = q.data_ptr(), 2 * q.stride(0)
+        k_at, v_at, k_bs = (k.data_ptr(), v.data_ptr(), 2 * k.stride(0)) if lk else (None, None, 0)
+        acc = m = l = o_at = None
+        if self._state is not None:
+            acc = self._state.data_ptr()
+            m = acc + 4 * b * rows * d
+            l = m + 4 * b * rows
+        if end:
+            o_at = self.ret.data_ptr()
         for bi in range(b):
-            acc, m, l = (None, None, None) if self._state is None else (
-                self._state[0][bi].data_ptr(), self._state[1][0, bi].data_ptr(), self._state[1][1, bi].data_ptr())
-            _lib.check(lib.infllm_attn_stage_ex(
-                q[bi].data_ptr(), q.stride(1), q.stride(2), k[bi].data_ptr() if lk else None, k_hs, k_ts,
-                v[bi].data_ptr() if lk else None, k_hs, k_ts, h, hkv, lq, lk, d, mode, off, size,
-                acc, m, l, int(self._first), None if scratch is None else scratch.data_ptr(), n_scratch,
-                out[bi].data_ptr() if end else None, out.stride(1) if end else 0, out.stride(2) if end else 0,
-                lse[bi].data_ptr() if lse is not None else None, self._code, stream))
+            rc = lib.infllm_attn_stage_ex(
+                q_at, q.stride(1), q.stride(2), k_at, k_hs, k_ts, v_at, k_hs, k_ts, h, hkv, lq, lk, d, mode, off, size,
+                acc, m, l, int(self._first), scratch_at, n_scratch, o_at, lq * d if end else 0, d if end else 0, lse_at,
+                self._code, stream)
+            if rc:
+                _lib.check(rc)
+            if bi + 1 < b:
+                q_at += q_bs
+                if lk:
+                    k_at, v_at = k_at + k_bs, v_at + k_bs
+                if acc is not None:
+                    acc, m, l = acc + 4 * rows * d, m + 4 * rows, l + 4 * rows
+                if end:
+                    o_at += 2 * rows * d
+                if lse_at is not None:
+                    lse_at += 4 * rows
         self._first = False
         self._stages.append((q, k, k_hs, k_ts, mode, off, size) if get_score else None)
         if end:
@@ -85,7 +104,7 @@ class CudaMultiStageDotProductionAttention:
         """The per-key scores of the stages that asked for them, from the final log-sum-exp of every row."""
         self.end = True
         b, h, lq, d = self.q_shape
-        stream = _lib.stream_ptr(self.device)
+        stream = _lib.raw_stream(self.device)
         for st in self._stages:
             if st is None:
                 self.score_list.append(None)
@@ -95,11 +114,15 @@ class CudaMultiStageDotProductionAttention:
             lk, hkv = k.size(2), k.size(1)
             # every column is written, unless there is nothing to sum
             score = (torch.empty if lq and lk else torch.zeros)((b, h, lk), dtype=torch.float32, device=self.device)
+            q_at, lse_at, score_at = q.data_ptr(), lse.data_ptr(), score.data_ptr()
+            k_at = k.data_ptr() if lk else None
             for bi in range(b):
-                _lib.check(_lib.lib.infllm_attn_colsum(
-                    q[bi].data_ptr(), q.stride(1), q.stride(2), k[bi].data_ptr() if lk else None, k_hs, k_ts, h, hkv,
-                    lq, lk, d, mode, off, size, lse[bi].data_ptr(), score[bi].data_ptr(),
-                    score.stride(1), 0, self._code, stream))
+                rc = _lib.lib.infllm_attn_colsum(
+                    q_at + 2 * bi * q.stride(0), q.stride(1), q.stride(2), k_at + 2 * bi * k.stride(0) if lk else None, k_hs, k_ts,
+                    h, hkv, lq, lk, d, mode, off, size, lse_at + 4 * bi * h * lq, score_at + 4 * bi * h * lk, lk, 0, self._code,
+                    stream)
+                if rc:
+                    _lib.check(rc)
             self.score_list_fp32.append(score)
             self.score_list.append(score.to(self.dtype))
         self._stages = []
