@@ -337,6 +337,12 @@ __global__ void __launch_bounds__(tc3::kThreads, 1) attn_tc3_kernel(const __grid
   const int rows_q = (int)((P.lq - i0) < kTile ? (P.lq - i0) : kTile);
   const int split = blockIdx.z;
 
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < T3_N_BARS; ++i) mbar_init(bar(i), i >= T3_P_FULL0 && i < T3_P_FULL0 + kBufs ? 4u * kCtas : 1u);
+    *abort_flag = 0;
+    mbar_fence_init();
+  }
+  if (kPair) cluster_arrive();  // (waited for below: the other CTA's barriers stand before anything is signalled on them)
   if (warp == kWarpQk && lane < P.n_stage) {  // the descriptors of the first loads are on their way while the run's parts are worked out
     const TcStage& S = P.stage[lane];
     tma_prefetch_map(&P.maps[S.map_q]);
@@ -354,18 +360,13 @@ __global__ void __launch_bounds__(tc3::kThreads, 1) attn_tc3_kernel(const __grid
     else make_plan<(kMaxSeg + 31) / 32>(P, u0, last, split, plan);
   }
 
-  if (threadIdx.x == 0) {
-    for (int i = 0; i < T3_N_BARS; ++i) mbar_init(bar(i), i >= T3_P_FULL0 && i < T3_P_FULL0 + kBufs ? 4u * kCtas : 1u);
-    *abort_flag = 0;
-    mbar_fence_init();
-  }
   if (warp == kWarpPv) {
     tmem_alloc<kPair>(smem_u32(tmem_slot), 512);
     tmem_relinquish<kPair>();
   }
   tc_fence_before();
   __syncthreads();
-  if (kPair) cluster_sync();  // the other CTA's barriers stand before anything is signalled on them
+  if (kPair) cluster_wait();
   tc_fence_after();
   chain_wait();  // up to here nothing has been read or written that the kernel before on the stream has to do with
   const uint32_t tmem = *tmem_slot;
@@ -559,10 +560,11 @@ __global__ void __launch_bounds__(tc3::kThreads, 1) attn_tc3_kernel(const __grid
           // a tile at an edge: what a row does not see is taken out of the scores where they are
 #pragma unroll 1
           for (int c = 0; c < kTile; c += 32) {
+            const int lo = c_lo - c, hi = c_hi - c;
+            if (__all_sync(0xffffffffu, lo <= 0 && hi >= 31)) continue;
             uint32_t u[32];
             tmem_ld32(tS + c, u);
             tmem_wait_ld32(u);
-            const int lo = c_lo - c, hi = c_hi - c;
 #pragma unroll
             for (int i = 0; i < 32; ++i) u[i] = i >= lo && i <= hi ? u[i] : 0xff800000u;
             tmem_st32(tS + c, u);
@@ -678,6 +680,7 @@ __global__ void __launch_bounds__(tc3::kThreads, 1) attn_tc3_kernel(const __grid
       asm volatile("bar.sync 1, 256;" ::: "memory");  // both halves of a row have read (m, l): they may be overwritten
     }
     if (ok && it >= 1) ok = warp_wait(bar(T3_O_FULL), 0, abort_flag, P.err, 624);
+    if (kPair) cluster_arrive();  // nothing more is signalled to or from this CTA (waited for at the end)
     if (ok) {
       tc_fence_after();
       const bool raw = P.part_acc != nullptr;
@@ -767,10 +770,11 @@ __global__ void __launch_bounds__(tc3::kThreads, 1) attn_tc3_kernel(const __grid
       }
     }
   }
+  if (kPair && warp >= 8) cluster_arrive();
   // ---- teardown
   tc_fence_before();
   __syncthreads();
-  if (kPair) cluster_sync();  // nothing is signalled in a CTA that has gone
+  if (kPair) cluster_wait();  // nothing is signalled in a CTA that has gone
   if (warp == kWarpPv) tmem_dealloc<kPair>(tmem, 512);
 }
 
