@@ -82,6 +82,11 @@ struct SealArgs {
   int32_t n_new, first_new, n_old, block_size, repr_topk, group, n_heads, head_dim, width;
   uint32_t seq;
 };
+__device__ __forceinline__ uint32_t float_key(float f) {
+  uint32_t u = __float_as_uint(f);
+  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);  // larger float <-> larger key
+}
+
 template <typename T>
 __global__ void __launch_bounds__(kSealThreads)
 seal_score_kernel(const __grid_constant__ SealArgs<T> A, const __grid_constant__ RowList list) {
@@ -102,32 +107,39 @@ seal_score_kernel(const __grid_constant__ SealArgs<T> A, const __grid_constant__
     const int64_t t0 = A.tok0 + (int64_t)b * A.block_size;
     T* row = A.bk + (int64_t)(A.first_new + b) * A.width;
     for (int h = warp; h < A.n_heads; h += 32) {
-      float v[kSealItems];
+      const int64_t at = (int64_t)h * A.head_dim + lane * vec;
+      float qb[4] = {0.f, 0.f, 0.f, 0.f};
+      if (A.qbar) {
 #pragma unroll
-      for (int i = 0; i < kSealItems; ++i)
-        v[i] = lane + 32 * i < A.block_size ? A.score[h * A.score_hs + t0 + lane + 32 * i] : -INFINITY;
+        for (int e = 0; e < 4; ++e)
+          if (e < vec) qb[e] = A.qbar[at + e];
+      }
+      uint32_t key[kSealItems];  // larger score <-> larger key; -inf and NaN are never picked: 0
+#pragma unroll
+      for (int i = 0; i < kSealItems; ++i) {
+        const float x = lane + 32 * i < A.block_size ? A.score[h * A.score_hs + t0 + lane + 32 * i] : -INFINITY;
+        key[i] = x > -INFINITY ? float_key(x + 0.f) : 0u;  // (-0 is 0)
+      }
       const T* kh = A.k + (int64_t)(h / A.group) * A.k_hs + t0 * A.k_ts + lane * vec;
       float acc[4] = {0.f, 0.f, 0.f, 0.f};
       for (int r0 = 0; r0 < A.repr_topk; r0 += 4) {
         int sel[4];
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
-          float bv = -INFINITY;
+          // the largest, of equals the first: one reduction over the keys, one over the places (a butterfly of both took 650 ns
+          // a round with 32 warps at it, of 6.2 us for the whole kernel; this takes 150)
+          uint32_t bk = 0;
           int bi = 0x7fffffff;
 #pragma unroll
           for (int i = 0; i < kSealItems; ++i)
-            if (v[i] > bv) bv = v[i], bi = lane + 32 * i;
-#pragma unroll
-          for (int o = 16; o > 0; o >>= 1) {
-            const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
-            const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-            if (ov > bv || (ov == bv && oi < bi)) bv = ov, bi = oi;
-          }
+            if (key[i] > bk) bk = key[i], bi = lane + 32 * i;
+          const uint32_t top = __reduce_max_sync(0xffffffffu, bk);
+          bi = (int)__reduce_min_sync(0xffffffffu, bk == top ? (uint32_t)bi : 0x7fffffffu);
           if (bi == 0x7fffffff) bi = 0;  // every remaining score is -inf or NaN
           sel[r] = bi;
 #pragma unroll
           for (int i = 0; i < kSealItems; ++i)
-            if (bi == lane + 32 * i) v[i] = -INFINITY;
+            if (bi == lane + 32 * i) key[i] = 0u;
         }
         uint2 raw[4];  // the rounds' rows, all on their way before the first is added
 #pragma unroll
@@ -145,14 +157,15 @@ seal_score_kernel(const __grid_constant__ SealArgs<T> A, const __grid_constant__
           for (int e = 0; e < 4; ++e) acc[e] += Act<T>::to_f(x[e]);
         }
       }
-      const int64_t at = (int64_t)h * A.head_dim + lane * vec;
       T o[4];
 #pragma unroll
       for (int e = 0; e < 4; ++e) o[e] = Act<T>::from_f(acc[e] / (float)A.repr_topk);
       if (vec == 4) *reinterpret_cast<uint2*>(row + at) = *reinterpret_cast<uint2*>(o);
       else *reinterpret_cast<uint32_t*>(row + at) = *reinterpret_cast<uint32_t*>(o);
       if (A.qbar) {
-        for (int e = 0; e < vec; ++e) dot = fmaf(Act<T>::to_f(o[e]), A.qbar[at + e], dot);
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (e < vec) dot = fmaf(Act<T>::to_f(o[e]), qb[e], dot);
       }
     }
   } else {  // kSealRows listed rows, eight warps to each
@@ -193,11 +206,6 @@ seal_score_kernel(const __grid_constant__ SealArgs<T> A, const __grid_constant__
     }
   }
   if (b >= A.n_new) chain_wait();  // whoever follows this kernel follows the one before it too
-}
-
-__device__ __forceinline__ uint32_t float_key(float f) {
-  uint32_t u = __float_as_uint(f);
-  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);  // larger float <-> larger key
 }
 
 constexpr int kTopkThreads = 1024;
