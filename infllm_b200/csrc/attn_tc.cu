@@ -629,22 +629,26 @@ __global__ void __launch_bounds__(tc3::kThreads, 1) attn_tc3_kernel(const __grid
           ok = warp_wait(bar(T3_PV_DONE0 + ((it - 1) % kBufs)), ((it - 1) / kBufs) & 1, abort_flag, P.err, 622);
           if (!ok) break;
           tc_fence_after();
-          // (all 128 columns at once: four rounds of 32, one behind the other, cost an attention with exact maxima 3 %: 4096 queries
-          // by 8192 keys 292.4 us, now 284.6)
-          uint32_t o[128];
-#pragma unroll
-          for (int c = 0; c < 128; c += 32) tmem_ld32(tO + lane_base + c, o + c);
-#pragma unroll
-          for (int c = 0; c < 128; c += 32) tmem_wait_ld32(o + c);
+          // kExact, where most tiles come here: all 128 columns at once (four rounds of 32, one behind the other: 292.4 us for 4096
+          // queries by 8192 keys, now 284.6)
+          constexpr int kRound = kExact ? 128 : 32;
           const float2 al = make_float2(alpha, alpha);
+#pragma unroll 1
+          for (int c0 = 0; c0 < 128; c0 += kRound) {
+            uint32_t o[kRound];
 #pragma unroll
-          for (int c = 0; c < 128; c += 32) {
+            for (int c = 0; c < kRound; c += 32) tmem_ld32(tO + lane_base + c0 + c, o + c);
 #pragma unroll
-            for (int i = c; i < c + 32; i += 2) {
-              const float2 x = fmul2(make_float2(__uint_as_float(o[i]), __uint_as_float(o[i + 1])), al);
-              o[i] = __float_as_uint(x.x), o[i + 1] = __float_as_uint(x.y);
+            for (int c = 0; c < kRound; c += 32) tmem_wait_ld32(o + c);
+#pragma unroll
+            for (int c = 0; c < kRound; c += 32) {
+#pragma unroll
+              for (int i = c; i < c + 32; i += 2) {
+                const float2 x = fmul2(make_float2(__uint_as_float(o[i]), __uint_as_float(o[i + 1])), al);
+                o[i] = __float_as_uint(x.x), o[i + 1] = __float_as_uint(x.y);
+              }
+              tmem_st32(tO + lane_base + c0 + c, o + c);
             }
-            tmem_st32(tO + lane_base + c, o + c);
           }
         }
         tmem_wait_st();
