@@ -1216,7 +1216,7 @@ int attn_tc_combine_launch(const float* acc, const float* m, const float* l, int
 }
 
 // Runs of key tiles per (128-query tile, head), as many as the SMs take at once and no more than pay: a run's tiles come one
-// after another, about 1.1 us each, and the partials cost a merge, two tiles' time for its launch and one more for every 40
+// after another, about 1.1 us each (0.92 in pairs of CTAs, where 4 runs of 32 items and 15 tiles, 16.9 us, and 8 of 12 and 24, 15.8, are still the best of 1 to 8), and the partials cost a merge, two tiles' time for its launch and one more for every 40
 // runs of the grid.  Measured over 4 to 60 tiles for 8 to 64 items (15 sizes each, bf16, both precisions, merge included): on
 // the average 0.7 % above the best count, 11 % at worst (6 tiles of 32 items: 16.5 us instead of 14.8).  At least seven tiles
 // to a run, which is what it was, is 13 % above it, 68 % at worst: 12 tiles of 8 items 24.2 us instead of 14.4.
