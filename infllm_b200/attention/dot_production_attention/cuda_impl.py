@@ -40,6 +40,8 @@ class CudaMultiStageDotProductionAttention:
                 raise TypeError(f"{n} dtype {t.dtype} != {self.dtype}")
         b, h, lq, d = self.q_shape
         hkv, lk = k.size(1), k.size(2)
+        if lk and (k.size(0) < b or v.size(0) < b):  # (addresses are worked out below: nothing else would notice)
+            raise IndexError(f"k and v have {k.size(0)} and {v.size(0)} batch elements, q has {b}")
         if sliding_window is None:
             mode, off, size = _lib.MASK_NONE, 0, 0
         else:
