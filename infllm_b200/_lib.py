@@ -235,6 +235,8 @@ def raw_stream(device):
     """The current stream's handle as an int (without building a Stream object: 3 us of a token's 15 on the host)."""
     import torch
 
+    if device.type != "cuda":  # (without an index it would be taken for the current CUDA device)
+        raise ValueError(f"a CUDA device is needed, got {device}")
     return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if device.index is None else device.index)
 
 

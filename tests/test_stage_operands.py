@@ -63,3 +63,15 @@ def test_a_stage_without_keys_has_no_batch_to_look_at(notes, monkeypatch):
     att = get_multi_stage_dot_production_attention(True)[0](q.shape, q.dtype, "cpu")
     att.append(q, _rand(1, 2, 0), _rand(1, 2, 0), end=True)
     assert len(notes.calls) == 2
+
+
+def test_a_class_made_for_another_device_than_cuda_is_refused(notes, monkeypatch):
+    # (a CUDA device that is there, so that only the class's own device is left to object to)
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 0)
+    monkeypatch.setattr(torch._C, "_cuda_getCurrentRawStream", lambda index: 0, raising=False)
+    q = _rand(1, 4, 5)
+    att = get_multi_stage_dot_production_attention(True)[0](q.shape, q.dtype, "cpu")
+    with pytest.raises(ValueError, match="cpu"):
+        att.append(q, _rand(1, 2, 9), _rand(1, 2, 9), end=True)
+    assert not notes.calls
+    assert _lib.raw_stream(torch.device("cuda")) == _lib.raw_stream(torch.device("cuda:0")) == 0
