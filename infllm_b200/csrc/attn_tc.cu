@@ -512,7 +512,8 @@ __global__ void __launch_bounds__(tc3::kThreads, 1) attn_tc3_kernel(const __grid
           }
           __syncwarp();
         }
-        if (ok && lead) tc_commit<kPair>(bar(T3_O_FULL));
+        // (without a product nobody waits for it, and it would arrive in the other CTA when that one may be gone)
+        if (ok && n > 0 && lead) tc_commit<kPair>(bar(T3_O_FULL));
       }
     }
   } else if (warp < 8) {

@@ -37,3 +37,29 @@ def test_pairs_and_lone_ctas_match_the_generic_kernel(monkeypatch, h, hkv, exec_
     err = (outs[0] - outs[1]).abs()
     assert err.norm() <= 8e-3 * outs[1].norm()
     assert err.max() <= 4e-2 * outs[1].abs().max()
+
+
+@pytest.mark.parametrize("h,hkv,lq", [(8, 2, 256), (7, 1, 256), (12, 12, 200), (7, 1, 300)])  # pairs of heads, of tiles, ragged; alone
+@pytest.mark.parametrize("hidden", [200, 3000])  # keys of the stage that no query sees: one run, and several
+@pytest.mark.parametrize("order", ["before", "behind", "only"])
+def test_a_stage_that_hides_every_pair_changes_nothing(h, hkv, lq, hidden, order):
+    from infllm_b200.attention import get_multi_stage_dot_production_attention
+
+    g = torch.Generator(device="cuda").manual_seed(h * lq + hidden)
+    q, k, v, hk, hv = (torch.randn((1, m, n, D), generator=g, device="cuda").to(torch.bfloat16)
+                       for m, n in ((h, lq), (hkv, 500), (hkv, 500), (hkv, hidden), (hkv, hidden)))
+    stages = [(k, v, 450, False)] * (order != "only")
+    stages.insert(order == "behind", (hk, hv, (-10 ** 6, 100), order != "before"))
+    att = get_multi_stage_dot_production_attention(True)[0](q.shape, q.dtype, "cuda")
+    for i, (sk, sv, win, comp) in enumerate(stages):
+        att.append(q, sk, sv, sliding_window=win, complement_sliding_window=comp, end=i == len(stages) - 1)
+    got = att.get_result()[0].float()
+    if order == "only":
+        assert not got.any()
+        return
+    s = q.float() @ k.float().repeat_interleave(h // hkv, 1).transpose(-1, -2) / D ** 0.5
+    dist = torch.arange(lq, device="cuda")[:, None] - torch.arange(500, device="cuda")[None] + 500 - lq
+    want = s.masked_fill((dist < 0) | (dist >= 450), float("-inf")).softmax(-1) @ v.float().repeat_interleave(h // hkv, 1)
+    err = (got - want).abs()
+    assert err.norm() <= 4e-3 * want.norm()  # (test_gpu_stage_kernels' bounds: one kernel against fp32)
+    assert err.max() <= 2e-2 * want.abs().max()
