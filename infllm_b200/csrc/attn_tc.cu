@@ -17,6 +17,7 @@
 
 #include "attn_common.cuh"
 #include "tc_common.cuh"
+#include "ring.cuh"
 #include "attn_tc.cuh"
 
 namespace infllm {
@@ -429,7 +430,10 @@ __global__ void __launch_bounds__(tc3::kThreads, 1) attn_tc3_kernel(const __grid
         }
         __syncwarp();
         if (pend.it >= 0) load_v();
-        if (!ok) break;
+        if (!ok) {
+          ++it;  // its K has been asked for
+          break;
+        }
         pend.it = it, pend.tok = tok, pend.c3 = R.c3_v, pend.map = R.map_v;
         ++it;
       }
@@ -437,11 +441,19 @@ __global__ void __launch_bounds__(tc3::kThreads, 1) attn_tc3_kernel(const __grid
     if (ok && pend.it >= 0) load_v();
     if (!ok && lane == 0) {
       // give loads that are still in flight a bounded chance to land before the CTA's memory goes away
-      for (int b = 0; b < kStages && rank == 0; ++b) {
-        for (uint32_t i = 0; i < 4096 && !mbar_try_wait(bar(T3_K_FULL0 + b), 0) && !mbar_try_wait(bar(T3_K_FULL0 + b), 1); ++i) __nanosleep(64);
-        for (uint32_t i = 0; i < 4096 && !mbar_try_wait(bar(T3_V_FULL0 + b), 0) && !mbar_try_wait(bar(T3_V_FULL0 + b), 1); ++i) __nanosleep(64);
+      auto land = [&](int first, int asked, int n) {
+        for (int b = 0; b < n; ++b) {
+          const int i = ring_last(asked, n, b);
+          for (uint32_t w = 0; i >= 0 && w < 4096 && !mbar_try_wait(bar(first + b), ring_parity(i, n)); ++w) __nanosleep(64);
+        }
+      };
+      if (rank == 0) {  // (of a pair, until the other CTA's share of the tile has landed there too)
+        land(T3_Q_FULL0, sidx, 2);
+        land(T3_K_FULL0, it, kStages);
+        land(T3_V_FULL0, pend.it >= 0 ? pend.it : it, kStages);
+      } else {  // its loads are counted in the first CTA, which may have given up before it asked for as many: a millisecond
+        for (uint32_t w = 0; w < 4096; ++w) __nanosleep(256);
       }
-      for (uint32_t i = 0; i < 4096 && rank != 0; ++i) __nanosleep(256);  // its loads are counted in the first CTA
     }
   } else if (warp == kWarpPv || warp == kWarpQk) {
     // ========================================================================== MMA issuers
@@ -999,13 +1011,13 @@ __global__ void __launch_bounds__(colsum_smem::kThreads, 1) colsum_tc_kernel(con
         }
         ++n;
       }
-      if (!ok) {
-        // give loads that are still in flight a bounded chance to land before the CTA's memory goes away
-        for (int b = 0; b < 2; ++b)
-          for (uint32_t i = 0; i < 4096 && !mbar_try_wait(bar(KF + b), 0) && !mbar_try_wait(bar(KF + b), 1); ++i) __nanosleep(64);
-        for (int t = q_first; t <= q_last; ++t)
-          for (uint32_t i = 0; i < 4096 && !mbar_try_wait(bar(QF + t), 0); ++i) __nanosleep(64);
+      // loads that are still in flight get a bounded chance to land before the CTA's memory goes away, whoever gave up
+      for (int b = 0; b < 2; ++b) {
+        const int i = ring_last(n, 2, b);
+        for (uint32_t w = 0; i >= 0 && w < 4096 && !mbar_try_wait(bar(KF + b), ring_parity(i, 2)); ++w) __nanosleep(64);
       }
+      for (int t = q_first; t <= q_last; ++t)
+        for (uint32_t w = 0; w < 4096 && !mbar_try_wait(bar(QF + t), 0); ++w) __nanosleep(64);
     }
   } else if (warp > 16) {
     // ====================================================================================== MMA issuers
