@@ -168,7 +168,7 @@ __device__ __forceinline__ bool seg_tiles(int64_t vis_lo, int64_t vis_hi, int64_
 // products (72.3); three teams.
 namespace tc3 {
 constexpr int kBufs = 3;                         // S/P buffers in TMEM
-constexpr int kQ = 0;                            // two stages
+constexpr int kQ = 0;                            // a tile for each of the two stages
 constexpr int kK = kQ + 4 * kSubTileBytes;       // two stages of a tile, or four of a CTA's half of one
 constexpr int kV = kK + 4 * kSubTileBytes;       // the same
 constexpr int kBar = kV + 4 * kSubTileBytes;
@@ -178,8 +178,8 @@ constexpr int kXsum = kXmax + 2 * 512;           // per team: row sums
 constexpr int kPlan = kXsum + 2 * 512;
 constexpr int kTotal = kPlan + 32 + kMaxSeg * 32;
 constexpr int kPolyEvery = 8;
-enum { T3_Q_FULL0 = 0, T3_Q_EMPTY0 = 2, T3_K_FULL0 = 4, T3_K_EMPTY0 = 8, T3_V_FULL0 = 12, T3_V_EMPTY0 = 16, T3_S_FULL0 = 20,
-       T3_P_FULL0 = 23, T3_PV_DONE0 = 26, T3_MAX0 = 29, T3_O_FULL = 45, T3_N_BARS };
+enum { T3_Q_FULL0 = 0, T3_K_FULL0 = 2, T3_K_EMPTY0 = 6, T3_V_FULL0 = 10, T3_V_EMPTY0 = 14, T3_S_FULL0 = 18,
+       T3_P_FULL0 = 21, T3_PV_DONE0 = 24, T3_MAX0 = 27, T3_O_FULL = 43, T3_N_BARS };
 constexpr int kWarpTma = 8, kWarpPv = 9, kWarpQk = 10;  // behind the eight softmax warps
 constexpr int kThreads = 11 * 32;
 // What a CTA does, worked out once, by one warp: the segments of its run that have tiles, in order.  Left to every role's own
@@ -404,15 +404,12 @@ __global__ void __launch_bounds__(tc3::kThreads, 1) attn_tc3_kernel(const __grid
     const int n_parts = plan->n_parts;
     for (int p = 0; p < n_parts && ok; ++p) {
       const Part R = plan->part[p];
-      if ((R.stage & 255) != stage) {  // the stage's queries; the buffer was the stage's before the last one's
+      if ((R.stage & 255) != stage) {  // the stage's queries, in a buffer of their own
         stage = R.stage & 255;
         const TcStage& S = P.stage[stage];
-        const int qb = sidx & 1;
-        if (sidx >= 2) ok = warp_wait(bar(T3_Q_EMPTY0 + qb), ((sidx >> 1) - 1) & 1, abort_flag, P.err, 600);
-        if (!ok) break;
         if (lead) {
-          const uint32_t dq = sQ + qb * 2 * kSubTileBytes, fb = lead_bar(T3_Q_FULL0 + qb);
-          if (rank == 0) mbar_expect_tx(bar(T3_Q_FULL0 + qb), 2 * kSubTileBytes * kCtas);
+          const uint32_t dq = sQ + sidx * 2 * kSubTileBytes, fb = lead_bar(T3_Q_FULL0 + sidx);
+          if (rank == 0) mbar_expect_tx(bar(T3_Q_FULL0 + sidx), 2 * kSubTileBytes * kCtas);
           tma_load_4d<kPair>(dq, &P.maps[S.map_q], fb, 0, S.q_row0 + (int)i0, 0, h);
         }
         __syncwarp();
@@ -439,9 +436,18 @@ __global__ void __launch_bounds__(tc3::kThreads, 1) attn_tc3_kernel(const __grid
       }
     }
     if (ok && pend.it >= 0) load_v();
+    // Nothing is on its way to this CTA any more when it says so (cluster_arrive below).  Of what the products signal, the releases
+    // of K and V are waited for above and not signalled behind the last loads, and the P V products before the last are waited for
+    // here: the softmax warps do so only where they scale O.  (Waiting for the last releases too cost 0.5 to 1.1 us a launch.)
+#pragma unroll 1
+    for (int b = 0; b < kBufs && ok; ++b) {
+      const int i = ring_last(it - 1, kBufs, b);
+      if (i >= 0) ok = warp_wait(bar(T3_PV_DONE0 + b), ring_parity(i, kBufs), abort_flag, P.err, 603);
+    }
+    // given up: loads that are still in flight get a bounded chance to land before the CTA's memory goes away
     if (!ok && lane == 0) {
-      // give loads that are still in flight a bounded chance to land before the CTA's memory goes away
       auto land = [&](int first, int asked, int n) {
+#pragma unroll 1
         for (int b = 0; b < n; ++b) {
           const int i = ring_last(asked, n, b);
           for (uint32_t w = 0; i >= 0 && w < 4096 && !mbar_try_wait(bar(first + b), ring_parity(i, n)); ++w) __nanosleep(64);
@@ -451,10 +457,11 @@ __global__ void __launch_bounds__(tc3::kThreads, 1) attn_tc3_kernel(const __grid
         land(T3_Q_FULL0, sidx, 2);
         land(T3_K_FULL0, it, kStages);
         land(T3_V_FULL0, pend.it >= 0 ? pend.it : it, kStages);
-      } else {  // its loads are counted in the first CTA, which may have given up before it asked for as many: a millisecond
+      } else if (!ok) {  // its loads are counted in the first CTA, which may have given up before it asked for as many: a millisecond
         for (uint32_t w = 0; w < 4096; ++w) __nanosleep(256);
       }
     }
+    __syncwarp();
   } else if (warp == kWarpPv || warp == kWarpQk) {
     // ========================================================================== MMA issuers
     // Two threads: one issues S = Q K^T, one O += P V.  One thread doing both was the longest serial
@@ -475,8 +482,8 @@ __global__ void __launch_bounds__(tc3::kThreads, 1) attn_tc3_kernel(const __grid
         for (int p = 0; p < n_parts && ok; ++p) {
           const int np = plan->part[p].n, last = plan->part[p].stage & 256;
           for (int t = 0; t < np && ok; ++t, ++iq) {
-            const int b = iq % kStages, qb = sq & 1;
-            if (q_due) ok = warp_wait(bar(T3_Q_FULL0 + qb), (sq >> 1) & 1, abort_flag, P.err, 610);
+            const int b = iq % kStages;
+            if (q_due) ok = warp_wait(bar(T3_Q_FULL0 + sq), 0, abort_flag, P.err, 610);
             q_due = false;
             if (ok) ok = warp_wait(bar(T3_K_FULL0 + b), (iq / kStages) & 1, abort_flag, P.err, 611);
             const int b3 = iq % kBufs;  // S/P buffer: free once the P V product of tile iq-3 has read P from it
@@ -492,10 +499,7 @@ __global__ void __launch_bounds__(tc3::kThreads, 1) attn_tc3_kernel(const __grid
               mma_ss<kPair>(tmem + b3 * 128, qd + qo, kd + ko, idesc_qk, ks > 0);
             }
             tc_commit<kPair>(bar(T3_S_FULL0 + b3));
-            tc_commit<kPair>(bar(T3_K_EMPTY0 + b));
-            if (last && t == np - 1) {
-              tc_commit<kPair>(bar(T3_Q_EMPTY0 + qb));  // the last product that reads this stage's Q tile
-            }
+            if (iq + kStages < n) tc_commit<kPair>(bar(T3_K_EMPTY0 + b));
             }
             if (last && t == np - 1) {
               ++sq;
@@ -519,8 +523,8 @@ __global__ void __launch_bounds__(tc3::kThreads, 1) attn_tc3_kernel(const __grid
             // A = P from TMEM, in the buffer's columns [0,64)
             mma_ts<kPair>(tO, tmem + b3 * 128 + 8 * ks, vd + (uint64_t)((ks * 2048) >> 4), idesc_pv, (ip > 0) || (ks > 0));
           }
-          tc_commit<kPair>(bar(T3_V_EMPTY0 + b));
-          tc_commit<kPair>(bar(T3_PV_DONE0 + b3));
+          if (ip + kStages < n) tc_commit<kPair>(bar(T3_V_EMPTY0 + b));
+          if (ip + 1 < n) tc_commit<kPair>(bar(T3_PV_DONE0 + b3));
           }
           __syncwarp();
         }
