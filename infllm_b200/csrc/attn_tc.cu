@@ -634,7 +634,7 @@ __global__ void __launch_bounds__(tc3::kThreads, 1) attn_tc3_kernel(const __grid
           float2 e[16];
           uint32_t pk[16];
           arg_chunk(sa, P.scale_log2, neg_m, e);
-          if (c < 3) tmem_ld32(tS + 32 * c + 32, ua);
+          tmem_ld32_if(c < 3, tS + 32 * c + 32, ua);
           exp_chunk<T, kExact>(e, rs, pk);
           tmem_st16(tS + 16 * c, pk);
           tmem_wait_ld32(ua);
