@@ -147,7 +147,8 @@ __device__ __forceinline__ bool seg_tiles(int64_t vis_lo, int64_t vis_hi, int64_
 // Pairs of CTAs (attn_tc3_pairs: where a KV head's query tiles, over all its query heads, come out even): the products are
 // cta_group::2, 256 rows of two CTAs by 128 keys, and a CTA fetches and holds half of every K and V tile.  That halves the
 // bytes from L2 to shared memory (a lone CTA's 64 KB a tile take 1600 cycles at 40 bytes per clock and SM) and leaves room for
-// four tiles in flight; the same code without pairs takes 78 us where pairs take 70.  Two query heads of a KV head make a pair, so
+// four tiles in flight.  Alone (7 heads by 3 tiles of a KV head, 12/12 heads by 3: 384 queries by 4480 + 2688 keys) the same code
+// takes 53.9 and 55.2 us where the eight-warp kernel before took 65.5 and 67.3.  Two query heads of a KV head make a pair, so
 // that both see the same keys; two tiles of one head where there is only one.
 // The softmax is two teams of four warps with the key tiles in turn, a thread per query row: no exchange within a row, and one
 // team's maximum and waits under the other's exponentials.  With all eight warps on one tile at a time (a row over four threads)
@@ -161,11 +162,12 @@ __device__ __forceinline__ bool seg_tiles(int64_t vis_lo, int64_t vis_hi, int64_
 // output against 64 bits); whenever a row's maximum grows, O is scaled.
 // What bounds it (clock stamps, cycles per 128-key tile): a period of 1600 at 1.75 GHz, a third of the way round of an S/P buffer:
 // product and commit 700, maximum 480, the other team's maximum 400, exponentials 1500, to the issuer 250, P V and back 800;
-// the tensor pipe needs 1024.  Per exec block of 32/8 heads, 512 queries by 4608 + 2688 keys: 64.3 us, 71.8 before (kExact: 70.6,
-// 84.6); 256 queries of 32/32 heads in two runs 45.5, 47.6; 4096 queries by 8192 keys, kExact, 306, 355.
-// Tried and not kept: four warps to half a tile's keys each, two tiles at once (70.5: more warps at the same pipes); the 64
-// score columns that a later tile needs first kept in registers, so that their buffer frees early (70.3); one issuer for both
-// products (72.3); three teams.
+// the tensor pipe needs 1024.  Per exec block of 32/8 heads, 512 queries by 4608 + 2688 keys, twenty launches in a row: 61.3 us where
+// the kernel before took 71.5 (kExact: 65.5, 83.7); 256 queries of 32/32 heads in two runs 42.6, 47.1; 4096 queries by 8192 keys,
+// kExact, 288.9, 354.3.
+// Tried and not kept, when the first of these took 70 us, timed by itself: four warps to half a tile's keys each, two tiles at once (70.5: more
+// warps at the same pipes); the 64 score columns that a later tile needs first kept in registers, so that their buffer frees early
+// (70.3); one issuer for both products (72.3); three teams.
 namespace tc3 {
 constexpr int kBufs = 3;                         // S/P buffers in TMEM
 constexpr int kQ = 0;                            // a tile for each of the two stages
@@ -457,18 +459,16 @@ __global__ void __launch_bounds__(tc3::kThreads, 1) attn_tc3_kernel(const __grid
         land(T3_Q_FULL0, sidx, 2);
         land(T3_K_FULL0, it, kStages);
         land(T3_V_FULL0, pend.it >= 0 ? pend.it : it, kStages);
-      } else if (!ok) {  // its loads are counted in the first CTA, which may have given up before it asked for as many: a millisecond
+      } else {  // its loads are counted in the first CTA, which may have given up before it asked for as many: a millisecond
         for (uint32_t w = 0; w < 4096; ++w) __nanosleep(256);
       }
     }
     __syncwarp();
   } else if (warp == kWarpPv || warp == kWarpQk) {
     // ========================================================================== MMA issuers
-    // Two threads: one issues S = Q K^T, one O += P V.  One thread doing both was the longest serial
-    // chain of a key tile (waits, 16 products that each hold the thread while the pipe is busy, commits: about
-    // 2500 cycles); apart they take about 1100 each and the softmax sets the pace.  What the tensor pipe ordered
-    // before - S of tile t+3 may overwrite its buffer only when P V of tile t has read P from it - is
-    // the wait for that product's commit.  Of a pair, the first CTA's issue for both.
+    // Two warps: one issues S = Q K^T, one O += P V, so that neither's waits hold up the other (one warp for both: 72.3 us
+    // instead of 70).  What the tensor pipe would order by itself then - S of tile t+3 may overwrite its buffer only when P V of
+    // tile t has read P from it - is the wait for that product's commit.  Of a pair, the first CTA's issue for both.
     if (rank == 0) {
       const bool lead = elect_one();
       const int n = plan->n_tiles;
@@ -613,8 +613,8 @@ __global__ void __launch_bounds__(tc3::kThreads, 1) attn_tc3_kernel(const __grid
           if (!ok) break;
           m_prev = next_ref<kExact>(m_prev, tmax[((it - 1) & 3) * kTile + row]);
         }
-        // (left behind the look at the other team's: a place is taken again by the tile after the next but one, whose team has
-        // then seen that it was read)
+        // (left behind the look at the other team's: a place is taken again four tiles later, by the same team, which by then has
+        // waited for the maximum of the tile before, and the other team left that one behind its own look at this place)
         tmax[(it & 3) * kTile + row] = m_tile;
         __syncwarp();
         if (lane == 0) mbar_arrive(bar(T3_MAX0 + (it & 3) * 4 + quad));
@@ -678,7 +678,7 @@ __global__ void __launch_bounds__(tc3::kThreads, 1) attn_tc3_kernel(const __grid
       }
       it0 += R.n;
     }
-    // ---- epilogue: the teams' row sums come together; then every warp of the first two teams writes 64 output columns of
+    // ---- epilogue: the teams' row sums come together; then every warp writes 64 output columns of
     // 32 rows
     xsum[team * kTile + row] = l_part;
     xmax[team * kTile + row] = m_ref;
@@ -1233,10 +1233,10 @@ int attn_tc_combine_launch(const float* acc, const float* m, const float* l, int
 }
 
 // Runs of key tiles per (128-query tile, head), as many as the SMs take at once and no more than pay: a run's tiles come one
-// after another, about 1.1 us each (0.92 in pairs of CTAs, where 4 runs of 32 items and 15 tiles, 16.9 us, and 8 of 12 and 24, 15.8, are still the best of 1 to 8), and the partials cost a merge, two tiles' time for its launch and one more for every 40
-// runs of the grid.  Measured over 4 to 60 tiles for 8 to 64 items (15 sizes each, bf16, both precisions, merge included): on
-// the average 0.7 % above the best count, 11 % at worst (6 tiles of 32 items: 16.5 us instead of 14.8).  At least seven tiles
-// to a run, which is what it was, is 13 % above it, 68 % at worst: 12 tiles of 8 items 24.2 us instead of 14.4.
+// after another, 0.9 us each, and the partials cost a merge, two tiles' time for its launch and one more for every 40 runs of the
+// grid.  Measured over 4 to 60 tiles for 8 to 64 items (nine kinds of 15 sizes, bf16, both precisions, merge included, every
+// count): on the average 1.0 % above the best count, 9.4 % at worst (4 tiles of 8 items: 11.5 us in four runs, 10.5 in one).  At
+// least seven tiles to a run, which is what it was, took 24.2 us for 12 tiles of 8 items instead of 14.4.
 int attn_tc3_splits(int64_t lq, int n_heads, int64_t keys) {
   const int64_t items = ceil_div(lq, kTile) * n_heads, tiles = ceil_div(keys, kTile);
   int best = 1;

@@ -13,7 +13,7 @@ namespace tc {
 // A wait that runs out records where it gave up and the kernel unwinds; the host reads the flag.
 constexpr int kErrNone = 0;
 constexpr int kErrWaitTimeout = 1;
-constexpr uint32_t kSpinLimit = 1u << 22;  // ~ a second with the back-off below
+constexpr uint32_t kSpinLimit = 1u << 22;  // of a bounded wait: about a second with its back-off
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -34,7 +34,10 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
-// arrival on a barrier of another CTA of the cluster (the address from cluster_map)
+// arrival on a barrier of another CTA of the cluster (the address from cluster_map), for tcgen05 work only: it says that loads from
+// and stores to TMEM are done, ordered by tcgen05.wait::ld / ::st and fence::before_thread_sync on this side and
+// fence::after_thread_sync on the other.  Without a scope it orders nothing else between the CTAs: data in shared or global
+// memory would need the .release.cluster form and an .acquire.cluster wait (1500 cycles an arrival instead of 100).
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
 }
@@ -43,12 +46,7 @@ __device__ __forceinline__ uint32_t cluster_map(uint32_t addr, uint32_t rank) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
   return r;
 }
-__device__ __forceinline__ uint32_t cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-// barrier of every thread of every CTA of the cluster, in two halves: what lies between them hides its way (600 cycles)
+// barrier of every thread of every CTA of the cluster, in two halves: what lies between them hides its way (1150 cycles)
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
 __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
@@ -61,14 +59,6 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
       : "r"(bar), "r"(parity)
       : "memory");
   return ok != 0;
-}
-// Bounded wait: false when the limit ran out (the caller records the error and unwinds).
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
-  for (uint32_t i = 0; i < kSpinLimit; ++i) {
-    if (mbar_try_wait(bar, parity)) return true;
-    if (i > 64) __nanosleep(i > 4096 ? 256 : 32);
-  }
-  return false;
 }
 
 // ----------------------------------------------------------------------------------------- TMA
@@ -245,7 +235,7 @@ constexpr int kSubTileBytes = 128 * 128;  // 128 rows x 64 elements x 2 bytes
 
 }  // namespace tc
 
-// host side: build a tiled tensor map (rank 3 or 4, 16-bit elements, 128-byte swizzle, zero fill)
+// host side: build a tiled tensor map (rank 4 or 5, 16-bit elements, 128-byte swizzle, zero fill)
 int encode_tensor_map(CUtensorMap* map, int dtype, const void* base, int rank, const uint64_t* dims,
                       const uint64_t* strides_bytes /* rank-1 */, const uint32_t* box);
 
