@@ -177,14 +177,14 @@ constexpr int kQ = 0;                            // a tile for each of the two s
 constexpr int kK = kQ + 4 * kSubTileBytes;       // two stages of a tile, or four of a CTA's half of one
 constexpr int kV = kK + 4 * kSubTileBytes;       // the same
 constexpr int kBar = kV + 4 * kSubTileBytes;
-constexpr int kTmax = kBar + 512;                // the rows' maxima in the last four tiles
-constexpr int kXmax = kTmax + 4 * 512;           // per team: the reference its row sums stand at
+constexpr int kTmax = kBar + 512;                // the rows' maxima in the last four tiles, each with its tile's number
+constexpr int kXmax = kTmax + 4 * 1024;          // per team: the reference its row sums stand at
 constexpr int kXsum = kXmax + 2 * 512;           // per team: row sums
 constexpr int kPlan = kXsum + 2 * 512;
 constexpr int kTotal = kPlan + 32 + kMaxSeg * 32;
 constexpr int kPolyEvery = 8;
 enum { T3_Q_FULL0 = 0, T3_K_FULL0 = 2, T3_K_EMPTY0 = 6, T3_V_FULL0 = 10, T3_V_EMPTY0 = 14, T3_S_FULL0 = 18,
-       T3_P_FULL0 = 21, T3_PV_DONE0 = 24, T3_MAX0 = 27, T3_O_FULL = 43, T3_N_BARS };
+       T3_P_FULL0 = 21, T3_PV_DONE0 = 24, T3_O_FULL = 27, T3_N_BARS };
 constexpr int kWarpTma = 8, kWarpPv = 9, kWarpQk = 10;  // behind the eight softmax warps
 constexpr int kThreads = 11 * 32;
 // What a CTA does, worked out once, by one warp: the segments of its run that have tiles, in order.  Left to every role's own
@@ -272,6 +272,13 @@ __device__ __forceinline__ void make_plan(const AttnTcParams& P, int64_t i0, int
     if (last[1] >= 0) plan->part[last[1]].stage |= 256;
   }
 }
+// a word of shared memory that another thread of the CTA watches: it is stored and loaded whole
+__device__ __forceinline__ uint64_t look_word(uint32_t addr) {
+  uint64_t v;
+  asm volatile("ld.volatile.shared.b64 %0, [%1];" : "=l"(v) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ void leave_word(uint32_t addr, uint64_t v) { asm volatile("st.volatile.shared.b64 [%0], %1;" ::"r"(addr), "l"(v) : "memory"); }
 // exponentials of 32 columns of a row, packed; sums into rs
 template <typename T, bool kExact>
 __device__ __forceinline__ void exp_chunk(const float2* a, float2* rs, uint32_t* pk) {
@@ -327,7 +334,7 @@ __global__ void __launch_bounds__(tc3::kThreads, 1) attn_tc3_kernel(const __grid
   const uint32_t bars = s_base + kBar;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + kBar + T3_N_BARS * 8);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + kBar + T3_N_BARS * 8 + 8);
-  float* tmax = reinterpret_cast<float*>(smem + kTmax);
+  const uint32_t tmax = s_base + kTmax;
   float* xmax = reinterpret_cast<float*>(smem + kXmax);
   float* xsum = reinterpret_cast<float*>(smem + kXsum);
   auto bar = [&](int i) { return bars + 8u * (uint32_t)i; };
@@ -348,6 +355,7 @@ __global__ void __launch_bounds__(tc3::kThreads, 1) attn_tc3_kernel(const __grid
     *abort_flag = 0;
     mbar_fence_init();
   }
+  for (int i = threadIdx.x; i < 4 * kTile; i += kThreads) reinterpret_cast<uint64_t*>(smem + kTmax)[i] = ~0ull;  // (no tile's number)
   if (kPair) cluster_arrive();  // (waited for below: the other CTA's barriers stand before anything is signalled on them)
   if (warp == kWarpQk && lane < P.n_stage) {  // the descriptors of the first loads are on their way while the run's parts are worked out
     const TcStage& S = P.stage[lane];
@@ -541,7 +549,7 @@ __global__ void __launch_bounds__(tc3::kThreads, 1) attn_tc3_kernel(const __grid
     // it, so that nothing is exchanged within a row.  What one team waits for - scores from TMEM, the maximum, the way
     // of P into TMEM - is covered by the other's exponentials.  There is one O and so one reference maximum per row; it follows
     // from the tiles' maxima, in order, and every thread works it out for itself from those of its own tiles and those that
-    // the other team leaves in shared memory (tmax, a barrier per tile and quarter of the rows).
+    // the other team leaves in shared memory (tmax).
     const int quad = warp & 3, team = warp >> 2, row = quad * 32 + lane;
     const uint32_t lane_base = ((uint32_t)(quad * 32)) << 16;
     const int64_t qi = i0 + row;
@@ -550,7 +558,7 @@ __global__ void __launch_bounds__(tc3::kThreads, 1) attn_tc3_kernel(const __grid
     float m_ref = -INFINITY, l_part = 0.f;  // the reference behind this team's last tile, and its sum relative to it
     int it0 = 0, stage = -1;
     bool ok = true;
-    int jlo = 0, jhi = 0;  // keys of the stage visible to this thread's query row
+    int jlo = 0, jhi = 0, wlo = 0, whi = 0;  // keys of the stage visible to this thread's query row, and to all rows of the warp
     const int n_parts = plan->n_parts, n_tiles = plan->n_tiles;
     for (int p = 0; p < n_parts && ok; ++p) {
       const Part R = plan->part[p];
@@ -567,16 +575,18 @@ __global__ void __launch_bounds__(tc3::kThreads, 1) attn_tc3_kernel(const __grid
           hi = qi + S.mask_offset - S.mask_size;
         }
         jlo = clamp(lo), jhi = clamp(hi);
+        wlo = __reduce_max_sync(0xffffffffu, jlo), whi = __reduce_min_sync(0xffffffffu, jhi);
       }
-      const int j_hi = jhi < R.lim ? jhi : R.lim;
+      const int j_hi = jhi < R.lim ? jhi : R.lim, w_hi = whi < R.lim ? whi : R.lim;
       for (int t = (team + it0) & 1; t < R.n && ok; t += 2) {
         const int it = it0 + t, b3 = it % kBufs;
         const uint32_t tS = tmem + b3 * 128 + lane_base;
         ok = warp_wait(bar(T3_S_FULL0 + b3), (it / kBufs) & 1, abort_flag, P.err, 620);
         if (!ok) break;
         tc_fence_after();
-        const int c_lo = jlo - R.j - t * kTile, c_hi = j_hi - R.j - t * kTile;
-        if (!__all_sync(0xffffffffu, c_lo <= 0 && c_hi >= kTile - 1)) {
+        const int j0 = R.j + t * kTile;
+        if (wlo > j0 || w_hi < j0 + kTile - 1) {
+          const int c_lo = jlo - j0, c_hi = j_hi - j0;
           // a tile at an edge: what a row does not see is taken out of the scores where they are
 #pragma unroll 1
           for (int c = 0; c < kTile; c += 32) {
@@ -610,24 +620,45 @@ __global__ void __launch_bounds__(tc3::kThreads, 1) attn_tc3_kernel(const __grid
           max_chunk(sa, mx);
         }
         const float m_tile = fmaxf(fmax3(mx[0], mx[1], mx[2]), mx[3]) * P.scale_log2;
-        float m_prev = m_ref;
-        if (it > 0) {
-          ok = warp_wait(bar(T3_MAX0 + ((it - 1) & 3) * 4 + quad), ((it - 1) >> 2) & 1, abort_flag, P.err, 621);
+        // What the other team left of the tile before, if it has.  The tile's number comes with the value, in one word, so that there
+        // is nothing else to wait for (a barrier per tile and quarter of the rows, a load behind it and two votes: 400 cycles, now 230).
+        const uint32_t there = tmax + (uint32_t)(((it - 1) & 3) * kTile + row) * 8;
+        uint64_t left = look_word(there);
+        float m_prev = it > 0 ? next_ref<kExact>(m_ref, __uint_as_float((uint32_t)left)) : m_ref, m_new = next_ref<kExact>(m_prev, m_tile), alpha = 1.f;
+        bool resc = false;
+        auto move_ref = [&]() {  // what the row's O and this team's sum are to be scaled by
+          resc = __any_sync(0xffffffffu, m_new != m_prev && m_prev != -INFINITY) && it >= 1;
+          alpha = m_prev == -INFINITY ? 1.f : ex2_approx(m_prev - m_new);
+          if (m_new != m_ref) {
+            l_part *= ex2_approx(m_ref - m_new);
+            m_ref = m_new;
+          }
+        };
+        // (lazy: nearly always the word is there and no reference moves, which one vote says)
+        const bool there_is = it == 0 || (int)(left >> 32) == it - 1;
+        if (!__all_sync(0xffffffffu, there_is && (kExact || m_new == m_ref))) {
+          for (uint32_t w = 0; it > 0 && (int)(left >> 32) != it - 1; ++w) {
+            if (*abort_flag || w >= kSpinLimit) {
+              ok = false;
+              break;
+            }
+            if (w > 64) __nanosleep(w > 4096 ? 256 : 32);
+            left = look_word(there);
+          }
+          if (!ok && !*abort_flag) {
+            *abort_flag = 1;
+            record_error(P.err, kErrWaitTimeout, 621);
+          }
+          ok = __all_sync(0xffffffffu, ok);
           if (!ok) break;
-          m_prev = next_ref<kExact>(m_prev, tmax[((it - 1) & 3) * kTile + row]);
+          if (it > 0) m_prev = next_ref<kExact>(m_ref, __uint_as_float((uint32_t)left));
+          m_new = next_ref<kExact>(m_prev, m_tile);
+          if (!kExact) move_ref();
         }
         // (left behind the look at the other team's: a place is taken again four tiles later, by the same team, which by then has
-        // waited for the maximum of the tile before, and the other team left that one behind its own look at this place)
-        tmax[(it & 3) * kTile + row] = m_tile;
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar(T3_MAX0 + (it & 3) * 4 + quad));
-        const float m_new = next_ref<kExact>(m_prev, m_tile);
-        const bool resc = __any_sync(0xffffffffu, m_new != m_prev && m_prev != -INFINITY) && it >= 1;
-        const float alpha = m_prev == -INFINITY ? 1.f : ex2_approx(m_prev - m_new);
-        if (m_new != m_ref) {
-          l_part *= ex2_approx(m_ref - m_new);
-          m_ref = m_new;
-        }
+        // seen the maximum of the tile before, and the other team left that one behind its own look at this place)
+        leave_word(tmax + (uint32_t)((it & 3) * kTile + row) * 8, (uint64_t)(uint32_t)it << 32 | __float_as_uint(m_tile));
+        if (kExact) move_ref();
         const float neg_m = m_new == -INFINITY ? 0.f : -m_new;
         float2 rs[4] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
         // P, packed, takes the place of the scores that have been read: 16 columns for 32.  (Rolled: the fetch of code is what
