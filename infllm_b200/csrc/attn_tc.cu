@@ -350,9 +350,10 @@ __global__ void __launch_bounds__(tc3::kThreads, 1) attn_tc3_kernel(const __grid
   const int rows_q = (int)((P.lq - i0) < kTile ? (P.lq - i0) : kTile);
   const int split = blockIdx.z;
 
-  if (threadIdx.x == 0) {
-    for (int i = 0; i < T3_N_BARS; ++i) mbar_init(bar(i), i >= T3_P_FULL0 && i < T3_P_FULL0 + kBufs ? 4u * kCtas : 1u);
-    *abort_flag = 0;
+  if (warp == 0) {
+    static_assert(T3_N_BARS <= 32, "");
+    if (lane < T3_N_BARS) mbar_init(bar(lane), lane >= T3_P_FULL0 && lane < T3_P_FULL0 + kBufs ? 4u * kCtas : 1u);
+    if (lane == 0) *abort_flag = 0;
     mbar_fence_init();
   }
   for (int i = threadIdx.x; i < 4 * kTile; i += kThreads) reinterpret_cast<uint64_t*>(smem + kTmax)[i] = ~0ull;  // (no tile's number)
