@@ -1033,7 +1033,6 @@ __global__ void __launch_bounds__(colsum_smem::kThreads, 1) colsum_tc_kernel(con
       }
     }
   }
-  for (int i = threadIdx.x; i < (kt1 - kt0) * NB * 128; i += blockDim.x) s_acc[i] = 0.f;
   if (warp == 17) {
     tmem_alloc(smem_u32(tmem_slot), 128 * NB);
     tmem_relinquish();
@@ -1194,7 +1193,8 @@ __global__ void __launch_bounds__(colsum_smem::kThreads, 1) colsum_tc_kernel(con
     float* dst = P.score + (int64_t)h * P.score_hs + (int64_t)kt0 * kTile;
     for (int i = threadIdx.x; i < cols; i += blockDim.x) {
       const float* sa = s_acc + (i >> 7) * NB * 128 + (i & 127);
-      const float v = (sa[0] + sa[128]) + (sa[256] + sa[384]);
+      int tf, tl;  // (the places of a key tile that no query sees have been written by nobody)
+      const float v = tile_q(kt0 + (i >> 7), &tf, &tl) ? (sa[0] + sa[128]) + (sa[256] + sa[384]) : 0.f;
       dst[i] = P.accumulate ? __ldcg(dst + i) + v : v;
     }
   }
