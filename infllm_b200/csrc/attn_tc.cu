@@ -1133,7 +1133,10 @@ __global__ void __launch_bounds__(colsum_smem::kThreads, 1) colsum_tc_kernel(con
       const int keys = (int)P.lk - j0 < kTile ? (int)P.lk - j0 : kTile;
       int tf, tl;
       colsum_q_tiles(P, j0, keys, &tf, &tl);
-      if (tl < tf) continue;
+      if (tl < tf) {
+        s_acc[((kt - kt0) * 4 + part) * 128 + krow] = 0.f;
+        continue;
+      }
       // queries [vi_lo, vi_hi] see this thread's key
       int vi_lo, vi_hi;
       colsum_range(P, j0 + krow, &vi_lo, &vi_hi);
@@ -1193,8 +1196,7 @@ __global__ void __launch_bounds__(colsum_smem::kThreads, 1) colsum_tc_kernel(con
     float* dst = P.score + (int64_t)h * P.score_hs + (int64_t)kt0 * kTile;
     for (int i = threadIdx.x; i < cols; i += blockDim.x) {
       const float* sa = s_acc + (i >> 7) * NB * 128 + (i & 127);
-      int tf, tl;  // (the places of a key tile that no query sees have been written by nobody)
-      const float v = tile_q(kt0 + (i >> 7), &tf, &tl) ? (sa[0] + sa[128]) + (sa[256] + sa[384]) : 0.f;
+      const float v = (sa[0] + sa[128]) + (sa[256] + sa[384]);
       dst[i] = P.accumulate ? __ldcg(dst + i) + v : v;
     }
   }
