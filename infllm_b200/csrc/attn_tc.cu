@@ -151,7 +151,7 @@ __device__ __forceinline__ bool seg_tiles(int64_t vis_lo, int64_t vis_hi, int64_
 // cta_group::2, 256 rows of two CTAs by 128 keys, and a CTA fetches and holds half of every K and V tile.  That halves the
 // bytes from L2 to shared memory (a lone CTA's 64 KB a tile take 1600 cycles at 40 bytes per clock and SM) and leaves room for
 // four tiles in flight.  Alone (7 heads by 3 tiles of a KV head, 12/12 heads by 3: 384 queries by 4480 + 2688 keys) the same code
-// takes 53.9 and 55.2 us where the eight-warp kernel before took 65.5 and 67.3.  Two query heads of a KV head make a pair, so
+// takes 51.2 and 50.3 us.  Two query heads of a KV head make a pair, so
 // that both see the same keys; two tiles of one head where there is only one.
 // The softmax is two teams of four warps with the key tiles in turn, a thread per query row: no exchange within a row, and one
 // team's maximum and waits under the other's exponentials.  With all eight warps on one tile at a time (a row over four threads)
@@ -163,11 +163,16 @@ __device__ __forceinline__ bool seg_tiles(int64_t vis_lo, int64_t vis_hi, int64_
 // kExact (see kExactQueries): that polynomial is as good as exp2f, and the reference
 // maximum of a row follows its maximum, so that the largest probabilities have no rounding (2 to 6 % less error of an
 // output against 64 bits); whenever a row's maximum grows, O is scaled.
-// What bounds it (clock stamps, cycles per 128-key tile): a period of 1600 at 1.75 GHz, a third of the way round of an S/P buffer:
-// product and commit 700, maximum 480, the other team's maximum 400, exponentials 1500, to the issuer 250, P V and back 800;
-// the tensor pipe needs 1024.  Per exec block of 32/8 heads, 512 queries by 4608 + 2688 keys, twenty launches in a row: 61.3 us where
-// the kernel before took 71.5 (kExact: 65.5, 83.7); 256 queries of 32/32 heads in two runs 42.6, 47.1; 4096 queries by 8192 keys,
-// kExact, 288.9, 354.3.
+// What bounds it (clock stamps, cycles): a key tile every 1420, of which the tensor pipe needs 1024.  Two ways round are equally long:
+// that of a team, two tiles in 2840 - exponentials 1500 (372 per 32 columns where one warp of a scheduler is at them, 265 where two
+// are), maximum 400, the other team's 230, the rest waits and hand-overs that are there already and cost 75 to 100 each - and that of
+// an S/P buffer, three tiles: product 700, softmax 2300, to the issuer 250, P V and back 850.  Set-up and first loads take 6000 and the
+// end 4500.  32/8 heads, 512 queries by 4608 + 2688 keys, twenty launches in a row: 52.7 us, with each wait through a loop, a barrier
+// for every maximum and ordering cluster barriers 58.2 (kExact: 57.5, 62.3); 256 queries of 32/32 heads in two runs 36.8, 40.7; 128
+// queries in four runs 14.8, 16.1; 4096 queries by 8192 keys, kExact, 264, 286.
+// Also not kept: S and P in buffers of their own with a tile's scores in registers (224 of them, setmaxnreg) and the next tile's loaded
+// under the exponentials.  A tile every 1470 from 1600 at the time, but straight code of 20 KB is fetched cold at every launch: 54.7
+// where the rolled loop went from 58.2 to 52.7, and 44.7 against 36.8 in two runs.
 // Tried and not kept, when the first of these took 70 us, timed by itself: four warps to half a tile's keys each, two tiles at once (70.5: more
 // warps at the same pipes); the 64 score columns that a later tile needs first kept in registers, so that their buffer frees early
 // (70.3); one issuer for both products (72.3); three teams.
@@ -905,11 +910,12 @@ __global__ void attn_tc_combine_kernel(const float* __restrict__ acc, const floa
 // four of the sixteen compute warps of its own, which turn it into sum_q exp2(s - lse_q).  A key tile is loaded once
 // per head and a query tile once per CTA, which keeps the L2 traffic an order of magnitude below one load per pair.
 // Bound: 16384 exponentials per pair, 768 cycles of the special-function unit with every fourth pair of them as a
-// quartic on the FMA pipe (a quintic, kExact, for exec blocks of one query tile), and the product, 514; a pair takes 1330 (the
-// special-function unit is busy for 54 % of the time, the schedulers for 56 %: what is waited for is latencies, and the
-// log-sum-exps out of shared memory share a queue with the exponentials).  512 queries x 32 heads over 4608 keys: 29.6 us, 37
-// over 4133: 10.8 (issued by lone threads: 30.2, 12.1).  Products of 64 queries, two buffers per group: 34.9 (half as many
-// columns are not half a product); two groups with two buffers each: 36.2.
+// quartic on the FMA pipe (a quintic, kExact, for exec blocks of one query tile; without any 29.0 us, with an eighth 27.9, three
+// eighths 27.0), the product, 514, whose operands want shared memory for all of that time, and 424 more there for the log-sum-exps
+// (685 in 16-byte loads); a pair takes 1030.  512 queries x 32 heads over 4608 keys: 26.5 us (28.3 with those loads, a loop at
+// every wait and sums cleared beforehand), 37 over 4133: 9.9 (10.7).  Products of 64 queries, two buffers per group: 34.9 (half as
+// many columns are not half a product); two groups with two buffers each: 36.2; queries as TMEM lanes, so that a log-sum-exp is a
+// register's and a key's sum is exchanged once per key tile: 28.7 (8 % more instructions), in eight warps 34.3.
 namespace colsum_smem {
 constexpr int kQTiles = 4;                     // resident query tiles
 constexpr int kMaxKeyTiles = 10;               // key tiles per CTA
