@@ -871,24 +871,42 @@ __global__ void attn_tc_combine_kernel(const float* __restrict__ acc, const floa
   const int lane = threadIdx.x & 31;
   const int64_t h = row / lq, i = row - h * lq;
   const int64_t stride = (int64_t)n_heads * lq;
+  // What bounds it is two loads behind one another and the launch: the first four partials are asked for whole, before their maximum is
+  // known (with the attention, 256 queries of 28/4 heads in two runs 32.5 -> 31.2 us, 37 of 32/8 in four 23.2 -> 22.6, 16 of 16/2 in four
+  // 10.0 -> 9.2; 128 of 32/8 in four 15.1, as before)
+  constexpr int kAhead = 4;
+  float4 pa[kAhead];
+  float pm[kAhead], pl[kAhead];
+#pragma unroll
+  for (int s = 0; s < kAhead; ++s) {
+    if (s >= n_split) continue;
+    pm[s] = m[s * stride + row], pl[s] = l ? l[s * stride + row] : 1.f;
+    pa[s] = *reinterpret_cast<const float4*>(acc + (s * stride + row) * 128 + lane * 4);
+  }
   float mx = st_acc ? st_m[row] : -INFINITY;
-  for (int s = 0; s < n_split; ++s) mx = fmaxf(mx, m[s * stride + row]);
+#pragma unroll
+  for (int s = 0; s < kAhead; ++s)
+    if (s < n_split) mx = fmaxf(mx, pm[s]);
+  for (int s = kAhead; s < n_split; ++s) mx = fmaxf(mx, m[s * stride + row]);
   float den = 0.f;
   float4 num = make_float4(0.f, 0.f, 0.f, 0.f);
   if (mx != -INFINITY) {
-    auto fold = [&](float ms, float ls, const float* ap) {
+    auto add = [&](float ms, float ls, float4 a) {
       if (ms == -INFINITY) return;
       const float w = exp2f(ms - mx);
       den = fmaf(w, ls, den);
-      const float4 a = *reinterpret_cast<const float4*>(ap + row * 128 + lane * 4);
       num.x = fmaf(w, a.x, num.x);
       num.y = fmaf(w, a.y, num.y);
       num.z = fmaf(w, a.z, num.z);
       num.w = fmaf(w, a.w, num.w);
     };
+    auto fold = [&](float ms, float ls, const float* ap) { add(ms, ls, *reinterpret_cast<const float4*>(ap + row * 128 + lane * 4)); };
     if (st_acc) fold(st_m[row], st_l[row], st_acc);
+#pragma unroll
+    for (int s = 0; s < kAhead; ++s)
+      if (s < n_split) add(pm[s], pl[s], pa[s]);
 #pragma unroll 4
-    for (int s = 0; s < n_split; ++s) fold(m[s * stride + row], l ? l[s * stride + row] : 1.f, acc + s * stride * 128);
+    for (int s = kAhead; s < n_split; ++s) fold(m[s * stride + row], l ? l[s * stride + row] : 1.f, acc + s * stride * 128);
   }
   if (out) {
     const float inv = den > 0.f ? 1.f / den : 0.f;
