@@ -155,8 +155,8 @@ __device__ __forceinline__ bool seg_tiles(int64_t vis_lo, int64_t vis_hi, int64_
 // that both see the same keys; two tiles of one head where there is only one.
 // The softmax is two teams of four warps with the key tiles in turn, a thread per query row: no exchange within a row, and one
 // team's maximum and waits under the other's exponentials.  With all eight warps on one tile at a time (a row over four threads)
-// a tile took 2000 cycles, 1700 of them theirs.  One pair of exponentials in eight is a polynomial on the FMA pipe: none to a
-// quarter make no difference to the time.
+// a tile took 2000 cycles, 1700 of them theirs.  One pair of exponentials in eight is a polynomial on the FMA pipe (none: 3 % more time;
+// a quarter: 1 % less, kExact 1 % more).
 // Issuers and producer are whole warps of which one lane issues: eight products in 120 cycles instead of 600, and one load per
 // tile and operand (both 64-dimension halves in one box) instead of four at about 390 cycles each, which was 1570 per tile
 // whatever their size.  The producer asks for K one tile ahead of V.
@@ -1311,10 +1311,10 @@ int attn_tc_combine_launch(const float* acc, const float* m, const float* l, int
 }
 
 // Runs of key tiles per (128-query tile, head), as many as the SMs take at once and no more than pay: a run's tiles come one
-// after another, 0.9 us each, and the partials cost a merge, two tiles' time for its launch and one more for every 40 runs of the
-// grid.  Measured over 4 to 60 tiles for 8 to 64 items (nine kinds of 15 sizes, bf16, both precisions, merge included, every
-// count): on the average 1.0 % above the best count, 9.4 % at worst (4 tiles of 8 items: 11.5 us in four runs, 10.5 in one).  At
-// least seven tiles to a run, which is what it was, took 24.2 us for 12 tiles of 8 items instead of 14.4.
+// after another, 0.8 us each, and the partials cost a merge, two tiles' time for its launch and one more for every 40 runs of the
+// grid.  Measured over 4 to 60 tiles for 8 to 64 items (eight kinds of 8 sizes, bf16, both precisions, merge included, every
+// count): on the average 0.9 % above the best count, 14 % at worst (4 tiles of 8 items: 10.6 us in four runs, 9.3 in one).  Half a
+// tile more or less for the merge, or one for every 32 or 50 runs: 0.8 to 1.3 % on the average.
 int attn_tc3_splits(int64_t lq, int n_heads, int64_t keys) {
   const int64_t items = ceil_div(lq, kTile) * n_heads, tiles = ceil_div(keys, kTile);
   int best = 1;
