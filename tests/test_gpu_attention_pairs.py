@@ -4,6 +4,8 @@ both see the same keys.
 
 Tolerance: each kernel rounds probabilities and outputs to bf16; test_gpu_stage_kernels bounds that by 4e-3 in the 2-norm and
 2e-2 of the largest output against fp32, two kernels differ by twice that."""
+import math
+
 import pytest
 import torch
 
@@ -20,7 +22,7 @@ D, UNIT = 128, 128
     (8, 2, 129, 1500),    # a second tile of one query
     (32, 8, 512, 3000),   # pairs of heads
 ])
-@pytest.mark.parametrize("step", [1.0, 4.0])  # keys that grow: the rows' reference maxima move in every tile
+@pytest.mark.parametrize("step", [1.0, 4.0])  # keys that grow: of a few rows the reference maximum moves, once
 def test_pairs_and_lone_ctas_match_the_generic_kernel(monkeypatch, h, hkv, exec_, n, step):
     from infllm_b200.attention import ContextManager, RotaryEmbeddingESM
     from infllm_b200.attention import context_manager as cmod
@@ -37,6 +39,75 @@ def test_pairs_and_lone_ctas_match_the_generic_kernel(monkeypatch, h, hkv, exec_
     err = (outs[0] - outs[1]).abs()
     assert err.norm() <= 8e-3 * outs[1].norm()
     assert err.max() <= 4e-2 * outs[1].abs().max()
+
+
+# what a row's maximum grows by from a key tile to the next, as a power of two.  A reference moves where that is more than 8.
+GROWTH = {
+    "every tile": [10] * 10,
+    "tiles of the first team": [0, 20] * 5,
+    "tiles of the second team": [20, 0] * 5,
+    "uneven": [9, 25, 0, 9, 9, 25, 0, 0, 9, 14],
+}
+
+
+@pytest.mark.parametrize("h,hkv,exec_", [
+    (32, 8, 512),   # pairs, one run
+    (36, 12, 384),  # alone, one run
+    (8, 2, 256),    # pairs, several runs
+    (7, 1, 384),    # alone, several runs
+])
+@pytest.mark.parametrize("growth", list(GROWTH))
+def test_references_that_move_from_tile_to_tile(h, hkv, exec_, growth):
+    """Exec blocks of more than one query tile (lazy references) over one window, against 64 bits, row by row.
+
+    One pair of dimensions that RoPE hardly turns carries the growth of the keys; of a tile's rows those of the first warp follow
+    it, one of the second's, every other of the third's and none of the fourth's.  The values fall as the weights of those rows
+    grow, so that every key tile has the same part of their outputs and a factor of O that is wrong or missing anywhere shows: at
+    least 1 / 11 of an output's square, 0.3 of its norm.  Of a row's sum only the last moves matter.
+
+    Tolerance: a row's error is the rounding of P (2^-9 of a weight at most, 1.1e-3 in the 2-norm), of rotated queries and keys
+    (1.1e-3 of a weight) and of the output (2^-9 at most).  Their worst sum over the few keys of an early row, with three standard
+    deviations for the middle one: 2^-9 + 3.3e-3 + 2^-9 = 7.2e-3, and twice that is allowed; over all rows 4e-3 (test_gpu_stage_kernels' bound)."""
+    from infllm_b200.attention import ContextManager, RotaryEmbeddingESM
+
+    step = torch.tensor([0] + GROWTH[growth], device="cuda")
+    n, tiles, c, base = 128 * step.numel(), step.numel(), D // 2 - 1, 1e6
+    s = step.cumsum(0).repeat_interleave(128).double()
+    log2 = 1 / (D ** 0.5 * math.log(2))  # of a score
+    g = torch.Generator(device="cuda").manual_seed(h * exec_ + tiles)
+    q, k, v = (torch.randn((1, m, n, D), generator=g, device="cuda") for m in (h, hkv, hkv))
+    r = torch.arange(n, device="cuda") % 128
+    follows = (r < 32) | (r == 37) | ((r >= 64) & (r < 96) & (r % 2 == 1))
+    q *= 0.25
+    for x, y in ((q, 8.0 * follows), (k, s / (8.0 * log2))):
+        x[..., c], x[..., c + D // 2] = y.float(), 0
+    v *= torch.exp2(s[-1] - s).float()[:, None]
+    q, k, v = (x.to(torch.bfloat16) for x in (q, k, v))
+    cm = ContextManager(RotaryEmbeddingESM(D, base, 1.0), 100, n, UNIT, 32, 32, exec_, None, True, 2)
+    got = cm.append(q, k, v, q, k, v).double()
+
+    ang = torch.arange(n, device="cuda")[:, None] / base ** (torch.arange(0, D, 2, device="cuda", dtype=torch.float64) / D)
+    cos, sin = ang.cos().repeat(1, 2), ang.sin().repeat(1, 2)
+
+    def turned(x):
+        a, b = x.double().chunk(2, -1)
+        return x.double() * cos + torch.cat((-b, a), -1) * sin
+
+    kk, vv = (x.repeat_interleave(h // hkv, 1) for x in (turned(k), v.double()))
+    score = turned(q) @ kk.transpose(-1, -2) * log2
+    score.masked_fill_(r.new_ones((n, n), dtype=torch.bool).triu(1), float("-inf"))
+    # the references of the last query tile's rows, which see whole tiles but the last
+    ref = torch.full((1, h, 128), float("-inf"), device="cuda", dtype=torch.float64)
+    for t in range(tiles):
+        m = score[:, :, -128:, t * 128:(t + 1) * 128].amax(-1)
+        moves = m - ref > 8
+        if t:
+            assert torch.equal(moves, (follows[-128:] & (step[t] > 0)).expand_as(moves))
+        ref = torch.where(moves, m, ref)
+    want = torch.softmax(score * math.log(2), -1) @ vv
+    err = (got - want).norm(dim=-1) / want.norm(dim=-1)
+    assert err.max() <= 1.5e-2
+    assert err.square().mean().sqrt() <= 4e-3
 
 
 @pytest.mark.parametrize("h,hkv,lq", [(8, 2, 256), (7, 1, 256), (12, 12, 200), (7, 1, 300)])  # pairs of heads, of tiles, ragged; alone
