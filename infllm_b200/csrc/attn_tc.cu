@@ -48,8 +48,8 @@ __device__ __forceinline__ bool wait_or_abort(uint32_t bar, uint32_t parity, vol
 }
 
 // the same for a whole (converged) warp, whose lanes go on or give up together.  Nearly always the phase has passed or is about
-// to: one look, in straight code, before the loop, in which lanes could part (110 cycles a wait, now 75; four such waits are in the way
-// of a key tile, and 512 queries by 4608 + 2688 keys took 58.2 us, now 55.4; 62.3 and 59.0 with exact maxima)
+// to: one look, in straight code, before the loop, in which lanes could part (75 cycles a wait instead of 110; four such waits are in
+// the way of a key tile: 512 queries by 4608 + 2688 keys 5 % less)
 __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* err, int where) {
   if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
   return __all_sync(0xffffffffu, wait_or_abort(bar, parity, abort_flag, err, where));
@@ -150,13 +150,11 @@ __device__ __forceinline__ bool seg_tiles(int64_t vis_lo, int64_t vis_hi, int64_
 // Pairs of CTAs (attn_tc3_pairs: where a KV head's query tiles, over all its query heads, come out even): the products are
 // cta_group::2, 256 rows of two CTAs by 128 keys, and a CTA fetches and holds half of every K and V tile.  That halves the
 // bytes from L2 to shared memory (a lone CTA's 64 KB a tile take 1600 cycles at 40 bytes per clock and SM) and leaves room for
-// four tiles in flight.  Alone (7 heads by 3 tiles of a KV head, 12/12 heads by 3: 384 queries by 4480 + 2688 keys) the same code
-// takes 51.2 and 50.3 us.  Two query heads of a KV head make a pair, so
-// that both see the same keys; two tiles of one head where there is only one.
+// four tiles in flight.  Alone (12/12 heads by 3 tiles: 384 queries by 4480 + 2688 keys) the same code takes 51.3 us, 55.5
+// with the waits that are named below.  Two query heads of a KV head make a pair, so that both see the same keys; two tiles of one head where there is only one.
 // The softmax is two teams of four warps with the key tiles in turn, a thread per query row: no exchange within a row, and one
-// team's maximum and waits under the other's exponentials.  With all eight warps on one tile at a time (a row over four threads)
-// a tile took 2000 cycles, 1700 of them theirs.  One pair of exponentials in eight is a polynomial on the FMA pipe (none: 3 % more time;
-// a quarter: 1 % less, kExact 1 % more).
+// team's maximum and waits under the other's exponentials.  One pair of exponentials in eight is a polynomial on the FMA pipe (none:
+// 3 % more time; a quarter: 1 % less, kExact 1 % more).
 // Issuers and producer are whole warps of which one lane issues: eight products in 120 cycles instead of 600, and one load per
 // tile and operand (both 64-dimension halves in one box) instead of four at about 390 cycles each, which was 1570 per tile
 // whatever their size.  The producer asks for K one tile ahead of V.
@@ -164,18 +162,12 @@ __device__ __forceinline__ bool seg_tiles(int64_t vis_lo, int64_t vis_hi, int64_
 // maximum of a row follows its maximum, so that the largest probabilities have no rounding (2 to 6 % less error of an
 // output against 64 bits); whenever a row's maximum grows, O is scaled.
 // What bounds it (clock stamps, cycles): a key tile every 1420, of which the tensor pipe needs 1024.  Two ways round are equally long:
-// that of a team, two tiles in 2840 - exponentials 1500 (372 per 32 columns where one warp of a scheduler is at them, 265 where two
-// are), maximum 400, the other team's 230, the rest waits and hand-overs that are there already and cost 75 to 100 each - and that of
-// an S/P buffer, three tiles: product 700, softmax 2300, to the issuer 250, P V and back 850.  Set-up and first loads take 6000 and the
-// end 4500.  32/8 heads, 512 queries by 4608 + 2688 keys, twenty launches in a row: 52.7 us, with each wait through a loop, a barrier
-// for every maximum and ordering cluster barriers 58.2 (kExact: 57.5, 62.3); 256 queries of 32/32 heads in two runs 36.8, 40.7; 128
-// queries in four runs 14.8, 16.1; 4096 queries by 8192 keys, kExact, 264, 286.
-// Also not kept: S and P in buffers of their own with a tile's scores in registers (224 of them, setmaxnreg) and the next tile's loaded
-// under the exponentials.  A tile every 1470 from 1600 at the time, but straight code of 20 KB is fetched cold at every launch: 54.7
-// where the rolled loop went from 58.2 to 52.7, and 44.7 against 36.8 in two runs.
-// Tried and not kept, when the first of these took 70 us, timed by itself: four warps to half a tile's keys each, two tiles at once (70.5: more
-// warps at the same pipes); the 64 score columns that a later tile needs first kept in registers, so that their buffer frees early
-// (70.3); one issuer for both products (72.3); three teams.
+// that of a team, two tiles in 2840 - exponentials 1500, maximum 400, the other team's 230, the rest waits and hand-overs that are
+// there already and cost 75 to 100 each - and that of an S/P buffer, three tiles: product 700, softmax 2300, to the issuer 250, P V and
+// back 850.  Set-up and first loads take 6000 and the end 4500.
+// 32/8 heads, 512 queries by 4608 + 2688 keys, twenty launches in a row: 54.7 us, with each wait through a loop, a barrier for every
+// maximum and ordering cluster barriers 60.6 (kExact: 60.3, 65.1; on another B200 52.7 and 58.2, 57.5 and 62.3); 256 queries of 32/32
+// heads in two runs, merge included, 37.3, 41.2; 128 queries by 1152 + 700 in four 15.2, 16.3; 4096 queries by 8192 keys, kExact, 264, 286.
 namespace tc3 {
 constexpr int kBufs = 3;                         // S/P buffers in TMEM
 constexpr int kQ = 0;                            // a tile for each of the two stages
@@ -686,8 +678,8 @@ __global__ void __launch_bounds__(tc3::kThreads, 1) attn_tc3_kernel(const __grid
           ok = warp_wait(bar(T3_PV_DONE0 + ((it - 1) % kBufs)), ((it - 1) / kBufs) & 1, abort_flag, P.err, 622);
           if (!ok) break;
           tc_fence_after();
-          // kExact, where most tiles come here: all 128 columns at once (four rounds of 32, one behind the other: 292.4 us for 4096
-          // queries by 8192 keys, now 284.6)
+          // kExact, where most tiles come here: all 128 columns at once (four rounds of 32, one behind the other, took 3 % more: 4096
+          // queries by 8192 keys)
           constexpr int kRound = kExact ? 128 : 32;
           const float2 al = make_float2(alpha, alpha);
 #pragma unroll 1
@@ -749,7 +741,10 @@ __global__ void __launch_bounds__(tc3::kThreads, 1) attn_tc3_kernel(const __grid
       asm volatile("bar.sync 1, 256;" ::: "memory");  // both halves of a row have read (m, l): they may be overwritten
     }
     if (ok && it >= 1) ok = warp_wait(bar(T3_O_FULL), 0, abort_flag, P.err, 624);
-    if (kPair) cluster_arrive();  // nothing more is signalled to or from this CTA (waited for at the end)
+    // Nothing more is signalled to or from this CTA, and no data goes with the arrival: O_FULL has said that the products are done, and so
+    // that the loads and probabilities that either CTA counted on the other's barriers have been taken; every S_FULL was waited for here, the
+    // PV_DONEs and the releases that are signalled at all by the producer.  (The other CTA's arrival is waited for at the end.)
+    if (kPair) cluster_arrive();
     if (ok) {
       tc_fence_after();
       const bool raw = P.part_acc != nullptr;
@@ -809,8 +804,8 @@ __global__ void __launch_bounds__(tc3::kThreads, 1) attn_tc3_kernel(const __grid
         const int cl = (lane & 15) * 4;
         const int64_t row0 = i0 + quad * 32, srow0 = (int64_t)h * P.lq + row0, prow0 = (int64_t)split * P.n_heads * P.lq + srow0;
         const float nrm = raw ? 1.f : inv;
-        // (a round's loads before its first store, rows past the last query with the last one's: one row after the other, 128 queries
-        // in four runs took 15.2 us, now 14.8)
+        // (a round's loads before its first store, rows past the last query with the last one's; one row after the other took 0.4 us
+        // more of 15 for 128 queries in four runs)
         const int n_rows = (int)((P.lq - row0) < 32 ? P.lq - row0 : 32);
 #pragma unroll 1
         for (int k0 = 0; k0 < 16; k0 += 8) {
@@ -872,8 +867,8 @@ __global__ void attn_tc_combine_kernel(const float* __restrict__ acc, const floa
   const int64_t h = row / lq, i = row - h * lq;
   const int64_t stride = (int64_t)n_heads * lq;
   // What bounds it is two loads behind one another and the launch: the first four partials are asked for whole, before their maximum is
-  // known (with the attention, 256 queries of 28/4 heads in two runs 32.5 -> 31.2 us, 37 of 32/8 in four 23.2 -> 22.6, 16 of 16/2 in four
-  // 10.0 -> 9.2; 128 of 32/8 in four 15.1, as before)
+  // known (with the attention, 256 queries of 28/4 heads in two runs 31.2 us, behind the maximum 32.5; 37 of 32/8 in four 22.6, 23.2; 16
+  // of 16/2 in four 9.2, 10.0; 128 of 32/8 in four no difference)
   constexpr int kAhead = 4;
   float4 pa[kAhead];
   float pm[kAhead], pl[kAhead];
@@ -930,10 +925,8 @@ __global__ void attn_tc_combine_kernel(const float* __restrict__ acc, const floa
 // Bound: 16384 exponentials per pair, 768 cycles of the special-function unit with every fourth pair of them as a
 // quartic on the FMA pipe (a quintic, kExact, for exec blocks of one query tile; without any 29.0 us, with an eighth 27.9, three
 // eighths 27.0), the product, 514, whose operands want shared memory for all of that time, and 424 more there for the log-sum-exps
-// (685 in 16-byte loads); a pair takes 1030.  512 queries x 32 heads over 4608 keys: 26.5 us (28.3 with those loads, a loop at
-// every wait and sums cleared beforehand), 37 over 4133: 9.9 (10.7).  Products of 64 queries, two buffers per group: 34.9 (half as
-// many columns are not half a product); two groups with two buffers each: 36.2; queries as TMEM lanes, so that a log-sum-exp is a
-// register's and a key's sum is exchanged once per key tile: 28.7 (8 % more instructions), in eight warps 34.3.
+// (709 in 16-byte loads); a pair takes 1030.  512 queries x 32 heads over 4608 keys: 26.7 us (28.5 with those loads, a loop at
+// every wait and sums cleared beforehand), 37 over 4133: 9.9 (10.7).
 namespace colsum_smem {
 constexpr int kQTiles = 4;                     // resident query tiles
 constexpr int kMaxKeyTiles = 10;               // key tiles per CTA
@@ -967,7 +960,7 @@ __device__ __forceinline__ void colsum_q_tiles(const ColsumTcParams& P, int j0, 
 }
 
 // eight bytes of shared memory that all lanes ask for.  (Sixteen at a time took 2.99 million turns of the path into the registers
-// for 512 queries x 32 heads over 4608 keys, these take 1.79, beside the operands of the products, which want all of it: 27.8 us, now 26.8)
+// for 512 queries x 32 heads over 4608 keys, these take 1.79, beside the operands of the products, which want all of it: 3 % less time)
 __device__ __forceinline__ float2 lds8(const float* p) {
   float2 v;
   asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(smem_u32(p)));
@@ -1313,8 +1306,9 @@ int attn_tc_combine_launch(const float* acc, const float* m, const float* l, int
 // Runs of key tiles per (128-query tile, head), as many as the SMs take at once and no more than pay: a run's tiles come one
 // after another, 0.8 us each, and the partials cost a merge, two tiles' time for its launch and one more for every 40 runs of the
 // grid.  Measured over 4 to 60 tiles for 8 to 64 items (eight kinds of 8 sizes, bf16, both precisions, merge included, every
-// count): on the average 0.9 % above the best count, 14 % at worst (4 tiles of 8 items: 10.6 us in four runs, 9.3 in one).  Half a
-// tile more or less for the merge, or one for every 32 or 50 runs: 0.8 to 1.3 % on the average.
+// count), three times: on the average 0.76 to 0.90 % above the best count, 9.3 % at worst (9 tiles of 8 items: 11.5 us in nine runs, 10.5
+// in four; in one of the three 14 %, 4 tiles of 8 items).  Two and a half tiles for the merge: 0.80 to 0.94 %, 9.3 to 9.6 at worst; one
+// and a half: 0.72 to 0.97, 9.3 to 14; three: 0.86 to 1.01; one more for every 32 runs 0.84 to 0.97, for every 50 1.05 to 1.31.
 int attn_tc3_splits(int64_t lq, int n_heads, int64_t keys) {
   const int64_t items = ceil_div(lq, kTile) * n_heads, tiles = ceil_div(keys, kTile);
   int best = 1;

@@ -19,8 +19,9 @@ constexpr TcBox box_v(bool pair) { return pair ? kBoxPairV : kBoxTile; }
 // multi-stage class and the sink + window types.  Up to 64 queries they used to be the shape-generic kernel's, which does;
 // up to 128 their key tiles are cut into runs, and where a row is one key's for the most part it matters which tiles share
 // a reference maximum (an 8192-token prompt in exec blocks of 128: largest error 2.6e-2 instead of 2.0e-2, 1.2 % more in
-// the 2-norm).  It costs them nothing that shows; larger exec blocks, which it would cost 4 to 5 %, have had the cubic and
-// the lazy maximum all along.
+// the 2-norm).  It costs them 3 % (128 queries by 1152 + 700 keys, merge included: 15.2 us instead of 14.8) to 9 % (128 by 4224 + 2304:
+// 24.5, 22.6; 37 by 4133 + 2200: 22.5, 20.7).  Larger exec blocks, which it would cost 7 to 10 % (256 of 32/32 heads in two runs: 40.0,
+// 37.3; 512 by 4608 + 2688: 60.3, 54.7), have had the cubic and the lazy maximum all along.
 constexpr int kExactQueries = kTile;
 
 struct TcSeg {
